@@ -92,6 +92,26 @@ def test_sgemm_is_true_float32(M, N, K):
     assert torch.equal(out1[0], out[M - 1])
 
 
+@pytest.mark.parametrize("M", [1, 15, 16, 17, 33, 65, 129, 300])
+@pytest.mark.parametrize("N,K,pad", [(31, 64, 0), (148 * 32, 68, 0), (1024, 260, 0), (4800, 96, 0), (130, 33, 0), (64, 128, 1), (10000, 20, 0)])
+def test_sgemm_same_sums_in_every_kernel(M, N, K, pad):
+    """Every kernel and tile size adds a row's products in the same order: bit by bit the row alone.  Strided and
+    unaligned operands take the same sums."""
+    from tokensprint_b200 import ops
+
+    a = torch.randn(M, K + pad, device=DEV)[:, pad:]
+    w = torch.randn(N, K + pad, device=DEV)[:, pad:]
+    out = torch.full((M, N), float("nan"), device=DEV)
+    ops.sgemm_nt(a, w, out)
+    assert float((out.double() - a.double() @ w.double().T).abs().max()) < 4e-7 * math.sqrt(K) * float(out.abs().max())
+    alone = torch.full((1, N), float("nan"), device=DEV)
+    ops.sgemm_nt(a[M - 1 :], w, alone)
+    assert torch.equal(alone[0], out[M - 1])
+    batch = torch.full((2, M, N), float("nan"), device=DEV)
+    ops.sgemm_nt_batched(a.expand(2, M, K), w.expand(2, N, K), batch)
+    assert torch.equal(batch[0], out) and torch.equal(batch[1], out)
+
+
 # ---------------------------------------------------------------------------
 # q/k norm + rope + store
 
@@ -248,6 +268,35 @@ def test_attention_simple(dtype, nq, nkv, d, page, window):
     got = run_simple(case, window)
     want = plain_attention(case, window)
     assert rel_err(got, want) < (3e-6 if dtype == torch.float32 else 1e-2)
+
+
+@pytest.mark.parametrize(
+    "nq,nkv,d,page,window,chunk,extra",
+    [(4, 2, 16, 16, 0, 0, 0), (5, 1, 48, 4, 0, 0, 1), (6, 3, 32, 32, 24, 0, 2), (2, 2, 84, 1, 7, 0, 3), (40, 1, 128, 16, 0, 50, 1), (3, 1, 256, 8, 33, 64, 0)],
+)
+def test_attention_float32_tiles(nq, nkv, d, page, window, chunk, extra):
+    """The tiled kernel beside the one-warp-a-query kernel: portions of all lengths, window, blocks of positions, sinks,
+    cap, distance penalty, pages given back (poisoned), a padded lane.  Both sum in float32: 1e-5 of the largest."""
+    from tokensprint_b200 import ops
+
+    case = finish_case(paged_case(MIXED, nq, nkv, d, page, torch.float32, seed=d))
+    more = [{}, {"softcap": 4.0, "head_sinks": torch.randn(nq, device=DEV)}, {"sink": 0.5},
+            {"distance": (torch.rand(nq, device=DEV), torch.rand(nq, device=DEV))}][extra]
+    q = torch.cat([case["q"], case["q"][:2]])
+    T, scale = case["q"].shape[0], d ** -0.5
+    want = torch.empty_like(q)
+    ops.attention_paged_simple(q[:T], case["kc"], case["vc"], want[:T], case["positions"], case["seq_index"], case["table"], page, nq, nkv, d, scale,
+                               window, chunk, **more)
+    table = case["table"].clone()
+    for b, (ql, ctx) in enumerate(case["seqs"]):  # pages that no query of the step sees any more
+        first = ctx - ql
+        lo = max(first - window + 1 if window else 0, first // chunk * chunk if chunk else 0, 0)
+        table[b, : lo // page] = -1
+    got = torch.full_like(q, float("nan"))
+    ops.attention_paged_float32(q, case["kc"], case["vc"], got, case["cu"], case["ctxs"], table, page, case["B"], max(n for n, _ in case["seqs"]),
+                                nq, nkv, d, scale, window, chunk, **more)
+    assert rel_err(got[:T], want[:T].double()) < 1e-5
+    assert torch.equal(got[T:], torch.zeros_like(got[T:]))
 
 
 @pytest.mark.parametrize(

@@ -34,6 +34,9 @@ _SIGNATURES = {
         _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
         _c_float, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p,
     ],
+    "ts_attention_paged_float32": [
+        _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
+        _c_int, _c_float, _c_int, _c_int, _c_int, _c_float, _c_float, _c_void_p, _c_void_p, _c_void_p, _c_void_p],
     "ts_attention_paged_simple": [
         _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
         _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_int, _c_int, _c_float, _c_float, _c_void_p, _c_void_p, _c_void_p,
@@ -481,6 +484,65 @@ def attention_paged_simple(
 def sample(
     logits: torch.Tensor,
     temperature: torch.Tensor,
+def attention_float32_supported(head_dim: int, *tensors: torch.Tensor) -> bool:
+    """Whether attention_paged_float32 takes these: float32, heads of 4 to 256 entries in fours, 16-byte aligned."""
+    return head_dim % 4 == 0 and 4 <= head_dim <= 256 and all(t.dtype == torch.float32 and t.data_ptr() % 16 == 0 for t in tensors)
+
+
+def attention_paged_float32(
+    q: torch.Tensor,
+    k_cache: torch.Tensor,
+    v_cache: torch.Tensor,
+    out: torch.Tensor,
+    cu_seqlens: torch.Tensor,
+    context_lens: torch.Tensor,
+    block_table: torch.Tensor,
+    page_size: int,
+    num_seqs: int,
+    max_seqlen_q: int,
+    num_heads: int,
+    num_kv_heads: int,
+    head_dim: int,
+    scale: float,
+    window: int = 0,
+    chunk: int = 0,
+    sink: Optional[float] = None,
+    softcap: float = 0.0,
+    head_sinks: Optional[torch.Tensor] = None,
+    distance: Optional[tuple[torch.Tensor, torch.Tensor]] = None,
+) -> None:
+    """attention_paged_simple in tiles, for float32 and a batch described by cu_seqlens [B + 1] and
+    context_lens [B] (i32); tokens behind the last sequence (padded lanes) get zeros."""
+    flush_gemm_chain()
+    nq, nkv, d = num_heads, num_kv_heads, head_dim
+    per_head = [("head_sinks", head_sinks)] + ([] if distance is None else list(zip(("distance r1", "distance r2"), distance)))
+    for name, t in per_head:
+        if t is not None:
+            _cuda_contig(name, t, torch.float32)
+            if t.numel() != nq:
+                raise KernelError(f"attention: {name} must have one entry per query head ({nq}), got {t.numel()}")
+    for name, t in (("q", q), ("k_cache", k_cache), ("v_cache", v_cache), ("out", out)):
+        _cuda_contig(name, t, torch.float32)
+    for name, t in (("cu_seqlens", cu_seqlens), ("context_lens", context_lens), ("block_table", block_table)):
+        _cuda_contig(name, t, torch.int32)
+    T = q.shape[0]
+    if not attention_float32_supported(d, q, k_cache, v_cache, out):
+        raise KernelError(f"attention_paged_float32: heads of 4 to 256 entries in fours, 16-byte aligned tensors; got heads of {d}")
+    if nq % nkv:
+        raise KernelError(f"attention: {nq} query heads are no multiple of {nkv} key/value heads")
+    if q.numel() != T * nq * d or out.numel() != T * nq * d:
+        raise KernelError("attention: q/out do not match [T, heads*head_dim]")
+    if tuple(k_cache.shape[-3:]) != (page_size, nkv, d) or k_cache.shape != v_cache.shape:
+        raise KernelError(f"attention: caches must be [pages,{page_size},{nkv},{d}], got {tuple(k_cache.shape)} and {tuple(v_cache.shape)}")
+    if block_table.dim() != 2 or block_table.shape[0] < num_seqs or cu_seqlens.numel() < num_seqs + 1 or context_lens.numel() < num_seqs:
+        raise KernelError("attention: block_table must be [B,max_blocks]; cu_seqlens needs B+1 and context_lens B entries")
+    _check("attention_paged_float32", _fn("ts_attention_paged_float32")(
+        q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), cu_seqlens.data_ptr(), context_lens.data_ptr(),
+        block_table.data_ptr(), block_table.shape[1], page_size, num_seqs, T, max_seqlen_q, nq, nkv, d, float(scale), int(window), int(chunk),
+        0 if sink is None else 1, 0.0 if sink is None else float(sink), float(softcap), _ptr(head_sinks),
+        None if distance is None else distance[0].data_ptr(), None if distance is None else distance[1].data_ptr(), _stream()))
+
+
     keys: Optional[torch.Tensor],
     out: torch.Tensor,
 ) -> None:
@@ -2668,7 +2730,7 @@ def library_mm(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor
 # Timers per kernel class, for eager steps (a replayed graph has no calls to time): switched on,
 # every launching function of this module is wrapped so that a pair of CUDA events brackets what it
 # launches; switched off, the functions are the plain ones again and nothing is paid.
-_TIMED = ("embed_gather", "feed_tokens", "add_rmsnorm", "residual_add", "swiglu", "qk_norm_rope_store", "attention_paged_simple",
+_TIMED = ("embed_gather", "feed_tokens", "add_rmsnorm", "residual_add", "swiglu", "qk_norm_rope_store", "attention_paged_simple", "attention_paged_float32",
           "sample", "sgemm_nt", "attention_paged_mma", "attention_decode_flat", "attention_prefill_tcgen05", "gemm_skinny_bf16",
           "gemm_skinny_fused", "rope_cos_sin", "gemm_qk_rope_store", "library_mm", "sgemm_nt_batched", "library_bmm", "pair_hash_embed",
           "rmsnorm_add", "round_rows", "latent_prepare", "latent_attention_simple", "latent_attention_mma", "gelu_tanh", "capped_glu", "gelu_gate_rows",

@@ -388,7 +388,12 @@ class AttentionMixer(Mixer):
                 step.seq_index, step.page_size, step.num_seqs, step.max_seqlen_q, nq, nkv, d, self.scale,
                 self.window, 1, None, 0, chunk=self.chunk, sink=self.sink, **scored)
             return
-        # float32 runs, and head sizes the tensor-core kernel does not take
+        if ops.attention_float32_supported(d, q, cache.k_pages, cache.v_pages, out):
+            ops.attention_paged_float32(
+                q, cache.k_pages, cache.v_pages, out, step.cu_seqlens_q, step.context_lens, tables.block_table, step.page_size,
+                step.num_seqs, step.max_seqlen_q, nq, nkv, d, self.scale, self.window, self.chunk, self.sink, **scored)
+            return
+        # head sizes that neither the tensor-core kernels nor the tiled one take
         ops.attention_paged_simple(
             q, cache.k_pages, cache.v_pages, out, step.positions, step.seq_index, tables.block_table,
             step.page_size, self.num_heads, self.num_kv_heads, d, self.scale, self.window, self.chunk, self.sink,
