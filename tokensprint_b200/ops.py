@@ -481,9 +481,6 @@ def attention_paged_simple(
         None if distance is None else distance[0].data_ptr(), None if distance is None else distance[1].data_ptr(), _stream()))
 
 
-def sample(
-    logits: torch.Tensor,
-    temperature: torch.Tensor,
 def attention_float32_supported(head_dim: int, *tensors: torch.Tensor) -> bool:
     """Whether attention_paged_float32 takes these: float32, heads of 4 to 256 entries in fours, 16-byte aligned."""
     return head_dim % 4 == 0 and 4 <= head_dim <= 256 and all(t.dtype == torch.float32 and t.data_ptr() % 16 == 0 for t in tensors)
@@ -543,6 +540,9 @@ def attention_paged_float32(
         None if distance is None else distance[0].data_ptr(), None if distance is None else distance[1].data_ptr(), _stream()))
 
 
+def sample(
+    logits: torch.Tensor,
+    temperature: torch.Tensor,
     keys: Optional[torch.Tensor],
     out: torch.Tensor,
 ) -> None:
