@@ -216,6 +216,82 @@ def test_latent_attention_finds_the_one_key(dtype, rank, rot, H, page, N, Q, win
                 assert bool(torch.isfinite(out2[:short].float()).all())
 
 
+REBUILT_CASES = [
+    # heads, rank, page, window, sinks, gates, portions (new tokens, context): tiles of 128 tokens in pairs, key blocks of 96
+    (1, 64, 16, 0, False, False, [(5, 5)]),
+    (2, 64, 16, 0, True, True, [(128, 128), (129, 130), (1, 95), (95, 96)]),
+    (3, 72, 8, 0, False, True, [(256, 256), (257, 353), (7, 384)]),
+    (2, 64, 4, 100, True, False, [(300, 700), (40, 40), (96, 193), (130, 1000)]),
+    (2, 512, 32, 1, False, False, [(33, 97), (385, 385)]),
+    (2, 512, 16, 4096, False, True, [(1, 2000), (515, 515)]),
+]
+
+
+@pytest.mark.parametrize("H, rank, page, window, sinks, gated, portions", REBUILT_CASES)
+def test_latent_portions_with_rebuilt_keys(H, rank, page, window, sinks, gated, portions):
+    """Gathered rows, keys and values made of them, and the tcgen05 attention, against float64 attention on the same rebuilt
+    (rounded) keys and values: what is left is P rounded to bfloat16 (2^-9 of a weight) and the result's rounding, 1e-2
+    of the largest entry as for the other bfloat16 attentions.  Pages that nobody sees are given back (NaN, table -1)."""
+    from tokensprint_b200 import ops
+
+    g = torch.Generator().manual_seed(H * 1000 + rank + page)
+    D, B = rank + 64, len(portions)
+    need = [-(-ctx // page) for _, ctx in portions]
+    pool = torch.full((sum(need) + 3, page, D), float("nan"), dtype=torch.bfloat16)
+    order, table, rows = torch.randperm(sum(need) + 3, generator=g).tolist(), torch.full((B, max(need)), -1, dtype=torch.int32), []
+    for b, (n, ctx) in enumerate(portions):
+        rows.append(torch.randn(ctx, D, generator=g).to(torch.bfloat16))
+        lo = max(0, ctx - n - window + 1) if window else 0
+        for j in range(lo // page * page, ctx):
+            table[b, j // page] = order[sum(need[:b]) + j // page]
+            pool[table[b, j // page], j % page] = rows[b][j]
+    ahead = 3 * (H - 1)  # tokens of other sequences in front
+    T = ahead + sum(n for n, _ in portions)
+    q = torch.randn(T, H * 192, generator=g).to(torch.bfloat16)
+    q_rot = torch.randn(T, H, 64, generator=g).to(torch.bfloat16)
+    weight = (torch.randn(H * 256, rank, generator=g) / rank ** 0.5).to(torch.bfloat16)
+    gates = torch.rand(T, H, generator=g) + 0.5 if gated else None
+    sink = torch.randn(H, generator=g) if sinks else None
+    cu = [ahead]
+    for n, _ in portions:
+        cu.append(cu[-1] + n)
+    kept = [ops.latent_kept_keys(window, n, ctx) for n, ctx in portions]
+    cached = torch.full((sum(kept), D), float("nan"), device="cuda", dtype=torch.bfloat16)
+    starts, lens = _i32(cu), _i32([ctx for _, ctx in portions])
+    ops.latent_gather(_dev(pool), cached, starts, lens, _dev(table), page, B, max(kept), window)
+    at = 0
+    for b, (n, ctx) in enumerate(portions):
+        lo = max(0, ctx - n - window + 1) if window else 0
+        want_rows = rows[b][ctx - kept[b]:].clone()
+        want_rows[: lo - (ctx - kept[b])] = 0
+        assert torch.equal(cached[at:at + kept[b]].cpu(), want_rows)
+        at += kept[b]
+    kv = ops.library_mm(cached[:, :rank], _dev(weight))
+    wide = torch.full((T, H * 192 + 8), float("nan"), device="cuda", dtype=torch.bfloat16)  # rows that are not side by side
+    wide[:, :-8] = _dev(q)
+    out = torch.full((T, H, 128), float("nan"), device="cuda", dtype=torch.bfloat16)
+    scale = 192 ** -0.5
+    ops.latent_rebuilt_attention(wide[:, :-8], _dev(q_rot[ahead:]), kv, cached, out, None if gates is None else _dev(gates), starts, lens, B,
+                                 max(n for n, _ in portions), H, rank, scale, window, None if sink is None else _dev(sink))
+    ops.check_device_errors()
+    made, at = kv.double().cpu(), 0
+    for b, (n, ctx) in enumerate(portions):
+        kb = made[at:at + kept[b]]
+        see = torch.arange(ctx - n, ctx)[:, None] - torch.arange(ctx - kept[b], ctx)[None, :]
+        see = (see >= 0) & (see < window) if window else see >= 0
+        want = torch.empty(n, H, 128, dtype=torch.float64)
+        for a in range(H):
+            qa = torch.cat([q[cu[b]:cu[b + 1], a * 192:a * 192 + 128], q_rot[cu[b]:cu[b + 1], a]], 1).double()
+            ka = torch.cat([kb[:, a * 128:a * 128 + 128], cached[at:at + kept[b], rank:].double().cpu()], 1)
+            s = (qa @ ka.T * scale).masked_fill(~see, -math.inf)
+            if sink is not None:
+                s = torch.cat([s, sink[a].double().expand(n, 1)], 1)
+            w = torch.softmax(s, 1)[:, :kept[b]]
+            want[:, a] = w @ kb[:, (H + a) * 128:(H + a + 1) * 128] * (1.0 if gates is None else gates[cu[b]:cu[b + 1], a, None].double())
+        assert _rel(out[cu[b]:cu[b + 1]], want) < 1e-2, f"portion {b}"
+        at += kept[b]
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("tag, layer", [("a", 0), ("b", 0), ("b", 1), ("c", 1)])
 def test_latent_mixer_whole_prompt(dtype, tag, layer):

@@ -7,7 +7,7 @@
 // and the head's output is U_v,a o'_a(t): every head reads the same cached rows, as keys over all
 // rank + rot entries and as values over the first `rank`.
 //
-// Two kernels here, both for any sizes and both element types:
+// The kernels here take any sizes and both element types (latent_gather: rows of 16-byte pieces):
 //   latent_prepare: per token, from the stacked projection [q heads | latent and key part | gate
 //     logits]: RMS norm of the latent, rotation of the key part and of every head's rotated
 //     query part (angles, sines and cosines in float32), store of [c ; r] into the cache by slot,
@@ -15,6 +15,11 @@
 //     sines may carry a `magnitude` (stretched frequencies come with one).  The queries may come
 //     from a tensor of their own (`q_src`: a layer whose queries pass a latent first), and a layer
 //     that reads another layer's cached rows has no latent of its own (`kv_off` < 0: queries only).
+//     Behind the first `absorbed` tokens the rotated parts go to a buffer [tokens, heads, rot] of their own
+//     (prompt portions whose keys are rebuilt).
+//   latent_gather: the cached rows that a step's prompt portions see, one sequence after the other in one
+//     matrix, for products that rebuild their keys and values (16-byte copies, bound by reading and writing the rows once:
+//     8,191 rows of 1,152 bytes 12 us).
 //   latent_attention_simple: CUDA cores, one warp per (token, head), scores, softmax and sums in
 //     float32: the float32 path's attention and the yardstick of the tensor-core kernel.
 #include "common.cuh"
@@ -51,7 +56,8 @@ __global__ void latent_prepare_kernel(const TA* __restrict__ proj, long long ld,
                                       TA* __restrict__ q_abs, TA* __restrict__ cache, const int* __restrict__ slot_mapping,
                                       const int* __restrict__ positions, const float* __restrict__ latent_weight, float eps,
                                       const float* __restrict__ inv_freq, int rot_dims, int pairing, float* __restrict__ gates,
-                                      int H, int nope, int rot, int rank, float magnitude, const TA* __restrict__ q_src, long long ld_q) {
+                                      int H, int nope, int rot, int rank, int absorbed, TA* __restrict__ q_rot, float magnitude,
+                                      const TA* __restrict__ q_src, long long ld_q) {
   ts_pdl_prologue();
   __shared__ float scratch[33];
   __shared__ float2 cs[LAT_MAX_PAIRS];  // (cos, sin) of the token's angles, shared by the key part and every head
@@ -81,11 +87,13 @@ __global__ void latent_prepare_kernel(const TA* __restrict__ proj, long long ld,
     for (int j = threadIdx.x; j < rot; j += blockDim.x)
       dst[rank + j] = ts_from_float<TA>(lat_rotated(lat + rank, j, rot_dims, pairing, cs));
   }
-  // every head's rotated query part, behind the place of its absorbed part
+  // every head's rotated query part, behind the place of its absorbed part or by itself
+  TA* q_dst = t < absorbed ? q_abs + (size_t)t * H * key_dim + rank : q_rot + (size_t)(t - absorbed) * H * rot;
+  const int q_step = t < absorbed ? key_dim : rot;
   for (int i = threadIdx.x; i < H * rot; i += blockDim.x) {
     const int a = i / rot, j = i - a * rot;
     const TA* qr = (q_src ? q_src + (size_t)t * ld_q : row + q_off) + (size_t)a * (nope + rot) + nope;
-    q_abs[((size_t)t * H + a) * key_dim + rank + j] = ts_from_float<TA>(lat_rotated(qr, j, rot_dims, pairing, cs));
+    q_dst[(size_t)a * q_step + j] = ts_from_float<TA>(lat_rotated(qr, j, rot_dims, pairing, cs));
   }
   if (gates)
     for (int a = threadIdx.x; a < H; a += blockDim.x) gates[(size_t)t * H + a] = 1.f / (1.f + expf(-ts_to_float(row[gate_off + a])));
@@ -94,10 +102,10 @@ __global__ void latent_prepare_kernel(const TA* __restrict__ proj, long long ld,
 TS_EXPORT int ts_latent_prepare(const void* proj, int act_dtype, long long ld, int q_off, int kv_off, int gate_off, void* q_abs,
                                 void* cache, const int* slot_mapping, const int* positions, const float* latent_weight, float eps,
                                 const float* inv_freq, int rot_dims, int pairing, float* gates, int T, int H, int nope, int rot,
-                                int rank, float magnitude, const void* q_src, long long ld_q, void* stream) {
+                                int rank, int absorbed, void* q_rot, float magnitude, const void* q_src, long long ld_q, void* stream) {
   if (T <= 0) return 0;
   if (rot_dims > 2 * LAT_MAX_PAIRS) return TS_ERR_UNSUPPORTED_SIZE;
-  if (H <= 0 || nope < 0 || rot < 0 || rank <= 0 || rot_dims < 0 || rot_dims > rot || (rot_dims & 1) || (rot_dims > 0 && !inv_freq) ||
+  if (H <= 0 || nope < 0 || rot < 0 || rank <= 0 || absorbed < 0 || (absorbed < T && !q_rot) || (absorbed > 0 && !q_abs) || rot_dims < 0 || rot_dims > rot || (rot_dims & 1) || (rot_dims > 0 && !inv_freq) ||
       (pairing != LAT_PAIR_HALF && pairing != LAT_PAIR_NEIGHBOURS) || (kv_off < 0 && cache != nullptr) || (proj == nullptr && (q_src == nullptr || kv_off >= 0 || gates)))
     return TS_ERR_BAD_ARGUMENT;
   cudaStream_t s = (cudaStream_t)stream;
@@ -105,12 +113,60 @@ TS_EXPORT int ts_latent_prepare(const void* proj, int act_dtype, long long ld, i
   if (act_dtype == TS_DTYPE_F32)
     return ts_launch(latent_prepare_kernel<float>, dim3(T), dim3(threads), 0, s, (const float*)proj, ld, q_off, kv_off, gate_off,
                      (float*)q_abs, (float*)cache, slot_mapping, positions, latent_weight, eps, inv_freq, rot_dims, pairing, gates, H,
-                     nope, rot, rank, magnitude, (const float*)q_src, ld_q);
+                     nope, rot, rank, absorbed, (float*)q_rot, magnitude, (const float*)q_src, ld_q);
   if (act_dtype == TS_DTYPE_BF16)
     return ts_launch(latent_prepare_kernel<__nv_bfloat16>, dim3(T), dim3(threads), 0, s, (const __nv_bfloat16*)proj, ld, q_off, kv_off,
                      gate_off, (__nv_bfloat16*)q_abs, (__nv_bfloat16*)cache, slot_mapping, positions, latent_weight, eps, inv_freq,
-                     rot_dims, pairing, gates, H, nope, rot, rank, magnitude, (const __nv_bfloat16*)q_src, ld_q);
+                     rot_dims, pairing, gates, H, nope, rot, rank, absorbed, (__nv_bfloat16*)q_rot, magnitude, (const __nv_bfloat16*)q_src, ld_q);
   return TS_ERR_BAD_ARGUMENT;
+}
+
+// ---------------------------------------------------------------------------------------------
+
+// Rows of `pieces` 16-byte pieces; GATHER_ROWS of them per CTA.  Sequence b keeps its keys from a multiple of `block`
+// positions on: the one at or below the first key that any token of its portion sees (window 0: all from 0
+// on).  Rows below that first key are zeros: their pages may have been given back.
+#define GATHER_ROWS 8
+__global__ void __launch_bounds__(256) latent_gather_kernel(const uint4* __restrict__ cache, uint4* __restrict__ out, const int* __restrict__ cu_seqlens,
+                                                            const int* __restrict__ context_lens, const int* __restrict__ block_table,
+                                                            int max_blocks, int page, int pieces, int window, int block) {
+  ts_pdl_prologue();
+  const int b = blockIdx.y;
+  auto first_seen = [&](int i, int n) { return window > 0 ? max(0, context_lens[i] - n - window + 1) : 0; };
+  const int q_len = cu_seqlens[b + 1] - cu_seqlens[b], end = context_lens[b];
+  if (q_len <= 0) return;
+  const int lo = first_seen(b, q_len), kept = lo / block * block;
+  const int key0 = kept + blockIdx.x * GATHER_ROWS;
+  if (key0 >= end) return;
+  __shared__ int before_s;
+  if (threadIdx.x < 32) {  // rows of the sequences ahead
+    int before = 0;
+    for (int i = threadIdx.x; i < b; i += 32) {
+      const int n = cu_seqlens[i + 1] - cu_seqlens[i];
+      if (n > 0) before += context_lens[i] - first_seen(i, n) / block * block;
+    }
+    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+    if (threadIdx.x == 0) before_s = before;
+  }
+  __syncthreads();
+  const size_t row0 = (size_t)before_s + (key0 - kept);
+  const int rows = min(GATHER_ROWS, end - key0);
+  for (int i = threadIdx.x; i < rows * pieces; i += blockDim.x) {
+    const int r = i / pieces, c = i - r * pieces, key = key0 + r;
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (key >= lo) v = cache[((size_t)block_table[(size_t)b * max_blocks + key / page] * page + key % page) * pieces + c];
+    out[(row0 + r) * pieces + c] = v;
+  }
+}
+
+// cache [slots, row_bytes], out [the sequences' kept keys, row_bytes], both 16-byte aligned; max_keys: the most of any sequence.
+TS_EXPORT int ts_latent_gather(const void* cache, void* out, const int* cu_seqlens, const int* context_lens, const int* block_table,
+                               int max_blocks, int page, int num_seqs, int max_keys, int row_bytes, int window, int block, void* stream) {
+  if (num_seqs <= 0 || max_keys <= 0) return 0;
+  if (page <= 0 || max_blocks <= 0 || row_bytes <= 0 || window < 0 || block <= 0) return TS_ERR_BAD_ARGUMENT;
+  if (row_bytes % 16 || num_seqs > 65535 || ((uintptr_t)cache | (uintptr_t)out) % 16) return TS_ERR_UNSUPPORTED_SIZE;
+  return ts_launch(latent_gather_kernel, dim3((max_keys + GATHER_ROWS - 1) / GATHER_ROWS, num_seqs), dim3(256), 0, (cudaStream_t)stream,
+                   (const uint4*)cache, (uint4*)out, cu_seqlens, context_lens, block_table, max_blocks, page, row_bytes / 16, window, block);
 }
 
 // ---------------------------------------------------------------------------------------------

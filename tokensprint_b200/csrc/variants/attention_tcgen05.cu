@@ -23,11 +23,20 @@
 //
 // Limits (the caller falls back to the mma.sync kernel otherwise): head size 128; at most 128
 // query heads per KV head; the page size is at least 8 and divides 64 or is a multiple of 128.
+//
+// Built with TS_ATT_ROT=64 the file holds another kernel made of the same parts: prompt portions of a
+// latent attention whose keys and values have been rebuilt from the cached rows (see "Rebuilt keys").
 #include "../common.cuh"
 #include "kv_tensor_map.cuh"
 
 #if TS_HEAD_DIM != 128
 #error "attention_tcgen05.cu is written for TS_HEAD_DIM=128"
+#endif
+#ifndef TS_ATT_ROT
+#define TS_ATT_ROT 0
+#endif
+#if TS_ATT_ROT != 0 && TS_ATT_ROT != 64
+#error "the rotated entries of a rebuilt key are one swizzled box of 64"
 #endif
 
 namespace {
@@ -48,17 +57,17 @@ constexpr uint32_t OFF_V = OFF_K + STAGES * KV_STAGE;
 // P of a block lies where that block's K lay: K is dead once S is computed, P is dead once
 // O_blk is, and only then is the stage filled again.
 static_assert(P_BYTES == KV_STAGE, "P takes the place of one K stage");
-constexpr uint32_t SMEM_TILES = OFF_V + STAGES * KV_STAGE;  // 98,304 bytes: two CTAs per SM
+[[maybe_unused]] constexpr uint32_t SMEM_TILES = OFF_V + STAGES * KV_STAGE;  // 98,304 bytes: two CTAs per SM
 constexpr int MAX_TABLE = 1024;                   // block-table entries kept in shared memory
-constexpr uint32_t TMEM_COLS = 256;               // S: 64 columns, O_blk: 128 columns
-constexpr uint32_t TMEM_S = 0, TMEM_O = 64;
+[[maybe_unused]] constexpr uint32_t TMEM_COLS = 256;               // S: 64 columns, O_blk: 128 columns
+[[maybe_unused]] constexpr uint32_t TMEM_S = 0, TMEM_O = 64;
 
 // Builds with TS_ATT_SCORED=1 also know a sink score per query head, a tanh cap on the scores and a logarithmic distance penalty; the others
 // carry none of that code (their callers are refused both).
 #ifndef TS_ATT_SCORED
 #define TS_ATT_SCORED 0
 #endif
-constexpr bool SCORED = TS_ATT_SCORED != 0;
+[[maybe_unused]] constexpr bool SCORED = TS_ATT_SCORED != 0;
 struct Params {
   __nv_bfloat16* out;     // [T, nq, D]
   const int* cu_q;        // [B + 1]
@@ -75,6 +84,9 @@ struct Params {
   float cap_raw, cap_inv;   // cap / scale and scale / cap: a raw score s becomes cap_raw * tanh(s * cap_inv); cap_raw 0: no cap
   const float* dist_r1;     // [nq] with dist_r2: the scaled score of key j for a query at position i loses r1 * ln(1 + r2 * (i - j)); null: no penalty
   const float* dist_r2;
+#endif
+#if TS_ATT_ROT
+  const float* gates;  // [T, nq] what a finished row is multiplied by, or null
 #endif
   float scale_log2;
   long long* probe;  // TS_ATT_PROBE builds: clock stamps of CTA 0's first softmax warp and of its MMA thread
@@ -115,12 +127,17 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   *abort_flag = 1;
   return false;
 }
+[[maybe_unused]] __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1) : "memory");
+}
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
       ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
 }
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2, int c3) {
+[[maybe_unused]] __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2, int c3) {
   asm volatile(
       "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
       ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
@@ -135,7 +152,7 @@ __device__ __forceinline__ uint64_t desc_mn_major(uint32_t addr, uint32_t lbo) {
   return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)((lbo >> 4) & 0x3FFF) << 16) | ((uint64_t)(1024 >> 4) << 32) |
          (1ull << 46) | (2ull << 61);
 }
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+[[maybe_unused]] __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
@@ -253,6 +270,7 @@ __host__ __device__ constexpr uint32_t idesc(int n, bool b_mn_major) {
          ((uint32_t)(BM >> 4) << 24);
 }
 
+#if TS_ATT_ROT == 0
 __global__ void __launch_bounds__(128, 2) attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q,
                                                                    const __grid_constant__ CUtensorMap map_k,
                                                                    const __grid_constant__ CUtensorMap map_v,
@@ -530,6 +548,7 @@ __global__ void __launch_bounds__(128, 2) attention_tcgen05_kernel(const __grid_
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
   }
 }
+#endif  // TS_ATT_ROT == 0
 
 // ---------------------------------------------------------------------------
 // Two tiles per CTA, roles in warps of their own (long prompt portions).
@@ -553,15 +572,30 @@ __global__ void __launch_bounds__(128, 2) attention_tcgen05_kernel(const __grid_
 // float32 range, and the final division by the row sum, taken with the same max, cancels it);
 // only then is the row of O rescaled in tensor memory.
 // Synchronisation is by mbarriers alone; every wait is bounded.
+//
+// Rebuilt keys (TS_ATT_ROT = 64): a head's query and key have 64 further entries behind the 128, and the
+// key's are the same for every head (the rotated part of a latent attention's cached row).  A KV head is
+// a query head of its own, so a tile is 128 tokens.  The keys and values lie as rows of two matrices, `kv`
+// [rows, nkv x 128 keys | nkv x 128 values] and `rows` [rows, rank + 64], the kept keys of the sequences one after
+// the other, each sequence from a multiple of PBN of its positions on (first_kept_key), so a block
+// begins at the same keys wherever a prompt was cut.  Q takes 3 x 16 KB per tile and K three
+// boxes a block: with blocks of 128 keys only one stage of V would fit the SM's shared memory, and V would be
+// asked for when its place is free, half a block before it is needed; blocks of 96 leave room for both rings of two.
+// Measured (16 heads, 8,191 tokens, window 4,096): 288 us a layer, 0.90 PFLOP/s of the 320 multiply-adds per (query, key,
+// head); latent_attention_mma.cu, on the cached rows themselves (1,088 multiply-adds, mma.sync), took 5,150.
 
-constexpr int PBN = 128;                          // keys per block of this kernel
-constexpr uint32_t PKV_HALF = PBN * 128;          // [128 keys x 128 B]: half a head
-constexpr uint32_t PKV_STAGE = 2 * PKV_HALF;      // both halves of the head
+constexpr bool REBUILT = TS_ATT_ROT != 0;
+constexpr int QK = D + TS_ATT_ROT;                // entries of a query and of a key
+constexpr int PBN = REBUILT ? 96 : 128;           // keys per block of this kernel
+constexpr int HALF = PBN / 2;                     // of them per softmax thread
+constexpr uint32_t PKV_HALF = PBN * 128;          // [PBN keys x 128 B]: half a head
+constexpr uint32_t PK_STAGE = QK / 64 * PKV_HALF, PV_STAGE = 2 * PKV_HALF;  // all parts of the head
+constexpr uint32_t PQ_BYTES = QK / 64 * BM * 128;
 constexpr int KV_RING = 2;
-constexpr uint32_t P2_OFF_Q = 0;                                   // 2 tiles x 32 KB
-constexpr uint32_t P2_OFF_K = P2_OFF_Q + 2 * Q_BYTES;
-constexpr uint32_t P2_OFF_V = P2_OFF_K + KV_RING * PKV_STAGE;
-constexpr uint32_t P2_SMEM = P2_OFF_V + KV_RING * PKV_STAGE;       // 196,608 bytes
+constexpr uint32_t P2_OFF_Q = 0;                                   // 2 tiles x 32 KB (REBUILT: 48 KB)
+constexpr uint32_t P2_OFF_K = P2_OFF_Q + 2 * PQ_BYTES;
+constexpr uint32_t P2_OFF_V = P2_OFF_K + KV_RING * PK_STAGE;
+constexpr uint32_t P2_SMEM = P2_OFF_V + KV_RING * PV_STAGE;        // 196,608 bytes (REBUILT: 221,184)
 constexpr uint32_t P2_TMEM_COLS = 512;
 // columns: S[tile] at tile * 128; O[tile] at 256 + tile * 128.  P of a block takes the first 64
 // columns of its tile's S.
@@ -645,9 +679,30 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
       : "memory");
 }
 
+// as many columns as the array has entries
+[[maybe_unused]] __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld32(taddr, r); }
+[[maybe_unused]] __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld16(taddr, r); }
+[[maybe_unused]] __device__ __forceinline__ void tmem_st(uint32_t taddr, const uint32_t (&r)[32]) { tmem_st32(taddr, r); }
+[[maybe_unused]] __device__ __forceinline__ void tmem_st(uint32_t taddr, const uint32_t (&r)[16]) { tmem_st16(taddr, r); }
+[[maybe_unused]] __device__ __forceinline__ void tmem_st(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+// Rebuilt keys: the first key of a sequence that has a row, a multiple of PBN (rows before the first one anybody
+// sees are zeros), for a portion of q_len tokens that ends at position ctx - 1.
+[[maybe_unused]] __device__ __forceinline__ int first_kept_key(int window, int q_len, int ctx) {
+  const int lo = window > 0 ? ctx - q_len - window + 1 : 0;
+  return lo > 0 ? lo / PBN * PBN : 0;
+}
+
 __global__ void __launch_bounds__(608, 1) attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_q,
                                                                         const __grid_constant__ CUtensorMap map_k,
                                                                         const __grid_constant__ CUtensorMap map_v,
+#if TS_ATT_ROT
+                                                                        const __grid_constant__ CUtensorMap map_q_rot,
+                                                                        const __grid_constant__ CUtensorMap map_k_rot,
+                                                                        int k_rot_column, int q_rot_first,
+#endif
                                                                         const Params p) {
   ts_pdl_wait();  // see the other kernel: tensor memory is never held while waiting for another kernel
   extern __shared__ unsigned char smem_unaligned[];
@@ -656,7 +711,7 @@ __global__ void __launch_bounds__(608, 1) attention_tcgen05_pair_kernel(const __
   __shared__ __align__(8) uint64_t s_done[2], p_ready[2], all_done;  // per tile
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
-  __shared__ int table_s[MAX_TABLE];
+  __shared__ int table_s[REBUILT ? 1 : MAX_TABLE];  // REBUILT: the row of the sequence's key 0 (may be negative)
   __shared__ int quit_s[2][4][2];   // [tile][quarter of the rows][block parity]: see the softmax warps
   __shared__ float sum_s[2][2][BM];  // [tile][half of the keys][row]: what the two threads of a row tell each other (a block's largest score; at the end their sums)
 
@@ -684,8 +739,10 @@ __global__ void __launch_bounds__(608, 1) attention_tcgen05_pair_kernel(const __
   // Both tiles walk all blocks of the later one (its last block may be fully masked for the
   // earlier tile): the two tiles stay in step.
   const int nblocks = hi / PBN - kb0 + 1;
+#if TS_ATT_ROT == 0
   const int box_rows = min(p.page, PBN);
   const int copies_per_block = PBN / box_rows;
+#endif
 
   if (tid == 0) {
     abort_s = 0;
@@ -704,6 +761,17 @@ __global__ void __launch_bounds__(608, 1) attention_tcgen05_pair_kernel(const __
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
+#if TS_ATT_ROT
+  if (warp == 16) {
+    int before = 0;  // rows of the sequences ahead
+    for (int i = lane; i < b; i += 32) {
+      const int n = p.cu_q[i + 1] - p.cu_q[i], end = p.ctx_len[i];
+      if (n > 0) before += end - first_kept_key(p.window, n, end);
+    }
+    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+    if (lane == 0) table_s[0] = before - first_kept_key(p.window, q_len, ctx);
+  }
+#else
   const int first_entry = (kb0 * PBN) / p.page;
   {
     const int n_entries = min(hi / p.page - first_entry + 1, MAX_TABLE);
@@ -713,12 +781,13 @@ __global__ void __launch_bounds__(608, 1) attention_tcgen05_pair_kernel(const __
       table_s[i] = e < p.max_blocks ? table[e] : -1;
     }
   }
+#endif
   if (RT < BM) {
     // the rows of the Q tiles that no copy fills (they belong to nobody): zeros, so that their scores are
     // numbers like any others
     for (int i = tid; i < 4 * (BM - RT) * 8; i += blockDim.x) {
       const int part = i / ((BM - RT) * 8), rest = i % ((BM - RT) * 8);  // part: tile * 2 + half of the head
-      *reinterpret_cast<uint4*>(smem + P2_OFF_Q + (part >> 1) * Q_BYTES + (part & 1) * (BM * 128) + (RT + rest / 8) * 128 + (rest % 8) * 16) =
+      *reinterpret_cast<uint4*>(smem + P2_OFF_Q + (part >> 1) * PQ_BYTES + (part & 1) * (BM * 128) + (RT + rest / 8) * 128 + (rest % 8) * 16) =
           make_uint4(0u, 0u, 0u, 0u);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -738,21 +807,35 @@ __global__ void __launch_bounds__(608, 1) attention_tcgen05_pair_kernel(const __
 
   if (warp == 16) {
     // ---------------- copies: lane 0 announces the bytes, lanes 0..2*copies-1 each ask for one box ----------------
+#if TS_ATT_ROT
+    if (lane == 0) {
+      mbar_expect_tx(smem_u32(&q_full), (uint32_t)ntiles * PQ_BYTES);
+      for (int t = 0; t < ntiles; ++t) {
+        const uint32_t q_tile = sm + P2_OFF_Q + t * PQ_BYTES;
+        tma_load_3d(q_tile, &map_q, smem_u32(&q_full), 0, hk, q_begin + r0 + t * BM);
+        tma_load_3d(q_tile + BM * 128, &map_q, smem_u32(&q_full), 64, hk, q_begin + r0 + t * BM);
+        tma_load_3d(q_tile + 2 * BM * 128, &map_q_rot, smem_u32(&q_full), 0, hk, q_begin + r0 + t * BM - q_rot_first);
+      }
+    }
+    const int key0_row = table_s[0];
+#else
     if (lane == 0) {
       mbar_expect_tx(smem_u32(&q_full), (uint32_t)(ntiles * 2 * RT * 128));  // per tile two half-head boxes of RT rows
       for (int t = 0; t < ntiles; ++t)
         for (int half = 0; half < 2; ++half)
-          tma_load_4d(sm + P2_OFF_Q + t * Q_BYTES + half * (BM * 128), &map_q, smem_u32(&q_full), half * 64, 0, hk,
+          tma_load_4d(sm + P2_OFF_Q + t * PQ_BYTES + half * (BM * 128), &map_q, smem_u32(&q_full), half * 64, 0, hk,
                       q_begin + (r0 + t * RT) / G);
     }
     const int c = lane >> 1, half = lane & 1;  // this lane's copy within a block, and its half of the head
     const bool copies = c < copies_per_block;
     const uint32_t lane_off = (uint32_t)half * PKV_HALF + (uint32_t)(c * box_rows) * 128u;
+#endif
     int issued[2] = {0, 0};  // K and V blocks asked for
     bool ok = true;
     for (int blk = 0; ok && blk < nblocks; ++blk) {
       const int st = blk % KV_RING;
       const uint32_t use = (uint32_t)(blk / KV_RING);
+#if TS_ATT_ROT == 0
       // where this lane's box starts in the cache
       int slot = p.total_slots;  // beyond the end: the copy engine fills zeros (a page that is not held)
       if (copies) {
@@ -763,6 +846,7 @@ __global__ void __launch_bounds__(608, 1) attention_tcgen05_pair_kernel(const __
           if (page_id >= 0) slot = page_id * p.page + (key0 - e * p.page);
         }
       }
+#endif
 #pragma unroll
       for (int which = 0; which < 2; ++which) {  // K first: S needs it first
         const uint32_t full = smem_u32(which == 0 ? &k_full[st] : &v_full[st]);
@@ -770,11 +854,19 @@ __global__ void __launch_bounds__(608, 1) attention_tcgen05_pair_kernel(const __
         if (blk >= KV_RING) ok = mbar_wait(empty, (use - 1) & 1, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
-        if (lane == 0) mbar_expect_tx(full, PKV_STAGE);
+        if (lane == 0) mbar_expect_tx(full, which == 0 ? PK_STAGE : PV_STAGE);
         __syncwarp();
-        if (copies)
-          tma_load_3d(sm + (which == 0 ? P2_OFF_K : P2_OFF_V) + st * PKV_STAGE + lane_off, which == 0 ? &map_k : &map_v, full,
-                      half * 64, hk, slot);
+        const uint32_t stage = sm + (which == 0 ? P2_OFF_K + st * PK_STAGE : P2_OFF_V + st * PV_STAGE);
+#if TS_ATT_ROT
+        // rows behind the last one are filled with zeros by the copy engine; rows of the next sequence count for nothing
+        const int row = key0_row + (kb0 + blk) * PBN;
+        if (lane < 2)
+          tma_load_2d(stage + lane * PKV_HALF, &map_k, full, (which * p.nkv + hk) * D + lane * 64, row);
+        else if (lane == 2 && which == 0)
+          tma_load_2d(stage + 2 * PKV_HALF, &map_k_rot, full, k_rot_column, row);
+#else
+        if (copies) tma_load_3d(stage + lane_off, which == 0 ? &map_k : &map_v, full, half * 64, hk, slot);
+#endif
         issued[which] = blk + 1;
       }
     }
@@ -812,12 +904,12 @@ __global__ void __launch_bounds__(608, 1) attention_tcgen05_pair_kernel(const __
     const uint64_t v_desc = desc_mn_major(sm + P2_OFF_V, PKV_HALF);
     auto issue_s = [&](int t, int blk) {  // S of block blk for tile t; the block's K is free again after the last tile's
       const int st = blk % KV_RING;
-      const uint64_t kd = k_desc + (uint64_t)((st * PKV_STAGE) >> 4);
-      const uint64_t qd = q_desc + (uint64_t)((t * Q_BYTES) >> 4);
+      const uint64_t kd = k_desc + (uint64_t)((st * PK_STAGE) >> 4);
+      const uint64_t qd = q_desc + (uint64_t)((t * PQ_BYTES) >> 4);
       const uint32_t s_addr = tmem_base + t * 128;
       if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks) {
+        for (int ks = 0; ks < QK / 16; ++ks) {
           const uint32_t off_q = ((ks >> 2) * (BM * 128) + (ks & 3) * 32) >> 4, off_k = ((ks >> 2) * PKV_HALF + (ks & 3) * 32) >> 4;
           if (ks == 0)
             umma_bf16_first(s_addr, qd + off_q, kd + off_k, idesc(PBN, false));
@@ -837,7 +929,7 @@ __global__ void __launch_bounds__(608, 1) attention_tcgen05_pair_kernel(const __
     }
     for (int j = 0; ok && j < nblocks; ++j) {
       const int st = j % KV_RING;
-      const uint64_t vd = v_desc + (uint64_t)((st * PKV_STAGE) >> 4);
+      const uint64_t vd = v_desc + (uint64_t)((st * PV_STAGE) >> 4);
       for (int t = 0; ok && t < ntiles; ++t) {
         if (lane == 0) PROBE(1, j, t * 3);
         ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&p_ready[t]), (uint32_t)j & 1, abort_flag));
@@ -845,14 +937,14 @@ __global__ void __launch_bounds__(608, 1) attention_tcgen05_pair_kernel(const __
         if (lane == 0) PROBE(1, j, t * 3 + 1);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t o_addr = tmem_base + 256 + t * 128;
-        const uint32_t p_addr = tmem_base + t * 128;  // 16 keys of P: 8 columns; keys 0..63 from column 0, keys 64..127 from column 64
+        const uint32_t p_addr = tmem_base + t * 128;  // 16 keys of P: 8 columns; the first half of the keys from column 0, the others from column HALF
         if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < PBN / 16; ++kk) {
             if (kk == 0 && j == 0)
               umma_bf16_tmem_a_first(o_addr, p_addr, vd, idesc(D, true));
             else
-              umma_bf16_tmem_a_more(o_addr, p_addr + (kk >> 2) * 64 + (kk & 3) * 8, vd + ((kk * 2048) >> 4), idesc(D, true));
+              umma_bf16_tmem_a_more(o_addr, p_addr + kk / (HALF / 16) * HALF + kk % (HALF / 16) * 8, vd + ((kk * 2048) >> 4), idesc(D, true));
           }
           if (t == ntiles - 1) umma_commit(smem_u32(&v_empty[st]));
         }
@@ -882,7 +974,7 @@ __global__ void __launch_bounds__(608, 1) attention_tcgen05_pair_kernel(const __
     const int tile_first_pos = start_pos + (r0 + t * RT) / G;
     const int tile_last_pos = start_pos + (min(r0 + t * RT + RT, rows_total) - 1) / G;  // of the tile's rows that belong to a token
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
-    const uint32_t s_addr = lane_addr + t * 128 + h * 64;        // this thread's 64 scores; its P goes over the first 32 of them
+    const uint32_t s_addr = lane_addr + t * 128 + h * HALF;      // this thread's 64 (REBUILT: 48) scores; its P goes over the first half of them
     const int pair_bar = 3 + t * 4 + quad;                       // hardware barrier of the two warps that share rows
     const uint32_t o_addr = lane_addr + 256 + t * 128 + h * 64;  // its half of the row of O
     // l_run: the sum over this thread's keys only; with a sink both threads of a row start from its score
@@ -891,56 +983,59 @@ __global__ void __launch_bounds__(608, 1) attention_tcgen05_pair_kernel(const __
     bool ok = true;
 
     for (int blk = 0; blk < nblocks; ++blk) {
-      const int kbase = (kb0 + blk) * PBN + h * 64;
+      const int kbase = (kb0 + blk) * PBN + h * HALF;
       if (h == 0 && row == 0) PROBE(t * 2, blk, 0);
       mbar_wait(smem_u32(&s_done[t]), (uint32_t)blk & 1, abort_flag);  // if it gives up: on to the barrier below, and out there
       __syncwarp();
       if (h == 0 && row == 0) PROBE(t * 2, blk, 1);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      // every one of these 64 keys is seen by every row of the tile that belongs to a token (rows that
+      // every one of these keys is seen by every row of the tile that belongs to a token (rows that
       // belong to nobody need no mask: a row's result depends on that row alone, and theirs is never stored)
-      const bool unmasked = (kbase + 63 <= tile_first_pos) && kbase >= first_visible_key(p, tile_last_pos);
-      // First walk over this thread's 64 scores: their largest.
+      const bool unmasked = (kbase + HALF - 1 <= tile_first_pos) && kbase >= first_visible_key(p, tile_last_pos);
+      // First walk over this thread's scores: their largest.
+      constexpr int PIECE = HALF % 32 == 0 ? 32 : 16, PIECES = HALF / PIECE;  // columns of tensor memory per load
       float m_blk;
       {
-        uint32_t v0[32], v1[32];
-        tmem_ld32(s_addr, v0);
-        tmem_ld32(s_addr + 32, v1);
+        uint32_t v[PIECES][PIECE];
+#pragma unroll
+        for (int g = 0; g < PIECES; ++g) tmem_ld(s_addr + g * PIECE, v[g]);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         if (has_cap(p) || has_distance(p)) {
           // the capped (and distance-charged) scores take the raw ones' place in tensor memory: the second walk reads them from there
           if (has_cap(p)) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              v0[i] = __float_as_uint(capped_score(p, __uint_as_float(v0[i])));
-              v1[i] = __float_as_uint(capped_score(p, __uint_as_float(v1[i])));
-            }
+            for (int g = 0; g < PIECES; ++g)
+#pragma unroll
+              for (int i = 0; i < PIECE; ++i) v[g][i] = __float_as_uint(capped_score(p, __uint_as_float(v[g][i])));
           }
           if (has_distance(p)) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              v0[i] = __float_as_uint(__uint_as_float(v0[i]) - distance_penalty(dist_a, dist_b, row_pos, kbase + i));
-              v1[i] = __float_as_uint(__uint_as_float(v1[i]) - distance_penalty(dist_a, dist_b, row_pos, kbase + 32 + i));
-            }
+            for (int g = 0; g < PIECES; ++g)
+#pragma unroll
+              for (int i = 0; i < PIECE; ++i)
+                v[g][i] = __float_as_uint(__uint_as_float(v[g][i]) - distance_penalty(dist_a, dist_b, row_pos, kbase + g * PIECE + i));
           }
-          tmem_st32(s_addr, v0);
-          tmem_st32(s_addr + 32, v1);
+#pragma unroll
+          for (int g = 0; g < PIECES; ++g) tmem_st(s_addr + g * PIECE, v[g]);
           asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         }
         float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // four chains: the warp has few others to hide latency behind
         if (unmasked) {
 #pragma unroll
-          for (int i = 0; i < 32; i += 4) {
+          for (int i = 0; i < PIECE; ++i) {
+            float top = __uint_as_float(v[PIECES - 1][i]);
 #pragma unroll
-            for (int u = 0; u < 4; ++u) mx[u] = fmaxf(mx[u], fmaxf(__uint_as_float(v0[i + u]), __uint_as_float(v1[i + u])));
+            for (int g = PIECES - 2; g >= 0; --g) top = fmaxf(__uint_as_float(v[g][i]), top);
+            mx[i & 3] = fmaxf(mx[i & 3], top);
           }
         } else {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int key0 = kbase + i, key1 = key0 + 32;
-            if (key0 <= row_pos && key0 >= row_lo) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(v0[i]));
-            if (key1 <= row_pos && key1 >= row_lo) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(v1[i]));
-          }
+          for (int i = 0; i < PIECE; ++i)
+#pragma unroll
+            for (int g = 0; g < PIECES; ++g) {
+              const int key = kbase + g * PIECE + i;
+              if (key <= row_pos && key >= row_lo) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(v[g][i]));
+            }
         }
         m_blk = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
       }
@@ -985,24 +1080,24 @@ __global__ void __launch_bounds__(608, 1) attention_tcgen05_pair_kernel(const __
       // (exp2_pair_fma).  (Measured at 8,192 tokens: none 543 us, one 524, two 525, three 566.)
       uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull};  // four chains of two float32 sums each (0 is +0.0 twice)
       const uint64_t scale2 = pack2(p.scale_log2, p.scale_log2), off2 = pack2(-m_off, -m_off);
-      // Second walk, 32 scores at a time.  P goes over the first half of the scores it came from
-      // (this thread's own lane and columns): P of keys 32 g .. 32 g + 31 to columns 16 g .. 16 g + 15,
+      // Second walk, PIECE scores at a time.  P goes over the first half of the scores it came from
+      // (this thread's own lane and columns): P of piece g to half as many columns from g * PIECE / 2 on,
       // over scores that have been read.
 #pragma unroll
-      for (int g = 0; g < 2; ++g) {
-        uint32_t v[32];
-        tmem_ld32(s_addr + g * 32, v);
+      for (int g = 0; g < PIECES; ++g) {
+        uint32_t v[PIECE];
+        tmem_ld(s_addr + g * PIECE, v);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         if (!unmasked) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int key = kbase + g * 32 + i;
+          for (int i = 0; i < PIECE; ++i) {
+            const int key = kbase + g * PIECE + i;
             if (!(key <= row_pos && key >= row_lo)) v[i] = __float_as_uint(-INFINITY);
           }
         }
-        uint32_t packed[16];
+        uint32_t packed[PIECE / 2];
 #pragma unroll
-        for (int j = 0; j < 32; j += 8) {
+        for (int j = 0; j < PIECE; j += 8) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             float p0, p1;
@@ -1017,7 +1112,7 @@ __global__ void __launch_bounds__(608, 1) attention_tcgen05_pair_kernel(const __
             packed[(j >> 1) + i] = pack_bf16(p0, p1);
           }
         }
-        tmem_st16(s_addr + g * 16, packed);
+        tmem_st(s_addr + g * (PIECE / 2), packed);
       }
       {
         float even, odd;
@@ -1037,7 +1132,7 @@ __global__ void __launch_bounds__(608, 1) attention_tcgen05_pair_kernel(const __
         const int first_bad = hi - (kb0 + blk) * PBN + 1;
         for (int i = h * BM + row; i < (PBN - first_bad) * 16; i += 2 * BM) {
           const int vrow = first_bad + i / 16, piece = i % 16;
-          *reinterpret_cast<uint4*>(smem + P2_OFF_V + st * PKV_STAGE + (piece >> 3) * PKV_HALF + vrow * 128 + ((piece & 7) << 4)) =
+          *reinterpret_cast<uint4*>(smem + P2_OFF_V + st * PV_STAGE + (piece >> 3) * PKV_HALF + vrow * 128 + ((piece & 7) << 4)) =
               make_uint4(0u, 0u, 0u, 0u);
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1055,8 +1150,11 @@ __global__ void __launch_bounds__(608, 1) attention_tcgen05_pair_kernel(const __
     sum_s[t][h][row] = l_run;
     asm volatile("bar.sync %0, 256;" ::"r"(1 + t) : "memory");
     l_run += sum_s[t][h ^ 1][row];
-    const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-    unsigned char* o_tile = smem + P2_OFF_Q + t * Q_BYTES;
+    float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+#if TS_ATT_ROT
+    if (p.gates != nullptr && row_pos >= 0) inv *= p.gates[(size_t)(q_begin + r) * p.nq + hk];
+#endif
+    unsigned char* o_tile = smem + P2_OFF_Q + t * PQ_BYTES;
     if (good) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       // The tile goes through shared memory (where its Q lay: the tensor core is done with it), so
@@ -1106,6 +1204,78 @@ __global__ void __launch_bounds__(608, 1) attention_tcgen05_pair_kernel(const __
 
 // ---------------------------------------------------------------------------
 // host side
+
+#if TS_ATT_ROT
+// A tensor of rank 2 or 3, boxes 64 entries (128 bytes, swizzled) wide.
+int rows_map(const void* ptr, int rank, const cuuint64_t (&dims)[3], const cuuint64_t (&strides)[2], const cuuint32_t (&box)[3], CUtensorMap* out) {
+  TsEncodeTiledFn fn = ts_encode_tiled();
+  if (!fn) return TS_ERR_UNSUPPORTED_SIZE;
+  const cuuint32_t estr[3] = {1, 1, 1};
+  return fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS
+             ? 0
+             : TS_ERR_BAD_ARGUMENT;
+}
+
+}  // namespace
+
+// Every sequence's kept keys begin at a multiple of this many positions.
+TS_EXPORT int ts_latent_rebuilt_block() { return PBN; }
+
+// q [T, H, 128 + 64] bf16, a token's row `ld_q` entries from the next one's (the last 64 of a head are not read), q_rot
+// [T - q_rot_first, H, 64] of the tokens from q_rot_first on (the sequences' tokens are among them);
+// kv [S, H x 128 | H x 128], rows [S, ld_rows] with the rotated key entries at column `rot_column`: the kept keys of
+// the sequences one after the other (first_kept_key; S is their sum); out [T, H, 128]; gates [T, H] f32 or null;
+// sinks [H] f32 or null; cu_q [B + 1] and ctx_len [B]; max_q: the most tokens of any sequence.
+TS_EXPORT int ts_latent_rebuilt_attention(const void* q, long long ld_q, const void* q_rot, int q_rot_first, const void* kv, const void* rows,
+                                          long long ld_rows, int rot_column, void* out, const float* gates, const float* sinks, const int* cu_q,
+                                          const int* ctx_len, long long S, int T, int B, int max_q, int H, float scale, int window, int* error,
+                                          void* stream) {
+  if (T <= 0 || B <= 0) return 0;
+  if (H <= 0 || max_q <= 0 || S <= 0 || q_rot_first < 0 || q_rot_first >= T || !(scale > 0.f) || error == nullptr || ld_q < (long long)H * QK ||
+      rot_column < 0 || ld_rows < rot_column + 64)
+    return TS_ERR_BAD_ARGUMENT;
+  const uintptr_t pointers = (uintptr_t)q | (uintptr_t)q_rot | (uintptr_t)kv | (uintptr_t)rows | (uintptr_t)out;
+  if (pointers % 16 || ld_q % 8 || ld_rows % 8 || rot_column % 8) return TS_ERR_UNSUPPORTED_SIZE;
+  const long long ctas = ((long long)max_q + 2 * BM - 1) / (2 * BM) * H * B;
+  if (S > 0x7fffffffLL - PBN || ctas > 0x7fffffffLL || H > 65535) return TS_ERR_UNSUPPORTED_SIZE;
+  Params p = {};
+  p.out = (__nv_bfloat16*)out;
+  p.cu_q = cu_q;
+  p.ctx_len = ctx_len;
+  p.error = error;
+  p.page = 1;
+  p.nq = p.nkv = H;
+  p.window = window;
+  p.num_seqs = B;
+  p.has_sink = sinks != nullptr ? 1 : 0;
+#if TS_ATT_SCORED
+  p.head_sinks = sinks;
+  p.inv_scale = 1.f / scale;
+#else
+  if (sinks != nullptr) return TS_ERR_BAD_ARGUMENT;
+#endif
+  p.gates = gates;
+  p.scale_log2 = scale * 1.4426950408889634f;
+  CUtensorMap mq, mqr, mkv, mkr;
+  const cuuint64_t UH = (cuuint64_t)H, UT = (cuuint64_t)T, US = (cuuint64_t)S;
+  int st = rows_map(q, 3, {QK, UH, UT}, {QK * 2, (cuuint64_t)ld_q * 2}, {64, 1, BM}, &mq);
+  if (!st) st = rows_map(q_rot, 3, {64, UH, UT - (cuuint64_t)q_rot_first}, {64 * 2, UH * 64 * 2}, {64, 1, BM}, &mqr);
+  if (!st) st = rows_map(kv, 2, {2 * UH * D, US, 1}, {2 * UH * D * 2, 0}, {64, PBN, 1}, &mkv);
+  if (!st) st = rows_map(rows, 2, {(cuuint64_t)rot_column + 64, US, 1}, {(cuuint64_t)ld_rows * 2, 0}, {64, PBN, 1}, &mkr);
+  if (st) return st;
+  const size_t smem = P2_SMEM + 1024;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(attention_tcgen05_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  return ts_launch(attention_tcgen05_pair_kernel, dim3((unsigned)ctas), dim3(608), smem, (cudaStream_t)stream, mq, mkv, mkv, mqr, mkr, rot_column,
+                   q_rot_first, p);
+}
+
+#else  // paged keys and values
 
 // q [T, nq, D] as a 4-d tensor {D, G, nkv, T}; boxes of {64, G, 1, 128 / G}: the rows of a box
 // come out ordered (token, head of the group), which is the tile's row order.
@@ -1239,3 +1409,4 @@ TS_EXPORT int ts_attention_prefill_tcgen05(const void* q, const void* kcache, co
   return ts_attention_prefill_tcgen05_scored(q, kcache, vcache, out, cu_q, ctx_len, block_table, max_blocks, page, total_slots, T, B, max_q,
                                              nq, nkv, scale, window, chunk, has_sink, sink_score, 0.f, nullptr, mode, error, stream_, nullptr, nullptr);
 }
+#endif  // TS_ATT_ROT

@@ -50,7 +50,9 @@ _SIGNATURES = {
     "ts_rmsnorm_add": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_float, _c_void_p],
     "ts_round_rows": [_c_void_p, _c_int, _c_void_p, _c_int, _c_ll, _c_void_p],
     "ts_latent_prepare": [_c_void_p, _c_int, _c_ll, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_float,
-                          _c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_void_p, _c_ll, _c_void_p],
+                          _c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_float, _c_void_p, _c_ll,
+                          _c_void_p],
+    "ts_latent_gather": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p],
     "ts_latent_attention_simple": [_c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int,
                                    _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_void_p, _c_void_p],
     "ts_gelu_tanh": [_c_void_p, _c_void_p, _c_int, _c_ll, _c_void_p],
@@ -1452,7 +1454,8 @@ LATENT_SIMPLE_MAX_KEY_DIM = 1024
 def latent_prepare(proj: Optional[torch.Tensor], q_off: int, kv_off: int, gate_off: int, q_abs: torch.Tensor, cache: Optional[torch.Tensor],
                    slot_mapping: Optional[torch.Tensor], positions: torch.Tensor, latent_weight: Optional[torch.Tensor], eps: float,
                    inv_freq: Optional[torch.Tensor], rot_dims: int, pairing: str, gates: Optional[torch.Tensor], num_heads: int,
-                   nope_dim: int, rot_dim: int, rank: int, magnitude: float = 1.0, q_src: Optional[torch.Tensor] = None) -> None:
+                   nope_dim: int, rot_dim: int, rank: int, magnitude: float = 1.0, q_src: Optional[torch.Tensor] = None,
+                   q_rot: Optional[torch.Tensor] = None) -> None:
     """What follows the stacked projection of a latent attention layer, per token: the latent (columns
     kv_off .. kv_off+rank of `proj`) RMS-normed with `latent_weight`, the key part behind it and
     every head's rotated query part turned by the token's position, [latent ; key part] stored in
@@ -1461,9 +1464,16 @@ def latent_prepare(proj: Optional[torch.Tensor], q_off: int, kv_off: int, gate_o
     Cosines and sines are multiplied by `magnitude`.  `q_src` [T, heads*(nope+rot)]: the queries come
     from this tensor instead of proj's columns from q_off on.  kv_off < 0: the layer has no latent of
     its own (it reads rows that another layer cached): only the queries are prepared, and `proj` may
-    then be None."""
+    then be None.  `q_rot` [t, heads, rot]: the step's last t tokens leave their rotated query parts there and
+    q_abs holds the others only."""
     flush_gemm_chain()
     H, dn, dr = num_heads, nope_dim, rot_dim
+    rotated_only = 0
+    if q_rot is not None:
+        _cuda_contig("q_rot", q_rot, q_abs.dtype)
+        rotated_only = q_rot.shape[0]
+        if q_rot.numel() != rotated_only * H * dr:
+            raise KernelError(f"latent_prepare: q_rot must be [tokens, {H}, {dr}], got {tuple(q_rot.shape)}")
     if q_src is not None:
         _cuda_contig("q_src", q_src, q_abs.dtype)
         if q_src.dim() != 2 or q_src.shape[1] != H * (dn + dr):
@@ -1481,8 +1491,8 @@ def latent_prepare(proj: Optional[torch.Tensor], q_off: int, kv_off: int, gate_o
         _cuda_contig("latent_weight", latent_weight, torch.float32)
     elif cache is not None or slot_mapping is not None:
         raise KernelError("latent_prepare: a layer without a latent of its own stores nothing")
-    if q_abs.numel() != T * H * (rank + dr):
-        raise KernelError(f"latent_prepare: q_abs must hold [{T}, {H}, {rank + dr}], got {tuple(q_abs.shape)}")
+    if rotated_only > T or q_abs.numel() != (T - rotated_only) * H * (rank + dr):
+        raise KernelError(f"latent_prepare: q_abs must hold [{T - rotated_only}, {H}, {rank + dr}], got {tuple(q_abs.shape)}")
     if (q_src is None and q_off + H * (dn + dr) > ld) or (kv_off >= 0 and kv_off + rank + dr > ld) or (gates is not None and gate_off + H > ld):
         raise KernelError("latent_prepare: the column ranges do not fit the projection's width")
     if slot_mapping is not None:
@@ -1503,9 +1513,9 @@ def latent_prepare(proj: Optional[torch.Tensor], q_off: int, kv_off: int, gate_o
         if inv_freq.numel() != rot_dims // 2 or rot_dims > dr or rot_dims % 2:
             raise KernelError(f"latent_prepare: {rot_dims} rotated entries of {dr} need {rot_dims // 2} frequencies")
     _check("latent_prepare", _fn("ts_latent_prepare")(
-        _ptr(proj), _act_code("q_abs", q_abs), ld, int(q_off), int(kv_off), int(gate_off), q_abs.data_ptr(), _ptr(cache),
+        _ptr(proj), _act_code("q_abs", q_abs), ld, int(q_off), int(kv_off), int(gate_off), q_abs.data_ptr() if T > rotated_only else None, _ptr(cache),
         _ptr(slot_mapping), positions.data_ptr(), _ptr(latent_weight), float(eps), _ptr(inv_freq), int(rot_dims),
-        ROTARY_PAIRINGS[pairing], _ptr(gates), T, H, dn, dr, int(rank), float(magnitude), _ptr(q_src),
+        ROTARY_PAIRINGS[pairing], _ptr(gates), T, H, dn, dr, int(rank), T - rotated_only, _ptr(q_rot), float(magnitude), _ptr(q_src),
         0 if q_src is None else q_src.stride(0), _stream()))
 
 
@@ -1901,6 +1911,88 @@ def latent_attention_mma(q_abs: torch.Tensor, cache: torch.Tensor, out: torch.Te
     if splits > 1:
         global launch_count
         launch_count += 1  # the merge kernel
+
+
+# Prompt portions with rebuilt keys and values (see csrc/variants/attention_tcgen05.cu).
+LATENT_REBUILT_SIZES = (128, 64, 128)  # the plain and the rotated entries of a query, and a value's
+_latent_rebuilt = None
+
+
+def _latent_rebuilt_fns():
+    global _latent_rebuilt
+    if _latent_rebuilt is None:
+        lib = _build.load_variant("attention_tcgen05", {"TS_HEAD_DIM": 128, "TS_ATT_SCORED": 1, "TS_ATT_ROT": LATENT_REBUILT_SIZES[1]})
+        run = lib.ts_latent_rebuilt_attention
+        run.argtypes = [_c_void_p, _c_ll, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_ll, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
+                        _c_void_p, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_void_p, _c_void_p]
+        run.restype = _c_int
+        lib.ts_latent_rebuilt_block.restype = _c_int
+        _latent_rebuilt = (run, lib.ts_latent_rebuilt_block())
+    return _latent_rebuilt
+
+
+def latent_kept_keys(window: int, q_len: int, context: int) -> int:
+    """How many rows latent_gather keeps of a sequence of `context` tokens whose last q_len are the step's."""
+    block = _latent_rebuilt_fns()[1]
+    first = max(0, context - q_len - window + 1) if window > 0 else 0
+    return context - first // block * block
+
+
+def latent_gather(cache: torch.Tensor, out: torch.Tensor, cu_seqlens: torch.Tensor, context_lens: torch.Tensor, block_table: torch.Tensor,
+                  page_size: int, num_seqs: int, max_keys: int, window: int = 0) -> None:
+    """The cached rows [pages, page, D] (bfloat16) that the sequences' portions see, one sequence after the other, in
+    out [sum of latent_kept_keys, D]; max_keys: the largest of latent_kept_keys."""
+    flush_gemm_chain()
+    _cuda_contig("cache", cache, torch.bfloat16)
+    _cuda_contig("out", out, torch.bfloat16)
+    for name, t in (("cu_seqlens", cu_seqlens), ("context_lens", context_lens)):
+        _cuda_contig(name, t, torch.int32)
+    if block_table.dtype != torch.int32 or block_table.dim() != 2 or block_table.stride(1) != 1:
+        raise KernelError("latent_gather: block_table must be an int32 matrix with unit inner stride")
+    if cu_seqlens.numel() < num_seqs + 1 or context_lens.numel() < num_seqs or block_table.shape[0] < num_seqs:
+        raise KernelError("latent_gather: the index arrays are shorter than the batch")
+    D = out.shape[-1]
+    if out.dim() != 2 or tuple(cache.shape[-2:]) != (page_size, D) or max_keys > out.shape[0]:
+        raise KernelError(f"latent_gather: cache {tuple(cache.shape)}, out {tuple(out.shape)} and pages of {page_size} disagree")
+    _check("latent_gather", _fn("ts_latent_gather")(
+        cache.data_ptr(), out.data_ptr(), cu_seqlens.data_ptr(), context_lens.data_ptr(), block_table.data_ptr(), block_table.stride(0), page_size,
+        num_seqs, max_keys, D * 2, int(window), _latent_rebuilt_fns()[1], _stream()))
+
+
+def latent_rebuilt_attention(q: torch.Tensor, q_rot: torch.Tensor, kv: torch.Tensor, rows: torch.Tensor, out: torch.Tensor,
+                             gates: Optional[torch.Tensor], cu_seqlens: torch.Tensor, context_lens: torch.Tensor, num_seqs: int,
+                             max_seqlen_q: int, num_heads: int, rank: int, scale: float, window: int = 0,
+                             sink: Optional[torch.Tensor] = None) -> None:
+    """Causal attention of prompt portions over rebuilt keys and values on the tcgen05 tensor cores (bfloat16).  q
+    [T, H * (128 + 64)] (rows may be strided; a head's last 64 are taken from q_rot instead, [t, H, 64] of the last t
+    tokens, the sequences' tokens among them), rows [S, rank + 64] as latent_gather leaves them, kv [S, H * 128 | H * 128]
+    the heads' keys and values made from rows[:, :rank]; out [T, H, 128], times gates [T, H] (float32) if given.
+    `sink` [H] float32 as in latent_attention_mma."""
+    flush_gemm_chain()
+    dn, dr, dv = LATENT_REBUILT_SIZES
+    T, H, S = q.shape[0], num_heads, rows.shape[0]
+    _check_sink("latent_rebuilt_attention", sink, H)
+    for name, t in (("q_rot", q_rot), ("kv", kv), ("rows", rows), ("out", out)):
+        _cuda_contig(name, t, torch.bfloat16)
+    for name, t in (("cu_seqlens", cu_seqlens), ("context_lens", context_lens)):
+        _cuda_contig(name, t, torch.int32)
+    if not q.is_cuda or q.dtype != torch.bfloat16 or q.dim() != 2 or q.stride(1) != 1 or q.shape[1] != H * (dn + dr):
+        raise KernelError(f"latent_rebuilt_attention: q must be [T, {H * (dn + dr)}] bfloat16 with unit inner stride, got {tuple(q.shape)} {q.dtype}")
+    if not 0 < q_rot.shape[0] <= T or q_rot.numel() != q_rot.shape[0] * H * dr or out.numel() != T * H * dv:
+        raise KernelError(f"latent_rebuilt_attention: q_rot {tuple(q_rot.shape)} and out {tuple(out.shape)} do not match {T} tokens")
+    if tuple(kv.shape) != (S, H * (dn + dv)) or tuple(rows.shape) != (S, rank + dr):
+        raise KernelError(f"latent_rebuilt_attention: kv {tuple(kv.shape)} and rows {tuple(rows.shape)} disagree")
+    if cu_seqlens.numel() < num_seqs + 1 or context_lens.numel() < num_seqs:
+        raise KernelError("latent_rebuilt_attention: the index arrays are shorter than the batch")
+    if gates is not None:
+        _cuda_contig("gates", gates, torch.float32)
+        if gates.numel() != T * H:
+            raise KernelError("latent_rebuilt_attention: gates must be [T, heads]")
+    _, error = _gemm_workspace(q.device)
+    _check("latent_rebuilt_attention", _latent_rebuilt_fns()[0](
+        q.data_ptr(), q.stride(0), q_rot.data_ptr(), T - q_rot.shape[0], kv.data_ptr(), rows.data_ptr(), rows.stride(0), rank, out.data_ptr(),
+        _ptr(gates), _ptr(sink), cu_seqlens.data_ptr(), context_lens.data_ptr(), S, T, num_seqs, max_seqlen_q, H, float(scale), int(window),
+        error.data_ptr(), _stream()))
 
 
 # ---------------------------------------------------------------------------
@@ -2733,7 +2825,8 @@ def library_mm(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor
 _TIMED = ("embed_gather", "feed_tokens", "add_rmsnorm", "residual_add", "swiglu", "qk_norm_rope_store", "attention_paged_simple", "attention_paged_float32",
           "sample", "sgemm_nt", "attention_paged_mma", "attention_decode_flat", "attention_prefill_tcgen05", "gemm_skinny_bf16",
           "gemm_skinny_fused", "rope_cos_sin", "gemm_qk_rope_store", "library_mm", "sgemm_nt_batched", "library_bmm", "pair_hash_embed",
-          "rmsnorm_add", "round_rows", "latent_prepare", "latent_attention_simple", "latent_attention_mma", "gelu_tanh", "capped_glu", "gelu_gate_rows",
+          "rmsnorm_add", "round_rows", "latent_prepare", "latent_attention_simple", "latent_attention_mma", "latent_gather",
+          "latent_rebuilt_attention", "gelu_tanh", "capped_glu", "gelu_gate_rows",
           "router_topk", "router", "moe_plan", "moe_gate_up", "moe_down", "moe_combine", "branch_norm_add", "stream_add",
           "qk_joint_norm_rope_store", "gla_scan", "gla_norm_gate", "linear_scan", "rows_dot_f32", "mlstm_gate_scan", "mlstm_norm_gate",
           "ssm_conv", "ssm_gate_norm", "scale_rows", "weighted_sum", "rope_table", "qkv_prepare", "gate_rows", "causal_conv", "delta_scan",

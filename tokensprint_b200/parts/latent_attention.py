@@ -4,7 +4,7 @@ latent row and one rotated key part, shared by all heads."""
 from __future__ import annotations
 
 import os
-from typing import Mapping, Optional
+from typing import Mapping, Optional, Sequence
 
 import torch
 
@@ -17,6 +17,30 @@ from tokensprint_b200.parts.linear import folding_possible, linear, linear_into_
 LATENT_ATTENTION_MMA = os.environ.get("TS_LATENT_ATTENTION_MMA", "1") != "0"
 # Up to this many tokens per sequence a step's keys are cut into ranges (decode, and the shortest portions).
 LATENT_DECODE_MAX_TOKENS = 4
+# TS_LATENT_REBUILD=0 (for measurements): prompt portions score the cached rows through absorbed queries too.
+LATENT_REBUILD = os.environ.get("TS_LATENT_REBUILD", "1") != "0"
+# Most bytes of rebuilt keys and values of a step; above it the portions go through absorbed queries.  A later portion of
+# a long prompt keeps more rows than the step that the page pool's size is measured with (a first portion):
+# the bound is the margin that the sizing leaves.
+LATENT_REBUILD_MAX_BYTES = 256 << 20
+
+
+def rebuilding_pays(portions: Sequence[tuple[int, int]], heads: int, sms: int) -> bool:
+    """Whether a step's prompt portions, as (new tokens, keys kept) each, are faster with rebuilt keys and values.
+
+    Both sides in microseconds, fitted to a sweep on B200 (16 and 32 heads, 1 and 4 portions of 5 to 512 tokens, 5 to 8,192
+    keys; the model is within a tenth or 4 us).  Absorbed queries: 32 rows a CTA, 3.75 us per block of 64 keys, one
+    CTA per SM.  Rebuilt: the product that makes keys and values, then 256 tokens of a head a CTA, 1.75 us per block of 96
+    keys.  16 heads, one portion: 128 tokens 25.6 against 29.7, 300 tokens 39.9 / 33.8, 32 tokens behind 480 48 / 36, 512 behind
+    7,680 965 / 220; 32 heads, 4 portions of 5 behind 507: 50 / 52."""
+    def passes(rows: int, keys: int, per_token: bool) -> float:
+        blocks = [-(-k // keys) for _, k in portions]
+        ctas = [-(-n * heads // rows) if per_token else -(-n // rows) * heads for n, _ in portions]
+        return max(max(blocks), sum(b * c for b, c in zip(blocks, ctas)) / sms)
+
+    absorbed = 18.0 + 3.75 * passes(32, 64, True)
+    rebuilt = 26.0 + 2.2e-4 * heads * sum(k for _, k in portions) + 1.75 * passes(256, 96, False)
+    return rebuilt < absorbed
 
 
 def batched_linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
@@ -37,11 +61,13 @@ class LatentAttentionMixer(Mixer):
         k_a = [U_k,a c ; r],  v_a = U_v,a c  (r is the same for every head)
         o_a = softmax(q_a . k_a * scale) v_a, times sigmoid(W_g x)_a if `gate` is named;  y = W_o [o_a]
 
-    Only [c ; r] is cached, one row of kv_rank + rot_dim entries per token in a single pool.  The
-    keys are never rebuilt: U_k,a^T q_plain,a (the absorbed query) is scored against c directly,
+    Only [c ; r] is cached, one row of kv_rank + rot_dim entries per token in a single pool.  Decode steps
+    and float32 runs never rebuild the keys: U_k,a^T q_plain,a (the absorbed query) is scored against c directly,
     the weighted sum runs over c, and U_v,a is applied to that sum.  A step is: one product for
     [q (or its latent) | c, r | gate logits], the prepare kernel (norm, rotation, store), the per-head absorbing
-    products, the attention kernel, the per-head value products, the output product.
+    products, the attention kernel, the per-head value products, the output product.  Prompt portions in bfloat16 with
+    heads of 128 + 64 and 128 do rebuild them (one product of the cached rows with [U_k ; U_v] for the step): a (query, key, head)
+    then costs 320 multiply-adds instead of 2 x 512 + 64, and the attention runs on the tcgen05 tensor cores.
 
     `q_rank` > 0: the queries pass a latent of their own first, q = W_uq norm(W_dq x) with an RMS
     norm and weight `dq_norm` over the q_rank entries (`q` then names W_uq [H (nope + rot), q_rank] and
@@ -144,6 +170,10 @@ class LatentAttentionMixer(Mixer):
         # U_v,a [value_dim, kv_rank] as it is stored
         self.uk_t = tensors[n["uk"]].view(H, self.nope_dim, self.kv_rank).transpose(1, 2).contiguous() if self.nope_dim else None
         self.uv = tensors[n["uv"]].view(H, self.value_dim, self.kv_rank).contiguous()
+        self.kv_weight: Optional[torch.Tensor] = None  # [U_k ; U_v], for portions whose keys and values are rebuilt
+        if self.uv.dtype == torch.bfloat16 and (self.nope_dim, self.rot_dim, self.value_dim) == ops.LATENT_REBUILT_SIZES and self.kv_rank % 8 == 0:
+            self.kv_weight = torch.cat([tensors[n["uk"]].reshape(-1, self.kv_rank), self.uv.view(-1, self.kv_rank)])
+            self.uv = self.kv_weight[H * self.nope_dim :].view(H, self.value_dim, self.kv_rank)
         self.o_weight = tensors[n["o"]]
         if self.position is not None:
             self.position.load(tensors)
@@ -170,22 +200,39 @@ class LatentAttentionMixer(Mixer):
             normed = torch.empty((T, self.q_rank), device=dev, dtype=dtype)
             ops.rmsnorm_rows(proj[:, q_off:q_off + self.q_rank], self.dq_norm_weight, normed, self.norm_eps)
             q_src = linear(normed, self.uq_weight)
-        q_abs = torch.empty((T, H, D), device=dev, dtype=dtype)
+        q_rows = q_src if q_src is not None else proj[:, q_off : q_off + H * (self.nope_dim + self.rot_dim)]
+        absorbed, kept = self._rebuild_plan(step, q_rows)  # tokens in front that go through absorbed queries; rows the others' portions keep
+        rebuilt = absorbed < T
+        q_abs = torch.empty((absorbed, H, D), device=dev, dtype=dtype)
+        q_rot = torch.empty((T - absorbed, H, self.rot_dim), device=dev, dtype=dtype) if rebuilt else None
         gates = torch.empty((T, H), device=dev, dtype=torch.float32) if self.names["gate"] is not None else None
         ops.latent_prepare(
             proj, q_off, kv_off, gate_off, q_abs, cache.k_pages if has_latent else None, tables.slot_mapping if has_latent else None,
             step.positions, self.latent_weight, self.norm_eps, None if self.position is None else self.position.frequencies(),
-            self.rot_dims, self.pairing, gates, H, self.nope_dim, self.rot_dim, R, magnitude=self.magnitude, q_src=q_src)
-        if self.nope_dim:
-            q_rows = q_src if q_src is not None else proj[:, : H * (self.nope_dim + self.rot_dim)]
-            q_plain = q_rows.view(T, H, self.nope_dim + self.rot_dim)[:, :, : self.nope_dim]
-            batched_linear(q_plain.transpose(0, 1), self.uk_t, q_abs[:, :, :R].transpose(0, 1))
-        else:
-            q_abs[:, :, :R].zero_()
-        latent_out = torch.empty((T, H, R), device=dev, dtype=dtype)
-        self._attend(q_abs, latent_out, gates, step, cache, tables)
+            self.rot_dims, self.pairing, gates, H, self.nope_dim, self.rot_dim, R, magnitude=self.magnitude, q_src=q_src, q_rot=q_rot)
         heads_out = torch.empty((T, H, self.value_dim), device=dev, dtype=dtype)
-        batched_linear(latent_out.transpose(0, 1), self.uv, heads_out.transpose(0, 1))
+        if absorbed:
+            if self.nope_dim:
+                q_plain = q_rows[:absorbed].view(absorbed, H, self.nope_dim + self.rot_dim)[:, :, : self.nope_dim]
+                batched_linear(q_plain.transpose(0, 1), self.uk_t, q_abs[:, :, :R].transpose(0, 1))
+            else:
+                q_abs[:, :, :R].zero_()
+            latent_out = torch.empty((absorbed, H, R), device=dev, dtype=dtype)
+            self._attend(q_abs, latent_out, None if gates is None else gates[:absorbed], step, cache, tables, portions=not rebuilt)
+            batched_linear(latent_out.transpose(0, 1), self.uv, heads_out[:absorbed].transpose(0, 1))
+        if rebuilt:
+            first = step.decode_seqs if absorbed else 0
+            count = step.num_seqs - first
+            cu, lens = step.cu_seqlens_q[first:], step.context_lens[first:]  # (the starts count from the step's first token)
+            # a layer that reads another one's rows finds them gathered already, where the windows agree
+            key = ("latent rows", cache.group, cache.k_pages.data_ptr(), self.window, first)
+            cached = None if has_latent else step.shared.get(key)
+            if cached is None:
+                cached = step.shared[key] = torch.empty((sum(kept), D), device=dev, dtype=dtype)
+                ops.latent_gather(cache.k_pages, cached, cu, lens, tables.block_table[first:], step.page_size, count, max(kept), self.window)
+            kv = ops.library_mm(cached[:, :R], self.kv_weight)
+            ops.latent_rebuilt_attention(q_rows, q_rot, kv, cached, heads_out, gates, cu, lens, count, step.max_seqlen_q, H, R, self.scale,
+                                         self.window, sink=self.sink)
         rows = heads_out.view(T, H * self.value_dim)
         if out_gate_off >= 0:
             gated = torch.empty_like(rows)
@@ -195,7 +242,23 @@ class LatentAttentionMixer(Mixer):
             return linear_into_residual(rows, self.o_weight, fold, next_weight=step.weight_after)
         return linear(rows, self.o_weight, next_weight=step.weight_after)
 
-    def _attend(self, q_abs, out, gates, step: StepContext, cache: LayerCache, tables) -> None:
+    def _rebuild_plan(self, step: StepContext, q_rows: torch.Tensor) -> tuple[int, list[int]]:
+        """How many tokens at the step's front go through absorbed queries (all of them, or the single decoded tokens
+        beside prompt portions), and how many cached rows each portion behind them keeps."""
+        T, B = step.num_tokens, step.num_seqs
+        if self.kv_weight is None or not LATENT_REBUILD or step.max_seqlen_q <= LATENT_DECODE_MAX_TOKENS or len(step.host_seq_lens) != B:
+            return T, []
+        if q_rows.stride(0) % 8 or q_rows.data_ptr() % 16:  # the copy engine's rows are 16-byte aligned
+            return T, []
+        first = step.decode_seqs if step.decode_seqs < B else 0
+        portions = [(n, ops.latent_kept_keys(self.window, n, start + n)) for start, n in zip(step.host_seq_starts[first:], step.host_seq_lens[first:])]
+        kept = [k for _, k in portions]
+        if sum(kept) * self.kv_weight.shape[0] * 2 > LATENT_REBUILD_MAX_BYTES or not rebuilding_pays(portions, self.num_heads, ops._sm_count(q_rows.device)):
+            return T, []
+        return first, kept
+
+    def _attend(self, q_abs, out, gates, step: StepContext, cache: LayerCache, tables, portions: bool) -> None:
+        """The absorbed queries over the cached rows; without `portions` only the single tokens at the step's front."""
         H, R, rot = self.num_heads, self.kv_rank, self.rot_dim
         if q_abs.dtype != torch.bfloat16 or not LATENT_ATTENTION_MMA or not ops.latent_attention_mma_supported(R, rot):
             # float32 runs, and sizes the tensor-core kernel is not made for
@@ -216,7 +279,9 @@ class LatentAttentionMixer(Mixer):
                 self.scale, self.window, splits, sink=self.sink)
 
         T = q_abs.shape[0]
-        if step.max_seqlen_q <= LATENT_DECODE_MAX_TOKENS:
+        if not portions:
+            run(0, singles, 0, T, 1, True)
+        elif step.max_seqlen_q <= LATENT_DECODE_MAX_TOKENS:
             run(0, B, 0, T, step.max_seqlen_q, True)  # few rows per sequence: the keys are spread over CTAs
         elif 0 < singles < B:
             # single decoded tokens beside portions of prompts (the runner put the single tokens' requests first)
