@@ -405,3 +405,47 @@ def test_expert_products_on_tensor_cores_against_cuda_cores(P, E, K, I, monkeypa
         for act, out in results:
             assert float((out[pair].double() - want).abs().max()) < 3e-2 * float(want.abs().max()) + 1e-3
     assert float((results[0][1] - results[1][1]).abs().max()) < 2e-2 * float(results[1][1].abs().max())
+
+
+@pytest.mark.parametrize("rows, E, K, I", [(1, 2, 64, 128), (31, 3, 72, 130), (32, 1, 200, 264), (33, 2, 64, 520), (127, 2, 136, 72), (128, 1, 64, 136),
+                                           (129, 2, 72, 264), (400, 2, 264, 200), (3, 1100, 64, 16)])
+@pytest.mark.parametrize("activation", ["capped_glu", "gelu"])
+def test_expert_products_at_the_edges_of_their_tiles(rows, E, K, I, activation):
+    """About `rows` pairs per expert (one expert gets none where there are several): row tiles of 32 and 128, weight tiles of 128
+    and 256 rows, remainders of all of them, more experts than shared memory holds offsets for; a pair that points past the experts has
+    no place.  Against float64 on the rounded inputs: the first product and the activation round to bfloat16 (2^-9 each)."""
+    from tokensprint_b200 import ops
+
+    g = torch.Generator().manual_seed(rows * 7 + E)
+    T = rows if E > 8 else rows * max(1, E - 1)
+    ids = torch.randint(0, max(1, E - 1), (T, 1), generator=g).to(torch.int32)
+    if E > 1:
+        ids[0] = E  # an identity expert: not in the plan
+    x = torch.randn(T, K, generator=g).to(torch.bfloat16).cuda()
+    matrix = lambda a, b: (torch.randn(E, a, b, generator=g) / b ** 0.5).to(torch.bfloat16).cuda()  # noqa: E731
+    gate, up, down = None if activation == "gelu" else matrix(I, K), matrix(I, K), matrix(K, I)
+    w = (torch.rand(T, generator=g) + 0.5).cuda()
+    for tile in (ops.moe_row_tile(True, 1, 1), ops.moe_row_tile(True, 99, 1)):
+        plan = ops.moe_plan(ids.cuda(), E, tile)
+        places = plan[2].cpu()[: int(plan[0][-1])].long().cuda()
+        e, h = ids.view(-1).cuda()[places].long(), x[places].double()
+        product = lambda m, r: torch.stack([m[int(n)].double() @ row for n, row in zip(e, r)])  # noqa: E731
+        for weight in (w, None):
+            act = torch.full((T, I), float("nan"), dtype=torch.bfloat16, device="cuda")
+            ops.moe_gate_up(x, weight, plan, gate, up, act, 1, 7.0, 1.702, activation)
+            if not len(places):  # nobody's pair has a place: nothing is written
+                assert bool(torch.isnan(act.float()).all())
+                continue
+            factor = 1.0 if weight is None else weight[places, None].double()
+            u = factor * product(up, h)
+            if gate is None:
+                want = torch.nn.functional.gelu(u)
+            else:
+                a, u = (factor * product(gate, h)).clamp(max=7.0), u.clamp(-7.0, 7.0)
+                want = a * torch.sigmoid(1.702 * a) * (u + 1.0)
+            assert _rel(act[: len(places)], want) < 1e-2
+        if len(places) and I % 8 == 0:
+            out = torch.full((T, K), float("nan"), dtype=torch.bfloat16, device="cuda")
+            ops.moe_down(act, plan, down, out)
+            assert _rel(out[places], product(down, act[: len(places)].double())) < 5e-3
+    ops.check_device_errors()

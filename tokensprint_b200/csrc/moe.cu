@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(256) moe_gate_up_kernel(const TA* __restrict__
     const int place = row0 + r;
     const int pair = place < row_end ? order[place] : -1;
     src_row[r] = pair < 0 ? -1 : pair / top;
-    src_scale[r] = pair < 0 ? 0.f : pair_weight[pair];
+    src_scale[r] = pair < 0 ? 0.f : pair_weight != nullptr ? pair_weight[pair] : 1.f;  // null: ones
   }
   __syncthreads();
   const TA* G = gate + (size_t)e * I * K;

@@ -62,9 +62,10 @@ _SIGNATURES = {
                        _c_void_p],
     "ts_router": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p,
                   _c_int, _c_int, _c_float, _c_void_p],
-    "ts_moe_gate_up_mma": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int,
-                           _c_int, _c_int, _c_float, _c_float, _c_int, _c_int, _c_void_p],
-    "ts_moe_down_mma": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p],
+    "ts_moe_gate_up_tcgen05": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int,
+                               _c_int, _c_int, _c_int, _c_float, _c_float, _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
+    "ts_moe_down_tcgen05": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
+                            _c_void_p, _c_void_p],
     "ts_moe_plan": [_c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p],
     "ts_moe_gate_up": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int,
                        _c_int, _c_int, _c_float, _c_float, _c_int, _c_void_p],
@@ -1677,7 +1678,7 @@ def moe_on_tensor_cores(dtype: torch.dtype, *inner_widths: int) -> bool:
     return MOE_MMA and dtype == torch.bfloat16 and all(k % 8 == 0 for k in inner_widths)
 
 
-_moe_mma_tiles: Optional[tuple[int, int]] = None
+_moe_tiles: Optional[tuple[int, int]] = None
 MOE_FEW_ROWS_PER_EXPERT = 12  # up to this many pairs per expert on average the short row tiles are planned
 
 
@@ -1685,14 +1686,14 @@ def moe_row_tile(tensor_cores: bool, pairs: int = 0, num_experts: int = 1) -> in
     """Places per row tile of the expert products' kernels: what a plan is made for.  The tensor-core
     kernels come in two shapes, for many rows per expert and for few (a function of the token count
     alone, so a captured step keeps its shape)."""
-    global _moe_mma_tiles
+    global _moe_tiles
     if not tensor_cores:
         return MOE_ROW_TILE
-    if _moe_mma_tiles is None:
-        fn = library().ts_moe_mma_row_tile
+    if _moe_tiles is None:
+        fn = library().ts_moe_tcgen05_row_tile
         fn.argtypes, fn.restype = [_c_int], _c_int
-        _moe_mma_tiles = (int(fn(0)), int(fn(1)))
-    return _moe_mma_tiles[1] if pairs <= MOE_FEW_ROWS_PER_EXPERT * num_experts else _moe_mma_tiles[0]
+        _moe_tiles = (int(fn(0)), int(fn(1)))
+    return _moe_tiles[1] if pairs <= MOE_FEW_ROWS_PER_EXPERT * num_experts else _moe_tiles[0]
 
 
 def moe_plan(ids: torch.Tensor, num_experts: int, tile_rows: int = MOE_ROW_TILE) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor, int]:
@@ -1717,7 +1718,7 @@ def _moe_path(name: str, plan, dtype: torch.dtype, *inner_widths: int) -> bool:
         return False
     if moe_on_tensor_cores(dtype, *inner_widths):
         moe_row_tile(True)
-        if plan[3] in _moe_mma_tiles:
+        if plan[3] in _moe_tiles:
             return True
     raise KernelError(f"{name}: the plan was made for row tiles of {plan[3]}, which no kernel for {dtype} and inner widths {inner_widths} takes")
 
@@ -1725,12 +1726,12 @@ def _moe_path(name: str, plan, dtype: torch.dtype, *inner_widths: int) -> bool:
 MOE_ACTIVATIONS = {"capped_glu": 0, "swiglu": 1, "gelu": 2}  # "gelu": experts without a gate matrix, W_down gelu_erf(W_up x)
 
 
-def moe_gate_up(x: torch.Tensor, pair_weight: torch.Tensor, plan: tuple, gate: Optional[torch.Tensor],
+def moe_gate_up(x: torch.Tensor, pair_weight: Optional[torch.Tensor], plan: tuple, gate: Optional[torch.Tensor],
                 up: torch.Tensor, act: torch.Tensor, top: int, limit: float, alpha: float, activation: str = "capped_glu") -> None:
     """For every pair, in the plan's order: act[place] = activation(gate_e (w x[token]), up_e (w x[token])), where
     activation is "capped_glu" (with `limit` and `alpha`) or "swiglu" (silu(gate) * up); or, for experts
     without a gate matrix (`gate` None, activation "gelu"), act[place] = gelu_erf(up_e (w x[token])).
-    x [T, K]; pair_weight [T*top] f32; gate, up [E, I, K]; act [T*top, I]."""
+    x [T, K]; pair_weight [T*top] f32, None: ones; gate, up [E, I, K]; act [T*top, I]."""
     flush_gemm_chain()
     offsets, tile_offsets, order, _ = plan
     _cuda_contig("x", x)
@@ -1743,19 +1744,22 @@ def moe_gate_up(x: torch.Tensor, pair_weight: torch.Tensor, plan: tuple, gate: O
         gate_ptr = gate.data_ptr()
     _cuda_contig("up", up, x.dtype)
     _cuda_contig("act", act, x.dtype)
-    _cuda_contig("pair_weight", pair_weight, torch.float32)
+    if pair_weight is not None:
+        _cuda_contig("pair_weight", pair_weight, torch.float32)
     T, K = x.shape
     E, I, K2 = up.shape
     P = T * top
-    if K2 != K or (gate is not None and up.shape != gate.shape) or act.shape != (P, I) or pair_weight.numel() != P or order.numel() != P:
+    if K2 != K or (gate is not None and up.shape != gate.shape) or act.shape != (P, I) or (pair_weight is not None and pair_weight.numel() != P) or order.numel() != P:
         raise KernelError(f"moe_gate_up: shapes disagree: x {tuple(x.shape)}, up {tuple(up.shape)}, act {tuple(act.shape)}")
     if _moe_path("moe_gate_up", plan, x.dtype, K):
-        _check("moe_gate_up", _fn("ts_moe_gate_up_mma")(
-            x.data_ptr(), pair_weight.data_ptr(), order.data_ptr(), offsets.data_ptr(), tile_offsets.data_ptr(), gate_ptr,
-            up.data_ptr(), act.data_ptr(), P, E, K, I, int(top), float(limit), float(alpha), MOE_ACTIVATIONS[activation], plan[3], _stream()))
+        _, error = _gemm_workspace(x.device)
+        _check("moe_gate_up", _fn("ts_moe_gate_up_tcgen05")(
+            x.data_ptr(), T, _ptr(pair_weight), order.data_ptr(), offsets.data_ptr(), tile_offsets.data_ptr(), gate_ptr,
+            up.data_ptr(), act.data_ptr(), P, E, K, I, int(top), float(limit), float(alpha), MOE_ACTIVATIONS[activation], plan[3],
+            _sm_count(x.device), error.data_ptr(), _stream()))
         return
     _check("moe_gate_up", _fn("ts_moe_gate_up")(
-        x.data_ptr(), _act_code("x", x), pair_weight.data_ptr(), order.data_ptr(), offsets.data_ptr(), tile_offsets.data_ptr(),
+        x.data_ptr(), _act_code("x", x), _ptr(pair_weight), order.data_ptr(), offsets.data_ptr(), tile_offsets.data_ptr(),
         gate_ptr, up.data_ptr(), act.data_ptr(), P, E, K, I, int(top), float(limit), float(alpha), MOE_ACTIVATIONS[activation], _stream()))
 
 
@@ -1771,9 +1775,10 @@ def moe_down(act: torch.Tensor, plan: tuple, down: torch.Tensor, pair_out: torch
     if I2 != I or pair_out.shape != (P, N) or order.numel() != P:
         raise KernelError(f"moe_down: shapes disagree: act {tuple(act.shape)}, down {tuple(down.shape)}, pair_out {tuple(pair_out.shape)}")
     if _moe_path("moe_down", plan, act.dtype, I):
-        _check("moe_down", _fn("ts_moe_down_mma")(
+        _, error = _gemm_workspace(act.device)
+        _check("moe_down", _fn("ts_moe_down_tcgen05")(
             act.data_ptr(), order.data_ptr(), offsets.data_ptr(), tile_offsets.data_ptr(), down.data_ptr(), pair_out.data_ptr(), P, E, I, N,
-            plan[3], _stream()))
+            plan[3], _sm_count(act.device), error.data_ptr(), _stream()))
         return
     _check("moe_down", _fn("ts_moe_down")(
         act.data_ptr(), _act_code("act", act), order.data_ptr(), offsets.data_ptr(), tile_offsets.data_ptr(), down.data_ptr(),

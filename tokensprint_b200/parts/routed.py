@@ -200,8 +200,7 @@ class RoutedExperts(FeedForward):
         plan = ops.moe_plan(chosen, self.num_experts, ops.moe_row_tile(tensor_cores, T * top, self.num_experts))
         act = torch.empty((T * top, self.intermediate_size), device=dev, dtype=x.dtype)
         on_input = self.weight_on == "input"
-        ones = None if on_input else torch.ones((T * top,), device=dev, dtype=torch.float32)
-        ops.moe_gate_up(x, weights.view(-1) if on_input else ones, plan, self.gate, self.up, act, top, self.limit, self.alpha,
+        ops.moe_gate_up(x, weights.view(-1) if on_input else None, plan, self.gate, self.up, act, top, self.limit, self.alpha,
                         activation=self.activation)
         pair_out = torch.empty((T * top, self.hidden_size), device=dev, dtype=x.dtype)
         ops.moe_down(act, plan, self.down, pair_out)
