@@ -2,30 +2,33 @@
 // sums in tensor memory, operands by TMA), over the plan that moe.cu makes: the (token, choice) pairs
 // sorted by expert, in row tiles (of 128 places, or of 32 in steps of few tokens) that never straddle two experts.
 //
-// A work item is one row tile and TN weight rows: for the first product the gate rows and the up rows of the same
-// TN / 2 outputs (so the activation is the epilogue), for the second TN rows of the down matrix.  CTAs are
-// persistent, one per SM, and take items in turn, the columns of a row tile side by side, so that an expert's
-// weights come from device memory once and from the L2 after that.  Roles in a CTA:
-//   warp 4      TMA: per slice of 64 along k two boxes of weight rows and, for the second product, one box of consecutive
-//               places, for the first with short row tiles the tokens' rows (tile::gather4, four rows a copy, only as many
-//               as the tile has), into a ring of slices with a full and an empty mbarrier each;
-//   warps 6-9   (first product, long row tiles) the tokens' rows by 16-byte cp.async in the swizzled layout.
-//               Each way where it is the faster one: the copy engine takes 40 ns per gather4, which a tile of 128 rows shows
-//               (16,384 pairs of 32 experts, 4,096 -> 2 x 1,536: 397 us by warps, 981 by gather4); the proxy fence behind a slice
-//               waits for the younger slices' copies too, so the slices of the warps follow one another at 0.45 us, which
-//               a tile of few rows shows (it then streams weights and little else);
-//   warp 5      one elected lane: every tcgen05.mma (M = 128 places, N = TN, K = 16; with row tiles of 32 the other 96 rows
-//               are whatever lies behind them in shared memory);
-//   warps 0-3   epilogue: thread r owns place r, reads its sums from tensor memory and writes its row.
-// Two accumulators take turns, so the epilogue of an item runs under the products of the next.  Rows of shared memory that no
-// copy fills hold old values: a place's sums read its own row only, and places without a pair are never stored.
+// Two kernels, both of persistent CTAs, one per SM, that take items in turn, the columns of a row tile side by side, so
+// that an expert's weights come from device memory once and from the L2 after that; operands pass through a ring of
+// slices of 64 along k with a full and an empty mbarrier each, and two accumulators take turns, so that the epilogue of an
+// item runs under the products of the next.  Rows of shared memory that no copy fills hold old values: a sum reads its own
+// place's row and its own weight row only, and sums that belong to no pair are never stored.
+//
+// Many rows (moe_many_kernel): an item is a row tile of 128 places, the MMA's M, and 256 weight rows, its N: for the first
+// product the gate rows and the up rows of the same 128 outputs (so the activation is the epilogue).
+//   warp 4       TMA: per slice two boxes of weight rows and, for the second product, one box of consecutive places;
+//   warps 6-9    (first product) the tokens' rows by 16-byte cp.async in the swizzled layout, only as many as the tile has
+//                (tile::gather4 copies, 40 ns each, took 981 us where this takes 397: 16,384 pairs of 32 experts, 4,096 -> 2 x 1,536);
+//   warp 5       one elected lane: every tcgen05.mma;
+//   the others   epilogue: a thread has a place and half of its columns, reads its sums from tensor memory and writes them.
+// Bound by the L2 at 48 KB a slice and SM (13 TB/s in all): 8,192 pairs of these experts 241 us, 0.86 PFLOP/s, and 121 us for
+// down (mma.sync tiles of 128 x 128: 863 and 450).
+//
+// Few rows (moe_few_kernel; up to 12 pairs per expert on average): the step streams the chosen experts' weights and little
+// else, at a rate that follows the bytes of weights in flight.  Row tiles of 32 places are the MMA's N and the weight rows
+// its M, two tiles of 128 (or one, see `narrow`), so 192 KB of weights are in flight per SM, and the epilogue, which nothing
+// hides where a CTA has one item, is spread over 128 threads that each have a weight row and only as many
+// columns as the tile has places (with the places as M one warp did all of it, 5 to 8 us of the 35).  The tokens' rows come by
+// tile::gather4, four rows a copy, only as many as the tile has.
+// 16 experts, 2,048 -> 2 x 1,024, in a graph, gate/up and down: 2 pairs 17.3 and 7.5 us, 10 pairs 17.8 and 9.2, 66 pairs 25.4 and 14.9
+// (5.3 and 4.5 TB/s); tiles of 16 rows on mma.sync, three CTAs an SM, took 22.6 and 11.8, 28.2 and 15.6, 32.6 and 17.5.
+//
 // The pair's routing weight multiplies the float32 sums, not the rounded input: (w x) . g = w (x . g) without
 // a second rounding of x.  Every output element is one chain of sums over k in a fixed order.
-//
-// Bounds.  Many rows: the L2, at 48 KB a slice and SM (13 TB/s in all; 8,192 pairs of 32 experts, 4,096 -> 2 x 1,536: 241 us, 0.86
-// PFLOP/s, and 121 us for down; mma.sync tiles of 128 x 128 took 863 and 450).  Few rows: the weights, at a rate
-// that follows the bytes of weights in flight, hence the short row tile (16 KB of a stage would hold A otherwise): 66 pairs
-// of the same experts 138 and 72 us (5.9 and 5.6 TB/s; mma.sync 153 and 86).
 // Every wait is on an mbarrier fed by this CTA's own copies, MMAs and warps, bounded; one that gives up raises the
 // error word, and the CTA lets its copies land, frees its tensor memory and returns.
 #include <cuda.h>
@@ -41,16 +44,6 @@ constexpr int BK = 64, SHARED_EXPERTS = 1024;  // up to this many experts the pl
 constexpr int ROWS_MANY = 128, ROWS_FEW = 32;  // places per row tile
 constexpr int GATHER_WARPS = 4, GATHER_THREADS = 32 * GATHER_WARPS;
 constexpr uint32_t SPIN_LIMIT = 1u << 22;
-__host__ __device__ constexpr bool by_warps(int mode, int bm) { return mode != 0 && bm == ROWS_MANY; }
-__host__ __device__ constexpr int threads(int mode, int bm) { return by_warps(mode, bm) ? 192 + GATHER_THREADS : 192; }
-
-template <int TN, int BM>
-struct Tile {
-  static constexpr uint32_t A_BYTES = BM * 128, B_BYTES = TN * 128, STAGE = A_BYTES + B_BYTES;
-  static constexpr int STAGES = 216 * 1024 / STAGE;
-  static constexpr uint32_t SMEM = STAGES * STAGE;
-  static constexpr uint32_t TMEM_COLS = 2 * TN;
-};
 
 struct Args {
   const float* pair_weight;
@@ -129,6 +122,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
 }
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
+}
+__device__ __forceinline__ uint32_t idesc(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+}
 __device__ __forceinline__ float rounded(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
 // 16 results of a row, from column n on
@@ -171,53 +171,84 @@ __device__ __forceinline__ Item item_at(const Args& a, const int* plan, int it) 
   return w;
 }
 
-// MODE 1: gate and up; MODE 2: the first product of experts without a gate; MODE 0: down.
-template <int MODE, int TN, int BM>
-__global__ void __launch_bounds__(threads(MODE, BM), 1) moe_tcgen05_kernel(const __nv_bfloat16* __restrict__ x, const __grid_constant__ CUtensorMap map_a,
-                                                                           const __grid_constant__ CUtensorMap map_b0,
-                                                                           const __grid_constant__ CUtensorMap map_b1, const Args a) {
-  using T = Tile<TN, BM>;
-  constexpr bool BY_TOKEN = MODE != 0, BY_WARPS = by_warps(MODE, BM);
-  constexpr int COLS = MODE == 1 ? TN / 2 : TN;  // outputs of an item
-  constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-  static_assert(T::A_BYTES + T::B_BYTES >= 128 * 128, "the 128 rows that an MMA reads lie inside the stage");
-  ts_pdl_wait();  // tensor memory is never held while waiting for another kernel
-  extern __shared__ unsigned char smem_unaligned[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_unaligned + 1023) & ~(uintptr_t)1023);
-  __shared__ __align__(8) uint64_t full[T::STAGES], empty[T::STAGES], acc_full[2], acc_empty[2], all_done;
-  __shared__ uint32_t tmem_base_s;
-  __shared__ int abort_s;
-  int* plan = a.E <= SHARED_EXPERTS ? reinterpret_cast<int*>(smem + T::SMEM) : nullptr;  // offsets and tile_offsets, looked up for every item
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+// What both kernels share: the ring's barriers, the plan in shared memory, tensor memory, and leaving.
+template <int STAGES>
+struct Common {
+  uint64_t full[STAGES], empty[STAGES], acc_full[2], acc_empty[2], all_done;
+  uint32_t tmem_base;
+  int abort;
+};
+template <int STAGES>
+__device__ __forceinline__ void begin(Common<STAGES>& c, const Args& a, int* plan, int fills, int readers, uint32_t tmem_cols) {
+  const int tid = threadIdx.x;
   if (tid == 0) {
-    abort_s = 0;
-    for (int s = 0; s < T::STAGES; ++s) {
-      mbar_init(smem_u32(&full[s]), BY_WARPS ? 1 + GATHER_WARPS : 1);
-      mbar_init(smem_u32(&empty[s]), 1);
+    c.abort = 0;
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(smem_u32(&c.full[s]), fills);
+      mbar_init(smem_u32(&c.empty[s]), 1);
     }
     for (int i = 0; i < 2; ++i) {
-      mbar_init(smem_u32(&acc_full[i]), 1);
-      mbar_init(smem_u32(&acc_empty[i]), 4);
+      mbar_init(smem_u32(&c.acc_full[i]), 1);
+      mbar_init(smem_u32(&c.acc_empty[i]), readers);
     }
-    mbar_init(smem_u32(&all_done), 1);
+    mbar_init(smem_u32(&c.all_done), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  for (int i = tid; plan != nullptr && i <= a.E; i += threads(MODE, BM)) {
+  for (int i = tid; plan != nullptr && i <= a.E; i += blockDim.x) {
     plan[i] = a.offsets[i];
     plan[a.E + 1 + i] = a.tile_offsets[i];
   }
-  if (warp == 0) {
+  if (tid < 32) {
     __syncwarp();
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(T::TMEM_COLS) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&c.tmem_base)), "r"(tmem_cols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   ts_pdl_launch_dependents();
-  const uint32_t tmem_base = tmem_base_s;
-  volatile int* abort_flag = &abort_s;
+}
+template <int STAGES>
+__device__ __forceinline__ void leave(Common<STAGES>& c, const Args& a, uint32_t tmem_cols) {
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (c.abort != 0 && threadIdx.x == 0) *a.error = 1;
+  if (threadIdx.x < 32) {
+    __syncwarp();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(c.tmem_base), "r"(tmem_cols) : "memory");
+  }
+}
+// the last copies of a CTA whose waits gave up: wait (bounded, on a count of its own) until they have landed
+template <int STAGES>
+__device__ __forceinline__ void let_land(Common<STAGES>& c, int asked) {
+  int patience = 0;
+  for (int i = max(0, asked - STAGES); i < asked; ++i) mbar_wait(smem_u32(&c.full[i % STAGES]), (uint32_t)(i / STAGES) & 1, &patience);
+}
+
+// ---- many rows ----
+
+constexpr int TN = 256;
+constexpr uint32_t MANY_A = ROWS_MANY * 128, MANY_B = TN * 128, MANY_STAGE = MANY_A + MANY_B;
+constexpr int MANY_STAGES = 4;
+constexpr uint32_t MANY_SMEM = MANY_STAGES * MANY_STAGE, MANY_TMEM = 2 * TN;
+__host__ __device__ constexpr int many_threads(int mode) { return 320 + (mode != 0 ? GATHER_THREADS : 0); }
+
+// MODE 1: gate and up; MODE 2: the first product of experts without a gate; MODE 0: down.
+template <int MODE>
+__global__ void __launch_bounds__(many_threads(MODE), 1) moe_many_kernel(const __nv_bfloat16* __restrict__ x, const __grid_constant__ CUtensorMap map_a,
+                                                                         const __grid_constant__ CUtensorMap map_b0,
+                                                                         const __grid_constant__ CUtensorMap map_b1, const Args a) {
+  constexpr bool BY_TOKEN = MODE != 0;
+  constexpr int COLS = MODE == 1 ? TN / 2 : TN;  // outputs of an item
+  ts_pdl_wait();  // tensor memory is never held while waiting for another kernel
+  extern __shared__ unsigned char smem_unaligned[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_unaligned + 1023) & ~(uintptr_t)1023);
+  __shared__ __align__(8) Common<MANY_STAGES> c;
+  int* plan = a.E <= SHARED_EXPERTS ? reinterpret_cast<int*>(smem + MANY_SMEM) : nullptr;  // offsets and tile_offsets, looked up for every item
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  begin(c, a, plan, BY_TOKEN ? 1 + GATHER_WARPS : 1, 8, MANY_TMEM);
+  volatile int* abort_flag = &c.abort;
   const uint32_t sm = smem_u32(smem);
   const int items = a.tile_offsets[a.E] * a.cols, slices = (a.K + BK - 1) / BK;
 
@@ -225,56 +256,44 @@ __global__ void __launch_bounds__(threads(MODE, BM), 1) moe_tcgen05_kernel(const
     int n = 0;  // slices asked for
     bool ok = true;
     for (int it = blockIdx.x; ok && it < items; it += gridDim.x) {
-      const Item w = item_at<COLS, BM>(a, plan, it);
-      const int quads = (w.rows + 3) >> 2;  // gathers of four rows; the last one repeats the tile's last row
-      int rows[4] = {0, 0, 0, 0};
-      if (BY_TOKEN && !BY_WARPS && lane < quads) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) rows[i] = a.order[w.row0 + min(4 * lane + i, w.rows - 1)] / a.top;
-      }
-      const uint32_t a_bytes = BY_WARPS ? 0u : BY_TOKEN ? (uint32_t)quads * 512u : T::A_BYTES;
+      const Item w = item_at<COLS, ROWS_MANY>(a, plan, it);
       const int b_row = w.e * a.NOUT + w.n0;
       for (int k = 0; k < slices; ++k, ++n) {
-        const int st = n % T::STAGES;
-        if (n >= T::STAGES) ok = mbar_wait(smem_u32(&empty[st]), (uint32_t)(n / T::STAGES - 1) & 1, abort_flag);
+        const int st = n % MANY_STAGES;
+        if (n >= MANY_STAGES) ok = mbar_wait(smem_u32(&c.empty[st]), (uint32_t)(n / MANY_STAGES - 1) & 1, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
-        const uint32_t bar = smem_u32(&full[st]), a_dst = sm + st * T::STAGE, b_dst = a_dst + T::A_BYTES;
-        if (lane == 0) mbar_expect_tx(bar, a_bytes + T::B_BYTES);
+        const uint32_t bar = smem_u32(&c.full[st]), a_dst = sm + st * MANY_STAGE, b_dst = a_dst + MANY_A;
+        if (lane == 0) mbar_expect_tx(bar, (BY_TOKEN ? 0u : MANY_A) + MANY_B);
         __syncwarp();
         if (lane < 2) {
           if (MODE == 1)
-            tma_load_2d(b_dst + lane * (T::B_BYTES / 2), lane == 0 ? &map_b0 : &map_b1, bar, k * BK, b_row);
+            tma_load_2d(b_dst + lane * (MANY_B / 2), lane == 0 ? &map_b0 : &map_b1, bar, k * BK, b_row);
           else
-            tma_load_2d(b_dst + lane * (T::B_BYTES / 2), &map_b0, bar, k * BK, b_row + lane * (TN / 2));
+            tma_load_2d(b_dst + lane * (MANY_B / 2), &map_b0, bar, k * BK, b_row + lane * (TN / 2));
         }
         if (!BY_TOKEN && lane == 2) tma_load_2d(a_dst, &map_a, bar, k * BK, w.row0);
-        if (BY_TOKEN && !BY_WARPS && lane < quads) tma_gather4(a_dst + lane * 512, &map_a, bar, k * BK, rows);
       }
     }
-    if (*abort_flag) {  // leave nothing in flight: wait (bounded, on a count of its own) for the copies already asked for
-      int patience = 0;
-      volatile int* own = &patience;
-      for (int i = max(0, n - T::STAGES); i < n; ++i) mbar_wait(smem_u32(&full[i % T::STAGES]), (uint32_t)(i / T::STAGES) & 1, own);
-    }
-  } else if (BY_WARPS && warp >= 6) {
+    if (*abort_flag) let_land(c, n);
+  } else if (BY_TOKEN && warp >= 6 && warp < 6 + GATHER_WARPS) {
     // thread g: piece g % 8 (16 bytes) of the rows g / 8, g / 8 + 16, ... of the tile
     const int g = tid - 192, piece = g & 7, first_row = g >> 3;
     const uint32_t to = (uint32_t)first_row * 128 + (uint32_t)((piece ^ (first_row & 7)) << 4);
-    constexpr int ROW_STEP = GATHER_THREADS / 8, PER = BM / ROW_STEP, AHEAD = T::STAGES - 1;
+    constexpr int ROW_STEP = GATHER_THREADS / 8, PER = ROWS_MANY / ROW_STEP, AHEAD = MANY_STAGES - 1;
     static_assert(ROW_STEP % 8 == 0, "a thread's rows swizzle alike");
     int n = 0;
     bool ok = true;
     auto hand_over = [&](int i) {  // slice i of this warp's rows has landed and the tensor core may read it
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&full[i % T::STAGES]));
+      if (lane == 0) mbar_arrive(smem_u32(&c.full[i % MANY_STAGES]));
     };
     int mine_next = 0, pairs_next[PER];  // of the item after this one: its trips to the plan run under this one's slices
     auto look_up = [&](int it) {
       mine_next = 0;
       if (it >= items) return;
-      const Item w = item_at<COLS, BM>(a, plan, it);
+      const Item w = item_at<COLS, ROWS_MANY>(a, plan, it);
       mine_next = w.rows > first_row ? (w.rows - first_row + ROW_STEP - 1) / ROW_STEP : 0;
 #pragma unroll
       for (int j = 0; j < PER; ++j) pairs_next[j] = j < mine_next ? a.order[w.row0 + first_row + j * ROW_STEP] : 0;
@@ -287,12 +306,12 @@ __global__ void __launch_bounds__(threads(MODE, BM), 1) moe_tcgen05_kernel(const
       for (int j = 0; j < PER; ++j) src[j] = x + (size_t)(j < mine ? pairs_next[j] / a.top : 0) * a.K + piece * 8;
       look_up(it + gridDim.x);
       for (int k = 0; k < slices; ++k, ++n) {
-        const int st = n % T::STAGES;
-        if (n >= T::STAGES) ok = mbar_wait(smem_u32(&empty[st]), (uint32_t)(n / T::STAGES - 1) & 1, abort_flag);
+        const int st = n % MANY_STAGES;
+        if (n >= MANY_STAGES) ok = mbar_wait(smem_u32(&c.empty[st]), (uint32_t)(n / MANY_STAGES - 1) & 1, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         const bool real = k * BK + piece * 8 < a.K;
-        const uint32_t dst = sm + st * T::STAGE + to;
+        const uint32_t dst = sm + st * MANY_STAGE + to;
 #pragma unroll
         for (int j = 0; j < PER; ++j)
           if (j < mine) cp_async16(dst + j * (ROW_STEP * 128), real ? src[j] + k * BK : x, real);
@@ -307,52 +326,55 @@ __global__ void __launch_bounds__(threads(MODE, BM), 1) moe_tcgen05_kernel(const
     if (ok)
       for (int i = max(0, n - (AHEAD - 1)); i < n; ++i) hand_over(i);
   } else if (warp == 5) {
-    const uint64_t a_desc = desc_k_major(sm), b_desc = desc_k_major(sm + T::A_BYTES);
+    const uint64_t a_desc = desc_k_major(sm), b_desc = desc_k_major(sm + MANY_A);
     int n = 0, turn = 0;
     bool ok = true;
     for (int it = blockIdx.x; ok && it < items; it += gridDim.x, ++turn) {
       const int acc = turn & 1;
-      if (turn >= 2) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&acc_empty[acc]), (uint32_t)(turn / 2 - 1) & 1, abort_flag));
+      if (turn >= 2) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.acc_empty[acc]), (uint32_t)(turn / 2 - 1) & 1, abort_flag));
       for (int k = 0; ok && k < slices; ++k, ++n) {
-        const int st = n % T::STAGES;
-        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&full[st]), (uint32_t)(n / T::STAGES) & 1, abort_flag));
+        const int st = n % MANY_STAGES;
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.full[st]), (uint32_t)(n / MANY_STAGES) & 1, abort_flag));
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (elect_one()) {
-          const uint64_t off = (uint64_t)((st * T::STAGE) >> 4);
+          const uint64_t off = (uint64_t)((st * MANY_STAGE) >> 4);
 #pragma unroll
           for (int ks = 0; ks < BK / 16; ++ks)
-            umma_bf16(tmem_base + acc * TN, a_desc + off + ks * 2, b_desc + off + ks * 2, IDESC, (k | ks) != 0 ? 1u : 0u);
-          umma_commit(smem_u32(&empty[st]));
-          if (k == slices - 1) umma_commit(smem_u32(&acc_full[acc]));
+            umma_bf16(c.tmem_base + acc * TN, a_desc + off + ks * 2, b_desc + off + ks * 2, idesc(TN), (k | ks) != 0 ? 1u : 0u);
+          umma_commit(smem_u32(&c.empty[st]));
+          if (k == slices - 1) umma_commit(smem_u32(&c.acc_full[acc]));
         }
         __syncwarp();
       }
     }
     // everything this CTA asked of the tensor core is done when this arrives: nobody leaves before
-    if (elect_one()) umma_commit(smem_u32(&all_done));
+    if (elect_one()) umma_commit(smem_u32(&c.all_done));
     __syncwarp();
-  } else if (warp < 4) {
+  } else {
+    // warps 0-3 have the first half of the columns, the last four the second; a warp reaches the 32 lanes of tensor memory
+    // of its number modulo 4
+    const int half = warp < 4 ? 0 : 1, quarter = warp & 3;
+    const int r = quarter * 32 + lane;
     int turn = 0;
     for (int it = blockIdx.x; it < items; it += gridDim.x, ++turn) {
-      const Item w = item_at<COLS, BM>(a, plan, it);
+      const Item w = item_at<COLS, ROWS_MANY>(a, plan, it);
       const int acc = turn & 1;
-      const int r = warp * 32 + lane;
       const bool mine = r < w.rows;
       const int pair = mine ? a.order[w.row0 + r] : 0;
       const float weight = (BY_TOKEN && mine && a.pair_weight != nullptr) ? a.pair_weight[pair] : 1.f;
-      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&acc_full[acc]), (uint32_t)(turn / 2) & 1, abort_flag))) break;
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&c.acc_full[acc]), (uint32_t)(turn / 2) & 1, abort_flag))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (warp * 32 < w.rows) {
-        const uint32_t addr = tmem_base + ((uint32_t)(warp * 32) << 16) + acc * TN;
+      if (quarter * 32 < w.rows) {
+        const uint32_t addr = c.tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * TN;
         __nv_bfloat16* dst = a.out + (size_t)(BY_TOKEN ? w.row0 + r : pair) * a.NOUT;
 #pragma unroll 1
-        for (int c = 0; c < COLS; c += 16) {
+        for (int col = half * (COLS / 2); col < (half + 1) * (COLS / 2); col += 16) {
           uint32_t v[16], u[16];
-          tmem_ld16(addr + c, v);
-          if (MODE == 1) tmem_ld16(addr + COLS + c, u);
+          tmem_ld16(addr + col, v);
+          if (MODE == 1) tmem_ld16(addr + COLS + col, u);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (mine && w.n0 + c < a.NOUT) {
+          if (mine && w.n0 + col < a.NOUT) {
             float y[16];
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
@@ -362,24 +384,158 @@ __global__ void __launch_bounds__(threads(MODE, BM), 1) moe_tcgen05_kernel(const
               else if (MODE == 2) y[i] = moe_gated_activation(a.act_mode, 0.f, rounded(weight * s), a.limit, a.alpha);
               else y[i] = s;
             }
-            store16(dst, w.n0 + c, a.NOUT, y);
+            store16(dst, w.n0 + col, a.NOUT, y);
           }
           __syncwarp();  // the next load from tensor memory is the whole warp's
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&acc_empty[acc]));
+      if (lane == 0) mbar_arrive(smem_u32(&c.acc_empty[acc]));
     }
-    mbar_wait(smem_u32(&all_done), 0, abort_flag);
+    mbar_wait(smem_u32(&c.all_done), 0, abort_flag);
   }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (abort_s != 0 && tid == 0) *a.error = 1;
-  if (warp == 0) {
+  leave(c, a, MANY_TMEM);
+}
+
+// ---- few rows ----
+
+// TILES: tiles of 128 weight rows per item.  MODE 1 with two: the gate rows and the up rows of 128 outputs; with one: of 64
+// outputs, 16 and 16 in turn, so that the two of an output sit in one warp, 16 lanes apart.
+template <int TILES>
+struct Few {
+  static constexpr uint32_t W_BYTES = TILES * 128 * 128, STAGE = W_BYTES + ROWS_FEW * 128;
+  static constexpr int STAGES = 216 * 1024 / STAGE;
+  static constexpr uint32_t SMEM = STAGES * STAGE;
+  static constexpr uint32_t ACC = TILES * ROWS_FEW, TMEM_COLS = 2 * ACC;  // columns of one accumulator, and of both
+};
+
+template <int MODE, int TILES>
+__global__ void __launch_bounds__(224, 1) moe_few_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w0,
+                                                         const __grid_constant__ CUtensorMap map_w1, const Args a) {
+  using F = Few<TILES>;
+  constexpr bool BY_TOKEN = MODE != 0, PAIRED = MODE == 1 && TILES == 1;
+  constexpr int COLS = MODE == 1 ? TILES * 64 : TILES * 128;
+  ts_pdl_wait();  // tensor memory is never held while waiting for another kernel
+  extern __shared__ unsigned char smem_unaligned[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_unaligned + 1023) & ~(uintptr_t)1023);
+  __shared__ __align__(8) Common<F::STAGES> c;
+  int* plan = a.E <= SHARED_EXPERTS ? reinterpret_cast<int*>(smem + F::SMEM) : nullptr;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  begin(c, a, plan, 2, 4, F::TMEM_COLS);
+  volatile int* abort_flag = &c.abort;
+  const uint32_t sm = smem_u32(smem);
+  const int items = a.tile_offsets[a.E] * a.cols, slices = (a.K + BK - 1) / BK;
+
+  if (warp == 4 || warp == 6) {  // the weight rows; the tokens' or places' rows
+    int n = 0;  // slices asked for
+    bool ok = true;
+    for (int it = blockIdx.x; ok && it < items; it += gridDim.x) {
+      const Item w = item_at<COLS, ROWS_FEW>(a, plan, it);
+      const int quads = (w.rows + 3) >> 2;  // gathers of four rows; the last one repeats the tile's last row
+      int rows[4] = {0, 0, 0, 0};
+      if (BY_TOKEN && warp == 6 && lane < quads) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) rows[i] = a.order[w.row0 + min(4 * lane + i, w.rows - 1)] / a.top;
+      }
+      const uint32_t bytes = warp == 4 ? F::W_BYTES : BY_TOKEN ? (uint32_t)quads * 512u : ROWS_FEW * 128u;
+      const int w_row = w.e * a.NOUT + w.n0;
+      for (int k = 0; k < slices; ++k, ++n) {
+        const int st = n % F::STAGES;
+        if (n >= F::STAGES) ok = mbar_wait(smem_u32(&c.empty[st]), (uint32_t)(n / F::STAGES - 1) & 1, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        const uint32_t bar = smem_u32(&c.full[st]), w_dst = sm + st * F::STAGE, x_dst = w_dst + F::W_BYTES;
+        if (lane == 0) mbar_expect_tx(bar, bytes);
+        __syncwarp();
+        if (warp == 4) {
+          if (PAIRED) {
+            if (lane < 8) tma_load_2d(w_dst + lane * 2048, (lane & 1) ? &map_w1 : &map_w0, bar, k * BK, w_row + (lane >> 1) * 16);
+          } else if (lane < TILES) {
+            tma_load_2d(w_dst + lane * 16384, MODE == 1 && lane == 1 ? &map_w1 : &map_w0, bar, k * BK, w_row + (MODE == 1 ? 0 : lane * 128));
+          }
+        } else if (BY_TOKEN) {
+          if (lane < quads) tma_gather4(x_dst + lane * 512, &map_x, bar, k * BK, rows);
+        } else if (lane == 0) {
+          tma_load_2d(x_dst, &map_x, bar, k * BK, w.row0);
+        }
+      }
+    }
+    if (*abort_flag) let_land(c, n);
+  } else if (warp == 5) {
+    const uint64_t w_desc = desc_k_major(sm), x_desc = desc_k_major(sm + F::W_BYTES);
+    int n = 0, turn = 0;
+    bool ok = true;
+    for (int it = blockIdx.x; ok && it < items; it += gridDim.x, ++turn) {
+      const int acc = turn & 1;
+      if (turn >= 2) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.acc_empty[acc]), (uint32_t)(turn / 2 - 1) & 1, abort_flag));
+      for (int k = 0; ok && k < slices; ++k, ++n) {
+        const int st = n % F::STAGES;
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.full[st]), (uint32_t)(n / F::STAGES) & 1, abort_flag));
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (elect_one()) {
+          const uint64_t off = (uint64_t)((st * F::STAGE) >> 4);
+#pragma unroll
+          for (int ks = 0; ks < BK / 16; ++ks)
+#pragma unroll
+            for (int t = 0; t < TILES; ++t)
+              umma_bf16(c.tmem_base + acc * F::ACC + t * ROWS_FEW, w_desc + off + t * 1024 + ks * 2, x_desc + off + ks * 2, idesc(ROWS_FEW),
+                        (k | ks) != 0 ? 1u : 0u);
+          umma_commit(smem_u32(&c.empty[st]));
+          if (k == slices - 1) umma_commit(smem_u32(&c.acc_full[acc]));
+        }
+        __syncwarp();
+      }
+    }
+    if (elect_one()) umma_commit(smem_u32(&c.all_done));  // nobody leaves before this has arrived (see the other kernel)
     __syncwarp();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(T::TMEM_COLS) : "memory");
+  } else if (warp < 4) {
+    int turn = 0;
+    for (int it = blockIdx.x; it < items; it += gridDim.x, ++turn) {
+      const Item w = item_at<COLS, ROWS_FEW>(a, plan, it);
+      const int acc = turn & 1;
+      // lane i looks place i's pair and weight up for everybody
+      const int pair_of = lane < w.rows ? a.order[w.row0 + lane] : 0;
+      const float weight_of = (BY_TOKEN && a.pair_weight != nullptr && lane < w.rows) ? a.pair_weight[pair_of] : 1.f;
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&c.acc_full[acc]), (uint32_t)(turn / 2) & 1, abort_flag))) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t addr = c.tmem_base + ((uint32_t)(warp * 32) << 16) + acc * F::ACC;
+      const int n = w.n0 + (PAIRED ? warp * 16 + (lane & 15) : tid);  // this thread's output (of tile 0)
+      for (int p0 = 0; p0 < w.rows; p0 += 8) {
+        uint32_t v[TILES][8];
+#pragma unroll
+        for (int t = 0; t < TILES; ++t) tmem_ld8(addr + t * ROWS_FEW + p0, v[t]);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          if (p0 + i >= w.rows) break;  // the same for the whole warp
+          const int pair = __shfl_sync(0xffffffffu, pair_of, p0 + i);
+          const float weight = __shfl_sync(0xffffffffu, weight_of, p0 + i);
+          __nv_bfloat16* dst = a.out + (size_t)(BY_TOKEN ? w.row0 + p0 + i : pair) * a.NOUT;
+          const float s0 = __uint_as_float(v[0][i]), s1 = __uint_as_float(v[TILES - 1][i]);
+          // the sums are rounded to bfloat16 before the activation, as a product stored to memory would be
+          if (MODE == 1) {
+            const float mate = PAIRED ? __shfl_xor_sync(0xffffffffu, s0, 16) : s1;  // of a gate row's lane: the up row's sum
+            if (n < a.NOUT && !(PAIRED && lane >= 16))
+              dst[n] = __float2bfloat16_rn(moe_gated_activation(a.act_mode, rounded(weight * s0), rounded(weight * mate), a.limit, a.alpha));
+          } else {
+#pragma unroll
+            for (int t = 0; t < TILES; ++t) {
+              const float s = t == 0 ? s0 : s1;
+              if (n + t * 128 < a.NOUT)
+                dst[n + t * 128] = __float2bfloat16_rn(MODE == 2 ? moe_gated_activation(a.act_mode, 0.f, rounded(weight * s), a.limit, a.alpha) : s);
+            }
+          }
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&c.acc_empty[acc]));
+    }
+    mbar_wait(smem_u32(&c.all_done), 0, abort_flag);
   }
+  leave(c, a, F::TMEM_COLS);
 }
 
 // A [rows, K] matrix, boxes of box_rows rows of 64 entries, 128-byte swizzle (box_rows 1: for gathers)
@@ -394,46 +550,70 @@ int rows_map(const void* ptr, long long rows, int K, int box_rows, CUtensorMap* 
              : TS_ERR_BAD_ARGUMENT;
 }
 
-template <int MODE, int TN, int BM>
-int launch(const void* A, int tokens, const void* B0, const void* B1, int P, Args a, int sms, cudaStream_t s) {
+// Bytes of dynamic shared memory behind `tiles` of ring, and the attribute that allows the most of it.
+size_t shared_bytes(uint32_t ring, int E) { return ring + 1024 + (E <= SHARED_EXPERTS ? 2 * (E + 1) * sizeof(int) : 0); }
+template <typename Kernel>
+int allow_shared(Kernel kernel, uint32_t ring) {
+  return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared_bytes(ring, SHARED_EXPERTS));
+}
+// How many CTAs: at most one per item, and every expert that got a pair may have one row tile that is not full.
+long long most_items(int P, int rows, const Args& a) { return ((long long)P / rows + min(a.E, P)) * a.cols; }
+
+template <int MODE>
+int launch_many(const void* A, const void* W0, const void* W1, int P, Args a, int sms, cudaStream_t s) {
   constexpr int COLS = MODE == 1 ? TN / 2 : TN;
   a.cols = (a.NOUT + COLS - 1) / COLS;
   CUtensorMap ma, m0, m1;
-  int st = MODE == 0 ? rows_map(A, P, a.K, BM, &ma) : by_warps(MODE, BM) ? 0 : rows_map(A, tokens, a.K, 1, &ma);
-  if (!st) st = rows_map(B0, (long long)a.E * a.NOUT, a.K, TN / 2, &m0);
-  if (!st) st = rows_map(B1 != nullptr ? B1 : B0, (long long)a.E * a.NOUT, a.K, TN / 2, &m1);
+  int st = rows_map(W0, (long long)a.E * a.NOUT, a.K, TN / 2, &m0);
+  if (!st) st = W1 != nullptr ? rows_map(W1, (long long)a.E * a.NOUT, a.K, TN / 2, &m1) : (m1 = m0, 0);
+  if (!st) st = MODE == 0 ? rows_map(A, P, a.K, ROWS_MANY, &ma) : (ma = m0, 0);
   if (st) return st;
-  if (by_warps(MODE, BM)) ma = m0;  // not used
   static bool configured = false;
-  const size_t smem = Tile<TN, BM>::SMEM + 1024 + (a.E <= SHARED_EXPERTS ? 2 * (a.E + 1) * sizeof(int) : 0);
   if (!configured) {
-    constexpr size_t most = Tile<TN, BM>::SMEM + 1024 + 2 * (SHARED_EXPERTS + 1) * sizeof(int);
-    cudaError_t e = cudaFuncSetAttribute(moe_tcgen05_kernel<MODE, TN, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
-    if (e != cudaSuccess) return (int)e;
+    if ((st = allow_shared(moe_many_kernel<MODE>, MANY_SMEM))) return st;
     configured = true;
   }
-  // at most this many items: every expert that got a pair may have one row tile that is not full
-  const long long most = ((long long)P / BM + min(a.E, P)) * a.cols;
+  const long long most = most_items(P, ROWS_MANY, a);
   if (most > 0x7fffffffLL) return TS_ERR_UNSUPPORTED_SIZE;
-  return ts_launch(moe_tcgen05_kernel<MODE, TN, BM>, dim3((unsigned)min((long long)sms, most)), dim3(threads(MODE, BM)), smem, s,
+  return ts_launch(moe_many_kernel<MODE>, dim3((unsigned)min((long long)sms, most)), dim3(many_threads(MODE)), shared_bytes(MANY_SMEM, a.E), s,
                    (const __nv_bfloat16*)A, ma, m0, m1, a);
 }
 
-// Items of 256 weight rows, or of 128 in steps of few pairs where the wide ones would leave SMs idle: the width whose
-// fullest CTA streams the fewest weight rows.  How many experts got a pair is known on the device only; on average P pairs meet
-// E (1 - (1 - 1/E)^P) of them.  (16 experts, 2,048 -> 2 x 1,024, one token's 2 pairs: 20.5 us with 128, 26.6 with 256 and nearly
-// twice with the 64 that would balance 16 pairs: a slice costs what it costs however few its rows.)
-bool narrow(int P, int E, int cols, int sms) {
-  const double met = E * (1.0 - pow(1.0 - 1.0 / E, (double)P));
-  return ceil(met * 2 * cols / sms) < 2 * ceil(met * cols / sms);
+template <int MODE, int TILES>
+int launch_few(const void* A, int rows, const void* W0, const void* W1, int P, Args a, int sms, cudaStream_t s) {
+  using F = Few<TILES>;
+  constexpr int COLS = MODE == 1 ? TILES * 64 : TILES * 128, BOX = MODE == 1 && TILES == 1 ? 16 : 128;
+  a.cols = (a.NOUT + COLS - 1) / COLS;
+  CUtensorMap mx, m0, m1;
+  int st = rows_map(W0, (long long)a.E * a.NOUT, a.K, BOX, &m0);
+  if (!st) st = W1 != nullptr ? rows_map(W1, (long long)a.E * a.NOUT, a.K, BOX, &m1) : (m1 = m0, 0);
+  if (!st) st = rows_map(A, rows, a.K, MODE == 0 ? ROWS_FEW : 1, &mx);
+  if (st) return st;
+  static bool configured = false;
+  if (!configured) {
+    if ((st = allow_shared(moe_few_kernel<MODE, TILES>, F::SMEM))) return st;
+    configured = true;
+  }
+  const long long most = most_items(P, ROWS_FEW, a);
+  if (most > 0x7fffffffLL) return TS_ERR_UNSUPPORTED_SIZE;
+  return ts_launch(moe_few_kernel<MODE, TILES>, dim3((unsigned)min((long long)sms, most)), dim3(224), shared_bytes(F::SMEM, a.E), s, mx, m0, m1, a);
 }
 
+// One tile of 128 weight rows per item instead of two where the wide items would leave SMs idle: the width whose fullest CTA
+// streams the fewest weight rows.  How many experts got a pair is known on the device only; on average P pairs meet
+// E (1 - (1 - 1/E)^P) of them.
+bool narrow(int P, int E, int wide_cols, int sms) {
+  const double met = E * (1.0 - pow(1.0 - 1.0 / E, (double)P));
+  return ceil(met * 2 * wide_cols / sms) < 2 * ceil(met * wide_cols / sms);
+}
+
+// A: `rows` rows (tokens of the first product, places of the second)
 template <int MODE>
-int launch_shape(int tile_rows, const void* A, int tokens, const void* B0, const void* B1, int P, const Args& a, int sms, cudaStream_t s) {
+int launch_shape(int tile_rows, const void* A, int rows, const void* W0, const void* W1, int P, const Args& a, int sms, cudaStream_t s) {
   constexpr int COLS = MODE == 1 ? 128 : 256;
-  if (tile_rows == ROWS_MANY) return launch<MODE, 256, ROWS_MANY>(A, tokens, B0, B1, P, a, sms, s);
-  if (narrow(P, a.E, (a.NOUT + COLS - 1) / COLS, sms)) return launch<MODE, 128, ROWS_FEW>(A, tokens, B0, B1, P, a, sms, s);
-  return launch<MODE, 256, ROWS_FEW>(A, tokens, B0, B1, P, a, sms, s);
+  if (tile_rows == ROWS_MANY) return launch_many<MODE>(A, W0, W1, P, a, sms, s);
+  if (narrow(P, a.E, (a.NOUT + COLS - 1) / COLS, sms)) return launch_few<MODE, 1>(A, rows, W0, W1, P, a, sms, s);
+  return launch_few<MODE, 2>(A, rows, W0, W1, P, a, sms, s);
 }
 
 }  // namespace
@@ -463,5 +643,5 @@ TS_EXPORT int ts_moe_down_tcgen05(const void* act, const int* order, const int* 
   if (E <= 0 || I <= 0 || N <= 0 || sms <= 0 || error == nullptr || (tile_rows != ROWS_MANY && tile_rows != ROWS_FEW)) return TS_ERR_BAD_ARGUMENT;
   if (I % 8 || (((uintptr_t)act | (uintptr_t)down) & 15) || (long long)E * N > 0x7fffffffLL - 256) return TS_ERR_UNSUPPORTED_SIZE;
   const Args a = {nullptr, order, offsets, tile_offsets, (__nv_bfloat16*)pair_out, error, E, I, N, 1, 0, 0.f, 0.f, 0};
-  return launch_shape<0>(tile_rows, act, 0, down, nullptr, P, a, sms, (cudaStream_t)stream);
+  return launch_shape<0>(tile_rows, act, P, down, nullptr, P, a, sms, (cudaStream_t)stream);
 }
