@@ -449,3 +449,24 @@ def test_expert_products_at_the_edges_of_their_tiles(rows, E, K, I, activation):
             ops.moe_down(act, plan, down, out)
             assert _rel(out[places], product(down, act[: len(places)].double())) < 5e-3
     ops.check_device_errors()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("T, W, E", [(1, 8, 1), (7, 2048, 16), (296, 4104, 33), (297, 136, 5), (1535, 64, 32), (1536, 200, 65), (1601, 1160, 31), (40, 44, 6), (300, 42, 7)])
+def test_router_logits_do_not_depend_on_the_kernel(dtype, T, W, E):
+    """A CTA a token, tiles of 8 and of 16 tokens, and the kernel for odd rows add a token's logits up in the same order: the weights
+    (sigmoid of the logits) are bit by bit those of the token alone, and close to float64."""
+    from tokensprint_b200 import ops
+
+    g = torch.Generator().manual_seed(T + W)
+    x, r, bias = torch.randn(T, W, generator=g).to(dtype).cuda(), (torch.randn(E, W, generator=g) / W ** 0.5).cuda(), torch.randn(E, generator=g).cuda()
+    top = min(E, 3)
+    ids, w = torch.full((T, top), -1, dtype=torch.int32, device="cuda"), torch.full((T, top), float("nan"), device="cuda")
+    ops.router(x, r, top, False, ids, w, bias=bias)
+    for t in sorted({0, T // 2, T - 1}):
+        one_id, one_w = torch.empty(1, top, dtype=torch.int32, device="cuda"), torch.empty(1, top, device="cuda")
+        ops.router(x[t:t + 1].clone(), r, top, False, one_id, one_w, bias=bias)
+        assert torch.equal(one_id[0], ids[t]) and torch.equal(one_w[0], w[t])
+    z = x.double() @ r.double().T + bias.double()
+    assert float((w.double() - torch.sigmoid(z.gather(1, ids.long()))).abs().max()) < 1e-5
+    assert float((torch.topk(z, top).values - z.gather(1, ids.long())).abs().max()) < 1e-5

@@ -446,12 +446,235 @@ __global__ void __launch_bounds__(256) router_kernel(const TX* __restrict__ x, c
                 weights + (size_t)(t0 + warp) * top, lane, correction, groups);
 }
 
+// The two kernels below add a logit up exactly as router_kernel does, so a token's logits are the same bit by bit whatever
+// else the step holds: chain l of 32 takes the 16-byte pieces l, l + 32, l + 64, ... of the row in order, and the chains meet
+// pairwise, l and l + 16 first.  Rows of whole 16-byte pieces (W % 4 == 0).
+
+template <typename TX>
+__device__ __forceinline__ float4 router_piece(const TX* p);
+template <>
+__device__ __forceinline__ float4 router_piece<float>(const float* p) {
+  return *reinterpret_cast<const float4*>(p);
+}
+template <>
+__device__ __forceinline__ float4 router_piece<__nv_bfloat16>(const __nv_bfloat16* p) {
+  const uint2 v = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ float router_fma(const float4& x, const float4& w, float acc) {
+  return fmaf(x.w, w.w, fmaf(x.z, w.z, fmaf(x.y, w.y, fmaf(x.x, w.x, acc))));
+}
+
+// Few tokens: one CTA a token, a warp an expert.  Such a step is a chain of trips to device memory and little else; the router's
+// rows are no kernel's output, so their first pieces are loaded, and the others asked into the L2, before the wait for the
+// kernels ahead.
+#define ROUTER_AHEAD 8
+template <typename TX>
+__global__ void __launch_bounds__(1024) router_few_kernel(const TX* __restrict__ x, const float* __restrict__ router, const float* __restrict__ bias,
+                                                          int W, int E, int top, int renormalize, int score_mode, int* __restrict__ ids,
+                                                          float* __restrict__ weights, const float* __restrict__ correction, RouterGroups groups) {
+  extern __shared__ float logits[];  // [E + groups]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5, pieces = W >> 2;
+  const float* row = router + (size_t)min(warp, E - 1) * W;
+  float4 w[ROUTER_AHEAD];
+#pragma unroll
+  for (int i = 0; i < ROUTER_AHEAD; ++i) w[i] = lane + 32 * i < pieces ? __ldg(reinterpret_cast<const float4*>(row) + lane + 32 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int k = (lane + 8 * ROUTER_AHEAD) * 16; k < W; k += 32 * 16)  // one request per 64 bytes of the rest
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(row + k));
+  ts_pdl_prologue();
+  const TX* xr = x + (size_t)blockIdx.x * W;
+  for (int e = warp; e < E; e += nwarps) {
+    const float* r = router + (size_t)e * W;
+    float acc = 0.f;
+    {
+      float4 xv[ROUTER_AHEAD];
+#pragma unroll
+      for (int i = 0; i < ROUTER_AHEAD; ++i) xv[i] = lane + 32 * i < pieces ? router_piece(xr + 4 * (lane + 32 * i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      if (e != warp) {
+#pragma unroll
+        for (int i = 0; i < ROUTER_AHEAD; ++i) w[i] = lane + 32 * i < pieces ? __ldg(reinterpret_cast<const float4*>(r) + lane + 32 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int i = 0; i < ROUTER_AHEAD; ++i) acc = router_fma(xv[i], w[i], acc);
+    }
+#pragma unroll 4
+    for (int k = lane + 32 * ROUTER_AHEAD; k < pieces; k += 32)
+      acc = router_fma(router_piece(xr + 4 * k), __ldg(reinterpret_cast<const float4*>(r) + k), acc);
+    acc = ts_warp_sum(acc);
+    if (lane == 0) logits[e] = acc + (bias ? bias[e] : 0.f);
+  }
+  __syncthreads();
+  if (warp == 0)
+    router_choose(logits, E, top, renormalize, score_mode, ids + (size_t)blockIdx.x * top, weights + (size_t)blockIdx.x * top, lane, correction, groups);
+}
+
+// Many tokens: TT tokens a CTA against EX experts at a time (16, or 32), slabs of 128 entries of both staged by 16-byte cp.async, NS - 1 in
+// flight.  Warp v has the chains 4 v .. 4 v + 3 of all TT x EX sums; a lane TT / 4 tokens x EX / 8 experts of each.  Bound by the trips of a slab to
+// the L2 and back while one or two CTAs an SM are there to hide them.  router_kernel re-read every router row
+// from the L2 per four tokens.
+constexpr int RT_SLAB = 128, RT_WS = RT_SLAB + 4;  // rows 16 bytes apart modulo 128: no two lanes meet in a bank
+template <typename TX>
+__host__ __device__ constexpr int rt_x_stride() { return RT_SLAB + 16 / (int)sizeof(TX); }
+template <typename TX, int TT, int EX>
+__host__ __device__ constexpr size_t rt_stage_bytes() { return (size_t)EX * RT_WS * 4 + (size_t)TT * rt_x_stride<TX>() * sizeof(TX); }
+template <typename TX, int TT, int EX, int NS>  // the slabs, or the chains' sums in their place
+__host__ __device__ constexpr size_t rt_ring_bytes() {
+  constexpr size_t slabs = NS * rt_stage_bytes<TX, TT, EX>(), sums = (size_t)32 * TT * (EX + 1) * 4;
+  return slabs > sums ? slabs : sums;
+}
+
+template <typename TX, int TT, int EX, int NS>
+__global__ void __launch_bounds__(256) router_tile_kernel(const TX* __restrict__ x, const float* __restrict__ router, const float* __restrict__ bias,
+                                                          int T, int W, int E, int top, int renormalize, int score_mode, int* __restrict__ ids,
+                                                          float* __restrict__ weights, const float* __restrict__ correction, RouterGroups groups) {
+  ts_pdl_prologue();
+  constexpr int XS = rt_x_stride<TX>(), TL = TT / 4;
+  constexpr size_t STAGE = rt_stage_bytes<TX, TT, EX>();
+  extern __shared__ __align__(16) unsigned char rsm[];
+  const int Z = E + groups.count;
+  float* logits = reinterpret_cast<float*>(rsm + rt_ring_bytes<TX, TT, EX, NS>());  // [TT][Z]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ti = lane >> 3, ej = lane & 7;
+  const int t0 = blockIdx.x * TT, nt = min(TT, T - t0), slabs = (W + RT_SLAB - 1) / RT_SLAB;
+  for (int e0 = 0; e0 < E; e0 += EX) {
+    auto copy16 = [&](void* dst, const void* src, bool real) {
+      const int bytes = real ? 16 : 0;  // 0: zeros
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
+    };
+    auto fetch = [&](int slab) {
+      unsigned char* st = rsm + (slab % NS) * STAGE;
+      float* ws = reinterpret_cast<float*>(st);
+      TX* xs = reinterpret_cast<TX*>(st + (size_t)EX * RT_WS * 4);
+      for (int i = tid; i < EX * (RT_SLAB / 4); i += 256) {
+        const int r = i / (RT_SLAB / 4), c = slab * RT_SLAB + (i % (RT_SLAB / 4)) * 4;
+        const bool real = e0 + r < E && c < W;
+        copy16(ws + r * RT_WS + (i % (RT_SLAB / 4)) * 4, real ? router + (size_t)(e0 + r) * W + c : router, real);
+      }
+      constexpr int PER = 16 / (int)sizeof(TX);  // W is a multiple of it: a piece lies inside the row or behind it
+      for (int i = tid; i < TT * (RT_SLAB / PER); i += 256) {
+        const int r = i / (RT_SLAB / PER), c = slab * RT_SLAB + (i % (RT_SLAB / PER)) * PER;
+        const bool real = r < nt && c < W;
+        copy16(xs + r * XS + (i % (RT_SLAB / PER)) * PER, real ? x + (size_t)(t0 + r) * W + c : x, real);
+      }
+    };
+    constexpr int EL = EX / 8;
+    float acc[4][TL][EL];
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+#pragma unroll
+      for (int i = 0; i < TL; ++i)
+#pragma unroll
+        for (int j = 0; j < EL; ++j) acc[p][i][j] = 0.f;
+    __syncthreads();  // the block of experts before has been read
+    for (int sl = 0; sl < NS - 1; ++sl) {
+      if (sl < slabs) fetch(sl);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    for (int sl = 0; sl < slabs; ++sl) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(NS - 2) : "memory");
+      __syncthreads();
+      if (sl + NS - 1 < slabs) fetch(sl + NS - 1);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      const unsigned char* st = rsm + (sl % NS) * STAGE;
+      const float* ws = reinterpret_cast<const float*>(st) + ej * RT_WS + warp * 16;
+      const TX* xs = reinterpret_cast<const TX*>(st + (size_t)EX * RT_WS * 4) + ti * XS + warp * 16;
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+        float4 wv[EL];
+#pragma unroll
+        for (int j = 0; j < EL; ++j) wv[j] = *reinterpret_cast<const float4*>(ws + j * 8 * RT_WS + p * 4);
+#pragma unroll
+        for (int i = 0; i < TL; ++i) {
+          const float4 xv = router_piece(xs + i * 4 * XS + p * 4);
+#pragma unroll
+          for (int j = 0; j < EL; ++j) acc[p][i][j] = router_fma(xv, wv[j], acc[p][i][j]);
+        }
+      }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    float* sums = reinterpret_cast<float*>(rsm);  // [32 chains][TT][EX + 1]
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+#pragma unroll
+      for (int i = 0; i < TL; ++i)
+#pragma unroll
+        for (int j = 0; j < EL; ++j) sums[((warp * 4 + p) * TT + ti + i * 4) * (EX + 1) + ej + j * 8] = acc[p][i][j];
+    __syncthreads();
+    for (int o = tid; o < TT * EX; o += 256) {
+      const int t = o / EX, e = o % EX;
+      float v[32];
+#pragma unroll
+      for (int l = 0; l < 32; ++l) v[l] = sums[(l * TT + t) * (EX + 1) + e];
+#pragma unroll
+      for (int half = 16; half > 0; half >>= 1)
+#pragma unroll
+        for (int l = 0; l < half; ++l) v[l] += v[l + half];
+      if (t < nt && e0 + e < E) logits[(size_t)t * Z + e0 + e] = v[0] + (bias ? bias[e0 + e] : 0.f);
+    }
+  }
+  __syncthreads();
+  for (int t = warp; t < nt; t += 8)
+    router_choose(logits + (size_t)t * Z, E, top, renormalize, score_mode, ids + (size_t)(t0 + t) * top, weights + (size_t)(t0 + t) * top, lane,
+                  correction, groups);
+}
+
+template <typename TX>
+static int launch_router_few(const void* x, const float* router, const float* bias, int T, int W, int E, int top, int renormalize, int score_mode, int* ids,
+                             float* weights, const float* correction, const RouterGroups& groups, cudaStream_t s) {
+  return ts_launch(router_few_kernel<TX>, dim3(T), dim3(32 * min(E, 32)), (size_t)(E + groups.count) * sizeof(float), s, (const TX*)x, router, bias, W, E,
+                   top, renormalize, score_mode, ids, weights, correction, groups);
+}
+template <typename TX, int TT, int EX, int NS>
+static int launch_router_tile(const void* x, const float* router, const float* bias, int T, int W, int E, int top, int renormalize, int score_mode, int* ids,
+                              float* weights, const float* correction, const RouterGroups& groups, cudaStream_t s) {
+  const size_t smem = rt_ring_bytes<TX, TT, EX, NS>() + (size_t)TT * (E + groups.count) * sizeof(float);
+  static bool configured = false;
+  if (!configured) {
+    const cudaError_t e = cudaFuncSetAttribute(router_tile_kernel<TX, TT, EX, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  return ts_launch(router_tile_kernel<TX, TT, EX, NS>, dim3((T + TT - 1) / TT), dim3(256), smem, s, (const TX*)x, router, bias, T, W, E, top, renormalize, score_mode,
+                   ids, weights, correction, groups);
+}
+template <int N>
+struct Const {
+  static constexpr int value = N;
+};
+#define ROUTER_FEW_TOKENS 296
+// Which kernel (the logits are the same): a CTA a token up to two tokens per SM, then tiles of 8 tokens, of 16 beyond 8 per SM,
+// with six slabs in the ring while a CTA has its SM to itself and four, two CTAs an SM, beyond that.  Rows that are no whole pieces, misaligned bases and more experts than shared memory has room for: router_kernel.
+// Measured, bfloat16 rows, us, router_kernel / these: 16 experts of 2,048: 64 tokens 7.7 / 4.8, 512 13.5 / 10.5, 2,048 20.3 / 21.9,
+// 8,192 72 / 40; 32 experts of 4,096: 64 tokens 20.3 / 8.4, 512 39.8 / 35.4, 2,048 95 / 38, 8,192 235 / 114.
+template <typename TX>
+static int launch_router(const void* x, const float* router, const float* bias, int T, int W, int E, int top, int renormalize, int score_mode, int* ids,
+                         float* weights, const float* correction, const RouterGroups& groups, cudaStream_t s, bool& taken) {
+  constexpr int PER = 16 / (int)sizeof(TX);
+  taken = W % PER == 0 && (((uintptr_t)x | (uintptr_t)router) & 15) == 0 && E <= 1024;
+  if (!taken) return 0;
+  if (T <= ROUTER_FEW_TOKENS) return launch_router_few<TX>(x, router, bias, T, W, E, top, renormalize, score_mode, ids, weights, correction, groups, s);
+  auto tiles = [&](auto tt, auto ns) {
+    if (E <= 16)
+      return launch_router_tile<TX, decltype(tt)::value, 16, decltype(ns)::value>(x, router, bias, T, W, E, top, renormalize, score_mode, ids, weights, correction, groups, s);
+    return launch_router_tile<TX, decltype(tt)::value, 32, decltype(ns)::value>(x, router, bias, T, W, E, top, renormalize, score_mode, ids, weights, correction, groups, s);
+  };
+  if (T <= 8 * 148) return tiles(Const<8>(), Const<4>());
+  return T <= 16 * 148 ? tiles(Const<16>(), Const<6>()) : tiles(Const<16>(), Const<4>());
+}
+
 TS_EXPORT int ts_router(const void* x, int x_dtype, const float* router, const float* bias, int T, int W, int E, int top, int renormalize,
                         int score_mode, int* ids, float* weights, const float* correction, int group_count, int group_keep, float scale,
                         void* stream) {
   if (T <= 0) return 0;
   if (W <= 0 || E <= 0 || top <= 0 || top > E || !router_groups_fit(E, top, group_count, group_keep)) return TS_ERR_BAD_ARGUMENT;
   const RouterGroups groups = {group_count, group_keep, scale};
+  if (x_dtype != TS_DTYPE_F32 && x_dtype != TS_DTYPE_BF16) return TS_ERR_BAD_ARGUMENT;
+  bool taken = false;
+  const int rc = x_dtype == TS_DTYPE_F32
+                     ? launch_router<float>(x, router, bias, T, W, E, top, renormalize, score_mode, ids, weights, correction, groups, (cudaStream_t)stream, taken)
+                     : launch_router<__nv_bfloat16>(x, router, bias, T, W, E, top, renormalize, score_mode, ids, weights, correction, groups, (cudaStream_t)stream, taken);
+  if (taken) return rc;
   const int Z = E + group_count;
   // tokens per CTA: four where there are CTAs enough for every SM several times over (a router row is
   // then read once per four tokens), fewer in steps of few tokens (more CTAs, shorter chains of loads)
