@@ -25,8 +25,10 @@ LATENT_REBUILD = os.environ.get("TS_LATENT_REBUILD", "1") != "0"
 LATENT_REBUILD_MAX_BYTES = 256 << 20
 
 
-def rebuilding_pays(portions: Sequence[tuple[int, int]], heads: int, sms: int) -> bool:
+def rebuilding_pays(portions: Sequence[tuple[int, int]], heads: int, sms: int, beside_decodes: bool = False) -> bool:
     """Whether a step's prompt portions, as (new tokens, keys kept) each, are faster with rebuilt keys and values.
+    Beside decoded tokens, which go through absorbed queries in any case, the step then has both paths: eight more calls a
+    layer, about 100 us of host time in a step that the host bounds (24 tokens beside 2 x 700: 2.13 against 2.01 ms).
 
     Both sides in microseconds, fitted to a sweep on B200 (16 and 32 heads, 1 and 4 portions of 5 to 512 tokens, 5 to 8,192
     keys; the model is within a tenth or 4 us).  Absorbed queries: 32 rows a CTA, 3.75 us per block of 64 keys, one
@@ -40,7 +42,7 @@ def rebuilding_pays(portions: Sequence[tuple[int, int]], heads: int, sms: int) -
 
     absorbed = 18.0 + 3.75 * passes(32, 64, True)
     rebuilt = 26.0 + 2.2e-4 * heads * sum(k for _, k in portions) + 1.75 * passes(256, 96, False)
-    return rebuilt < absorbed
+    return rebuilt + (150.0 if beside_decodes else 0.0) < absorbed
 
 
 def batched_linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
@@ -253,7 +255,8 @@ class LatentAttentionMixer(Mixer):
         first = step.decode_seqs if step.decode_seqs < B else 0
         portions = [(n, ops.latent_kept_keys(self.window, n, start + n)) for start, n in zip(step.host_seq_starts[first:], step.host_seq_lens[first:])]
         kept = [k for _, k in portions]
-        if sum(kept) * self.kv_weight.shape[0] * 2 > LATENT_REBUILD_MAX_BYTES or not rebuilding_pays(portions, self.num_heads, ops._sm_count(q_rows.device)):
+        if sum(kept) * self.kv_weight.shape[0] * 2 > LATENT_REBUILD_MAX_BYTES or not rebuilding_pays(
+                portions, self.num_heads, ops._sm_count(q_rows.device), first > 0):
             return T, []
         return first, kept
 
