@@ -37,6 +37,9 @@
 #define GLA_UNROLL 4     // tokens of a round whose loads and shuffles are in flight together
 #endif
 constexpr int GLA_UNROLL_TOKENS = GLA_UNROLL;
+#ifndef GLA_TWO_COLUMNS_CTAS
+#define GLA_TWO_COLUMNS_CTAS 296  // fewest CTAs of two columns a thread
+#endif
 
 __device__ __forceinline__ float gla_log_sigmoid(float z) {
   // log(1 / (1 + exp(-z))) without overflow on either side
@@ -57,6 +60,24 @@ __device__ __forceinline__ __nv_bfloat16 gla_load(const __nv_bfloat16* p) {
   return __ushort_as_bfloat16(v);
 }
 
+// two float32 in one 64-bit register, and the packed arithmetic on them (each half rounds as the scalar operation does)
+__device__ __forceinline__ uint64_t gla_pack(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void gla_unpack(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t gla_fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t gla_mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
 // The rounds are pipelined: while the threads run the updates of one round from shared memory, the
 // loads of the next round's q, k, z and v are in flight into registers (issued before the updates,
 // used after them), so the recurrence never waits for device memory.
@@ -67,8 +88,8 @@ __device__ __forceinline__ __nv_bfloat16 gla_load(const __nv_bfloat16* p) {
 // MODE 2 starts every segment from what the segments before it left, folded in order
 // (S <- product * S + state), writes the read-outs, and the last segment writes the request's slot.
 // MODE 0 is the whole portion in one piece (decode steps, short portions: the same sums whatever the cut).
-template <typename TA, int KP, int MODE>
-__global__ void __launch_bounds__(GLA_THREADS, GLA_MIN_BLOCKS) gla_scan_kernel(
+template <typename TA, int KP, int MODE, int NC>
+__global__ void __launch_bounds__(GLA_THREADS, NC == 2 ? 3 : GLA_MIN_BLOCKS) gla_scan_kernel(
     const TA* __restrict__ q, const TA* __restrict__ k, const TA* __restrict__ v, long long ld_qkv, const float* __restrict__ decay,
     float q_scale, float* __restrict__ state, const int* __restrict__ state_slots, const int* __restrict__ cu_seqlens,
     float* __restrict__ o, int H, int d, int e, int R, int cols_per_cta, int tb, int segs, int seg_len, float* __restrict__ seg_state,
@@ -89,8 +110,15 @@ __global__ void __launch_bounds__(GLA_THREADS, GLA_MIN_BLOCKS) gla_scan_kernel(
   const bool last = t_end == cu_seqlens[b + 1];
   if (MODE == 1 && last) return;  // nobody starts from what a sequence's last segment leaves
   const int r = threadIdx.x % R, cj = threadIdx.x / R;  // lanes of one column sit side by side
-  const int col = col0 + cj;
-  const bool has_col = col < e;
+  constexpr int PFV = GLA_PFV * NC;
+  const int lanes = GLA_THREADS / R;  // columns side by side; a thread has NC of them, `lanes` apart
+  int col[NC];
+  bool has_col[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    col[c] = col0 + cj + c * lanes;
+    has_col[c] = col[c] < e;
+  }
   // Register i of a thread holds key channel CH(i): its channels come in fours, and the fours of the R lanes of a column
   // are interleaved (lane r owns fours r, r + R, r + 2 R, ...), so that the 16-byte loads of a warp's lanes fall on
   // consecutive 16-byte pieces of the staged rows: no two of them meet in a bank of shared memory.
@@ -100,44 +128,61 @@ __global__ void __launch_bounds__(GLA_THREADS, GLA_MIN_BLOCKS) gla_scan_kernel(
   float* seg_L = MODE == 0 ? nullptr : seg_state + (((size_t)b * segs + seg) * H + h) * state_elems;   // this segment's end state
   float* seg_P = MODE == 0 ? nullptr : seg_decay + (((size_t)b * segs + seg) * H + h) * d;             // this segment's decay product
   float* seg_S0 = MODE == 0 ? nullptr : seg_start + ((size_t)b * H + h) * state_elems;                 // the request's state as the step found it
-  float s_reg[KP];
-  float p_reg[MODE == 1 ? KP : 1];
-  if (MODE == 0 || (seg == 0 && (MODE == 1 || last))) {
-    // the request's state (MODE 2: only a sequence of one segment reads the slot, which it alone writes in this launch)
+  // pairs of neighbouring channels (CH(2 i), CH(2 i) + 1) of a column in one 64-bit register
+  uint64_t s_reg[NC][KP / 2];
+  uint64_t p_reg[MODE == 1 ? KP / 2 : 1];
+  auto load_pair = [&](const float* from, int i, int c) {
+    const int ch = CH(2 * i);
+    return gla_pack((has_col[c] && ch < d) ? from[(size_t)ch * e + col[c]] : 0.f, (has_col[c] && ch + 1 < d) ? from[(size_t)(ch + 1) * e + col[c]] : 0.f);
+  };
+  auto store_pair = [&](float* to, int i, int c, uint64_t v) {
+    const int ch = CH(2 * i);
+    float lo, hi;
+    gla_unpack(v, lo, hi);
+    if (has_col[c] && ch < d) to[(size_t)ch * e + col[c]] = lo;
+    if (has_col[c] && ch + 1 < d) to[(size_t)(ch + 1) * e + col[c]] = hi;
+  };
 #pragma unroll
-    for (int i = 0; i < KP; ++i) s_reg[i] = (has_col && CH(i) < d) ? S[(size_t)(CH(i)) * e + col] : 0.f;
-    if (MODE == 1 && has_col) {
+  for (int c = 0; c < NC; ++c) {
+    if (MODE == 0 || (seg == 0 && (MODE == 1 || last))) {
+      // the request's state (MODE 2: only a sequence of one segment reads the slot, which it alone writes in this launch)
 #pragma unroll
-      for (int i = 0; i < KP; ++i)
-        if (CH(i) < d) seg_S0[(size_t)(CH(i)) * e + col] = s_reg[i];
-    }
-  } else if (MODE == 1) {
+      for (int i = 0; i < KP / 2; ++i) s_reg[c][i] = load_pair(S, i, c);
+      if (MODE == 1) {
 #pragma unroll
-    for (int i = 0; i < KP; ++i) s_reg[i] = 0.f;
-  } else if (seg == 0) {
+        for (int i = 0; i < KP / 2; ++i) store_pair(seg_S0, i, c, s_reg[c][i]);
+      }
+    } else if (MODE == 1) {
 #pragma unroll
-    for (int i = 0; i < KP; ++i) s_reg[i] = (has_col && CH(i) < d) ? seg_S0[(size_t)(CH(i)) * e + col] : 0.f;
-  } else {
-    // what the segments before left, folded in order (the first one's end state already holds the request's state)
-    const float* L = seg_state + (((size_t)b * segs) * H + h) * state_elems;
+      for (int i = 0; i < KP / 2; ++i) s_reg[c][i] = 0ull;  // +0.0 twice
+    } else if (seg == 0) {
 #pragma unroll
-    for (int i = 0; i < KP; ++i) s_reg[i] = (has_col && CH(i) < d) ? L[(size_t)(CH(i)) * e + col] : 0.f;
-    for (int j = 1; j < seg; ++j) {
-      L = seg_state + (((size_t)b * segs + j) * H + h) * state_elems;
-      const float* P = seg_decay + (((size_t)b * segs + j) * H + h) * d;
+      for (int i = 0; i < KP / 2; ++i) s_reg[c][i] = load_pair(seg_S0, i, c);
+    } else {
+      // what the segments before left, folded in order (the first one's end state already holds the request's state)
+      const float* L = seg_state + (((size_t)b * segs) * H + h) * state_elems;
 #pragma unroll
-      for (int i = 0; i < KP; ++i)
-        if (has_col && CH(i) < d) s_reg[i] = fmaf(P[CH(i)], s_reg[i], L[(size_t)(CH(i)) * e + col]);
+      for (int i = 0; i < KP / 2; ++i) s_reg[c][i] = load_pair(L, i, c);
+      for (int j = 1; j < seg; ++j) {
+        L = seg_state + (((size_t)b * segs + j) * H + h) * state_elems;
+        const float* P = seg_decay + (((size_t)b * segs + j) * H + h) * d;
+#pragma unroll
+        for (int i = 0; i < KP / 2; ++i) {
+          const int ch = CH(2 * i);
+          const uint64_t p2 = gla_pack(ch < d ? P[ch] : 0.f, ch + 1 < d ? P[ch + 1] : 0.f);
+          s_reg[c][i] = gla_fma2(p2, s_reg[c][i], load_pair(L, i, c));
+        }
+      }
     }
   }
   if (MODE == 1) {
 #pragma unroll
-    for (int i = 0; i < KP; ++i) p_reg[i] = 1.f;
+    for (int i = 0; i < KP / 2; ++i) p_reg[i] = gla_pack(1.f, 1.f);
   }
 
   const size_t qk_off = (size_t)(h / (H / groups)) * d, a_off = (size_t)h * d, v_off = (size_t)h * ev + col0;
   // what this thread fetches for a round: entries threadIdx.x + j * GLA_THREADS of the round's [tokens][dp] and [tokens][cols]
-  TA fq[GLA_PF], fk[GLA_PF], fv[GLA_PFV];
+  TA fq[GLA_PF], fk[GLA_PF], fv[PFV];
   float fa[GLA_PF], fb[GLA_PF];
   // Entry i of a round is channel i % dp of token i / dp (for v: column i % cols of token i / cols); a thread's
   // entries lie GLA_THREADS apart, so their places are found once, by steps, without a division per entry.
@@ -163,7 +208,7 @@ __global__ void __launch_bounds__(GLA_THREADS, GLA_MIN_BLOCKS) gla_scan_kernel(
     }
     tt = vfirst_t, c = vfirst_c;
 #pragma unroll
-    for (int j = 0; j < GLA_PFV; ++j) {
+    for (int j = 0; j < PFV; ++j) {
       fv[j] = gla_load(v + (size_t)(t0 + min(tt, nt - 1)) * ld_qkv + v_off + min(c, ev - 1 - col0));
       tt += vstep_t, c += vstep_c;
       if (c >= cols_per_cta) c -= cols_per_cta, ++tt;
@@ -186,7 +231,7 @@ __global__ void __launch_bounds__(GLA_THREADS, GLA_MIN_BLOCKS) gla_scan_kernel(
     }
     tt = vfirst_t, c = vfirst_c;
 #pragma unroll
-    for (int j = 0; j < GLA_PFV; ++j) {
+    for (int j = 0; j < PFV; ++j) {
       if (tt < nt) sv[tt * cols_per_cta + c] = (col0 + c < ev) ? ts_to_float(fv[j]) : (col0 + c < e ? 1.f : 0.f);
       tt += vstep_t, c += vstep_c;
       if (c >= cols_per_cta) c -= cols_per_cta, ++tt;
@@ -200,59 +245,76 @@ __global__ void __launch_bounds__(GLA_THREADS, GLA_MIN_BLOCKS) gla_scan_kernel(
     stage(t0);
     __syncthreads();
     if (t0 + tb < t_end) fetch(t0 + tb);  // in flight while this round's updates run
-#pragma unroll(KP > 16 ? 1 : GLA_UNROLL_TOKENS)  // several tokens' loads and shuffles in flight where the registers allow
+#pragma unroll(KP * NC > 16 ? 1 : GLA_UNROLL_TOKENS)  // several tokens' loads and shuffles in flight where the registers allow
     for (int tt = 0; tt < nt; ++tt) {
-      const float vv = sv[tt * cols_per_cta + cj];
-      // a thread's channels come in fours that start on 16-byte boundaries: 16-byte loads
-      const float4* pq = reinterpret_cast<const float4*>(sq + tt * dp) + r;
-      const float4* pk = reinterpret_cast<const float4*>(sk + tt * dp) + r;
-      const float4* pa = reinterpret_cast<const float4*>(sa + tt * dp) + r;
-      float acc[4] = {0.f, 0.f, 0.f, 0.f};  // four chains: the read-out is a sum of KP terms, its order is fixed by KP alone
+      uint64_t vv[NC];
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const float v1 = sv[tt * cols_per_cta + cj + c * lanes];
+        vv[c] = gla_pack(v1, v1);
+      }
+      // a thread's channels come in fours that start on 16-byte boundaries: 16-byte loads, two pairs each, shared by its columns
+      const ulonglong2* pq = reinterpret_cast<const ulonglong2*>(sq + tt * dp) + r;
+      const ulonglong2* pk = reinterpret_cast<const ulonglong2*>(sk + tt * dp) + r;
+      const ulonglong2* pa = reinterpret_cast<const ulonglong2*>(sa + tt * dp) + r;
+      uint64_t acc[NC][2];  // four chains: the read-out is a sum of KP terms, its order is fixed by KP alone
+#pragma unroll
+      for (int c = 0; c < NC; ++c) acc[c][0] = acc[c][1] = 0ull;
 #pragma unroll
       for (int i = 0; i < KP / 4; ++i) {
-        const float4 a4 = pa[i * R], k4 = pk[i * R];
-        s_reg[4 * i + 0] = fmaf(a4.x, s_reg[4 * i + 0], k4.x * vv);
-        s_reg[4 * i + 1] = fmaf(a4.y, s_reg[4 * i + 1], k4.y * vv);
-        s_reg[4 * i + 2] = fmaf(a4.z, s_reg[4 * i + 2], k4.z * vv);
-        s_reg[4 * i + 3] = fmaf(a4.w, s_reg[4 * i + 3], k4.w * vv);
+        const ulonglong2 a4 = pa[i * R], k4 = pk[i * R];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          s_reg[c][2 * i] = gla_fma2(a4.x, s_reg[c][2 * i], gla_mul2(k4.x, vv[c]));
+          s_reg[c][2 * i + 1] = gla_fma2(a4.y, s_reg[c][2 * i + 1], gla_mul2(k4.y, vv[c]));
+        }
         if (MODE == 1) {  // no read-outs yet: the product of the segment's decays instead
-          p_reg[(MODE == 1 ? 4 * i : 0) + 0] *= a4.x;
-          p_reg[(MODE == 1 ? 4 * i + 1 : 0)] *= a4.y;
-          p_reg[(MODE == 1 ? 4 * i + 2 : 0)] *= a4.z;
-          p_reg[(MODE == 1 ? 4 * i + 3 : 0)] *= a4.w;
+          p_reg[MODE == 1 ? 2 * i : 0] = gla_mul2(p_reg[MODE == 1 ? 2 * i : 0], a4.x);
+          p_reg[MODE == 1 ? 2 * i + 1 : 0] = gla_mul2(p_reg[MODE == 1 ? 2 * i + 1 : 0], a4.y);
         } else {
-          const float4 q4 = pq[i * R];
-          acc[0] = fmaf(s_reg[4 * i + 0], q4.x, acc[0]);
-          acc[1] = fmaf(s_reg[4 * i + 1], q4.y, acc[1]);
-          acc[2] = fmaf(s_reg[4 * i + 2], q4.z, acc[2]);
-          acc[3] = fmaf(s_reg[4 * i + 3], q4.w, acc[3]);
+          const ulonglong2 q4 = pq[i * R];
+#pragma unroll
+          for (int c = 0; c < NC; ++c) {
+            acc[c][0] = gla_fma2(s_reg[c][2 * i], q4.x, acc[c][0]);
+            acc[c][1] = gla_fma2(s_reg[c][2 * i + 1], q4.y, acc[c][1]);
+          }
         }
       }
       if (MODE != 1) {
-        float sum = (acc[0] + acc[1]) + (acc[2] + acc[3]);
-        for (int w = 1; w < R; w <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, w);
-        if (r == 0 && has_col) o[((size_t)(t0 + tt) * H + h) * e + col] = sum;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          float a0, a1, a2, a3;
+          gla_unpack(acc[c][0], a0, a1);
+          gla_unpack(acc[c][1], a2, a3);
+          float sum = (a0 + a1) + (a2 + a3);
+          for (int w = 1; w < R; w <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, w);
+          if (r == 0 && has_col[c]) o[((size_t)(t0 + tt) * H + h) * e + col[c]] = sum;
+        }
       }
     }
   }
   if (MODE == 1) {
-    if (has_col) {
 #pragma unroll
-      for (int i = 0; i < KP; ++i)
-        if (CH(i) < d) seg_L[(size_t)(CH(i)) * e + col] = s_reg[i];
-    }
+    for (int c = 0; c < NC; ++c)
+#pragma unroll
+      for (int i = 0; i < KP / 2; ++i) store_pair(seg_L, i, c, s_reg[c][i]);
     if (blockIdx.z == 0 && cj == 0) {  // the decays do not depend on the column: one thread per group of channels writes them
 #pragma unroll
-      for (int i = 0; i < KP; ++i)
-        if (CH(i) < d) seg_P[CH(i)] = p_reg[MODE == 1 ? i : 0];
+      for (int i = 0; i < KP / 2; ++i) {
+        const int ch = CH(2 * i);
+        float lo, hi;
+        gla_unpack(p_reg[MODE == 1 ? i : 0], lo, hi);
+        if (ch < d) seg_P[ch] = lo;
+        if (ch + 1 < d) seg_P[ch + 1] = hi;
+      }
     }
-  } else if (has_col && (MODE == 0 || last)) {
+  } else if (MODE == 0 || last) {
 #pragma unroll
-    for (int i = 0; i < KP; ++i)
-      if (CH(i) < d) S[(size_t)(CH(i)) * e + col] = s_reg[i];
+    for (int c = 0; c < NC; ++c)
+#pragma unroll
+      for (int i = 0; i < KP / 2; ++i) store_pair(S, i, c, s_reg[c][i]);
   }
 }
-
 
 // A step in which every sequence brings one token at most (decode): nothing is staged, no barrier is met.  One CTA per
 // (sequence, head, block of value columns) as above; a thread reads the token's q, k and decay entries of its own
@@ -310,24 +372,43 @@ struct GlaExtra {
   long long slot_stride;  // floats from one request's state to the next
 };
 
-template <typename TA, int KP, int MODE>
+template <typename TA, int KP, int MODE, int NC>
 static int launch_gla_scan(const void* q, const void* k, const void* v, long long ld_qkv, const float* decay, float q_scale, float* state,
                            const int* state_slots, const int* cu_seqlens, float* o, int B, int H, int d, int e, int R, int segs, int seg_len,
                            float* scratch, cudaStream_t s, const GlaExtra& x) {
-  const int cols = GLA_THREADS / R, dp = R * KP;
+  const int cols = NC * GLA_THREADS / R, dp = R * KP;
   // tokens per round: what the threads' fetch registers hold, at most GLA_TB
-  const int tb = min(GLA_TB, min(GLA_THREADS * GLA_PF / dp, GLA_THREADS * GLA_PFV / cols));
+  const int tb = min(GLA_TB, min(GLA_THREADS * GLA_PF / dp, GLA_THREADS * GLA_PFV * NC / cols));
   if (tb < 1) return TS_ERR_UNSUPPORTED_SIZE;
-  const size_t smem = (size_t)tb * (3 * dp + cols) * sizeof(float);  // at most 16 * (3 * 64 + 128) or 1 * (3 * 1024 + 4) floats: below 48 KB
+  const size_t smem = (size_t)tb * (3 * dp + cols) * sizeof(float);  // at most 16 * (3 * 64 + 256) or 1 * (3 * 1024 + 8) floats: below 48 KB
   const dim3 grid(B * segs, H, (e + cols - 1) / cols);
   if (grid.y > 65535 || grid.z > 65535) return TS_ERR_UNSUPPORTED_SIZE;
   // scratch of the segmented scan: end states [B, segs, H, d, e], decay products [B, segs, H, d], start states [B, H, d, e]
   float* seg_state = scratch;
   float* seg_decay = scratch ? seg_state + (size_t)B * segs * H * d * e : nullptr;
   float* seg_start = scratch ? seg_decay + (size_t)B * segs * H * d : nullptr;
-  return ts_launch(gla_scan_kernel<TA, KP, MODE>, grid, dim3(GLA_THREADS), smem, s, (const TA*)q, (const TA*)k, (const TA*)v, ld_qkv, decay,
+  return ts_launch(gla_scan_kernel<TA, KP, MODE, NC>, grid, dim3(GLA_THREADS), smem, s, (const TA*)q, (const TA*)k, (const TA*)v, ld_qkv, decay,
                    q_scale, state, state_slots, cu_seqlens, o, H, d, e, R, cols, tb, segs, seg_len, seg_state, seg_decay, seg_start, x.kscale,
                    x.decay_scalar, x.groups, x.ev, x.slot_stride);
+}
+
+// Whether a thread takes two columns: its loads of q, k and the decay from shared memory then serve both.  Not where the grid
+// would no longer fill the SMs, nor where the state of two columns does not fit the registers.
+template <int KP>
+static bool two_columns(int B, int segs, int H, int e, int R) {
+  const long long cols = 2 * GLA_THREADS / R;
+  return KP <= 16 && e > GLA_THREADS / R && (long long)B * segs * H * ((e + cols - 1) / cols) >= GLA_TWO_COLUMNS_CTAS;
+}
+
+template <typename TA, int KP, int MODE>
+static int launch_gla_scan_columns(const void* q, const void* k, const void* v, long long ld_qkv, const float* decay, float q_scale, float* state,
+                                   const int* state_slots, const int* cu_seqlens, float* o, int B, int H, int d, int e, int R, int segs,
+                                   int seg_len, float* scratch, cudaStream_t s, const GlaExtra& x) {
+  if constexpr (KP <= 16)
+    if (two_columns<KP>(B, segs, H, e, R))
+      return launch_gla_scan<TA, KP, MODE, 2>(q, k, v, ld_qkv, decay, q_scale, state, state_slots, cu_seqlens, o, B, H, d, e, R, segs, seg_len,
+                                              scratch, s, x);
+  return launch_gla_scan<TA, KP, MODE, 1>(q, k, v, ld_qkv, decay, q_scale, state, state_slots, cu_seqlens, o, B, H, d, e, R, segs, seg_len, scratch, s, x);
 }
 
 template <typename TA, int KP>
@@ -335,11 +416,11 @@ static int launch_gla_scan_modes(const void* q, const void* k, const void* v, lo
                                  const int* state_slots, const int* cu_seqlens, float* o, int B, int H, int d, int e, int R, int segs,
                                  int seg_len, float* scratch, cudaStream_t s, const GlaExtra& x) {
   if (segs <= 1)
-    return launch_gla_scan<TA, KP, 0>(q, k, v, ld_qkv, decay, q_scale, state, state_slots, cu_seqlens, o, B, H, d, e, R, 1, 0, nullptr, s, x);
-  const int st = launch_gla_scan<TA, KP, 1>(q, k, v, ld_qkv, decay, q_scale, state, state_slots, cu_seqlens, o, B, H, d, e, R, segs, seg_len,
+    return launch_gla_scan_columns<TA, KP, 0>(q, k, v, ld_qkv, decay, q_scale, state, state_slots, cu_seqlens, o, B, H, d, e, R, 1, 0, nullptr, s, x);
+  const int st = launch_gla_scan_columns<TA, KP, 1>(q, k, v, ld_qkv, decay, q_scale, state, state_slots, cu_seqlens, o, B, H, d, e, R, segs, seg_len,
                                             scratch, s, x);
   if (st != 0) return st;
-  return launch_gla_scan<TA, KP, 2>(q, k, v, ld_qkv, decay, q_scale, state, state_slots, cu_seqlens, o, B, H, d, e, R, segs, seg_len, scratch, s, x);
+  return launch_gla_scan_columns<TA, KP, 2>(q, k, v, ld_qkv, decay, q_scale, state, state_slots, cu_seqlens, o, B, H, d, e, R, segs, seg_len, scratch, s, x);
 }
 
 template <typename TA>
