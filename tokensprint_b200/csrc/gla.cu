@@ -60,21 +60,26 @@ __device__ __forceinline__ __nv_bfloat16 gla_load(const __nv_bfloat16* p) {
   return __ushort_as_bfloat16(v);
 }
 
-// two float32 in one 64-bit register, and the packed arithmetic on them (each half rounds as the scalar operation does)
-__device__ __forceinline__ uint64_t gla_pack(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+// Two float32 at a time: by the packed instructions, or one after the other (each half rounds alike).  The pass in one piece takes
+// the scalar ones: pairs of registers cost it spills (50 decoded tokens beside a prompt of 944: the step 2.08 ms packed, 2.05 scalar).
+template <bool PACKED>
+__device__ __forceinline__ float2 gla_fma2(float2 a, float2 b, float2 c) {
+  if (!PACKED) return make_float2(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y));
+  float2 r;
+  asm("{\n\t.reg .b64 a, b, c;\n\t"
+      "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+      "fma.rn.f32x2 c, a, b, c;\n\tmov.b64 {%0, %1}, c;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
   return r;
 }
-__device__ __forceinline__ void gla_unpack(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ uint64_t gla_fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t gla_mul2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+template <bool PACKED>
+__device__ __forceinline__ float2 gla_mul2(float2 a, float2 b) {
+  if (!PACKED) return make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
+  float2 r;
+  asm("{\n\t.reg .b64 a, b;\n\t"
+      "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+      "mul.rn.f32x2 a, a, b;\n\tmov.b64 {%0, %1}, a;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return r;
 }
 
@@ -128,19 +133,18 @@ __global__ void __launch_bounds__(GLA_THREADS, NC == 2 ? 3 : GLA_MIN_BLOCKS) gla
   float* seg_L = MODE == 0 ? nullptr : seg_state + (((size_t)b * segs + seg) * H + h) * state_elems;   // this segment's end state
   float* seg_P = MODE == 0 ? nullptr : seg_decay + (((size_t)b * segs + seg) * H + h) * d;             // this segment's decay product
   float* seg_S0 = MODE == 0 ? nullptr : seg_start + ((size_t)b * H + h) * state_elems;                 // the request's state as the step found it
-  // pairs of neighbouring channels (CH(2 i), CH(2 i) + 1) of a column in one 64-bit register
-  uint64_t s_reg[NC][KP / 2];
-  uint64_t p_reg[MODE == 1 ? KP / 2 : 1];
+  constexpr bool PACKED = MODE != 0;
+  // pairs of neighbouring channels, CH(2 i) and CH(2 i) + 1, of a column
+  float2 s_reg[NC][KP / 2];
+  float2 p_reg[MODE == 1 ? KP / 2 : 1];
   auto load_pair = [&](const float* from, int i, int c) {
     const int ch = CH(2 * i);
-    return gla_pack((has_col[c] && ch < d) ? from[(size_t)ch * e + col[c]] : 0.f, (has_col[c] && ch + 1 < d) ? from[(size_t)(ch + 1) * e + col[c]] : 0.f);
+    return make_float2((has_col[c] && ch < d) ? from[(size_t)ch * e + col[c]] : 0.f, (has_col[c] && ch + 1 < d) ? from[(size_t)(ch + 1) * e + col[c]] : 0.f);
   };
-  auto store_pair = [&](float* to, int i, int c, uint64_t v) {
+  auto store_pair = [&](float* to, int i, int c, float2 v) {
     const int ch = CH(2 * i);
-    float lo, hi;
-    gla_unpack(v, lo, hi);
-    if (has_col[c] && ch < d) to[(size_t)ch * e + col[c]] = lo;
-    if (has_col[c] && ch + 1 < d) to[(size_t)(ch + 1) * e + col[c]] = hi;
+    if (has_col[c] && ch < d) to[(size_t)ch * e + col[c]] = v.x;
+    if (has_col[c] && ch + 1 < d) to[(size_t)(ch + 1) * e + col[c]] = v.y;
   };
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
@@ -154,7 +158,7 @@ __global__ void __launch_bounds__(GLA_THREADS, NC == 2 ? 3 : GLA_MIN_BLOCKS) gla
       }
     } else if (MODE == 1) {
 #pragma unroll
-      for (int i = 0; i < KP / 2; ++i) s_reg[c][i] = 0ull;  // +0.0 twice
+      for (int i = 0; i < KP / 2; ++i) s_reg[c][i] = make_float2(0.f, 0.f);
     } else if (seg == 0) {
 #pragma unroll
       for (int i = 0; i < KP / 2; ++i) s_reg[c][i] = load_pair(seg_S0, i, c);
@@ -169,15 +173,15 @@ __global__ void __launch_bounds__(GLA_THREADS, NC == 2 ? 3 : GLA_MIN_BLOCKS) gla
 #pragma unroll
         for (int i = 0; i < KP / 2; ++i) {
           const int ch = CH(2 * i);
-          const uint64_t p2 = gla_pack(ch < d ? P[ch] : 0.f, ch + 1 < d ? P[ch + 1] : 0.f);
-          s_reg[c][i] = gla_fma2(p2, s_reg[c][i], load_pair(L, i, c));
+          const float2 p2 = make_float2(ch < d ? P[ch] : 0.f, ch + 1 < d ? P[ch + 1] : 0.f);
+          s_reg[c][i] = gla_fma2<PACKED>(p2, s_reg[c][i], load_pair(L, i, c));
         }
       }
     }
   }
   if (MODE == 1) {
 #pragma unroll
-    for (int i = 0; i < KP / 2; ++i) p_reg[i] = gla_pack(1.f, 1.f);
+    for (int i = 0; i < KP / 2; ++i) p_reg[i] = make_float2(1.f, 1.f);
   }
 
   const size_t qk_off = (size_t)(h / (H / groups)) * d, a_off = (size_t)h * d, v_off = (size_t)h * ev + col0;
@@ -247,46 +251,43 @@ __global__ void __launch_bounds__(GLA_THREADS, NC == 2 ? 3 : GLA_MIN_BLOCKS) gla
     if (t0 + tb < t_end) fetch(t0 + tb);  // in flight while this round's updates run
 #pragma unroll(KP * NC > 16 ? 1 : GLA_UNROLL_TOKENS)  // several tokens' loads and shuffles in flight where the registers allow
     for (int tt = 0; tt < nt; ++tt) {
-      uint64_t vv[NC];
+      float2 vv[NC];
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
         const float v1 = sv[tt * cols_per_cta + cj + c * lanes];
-        vv[c] = gla_pack(v1, v1);
+        vv[c] = make_float2(v1, v1);
       }
       // a thread's channels come in fours that start on 16-byte boundaries: 16-byte loads, two pairs each, shared by its columns
-      const ulonglong2* pq = reinterpret_cast<const ulonglong2*>(sq + tt * dp) + r;
-      const ulonglong2* pk = reinterpret_cast<const ulonglong2*>(sk + tt * dp) + r;
-      const ulonglong2* pa = reinterpret_cast<const ulonglong2*>(sa + tt * dp) + r;
-      uint64_t acc[NC][2];  // four chains: the read-out is a sum of KP terms, its order is fixed by KP alone
+      const float4* pq = reinterpret_cast<const float4*>(sq + tt * dp) + r;
+      const float4* pk = reinterpret_cast<const float4*>(sk + tt * dp) + r;
+      const float4* pa = reinterpret_cast<const float4*>(sa + tt * dp) + r;
+      float2 acc[NC][2];  // four chains: the read-out is a sum of KP terms, its order is fixed by KP alone
 #pragma unroll
-      for (int c = 0; c < NC; ++c) acc[c][0] = acc[c][1] = 0ull;
+      for (int c = 0; c < NC; ++c) acc[c][0] = acc[c][1] = make_float2(0.f, 0.f);
 #pragma unroll
       for (int i = 0; i < KP / 4; ++i) {
-        const ulonglong2 a4 = pa[i * R], k4 = pk[i * R];
+        const float4 a4 = pa[i * R], k4 = pk[i * R];
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-          s_reg[c][2 * i] = gla_fma2(a4.x, s_reg[c][2 * i], gla_mul2(k4.x, vv[c]));
-          s_reg[c][2 * i + 1] = gla_fma2(a4.y, s_reg[c][2 * i + 1], gla_mul2(k4.y, vv[c]));
+          s_reg[c][2 * i] = gla_fma2<PACKED>(make_float2(a4.x, a4.y), s_reg[c][2 * i], gla_mul2<PACKED>(make_float2(k4.x, k4.y), vv[c]));
+          s_reg[c][2 * i + 1] = gla_fma2<PACKED>(make_float2(a4.z, a4.w), s_reg[c][2 * i + 1], gla_mul2<PACKED>(make_float2(k4.z, k4.w), vv[c]));
         }
         if (MODE == 1) {  // no read-outs yet: the product of the segment's decays instead
-          p_reg[MODE == 1 ? 2 * i : 0] = gla_mul2(p_reg[MODE == 1 ? 2 * i : 0], a4.x);
-          p_reg[MODE == 1 ? 2 * i + 1 : 0] = gla_mul2(p_reg[MODE == 1 ? 2 * i + 1 : 0], a4.y);
+          p_reg[MODE == 1 ? 2 * i : 0] = gla_mul2<PACKED>(p_reg[MODE == 1 ? 2 * i : 0], make_float2(a4.x, a4.y));
+          p_reg[MODE == 1 ? 2 * i + 1 : 0] = gla_mul2<PACKED>(p_reg[MODE == 1 ? 2 * i + 1 : 0], make_float2(a4.z, a4.w));
         } else {
-          const ulonglong2 q4 = pq[i * R];
+          const float4 q4 = pq[i * R];
 #pragma unroll
           for (int c = 0; c < NC; ++c) {
-            acc[c][0] = gla_fma2(s_reg[c][2 * i], q4.x, acc[c][0]);
-            acc[c][1] = gla_fma2(s_reg[c][2 * i + 1], q4.y, acc[c][1]);
+            acc[c][0] = gla_fma2<PACKED>(s_reg[c][2 * i], make_float2(q4.x, q4.y), acc[c][0]);
+            acc[c][1] = gla_fma2<PACKED>(s_reg[c][2 * i + 1], make_float2(q4.z, q4.w), acc[c][1]);
           }
         }
       }
       if (MODE != 1) {
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-          float a0, a1, a2, a3;
-          gla_unpack(acc[c][0], a0, a1);
-          gla_unpack(acc[c][1], a2, a3);
-          float sum = (a0 + a1) + (a2 + a3);
+          float sum = (acc[c][0].x + acc[c][0].y) + (acc[c][1].x + acc[c][1].y);
           for (int w = 1; w < R; w <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, w);
           if (r == 0 && has_col[c]) o[((size_t)(t0 + tt) * H + h) * e + col[c]] = sum;
         }
@@ -302,10 +303,9 @@ __global__ void __launch_bounds__(GLA_THREADS, NC == 2 ? 3 : GLA_MIN_BLOCKS) gla
 #pragma unroll
       for (int i = 0; i < KP / 2; ++i) {
         const int ch = CH(2 * i);
-        float lo, hi;
-        gla_unpack(p_reg[MODE == 1 ? i : 0], lo, hi);
-        if (ch < d) seg_P[ch] = lo;
-        if (ch + 1 < d) seg_P[ch + 1] = hi;
+        const float2 p2 = p_reg[MODE == 1 ? i : 0];
+        if (ch < d) seg_P[ch] = p2.x;
+        if (ch + 1 < d) seg_P[ch + 1] = p2.y;
       }
     }
   } else if (MODE == 0 || last) {
@@ -393,7 +393,9 @@ static int launch_gla_scan(const void* q, const void* k, const void* v, long lon
 }
 
 // Whether a thread takes two columns: its loads of q, k and the decay from shared memory then serve both.  Not where the grid
-// would no longer fill the SMs, nor where the state of two columns does not fit the registers.
+// would no longer fill the SMs, nor where the state of two columns does not fit the registers, nor in one piece: the longest portion's chain of
+// tokens then sets the time, and it is longer with two (64 heads of 128 x 64, 50 decoded tokens beside a prompt of 944: the
+// step 2.37 ms against 2.05).  Passes over 16 segments of 64 tokens of the same heads, without and with read-outs: 235 -> 131 and 487 -> 471 us.
 template <int KP>
 static bool two_columns(int B, int segs, int H, int e, int R) {
   const long long cols = 2 * GLA_THREADS / R;
@@ -404,7 +406,7 @@ template <typename TA, int KP, int MODE>
 static int launch_gla_scan_columns(const void* q, const void* k, const void* v, long long ld_qkv, const float* decay, float q_scale, float* state,
                                    const int* state_slots, const int* cu_seqlens, float* o, int B, int H, int d, int e, int R, int segs,
                                    int seg_len, float* scratch, cudaStream_t s, const GlaExtra& x) {
-  if constexpr (KP <= 16)
+  if constexpr (KP <= 16 && MODE != 0)
     if (two_columns<KP>(B, segs, H, e, R))
       return launch_gla_scan<TA, KP, MODE, 2>(q, k, v, ld_qkv, decay, q_scale, state, state_slots, cu_seqlens, o, B, H, d, e, R, segs, seg_len,
                                               scratch, s, x);
