@@ -30,7 +30,7 @@
 // The pair's routing weight multiplies the float32 sums, not the rounded input: (w x) . g = w (x . g) without
 // a second rounding of x.  Every output element is one chain of sums over k in a fixed order.
 // Every wait is on an mbarrier fed by this CTA's own copies, MMAs and warps, bounded; one that gives up raises the
-// error word, and the CTA lets its copies land, frees its tensor memory and returns.
+// error word, and the CTA lets its copies land and its products end, frees its tensor memory and returns.
 #include <cuda.h>
 #include <math.h>
 
@@ -226,6 +226,18 @@ __device__ __forceinline__ void let_land(Common<STAGES>& c, int asked) {
   for (int i = max(0, asked - STAGES); i < asked; ++i) mbar_wait(smem_u32(&c.full[i % STAGES]), (uint32_t)(i / STAGES) & 1, &patience);
 }
 
+// Everything this CTA asked of the tensor core is done when the commit arrives.  The warp that asked waits for it, on a count
+// of its own: leave()'s barrier then holds everybody until no product writes tensor memory and no commit has yet to
+// arrive, also where a wait gave up before.
+template <int STAGES>
+__device__ __forceinline__ void let_finish(Common<STAGES>& c) {
+  if (elect_one()) umma_commit(smem_u32(&c.all_done));
+  __syncwarp();
+  int patience = 0;
+  mbar_wait(smem_u32(&c.all_done), 0, &patience);
+  if (patience != 0) c.abort = 1;
+}
+
 // ---- many rows ----
 
 constexpr int TN = 256;
@@ -348,9 +360,7 @@ __global__ void __launch_bounds__(many_threads(MODE), 1) moe_many_kernel(const _
         __syncwarp();
       }
     }
-    // everything this CTA asked of the tensor core is done when this arrives: nobody leaves before
-    if (elect_one()) umma_commit(smem_u32(&c.all_done));
-    __syncwarp();
+    let_finish(c);
   } else {
     // warps 0-3 have the first half of the columns, the last four the second; a warp reaches the 32 lanes of tensor memory
     // of its number modulo 4
@@ -393,7 +403,6 @@ __global__ void __launch_bounds__(many_threads(MODE), 1) moe_many_kernel(const _
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&c.acc_empty[acc]));
     }
-    mbar_wait(smem_u32(&c.all_done), 0, abort_flag);
   }
   leave(c, a, MANY_TMEM);
 }
@@ -488,8 +497,7 @@ __global__ void __launch_bounds__(224, 1) moe_few_kernel(const __grid_constant__
         __syncwarp();
       }
     }
-    if (elect_one()) umma_commit(smem_u32(&c.all_done));  // nobody leaves before this has arrived (see the other kernel)
-    __syncwarp();
+    let_finish(c);
   } else if (warp < 4) {
     int turn = 0;
     for (int it = blockIdx.x; it < items; it += gridDim.x, ++turn) {
@@ -533,7 +541,6 @@ __global__ void __launch_bounds__(224, 1) moe_few_kernel(const __grid_constant__
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&c.acc_empty[acc]));
     }
-    mbar_wait(smem_u32(&c.all_done), 0, abort_flag);
   }
   leave(c, a, F::TMEM_COLS);
 }

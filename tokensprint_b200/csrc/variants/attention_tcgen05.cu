@@ -955,9 +955,14 @@ __global__ void __launch_bounds__(608, 1) attention_tcgen05_pair_kernel(const __
     }
     // Everything this CTA asked of the tensor core is done when this arrives, the arrivals of
     // the commits above included: nobody leaves before (an arrival after the CTA's end would
-    // land in the barriers of the next CTA on this SM).
+    // land in the barriers of the next CTA on this SM).  Where a wait gave up the others look at this
+    // barrier once only: this warp waits for it, on a count of its own, and they wait for this warp
+    // at the barrier ahead of the end.
     if (elect_one()) umma_commit(smem_u32(&all_done));
     __syncwarp();
+    int patience = 0;
+    mbar_wait(smem_u32(&all_done), 0, &patience);
+    if (patience != 0) *abort_flag = 1;
   } else if (warp < 8 * ntiles) {
     // ---------------- softmax: two threads per row, 64 of a block's 128 keys each ----------------
     // Warps 8 t .. 8 t + 7 belong to tile t; warp 8 t + 4 h + quad takes keys 64 h .. 64 h + 63 of
