@@ -292,6 +292,53 @@ def test_latent_portions_with_rebuilt_keys(H, rank, page, window, sinks, gated, 
         at += kept[b]
 
 
+def _rebuilt_one_head(keys, values, scale, gates=None):
+    """latent_rebuilt_attention of a whole prompt of len(keys) tokens, one head; every query is the first unit vector."""
+    from tokensprint_b200 import ops
+
+    n = keys.shape[0]
+    q = torch.zeros(n, 192)
+    q[:, 0] = 1.0
+    rows, out = torch.zeros(n, 128, device="cuda", dtype=torch.bfloat16), torch.empty(n, 1, 128, device="cuda", dtype=torch.bfloat16)
+    q = _dev(q, torch.bfloat16)
+    ops.latent_rebuilt_attention(q, q[:, 128:].contiguous(), _dev(torch.cat([keys, values], 1), torch.bfloat16), rows, out, gates, _i32([0, n]),
+                                 _i32([n]), 1, n, 1, 64, scale)
+    ops.check_device_errors()
+    return out[:, 0].double().cpu()
+
+
+@pytest.mark.parametrize("mantissa", [0, 3, 17, 40, 64, 71, 97, 110, 127])
+@pytest.mark.parametrize("side", [2e-5, -2e-5])
+def test_latent_rebuilt_weights_are_rounded_exponentials(mantissa, side):
+    """Key 0 scores `scale`, all others 0, and exp(-scale) lies 2e-5 above or below the middle of two bfloat16
+    numbers: every weight must round to the right one of them, wherever in a block its key stands.  Value entry c is 1 for the
+    keys c modulo 8.  A wrong unit is at least 2^-8 of a weight and moves its columns by 7/8 of that; the results' own rounding, up
+    to 2^-8 either way with a deviation of 1.6e-3, averages out over the rows (1.2e-4 for 190 of them; five times that is 6e-4)."""
+    n = 200
+    middle = (1 + (mantissa + 0.5) / 128) / 2 * (1 + side)
+    w = float(torch.tensor(middle, dtype=torch.float64).to(torch.bfloat16))
+    keys, values = torch.zeros(n, 128), torch.zeros(n, 128)
+    keys[0, 0] = 1.0
+    for j in range(1, n):
+        values[j, j % 8] = 1.0
+    out = _rebuilt_one_head(keys, values, -math.log(middle))
+    count = values[:, :8].double().cumsum(0)
+    want = count * w / (1.0 + torch.arange(n).double()[:, None] * w)
+    assert float(((out[8:, :8] - want[8:]) / want[8:]).mean(0).abs().max()) < 1e-3
+
+
+def test_latent_rebuilt_weights_add_up_to_one():
+    """All values alike: the result is that value, whatever the weights were rounded to, up to float32 sums (200 terms, 2e-5).
+    The gates bring the product within 1e-4 of the middle of two bfloat16 numbers, so a bias of the sum would show."""
+    n = 200
+    keys, values = torch.randn(n, 128, generator=torch.Generator().manual_seed(3)) * 3.0, torch.full((n, 128), 1.5)
+    keys[0, 0] = 4.0
+    for side in (1e-4, -1e-4):
+        gate = torch.full((n, 1), (1.0 + 1.0 / 256) * (1.0 + side) / 1.5)
+        out = _rebuilt_one_head(keys, values, 1.0, _dev(gate))
+        assert torch.equal(out, torch.full_like(out, 1.0 + (1.0 / 128 if side > 0 else 0.0)))
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("tag, layer", [("a", 0), ("b", 0), ("b", 1), ("c", 1)])
 def test_latent_mixer_whole_prompt(dtype, tag, layer):

@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(128, 2) attention_tcgen05_kernel(const __grid_
 // begins at the same keys wherever a prompt was cut.  Q takes 3 x 16 KB per tile and K three
 // boxes a block: with blocks of 128 keys only one stage of V would fit the SM's shared memory, and V would be
 // asked for when its place is free, half a block before it is needed; blocks of 96 leave room for both rings of two.
-// Measured (16 heads, 8,191 tokens, window 4,096): 288 us a layer, 0.90 PFLOP/s of the 320 multiply-adds per (query, key,
+// Measured (16 heads, 8,191 tokens, window 4,096): 294 us a layer, 0.88 PFLOP/s of the 320 multiply-adds per (query, key,
 // head); latent_attention_mma.cu, on the cached rows themselves (1,088 multiply-adds, mma.sync), took 5,150.
 
 constexpr bool REBUILT = TS_ATT_ROT != 0;
@@ -604,6 +604,7 @@ constexpr float RESCALE_THRESHOLD = 8.f;
 #ifndef TS_ATT_FMA_PAIRS
 #define TS_ATT_FMA_PAIRS 1
 #endif
+constexpr int FMA_PAIRS = REBUILT ? 0 : TS_ATT_FMA_PAIRS;
 
 // two float32 in one 64-bit register, and the packed arithmetic on them
 __device__ __forceinline__ uint64_t pack2(float lo, float hi) {
@@ -1083,6 +1084,9 @@ __global__ void __launch_bounds__(608, 1) attention_tcgen05_pair_kernel(const __
       // Weights p = 2^(s * scale - m * scale), two at a time.  The special-function unit does 16
       // exponentials a clock per SM; one pair in four is computed on the FMA pipe instead
       // (exp2_pair_fma).  (Measured at 8,192 tokens: none 543 us, one 524, two 525, three 566.)
+      // REBUILT: none, and the row's sum runs over the rounded weights, the ones that the value product uses, as in
+      // latent_attention_mma.cu, which takes the steps that are not rebuilt (16 heads, 8,191 tokens: 284 us with one
+      // and the unrounded sum, 288 with none, 294 as it is; where few weights count the distance from float64 falls by 3 %).
       uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull};  // four chains of two float32 sums each (0 is +0.0 twice)
       const uint64_t scale2 = pack2(p.scale_log2, p.scale_log2), off2 = pack2(-m_off, -m_off);
       // Second walk, PIECE scores at a time.  P goes over the first half of the scores it came from
@@ -1106,15 +1110,17 @@ __global__ void __launch_bounds__(608, 1) attention_tcgen05_pair_kernel(const __
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             float p0, p1;
-            if (i < TS_ATT_FMA_PAIRS) {
+            if (i < FMA_PAIRS) {
               const uint64_t x = fma2(pack2(__uint_as_float(v[j + 2 * i]), __uint_as_float(v[j + 2 * i + 1])), scale2, off2);
               exp2_pair_fma(x, p0, p1);
             } else {
               p0 = fast_exp2(fmaf(__uint_as_float(v[j + 2 * i]), p.scale_log2, -m_off));
               p1 = fast_exp2(fmaf(__uint_as_float(v[j + 2 * i + 1]), p.scale_log2, -m_off));
             }
+            const uint32_t both = pack_bf16(p0, p1);
+            packed[(j >> 1) + i] = both;
+            if (REBUILT) p0 = __uint_as_float(both << 16), p1 = __uint_as_float(both & 0xffff0000u);
             sum2[i] = add2(sum2[i], pack2(p0, p1));
-            packed[(j >> 1) + i] = pack_bf16(p0, p1);
           }
         }
         tmem_st(s_addr + g * (PIECE / 2), packed);
