@@ -517,3 +517,32 @@ def test_router_logits_do_not_depend_on_the_kernel(dtype, T, W, E):
     z = x.double() @ r.double().T + bias.double()
     assert float((w.double() - torch.sigmoid(z.gather(1, ids.long()))).abs().max()) < 1e-5
     assert float((torch.topk(z, top).values - z.gather(1, ids.long())).abs().max()) < 1e-5
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("T, W, E, groups", [
+    (600, 136, 33, None), (1184, 64, 17, None), (1185, 64, 17, (17, 2)), (2368, 136, 16, None), (2369, 136, 40, (8, 3)), (2500, 72, 16, (4, 2)),
+    # the logits of 16 tokens beside six slabs: up to 824 float32 entries (experts and groups), 1,208 of bfloat16 rows; four slabs
+    # up to 1,616; beyond that the kernel without tiles
+    (1185, 64, 824, None), (1185, 64, 825, None), (2368, 64, 1024, None), (2368, 64, 1024, (256, 200)), (1200, 64, 1024, (1024, 900)), (2400, 64, 1024, None),
+])
+def test_router_takes_every_number_of_experts(dtype, T, W, E, groups):
+    """Every tile and ring that the sizes choose gives a token the choice and, bit by bit, the weights of the token alone (the kernel
+    with a CTA a token), with expert groups and a correction too; the logits behind the weights are those of float64."""
+    from tokensprint_b200 import ops
+
+    g = torch.Generator().manual_seed(T + E)
+    x, r = torch.randn(T, W, generator=g).to(dtype).cuda(), (torch.randn(E, W, generator=g) / W ** 0.5).cuda()
+    correction = 0.1 * torch.randn(E, generator=g).cuda()
+    top = min(E, 6)
+    if groups is not None:
+        top = min(top, groups[1] * (E // groups[0]))
+    ids, w = torch.full((T, top), -1, dtype=torch.int32, device="cuda"), torch.full((T, top), float("nan"), device="cuda")
+    ops.router(x, r, top, False, ids, w, score="softmax_all", correction=correction, groups=groups)
+    for t in sorted({0, 7, 8, 15, 16, T // 2, T - 9, T - 1}):
+        one_id, one_w = torch.empty(1, top, dtype=torch.int32, device="cuda"), torch.empty(1, top, device="cuda")
+        ops.router(x[t:t + 1].clone(), r, top, False, one_id, one_w, score="softmax_all", correction=correction, groups=groups)
+        assert torch.equal(one_id[0], ids[t]) and torch.equal(one_w[0], w[t])
+    assert int(ids.min()) >= 0 and int(ids.max()) < E
+    z = x.double() @ r.double().T
+    assert float((w.double() - torch.softmax(z, 1).gather(1, ids.long())).abs().max()) < 1e-5

@@ -625,13 +625,17 @@ static int launch_router_few(const void* x, const float* router, const float* bi
   return ts_launch(router_few_kernel<TX>, dim3(T), dim3(32 * min(E, 32)), (size_t)(E + groups.count) * sizeof(float), s, (const TX*)x, router, bias, W, E,
                    top, renormalize, score_mode, ids, weights, correction, groups);
 }
+// `taken` says whether the shared memory has room for the slabs and the logits of a tile's tokens.
+constexpr size_t ROUTER_TILE_SMEM = 200 * 1024;
 template <typename TX, int TT, int EX, int NS>
 static int launch_router_tile(const void* x, const float* router, const float* bias, int T, int W, int E, int top, int renormalize, int score_mode, int* ids,
-                              float* weights, const float* correction, const RouterGroups& groups, cudaStream_t s) {
+                              float* weights, const float* correction, const RouterGroups& groups, cudaStream_t s, bool& taken) {
   const size_t smem = rt_ring_bytes<TX, TT, EX, NS>() + (size_t)TT * (E + groups.count) * sizeof(float);
+  taken = smem <= ROUTER_TILE_SMEM;
+  if (!taken) return 0;
   static bool configured = false;
   if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(router_tile_kernel<TX, TT, EX, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    const cudaError_t e = cudaFuncSetAttribute(router_tile_kernel<TX, TT, EX, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ROUTER_TILE_SMEM);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
@@ -644,7 +648,8 @@ struct Const {
 };
 #define ROUTER_FEW_TOKENS 296
 // Which kernel (the logits are the same): a CTA a token up to two tokens per SM, then tiles of 8 tokens, of 16 beyond 8 per SM,
-// with six slabs in the ring while a CTA has its SM to itself and four, two CTAs an SM, beyond that.  Rows that are no whole pieces, misaligned bases and more experts than shared memory has room for: router_kernel.
+// with six slabs in the ring while a CTA has its SM to itself (where that leaves room for the logits: 824 float32 experts) and four, two CTAs an SM, beyond
+// that.  Rows that are no whole pieces, misaligned bases and more experts than shared memory has room for: router_kernel.
 // Measured, bfloat16 rows, us, router_kernel / these: 16 experts of 2,048: 64 tokens 7.7 / 4.8, 512 13.5 / 10.5, 2,048 20.3 / 21.9,
 // 8,192 72 / 40; 32 experts of 4,096: 64 tokens 20.3 / 8.4, 512 39.8 / 35.4, 2,048 95 / 38, 8,192 235 / 114.
 template <typename TX>
@@ -656,11 +661,15 @@ static int launch_router(const void* x, const float* router, const float* bias, 
   if (T <= ROUTER_FEW_TOKENS) return launch_router_few<TX>(x, router, bias, T, W, E, top, renormalize, score_mode, ids, weights, correction, groups, s);
   auto tiles = [&](auto tt, auto ns) {
     if (E <= 16)
-      return launch_router_tile<TX, decltype(tt)::value, 16, decltype(ns)::value>(x, router, bias, T, W, E, top, renormalize, score_mode, ids, weights, correction, groups, s);
-    return launch_router_tile<TX, decltype(tt)::value, 32, decltype(ns)::value>(x, router, bias, T, W, E, top, renormalize, score_mode, ids, weights, correction, groups, s);
+      return launch_router_tile<TX, decltype(tt)::value, 16, decltype(ns)::value>(x, router, bias, T, W, E, top, renormalize, score_mode, ids, weights, correction, groups, s, taken);
+    return launch_router_tile<TX, decltype(tt)::value, 32, decltype(ns)::value>(x, router, bias, T, W, E, top, renormalize, score_mode, ids, weights, correction, groups, s, taken);
   };
   if (T <= 8 * 148) return tiles(Const<8>(), Const<4>());
-  return T <= 16 * 148 ? tiles(Const<16>(), Const<6>()) : tiles(Const<16>(), Const<4>());
+  if (T <= 16 * 148) {
+    const int rc = tiles(Const<16>(), Const<6>());
+    if (taken) return rc;
+  }
+  return tiles(Const<16>(), Const<4>());
 }
 
 TS_EXPORT int ts_router(const void* x, int x_dtype, const float* router, const float* bias, int T, int W, int E, int top, int renormalize,
