@@ -546,3 +546,30 @@ def test_router_takes_every_number_of_experts(dtype, T, W, E, groups):
     assert int(ids.min()) >= 0 and int(ids.max()) < E
     z = x.double() @ r.double().T
     assert float((w.double() - torch.softmax(z, 1).gather(1, ids.long())).abs().max()) < 1e-5
+
+
+@pytest.mark.parametrize("T, E, top", [(3, 40, 40), (20, 33, 32), (2, 70, 33), (300, 70, 66), (1200, 100, 64), (4, 16, 8)])
+@pytest.mark.parametrize("renormalize, scale", [(True, 1.0), (False, 2.5), (False, 1.0), (True, 0.5)])
+def test_router_choices_in_order(T, E, top, renormalize, scale):
+    """Many choices (a lane keeps every 32nd), ties, infinities: the order of the choices and the weights are those of a stable
+    sort.  Weights: float32 sums of up to 66 sigmoids, 1e-5."""
+    from tokensprint_b200 import ops
+
+    g = torch.Generator().manual_seed(T + E + top)
+    z = torch.round(torch.randn(T, E, generator=g) * 4) / 4  # quarters: many ties
+    z[0, : E // 2] = -math.inf
+    z[T - 1, E - 1] = math.inf
+    r = torch.eye(E)  # rows are the logits themselves
+    finite = z.clamp(-1e4, 1e4)
+    order = torch.sort(finite, dim=1, descending=True, stable=True).indices[:, :top]
+    for through in ("logits", "rows"):
+        ids, w = torch.empty((T, top), dtype=torch.int32, device="cuda"), torch.empty((T, top), device="cuda")
+        if through == "logits":
+            ops.router_topk(z.cuda(), top, renormalize, ids, w, scale=scale)
+        else:
+            ops.router(finite.cuda(), r.cuda(), top, renormalize, ids, w, scale=scale)
+        assert torch.equal(ids.cpu().long(), order)
+        want = torch.sigmoid((z if through == "logits" else finite).double().gather(1, order))
+        if renormalize:
+            want = want / (want.sum(1, keepdim=True) + 1e-20)
+        assert float((w.cpu().double() - want * scale).abs().max()) < 1e-5

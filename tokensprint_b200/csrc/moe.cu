@@ -43,7 +43,9 @@ struct RouterGroups {
 };
 
 // The choice of one token by one warp: logits z [E + groups.count] (shared memory; the entries behind the
-// logits are scratch), the bias already in.
+// logits are scratch), the bias already in.  A chosen entry becomes NaN, which no comparison prefers, and lane k % 32 keeps
+// choice k: nothing is read back from device memory.  (With earlier choices and weights read back where they had been stored, eight
+// warps of a CTA took 25 us for a choice of 8.)
 __device__ __forceinline__ void router_choose(float* z, int E, int top, int renormalize, int score_mode, int* my_ids, float* my_w,
                                               int lane, const float* __restrict__ correction, const RouterGroups& groups) {
   if (score_mode == ROUTER_SCORE_SOFTMAX_ALL) {
@@ -73,15 +75,15 @@ __device__ __forceinline__ void router_choose(float* z, int E, int top, int reno
     }
     __syncwarp();
   }
-  float total = 0.f, first = 0.f;
+  float total = 0.f, first = 0.f, my_score = 0.f;
+  int my_choice = 0;
+  const bool divided = renormalize || score_mode == ROUTER_SCORE_SOFTMAX_CHOSEN;
   for (int k = 0; k < top; ++k) {
     float best = -INFINITY;
     int best_e = 0x7fffffff;
     for (int e = lane; e < E; e += 32) {
-      bool taken = false;
-      for (int j = 0; j < k; ++j) taken |= (my_ids[j] == e);
       const float v = z[e] + (correction ? correction[e] : 0.f);
-      if (!taken && (v > best || (v == best && e < best_e))) {
+      if (v > best || (v == best && e < best_e)) {
         best = v;
         best_e = e;
       }
@@ -99,17 +101,26 @@ __device__ __forceinline__ void router_choose(float* z, int E, int top, int reno
     const float score = score_mode == ROUTER_SCORE_SOFTMAX_ALL ? z[best_e < E ? best_e : 0]
                       : score_mode == ROUTER_SCORE_SOFTMAX_CHOSEN ? expf(best - first) : 1.f / (1.f + expf(-best));
     total += score;
-    if (lane == 0) {
-      my_ids[k] = best_e < E ? best_e : 0;
-      my_w[k] = score;
-    }
+    const int chosen = best_e < E ? best_e : 0;
+    if (lane == (k & 31)) my_choice = chosen, my_score = score;
+    __syncwarp();  // everybody has read the scores
+    if (lane == 0) z[chosen] = __int_as_float(0x7fffffff);
     __syncwarp();
+    if ((k & 31) == 31 && k + 1 < top) {  // more than 32 choices: the weights are finished below
+      my_ids[k - 31 + lane] = my_choice;
+      my_w[k - 31 + lane] = my_score;
+    }
   }
-  if (lane == 0) {
-    if (renormalize || score_mode == ROUTER_SCORE_SOFTMAX_CHOSEN)
-      for (int k = 0; k < top; ++k) my_w[k] /= total + 1e-20f;
-    if (groups.scale != 1.f)
-      for (int k = 0; k < top; ++k) my_w[k] *= groups.scale;
+  const int rest = (top - 1) / 32 * 32;
+  if (rest + lane < top) {
+    my_ids[rest + lane] = my_choice;
+    my_w[rest + lane] = my_score;
+  }
+  for (int k = lane; k < top; k += 32) {  // every lane finishes what it wrote
+    float w = k >= rest ? my_score : my_w[k];
+    if (divided) w /= total + 1e-20f;
+    if (groups.scale != 1.f) w *= groups.scale;
+    if (k < rest || divided || groups.scale != 1.f) my_w[k] = w;
   }
 }
 
