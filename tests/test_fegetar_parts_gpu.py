@@ -521,6 +521,7 @@ def test_router_logits_do_not_depend_on_the_kernel(dtype, T, W, E):
 
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("T, W, E, groups", [
+    (592, 64, 8, None), (593, 64, 8, None), (148, 128, 20, None), (149, 128, 20, (4, 2)), (296, 1024, 20, None), (297, 1024, 20, None),
     (600, 136, 33, None), (1184, 64, 17, None), (1185, 64, 17, (17, 2)), (2368, 136, 16, None), (2369, 136, 40, (8, 3)), (2500, 72, 16, (4, 2)),
     # the logits of 16 tokens beside six slabs: up to 824 float32 entries (experts and groups), 1,208 of bfloat16 rows; four slabs
     # up to 1,616; beyond that the kernel without tiles

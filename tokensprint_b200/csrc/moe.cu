@@ -657,19 +657,23 @@ template <int N>
 struct Const {
   static constexpr int value = N;
 };
-#define ROUTER_FEW_TOKENS 296
-// Which kernel (the logits are the same): a CTA a token up to two tokens per SM, then tiles of 8 tokens, of 16 beyond 8 per SM,
+// Up to how many tokens a CTA takes one: the CTAs (a warp an expert, at most 32) then stand on the SMs at once, 4 of 8 experts
+// on each, 2 of 16, 1 of more; with wide rows twice as many of the last, while tiles would wait longer for
+// their slabs.  A CTA a token / tiles / router_kernel, us, choice of 2: 8 experts of 1,024, 297 to 512 tokens 4.0 / 6.6 / 5.6 to 7.7;
+// 32 of 256, 149 to 296 tokens 7.4 to 8.0 / 4.8 / 5.7 to 6.4; 64 of 1,024, 13.0 to 14.1 / 15.6 / 13.6 to 18.4.
+static int router_few_tokens(int E, int W) { return 148 * (E <= 8 ? 4 : E <= 16 || W > 512 ? 2 : 1); }
+// Which kernel (the logits are the same): a CTA a token for few of them, then tiles of 8 tokens, of 16 beyond 8 per SM,
 // with six slabs in the ring while a CTA has its SM to itself (where that leaves room for the logits: 824 float32 experts) and four, two CTAs an SM, beyond
 // that.  Rows that are no whole pieces, misaligned bases and more experts than shared memory has room for: router_kernel.
-// Measured, bfloat16 rows, us, router_kernel / these: 16 experts of 2,048: 64 tokens 7.7 / 4.8, 512 13.5 / 10.5, 2,048 20.3 / 21.9,
-// 8,192 72 / 40; 32 experts of 4,096: 64 tokens 20.3 / 8.4, 512 39.8 / 35.4, 2,048 95 / 38, 8,192 235 / 114.
+// Measured, bfloat16 rows, us, router_kernel / these: choice of 2 of 16 experts of 2,048: 64 tokens 8.2 / 4.7, 512 14.4 / 10.3,
+// 2,048 22.4 / 20.0, 8,192 76 / 40; of 4 of 32 experts of 4,096: 64 tokens 20.9 / 8.6, 512 40 / 27.8, 2,048 99 / 36, 8,192 245 / 110.
 template <typename TX>
 static int launch_router(const void* x, const float* router, const float* bias, int T, int W, int E, int top, int renormalize, int score_mode, int* ids,
                          float* weights, const float* correction, const RouterGroups& groups, cudaStream_t s, bool& taken) {
   constexpr int PER = 16 / (int)sizeof(TX);
   taken = W % PER == 0 && (((uintptr_t)x | (uintptr_t)router) & 15) == 0 && E <= 1024;
   if (!taken) return 0;
-  if (T <= ROUTER_FEW_TOKENS) return launch_router_few<TX>(x, router, bias, T, W, E, top, renormalize, score_mode, ids, weights, correction, groups, s);
+  if (T <= router_few_tokens(E, W)) return launch_router_few<TX>(x, router, bias, T, W, E, top, renormalize, score_mode, ids, weights, correction, groups, s);
   auto tiles = [&](auto tt, auto ns) {
     if (E <= 16)
       return launch_router_tile<TX, decltype(tt)::value, 16, decltype(ns)::value>(x, router, bias, T, W, E, top, renormalize, score_mode, ids, weights, correction, groups, s, taken);
