@@ -20,12 +20,12 @@
 //
 // Few rows (moe_few_kernel; up to 12 pairs per expert on average): the step streams the chosen experts' weights and little
 // else, at a rate that follows the bytes of weights in flight.  Row tiles of 32 places are the MMA's N and the weight rows
-// its M, two tiles of 128 (or one, see `narrow`), so 192 KB of weights are in flight per SM, and the epilogue, which nothing
+// its M, two tiles of 128 (or, without a gate, one: see `narrow`), so 192 KB of weights are in flight per SM, and the epilogue, which nothing
 // hides where a CTA has one item, is spread over 128 threads that each have a weight row and only as many
 // columns as the tile has places (with the places as M one warp did all of it, 5 to 8 us of the 35).  The tokens' rows come by
 // tile::gather4, four rows a copy, only as many as the tile has.
-// 16 experts, 2,048 -> 2 x 1,024, in a graph, gate/up and down: 2 pairs 17.3 and 7.5 us, 10 pairs 17.8 and 9.2, 66 pairs 25.4 and 14.9
-// (5.3 and 4.5 TB/s); tiles of 16 rows on mma.sync, three CTAs an SM, took 22.6 and 11.8, 28.2 and 15.6, 32.6 and 17.5.
+// 16 experts, 2,048 -> 2 x 1,024, six calls in a graph, gate/up and down: 2 pairs 15.5 and 8.1 us, 8 pairs 15.8 and 8.9, 66 pairs 26.3 and 10.6
+// (the down matrices stay in the L2 in part); tiles of 16 rows on mma.sync, three CTAs an SM, took 22.2 and 11.8, 26.6 and 14.3, 33.1 and 17.6.
 //
 // The pair's routing weight multiplies the float32 sums, not the rounded input: (w x) . g = w (x . g) without
 // a second rounding of x.  Every output element is one chain of sums over k in a fixed order.
@@ -409,8 +409,7 @@ __global__ void __launch_bounds__(many_threads(MODE), 1) moe_many_kernel(const _
 
 // ---- few rows ----
 
-// TILES: tiles of 128 weight rows per item.  MODE 1 with two: the gate rows and the up rows of 128 outputs; with one: of 64
-// outputs, 16 and 16 in turn, so that the two of an output sit in one warp, 16 lanes apart.
+// TILES: tiles of 128 weight rows per item; MODE 1 has two, the gate rows and the up rows of 128 outputs.
 template <int TILES>
 struct Few {
   static constexpr uint32_t W_BYTES = TILES * 128 * 128, STAGE = W_BYTES + ROWS_FEW * 128;
@@ -423,8 +422,9 @@ template <int MODE, int TILES>
 __global__ void __launch_bounds__(224, 1) moe_few_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w0,
                                                          const __grid_constant__ CUtensorMap map_w1, const Args a) {
   using F = Few<TILES>;
-  constexpr bool BY_TOKEN = MODE != 0, PAIRED = MODE == 1 && TILES == 1;
-  constexpr int COLS = MODE == 1 ? TILES * 64 : TILES * 128;
+  static_assert(MODE != 1 || TILES == 2, "gate rows and up rows");
+  constexpr bool BY_TOKEN = MODE != 0;
+  constexpr int COLS = MODE == 1 ? 128 : TILES * 128;
   ts_pdl_wait();  // tensor memory is never held while waiting for another kernel
   extern __shared__ unsigned char smem_unaligned[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_unaligned + 1023) & ~(uintptr_t)1023);
@@ -458,11 +458,8 @@ __global__ void __launch_bounds__(224, 1) moe_few_kernel(const __grid_constant__
         if (lane == 0) mbar_expect_tx(bar, bytes);
         __syncwarp();
         if (warp == 4) {
-          if (PAIRED) {
-            if (lane < 8) tma_load_2d(w_dst + lane * 2048, (lane & 1) ? &map_w1 : &map_w0, bar, k * BK, w_row + (lane >> 1) * 16);
-          } else if (lane < TILES) {
+          if (lane < TILES)
             tma_load_2d(w_dst + lane * 16384, MODE == 1 && lane == 1 ? &map_w1 : &map_w0, bar, k * BK, w_row + (MODE == 1 ? 0 : lane * 128));
-          }
         } else if (BY_TOKEN) {
           if (lane < quads) tma_gather4(x_dst + lane * 512, &map_x, bar, k * BK, rows);
         } else if (lane == 0) {
@@ -509,8 +506,9 @@ __global__ void __launch_bounds__(224, 1) moe_few_kernel(const __grid_constant__
       if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&c.acc_full[acc]), (uint32_t)(turn / 2) & 1, abort_flag))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t addr = c.tmem_base + ((uint32_t)(warp * 32) << 16) + acc * F::ACC;
-      const int n = w.n0 + (PAIRED ? warp * 16 + (lane & 15) : tid);  // this thread's output (of tile 0)
+      const int n = w.n0 + tid;  // this thread's output (of tile 0)
       for (int p0 = 0; p0 < w.rows; p0 += 8) {
+        __syncwarp();  // the load from tensor memory is the whole warp's
         uint32_t v[TILES][8];
 #pragma unroll
         for (int t = 0; t < TILES; ++t) tmem_ld8(addr + t * ROWS_FEW + p0, v[t]);
@@ -524,9 +522,7 @@ __global__ void __launch_bounds__(224, 1) moe_few_kernel(const __grid_constant__
           const float s0 = __uint_as_float(v[0][i]), s1 = __uint_as_float(v[TILES - 1][i]);
           // the sums are rounded to bfloat16 before the activation, as a product stored to memory would be
           if (MODE == 1) {
-            const float mate = PAIRED ? __shfl_xor_sync(0xffffffffu, s0, 16) : s1;  // of a gate row's lane: the up row's sum
-            if (n < a.NOUT && !(PAIRED && lane >= 16))
-              dst[n] = __float2bfloat16_rn(moe_gated_activation(a.act_mode, rounded(weight * s0), rounded(weight * mate), a.limit, a.alpha));
+            if (n < a.NOUT) dst[n] = __float2bfloat16_rn(moe_gated_activation(a.act_mode, rounded(weight * s0), rounded(weight * s1), a.limit, a.alpha));
           } else {
 #pragma unroll
             for (int t = 0; t < TILES; ++t) {
@@ -589,7 +585,7 @@ int launch_many(const void* A, const void* W0, const void* W1, int P, Args a, in
 template <int MODE, int TILES>
 int launch_few(const void* A, int rows, const void* W0, const void* W1, int P, Args a, int sms, cudaStream_t s) {
   using F = Few<TILES>;
-  constexpr int COLS = MODE == 1 ? TILES * 64 : TILES * 128, BOX = MODE == 1 && TILES == 1 ? 16 : 128;
+  constexpr int COLS = MODE == 1 ? 128 : TILES * 128, BOX = 128;
   a.cols = (a.NOUT + COLS - 1) / COLS;
   CUtensorMap mx, m0, m1;
   int st = rows_map(W0, (long long)a.E * a.NOUT, a.K, BOX, &m0);
@@ -608,7 +604,9 @@ int launch_few(const void* A, int rows, const void* W0, const void* W1, int P, A
 
 // One tile of 128 weight rows per item instead of two where the wide items would leave SMs idle: the width whose fullest CTA
 // streams the fewest weight rows.  How many experts got a pair is known on the device only; on average P pairs meet
-// E (1 - (1 - 1/E)^P) of them.
+// E (1 - (1 - 1/E)^P) of them.  Down, one / two tiles, us: 2 pairs of 16 experts of 1,024 -> 2,048 8.2 / 9.5, 128 pairs 13.8 / 10.7; 2
+// to 32 pairs of 8 experts of 3,584 -> 1,024 19 / 24.  Not for gate and up, whose narrow items would be 64 outputs in boxes of 16 rows: 4 to 384
+// pairs of 32 experts, 4,096 -> 2 x 1,536, 33 / 28 to 180 / 130; 32 to 1,024 of 128, 2,048 -> 2 x 768, 48 / 38 to 170 / 126.
 bool narrow(int P, int E, int wide_cols, int sms) {
   const double met = E * (1.0 - pow(1.0 - 1.0 / E, (double)P));
   return ceil(met * 2 * wide_cols / sms) < 2 * ceil(met * wide_cols / sms);
@@ -619,7 +617,8 @@ template <int MODE>
 int launch_shape(int tile_rows, const void* A, int rows, const void* W0, const void* W1, int P, const Args& a, int sms, cudaStream_t s) {
   constexpr int COLS = MODE == 1 ? 128 : 256;
   if (tile_rows == ROWS_MANY) return launch_many<MODE>(A, W0, W1, P, a, sms, s);
-  if (narrow(P, a.E, (a.NOUT + COLS - 1) / COLS, sms)) return launch_few<MODE, 1>(A, rows, W0, W1, P, a, sms, s);
+  if constexpr (MODE != 1)
+    if (narrow(P, a.E, (a.NOUT + COLS - 1) / COLS, sms)) return launch_few<MODE, 1>(A, rows, W0, W1, P, a, sms, s);
   return launch_few<MODE, 2>(A, rows, W0, W1, P, a, sms, s);
 }
 
