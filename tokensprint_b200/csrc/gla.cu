@@ -37,9 +37,6 @@
 #define GLA_UNROLL 4     // tokens of a round whose loads and shuffles are in flight together
 #endif
 constexpr int GLA_UNROLL_TOKENS = GLA_UNROLL;
-#ifndef GLA_TWO_COLUMNS_CTAS
-#define GLA_TWO_COLUMNS_CTAS 296  // fewest CTAs of two columns a thread
-#endif
 
 __device__ __forceinline__ float gla_log_sigmoid(float z) {
   // log(1 / (1 + exp(-z))) without overflow on either side
@@ -60,11 +57,8 @@ __device__ __forceinline__ __nv_bfloat16 gla_load(const __nv_bfloat16* p) {
   return __ushort_as_bfloat16(v);
 }
 
-// Two float32 at a time: by the packed instructions, or one after the other (each half rounds alike).  The pass in one piece takes
-// the scalar ones: pairs of registers cost it spills (50 decoded tokens beside a prompt of 944: the step 2.08 ms packed, 2.05 scalar).
-template <bool PACKED>
+// Two float32 at a time by the packed instructions; each half rounds as the scalar ones do.
 __device__ __forceinline__ float2 gla_fma2(float2 a, float2 b, float2 c) {
-  if (!PACKED) return make_float2(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y));
   float2 r;
   asm("{\n\t.reg .b64 a, b, c;\n\t"
       "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
@@ -72,9 +66,7 @@ __device__ __forceinline__ float2 gla_fma2(float2 a, float2 b, float2 c) {
       : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
   return r;
 }
-template <bool PACKED>
 __device__ __forceinline__ float2 gla_mul2(float2 a, float2 b) {
-  if (!PACKED) return make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
   float2 r;
   asm("{\n\t.reg .b64 a, b;\n\t"
       "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
@@ -83,18 +75,149 @@ __device__ __forceinline__ float2 gla_mul2(float2 a, float2 b) {
   return r;
 }
 
+// Register i of a thread holds key channel CH(i): its channels come in fours, and the fours of the R lanes of a column
+// are interleaved (lane r owns fours r, r + R, r + 2 R, ...), so that the 16-byte loads of a warp's lanes fall on
+// consecutive 16-byte pieces of the staged rows: no two of them meet in a bank of shared memory.
+#define CH(i) (((((i) >> 2) * R + r) << 2) + ((i) & 3))
+
 // The rounds are pipelined: while the threads run the updates of one round from shared memory, the
 // loads of the next round's q, k, z and v are in flight into registers (issued before the updates,
 // used after them), so the recurrence never waits for device memory.
 //
+// The whole portion in one piece (short portions, and steps whose sequences fill the SMs: the same sums whatever the cut).  Scalar
+// arithmetic: in packed pairs (the kernel below with a segment as long as the portion) the longest chain of tokens
+// takes longer, one portion of 500 tokens, 16 heads of 64 x 128: 154 us here, 164 there.
+template <typename TA, int KP>
+__global__ void __launch_bounds__(GLA_THREADS, GLA_MIN_BLOCKS) gla_scan_kernel(
+    const TA* __restrict__ q, const TA* __restrict__ k, const TA* __restrict__ v, long long ld_qkv, const float* __restrict__ decay,
+    float q_scale, float* __restrict__ state, const int* __restrict__ state_slots, const int* __restrict__ cu_seqlens,
+    float* __restrict__ o, int H, int d, int e, int R, int cols_per_cta, int tb, const float* __restrict__ kscale, int decay_scalar,
+    int groups, int ev, long long slot_stride) {
+  ts_pdl_prologue();
+  extern __shared__ __align__(16) float sm[];
+  // staged per token: q, k, decay [dp] each, v [cols]
+  const int dp = R * KP;  // d padded to the channels the threads cover
+  float* sq = sm;
+  float* sk = sq + tb * dp;
+  float* sa = sk + tb * dp;
+  float* sv = sa + tb * dp;  // [tb][cols_per_cta]
+  const int b = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * cols_per_cta;
+  const int t_begin = cu_seqlens[b], t_end = cu_seqlens[b + 1];
+  if (t_end <= t_begin) return;
+  const int r = threadIdx.x % R, cj = threadIdx.x / R;  // lanes of one column sit side by side
+  const int col = col0 + cj;
+  const bool has_col = col < e;
+  float* S = state + (size_t)state_slots[b] * slot_stride + ((size_t)h * d) * e;
+  float s_reg[KP];
+#pragma unroll
+  for (int i = 0; i < KP; ++i) s_reg[i] = (has_col && CH(i) < d) ? S[(size_t)(CH(i)) * e + col] : 0.f;
+
+  const size_t qk_off = (size_t)(h / (H / groups)) * d, a_off = (size_t)h * d, v_off = (size_t)h * ev + col0;
+  // what this thread fetches for a round: entries threadIdx.x + j * GLA_THREADS of the round's [tokens][dp] and [tokens][cols]
+  TA fq[GLA_PF], fk[GLA_PF], fv[GLA_PFV];
+  float fa[GLA_PF], fb[GLA_PF];
+  // Entry i of a round is channel i % dp of token i / dp (for v: column i % cols of token i / cols); a thread's
+  // entries lie GLA_THREADS apart, so their places are found once, by steps, without a division per entry.
+  const int Hd = H * d;
+  const int step_t = GLA_THREADS / dp, step_c = GLA_THREADS % dp, first_t = (int)threadIdx.x / dp, first_c = (int)threadIdx.x % dp;
+  const int vstep_t = GLA_THREADS / cols_per_cta, vstep_c = GLA_THREADS % cols_per_cta;
+  const int vfirst_t = (int)threadIdx.x / cols_per_cta, vfirst_c = (int)threadIdx.x % cols_per_cta;
+  auto fetch = [&](int t0) {
+    const int nt = min(tb, t_end - t0);
+    int tt = first_t, c = first_c;
+#pragma unroll
+    for (int j = 0; j < GLA_PF; ++j) {
+      {  // an entry beyond the round's tokens or the head's channels reads a valid place and is not used
+        const int tr = t0 + min(tt, nt - 1), cr = min(c, d - 1);
+        const size_t at = (size_t)tr * ld_qkv + qk_off + cr;
+        fq[j] = gla_load(q + at);
+        fk[j] = gla_load(k + at);
+        fa[j] = decay_scalar ? gla_load(decay + (size_t)tr * H + h) : gla_load(decay + (size_t)tr * Hd + a_off + cr);
+        fb[j] = kscale ? gla_load(kscale + (size_t)tr * H + h) : 1.f;
+      }
+      tt += step_t, c += step_c;
+      if (c >= dp) c -= dp, ++tt;
+    }
+    tt = vfirst_t, c = vfirst_c;
+#pragma unroll
+    for (int j = 0; j < GLA_PFV; ++j) {
+      fv[j] = gla_load(v + (size_t)(t0 + min(tt, nt - 1)) * ld_qkv + v_off + min(c, ev - 1 - col0));
+      tt += vstep_t, c += vstep_c;
+      if (c >= cols_per_cta) c -= cols_per_cta, ++tt;
+    }
+  };
+  auto stage = [&](int t0) {  // the fetched entries into shared memory as float32, q scaled
+    const int nt = min(tb, t_end - t0);
+    int tt = first_t, c = first_c;
+#pragma unroll
+    for (int j = 0; j < GLA_PF; ++j) {
+      if (tt < nt) {
+        const bool real = c < d;
+        const int i = tt * dp + c;
+        sq[i] = real ? ts_to_float(fq[j]) * q_scale : 0.f;
+        sk[i] = real ? ts_to_float(fk[j]) * fb[j] : 0.f;
+        sa[i] = real ? fa[j] : 1.f;
+      }
+      tt += step_t, c += step_c;
+      if (c >= dp) c -= dp, ++tt;
+    }
+    tt = vfirst_t, c = vfirst_c;
+#pragma unroll
+    for (int j = 0; j < GLA_PFV; ++j) {
+      if (tt < nt) sv[tt * cols_per_cta + c] = (col0 + c < ev) ? ts_to_float(fv[j]) : (col0 + c < e ? 1.f : 0.f);
+      tt += vstep_t, c += vstep_c;
+      if (c >= cols_per_cta) c -= cols_per_cta, ++tt;
+    }
+  };
+
+  fetch(t_begin);
+  for (int t0 = t_begin; t0 < t_end; t0 += tb) {
+    const int nt = min(tb, t_end - t0);
+    __syncthreads();  // the round before has been read
+    stage(t0);
+    __syncthreads();
+    if (t0 + tb < t_end) fetch(t0 + tb);  // in flight while this round's updates run
+#pragma unroll(KP > 16 ? 1 : GLA_UNROLL_TOKENS)  // several tokens' loads and shuffles in flight where the registers allow
+    for (int tt = 0; tt < nt; ++tt) {
+      const float vv = sv[tt * cols_per_cta + cj];
+      // a thread's channels come in fours that start on 16-byte boundaries: 16-byte loads
+      const float4* pq = reinterpret_cast<const float4*>(sq + tt * dp) + r;
+      const float4* pk = reinterpret_cast<const float4*>(sk + tt * dp) + r;
+      const float4* pa = reinterpret_cast<const float4*>(sa + tt * dp) + r;
+      float acc[4] = {0.f, 0.f, 0.f, 0.f};  // four chains: the read-out is a sum of KP terms, its order is fixed by KP alone
+#pragma unroll
+      for (int i = 0; i < KP / 4; ++i) {
+        const float4 a4 = pa[i * R], k4 = pk[i * R];
+        s_reg[4 * i + 0] = fmaf(a4.x, s_reg[4 * i + 0], k4.x * vv);
+        s_reg[4 * i + 1] = fmaf(a4.y, s_reg[4 * i + 1], k4.y * vv);
+        s_reg[4 * i + 2] = fmaf(a4.z, s_reg[4 * i + 2], k4.z * vv);
+        s_reg[4 * i + 3] = fmaf(a4.w, s_reg[4 * i + 3], k4.w * vv);
+        const float4 q4 = pq[i * R];
+        acc[0] = fmaf(s_reg[4 * i + 0], q4.x, acc[0]);
+        acc[1] = fmaf(s_reg[4 * i + 1], q4.y, acc[1]);
+        acc[2] = fmaf(s_reg[4 * i + 2], q4.z, acc[2]);
+        acc[3] = fmaf(s_reg[4 * i + 3], q4.w, acc[3]);
+      }
+      float sum = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+      for (int w = 1; w < R; w <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, w);
+      if (r == 0 && has_col) o[((size_t)(t0 + tt) * H + h) * e + col] = sum;
+    }
+  }
+  if (has_col) {
+#pragma unroll
+    for (int i = 0; i < KP; ++i)
+      if (CH(i) < d) S[(size_t)(CH(i)) * e + col] = s_reg[i];
+  }
+}
+
 // Long portions are cut into `segs` segments of `seg_len` tokens that run side by side (the recurrence
 // is linear in the state): MODE 1 runs every segment but a sequence's last from a zero state (the
 // first from the request's state) and leaves the state it ends with and the product of its decays;
 // MODE 2 starts every segment from what the segments before it left, folded in order
 // (S <- product * S + state), writes the read-outs, and the last segment writes the request's slot.
-// MODE 0 is the whole portion in one piece (decode steps, short portions: the same sums whatever the cut).
+// Pairs of neighbouring channels go through the packed instructions, and a thread has NC columns.
 template <typename TA, int KP, int MODE, int NC>
-__global__ void __launch_bounds__(GLA_THREADS, NC == 2 ? 3 : GLA_MIN_BLOCKS) gla_scan_kernel(
+__global__ void __launch_bounds__(GLA_THREADS, NC == 2 ? 3 : GLA_MIN_BLOCKS) gla_segment_kernel(
     const TA* __restrict__ q, const TA* __restrict__ k, const TA* __restrict__ v, long long ld_qkv, const float* __restrict__ decay,
     float q_scale, float* __restrict__ state, const int* __restrict__ state_slots, const int* __restrict__ cu_seqlens,
     float* __restrict__ o, int H, int d, int e, int R, int cols_per_cta, int tb, int segs, int seg_len, float* __restrict__ seg_state,
@@ -108,9 +231,9 @@ __global__ void __launch_bounds__(GLA_THREADS, NC == 2 ? 3 : GLA_MIN_BLOCKS) gla
   float* sk = sq + tb * dp;
   float* sa = sk + tb * dp;
   float* sv = sa + tb * dp;  // [tb][cols_per_cta]
-  const int b = MODE == 0 ? blockIdx.x : blockIdx.x / segs, seg = MODE == 0 ? 0 : blockIdx.x - b * segs;
+  const int b = blockIdx.x / segs, seg = blockIdx.x - b * segs;
   const int h = blockIdx.y, col0 = blockIdx.z * cols_per_cta;
-  const int t_begin = cu_seqlens[b] + seg * seg_len, t_end = MODE == 0 ? cu_seqlens[b + 1] : min(cu_seqlens[b + 1], t_begin + seg_len);
+  const int t_begin = cu_seqlens[b] + seg * seg_len, t_end = min(cu_seqlens[b + 1], t_begin + seg_len);
   if (t_end <= t_begin) return;
   const bool last = t_end == cu_seqlens[b + 1];
   if (MODE == 1 && last) return;  // nobody starts from what a sequence's last segment leaves
@@ -124,16 +247,11 @@ __global__ void __launch_bounds__(GLA_THREADS, NC == 2 ? 3 : GLA_MIN_BLOCKS) gla
     col[c] = col0 + cj + c * lanes;
     has_col[c] = col[c] < e;
   }
-  // Register i of a thread holds key channel CH(i): its channels come in fours, and the fours of the R lanes of a column
-  // are interleaved (lane r owns fours r, r + R, r + 2 R, ...), so that the 16-byte loads of a warp's lanes fall on
-  // consecutive 16-byte pieces of the staged rows: no two of them meet in a bank of shared memory.
-#define CH(i) (((((i) >> 2) * R + r) << 2) + ((i) & 3))
   float* S = state + (size_t)state_slots[b] * slot_stride + ((size_t)h * d) * e;
   const size_t state_elems = (size_t)d * e;
-  float* seg_L = MODE == 0 ? nullptr : seg_state + (((size_t)b * segs + seg) * H + h) * state_elems;   // this segment's end state
-  float* seg_P = MODE == 0 ? nullptr : seg_decay + (((size_t)b * segs + seg) * H + h) * d;             // this segment's decay product
-  float* seg_S0 = MODE == 0 ? nullptr : seg_start + ((size_t)b * H + h) * state_elems;                 // the request's state as the step found it
-  constexpr bool PACKED = MODE != 0;
+  float* seg_L = seg_state + (((size_t)b * segs + seg) * H + h) * state_elems;   // this segment's end state
+  float* seg_P = seg_decay + (((size_t)b * segs + seg) * H + h) * d;             // this segment's decay product
+  float* seg_S0 = seg_start + ((size_t)b * H + h) * state_elems;                 // the request's state as the step found it
   // pairs of neighbouring channels, CH(2 i) and CH(2 i) + 1, of a column
   float2 s_reg[NC][KP / 2];
   float2 p_reg[MODE == 1 ? KP / 2 : 1];
@@ -148,7 +266,7 @@ __global__ void __launch_bounds__(GLA_THREADS, NC == 2 ? 3 : GLA_MIN_BLOCKS) gla
   };
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
-    if (MODE == 0 || (seg == 0 && (MODE == 1 || last))) {
+    if (seg == 0 && (MODE == 1 || last)) {
       // the request's state (MODE 2: only a sequence of one segment reads the slot, which it alone writes in this launch)
 #pragma unroll
       for (int i = 0; i < KP / 2; ++i) s_reg[c][i] = load_pair(S, i, c);
@@ -174,7 +292,7 @@ __global__ void __launch_bounds__(GLA_THREADS, NC == 2 ? 3 : GLA_MIN_BLOCKS) gla
         for (int i = 0; i < KP / 2; ++i) {
           const int ch = CH(2 * i);
           const float2 p2 = make_float2(ch < d ? P[ch] : 0.f, ch + 1 < d ? P[ch + 1] : 0.f);
-          s_reg[c][i] = gla_fma2<PACKED>(p2, s_reg[c][i], load_pair(L, i, c));
+          s_reg[c][i] = gla_fma2(p2, s_reg[c][i], load_pair(L, i, c));
         }
       }
     }
@@ -269,18 +387,18 @@ __global__ void __launch_bounds__(GLA_THREADS, NC == 2 ? 3 : GLA_MIN_BLOCKS) gla
         const float4 a4 = pa[i * R], k4 = pk[i * R];
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-          s_reg[c][2 * i] = gla_fma2<PACKED>(make_float2(a4.x, a4.y), s_reg[c][2 * i], gla_mul2<PACKED>(make_float2(k4.x, k4.y), vv[c]));
-          s_reg[c][2 * i + 1] = gla_fma2<PACKED>(make_float2(a4.z, a4.w), s_reg[c][2 * i + 1], gla_mul2<PACKED>(make_float2(k4.z, k4.w), vv[c]));
+          s_reg[c][2 * i] = gla_fma2(make_float2(a4.x, a4.y), s_reg[c][2 * i], gla_mul2(make_float2(k4.x, k4.y), vv[c]));
+          s_reg[c][2 * i + 1] = gla_fma2(make_float2(a4.z, a4.w), s_reg[c][2 * i + 1], gla_mul2(make_float2(k4.z, k4.w), vv[c]));
         }
         if (MODE == 1) {  // no read-outs yet: the product of the segment's decays instead
-          p_reg[MODE == 1 ? 2 * i : 0] = gla_mul2<PACKED>(p_reg[MODE == 1 ? 2 * i : 0], make_float2(a4.x, a4.y));
-          p_reg[MODE == 1 ? 2 * i + 1 : 0] = gla_mul2<PACKED>(p_reg[MODE == 1 ? 2 * i + 1 : 0], make_float2(a4.z, a4.w));
+          p_reg[MODE == 1 ? 2 * i : 0] = gla_mul2(p_reg[MODE == 1 ? 2 * i : 0], make_float2(a4.x, a4.y));
+          p_reg[MODE == 1 ? 2 * i + 1 : 0] = gla_mul2(p_reg[MODE == 1 ? 2 * i + 1 : 0], make_float2(a4.z, a4.w));
         } else {
           const float4 q4 = pq[i * R];
 #pragma unroll
           for (int c = 0; c < NC; ++c) {
-            acc[c][0] = gla_fma2<PACKED>(s_reg[c][2 * i], make_float2(q4.x, q4.y), acc[c][0]);
-            acc[c][1] = gla_fma2<PACKED>(s_reg[c][2 * i + 1], make_float2(q4.z, q4.w), acc[c][1]);
+            acc[c][0] = gla_fma2(s_reg[c][2 * i], make_float2(q4.x, q4.y), acc[c][0]);
+            acc[c][1] = gla_fma2(s_reg[c][2 * i + 1], make_float2(q4.z, q4.w), acc[c][1]);
           }
         }
       }
@@ -308,7 +426,7 @@ __global__ void __launch_bounds__(GLA_THREADS, NC == 2 ? 3 : GLA_MIN_BLOCKS) gla
         if (ch + 1 < d) seg_P[ch + 1] = p2.y;
       }
     }
-  } else if (MODE == 0 || last) {
+  } else if (last) {
 #pragma unroll
     for (int c = 0; c < NC; ++c)
 #pragma unroll
@@ -372,57 +490,77 @@ struct GlaExtra {
   long long slot_stride;  // floats from one request's state to the next
 };
 
-template <typename TA, int KP, int MODE, int NC>
+// The grid, the tokens per round (what the threads' fetch registers hold, at most GLA_TB) and the shared memory of a scan whose
+// threads have `nc` columns each.
+struct GlaShape {
+  int cols, tb;
+  size_t smem;
+  dim3 grid;
+  bool fits;
+};
+static GlaShape gla_shape(int parts, int H, int e, int R, int dp, int nc) {
+  GlaShape g;
+  g.cols = nc * GLA_THREADS / R;
+  g.tb = min(GLA_TB, min(GLA_THREADS * GLA_PF / dp, GLA_THREADS * GLA_PFV * nc / g.cols));
+  g.smem = (size_t)g.tb * (3 * dp + g.cols) * sizeof(float);  // at most 16 * (3 * 64 + 256) or 1 * (3 * 1024 + 8) floats: below 48 KB
+  g.grid = dim3(parts, H, (e + g.cols - 1) / g.cols);
+  g.fits = g.tb >= 1 && g.grid.y <= 65535 && g.grid.z <= 65535;
+  return g;
+}
+
+template <typename TA, int KP>
 static int launch_gla_scan(const void* q, const void* k, const void* v, long long ld_qkv, const float* decay, float q_scale, float* state,
-                           const int* state_slots, const int* cu_seqlens, float* o, int B, int H, int d, int e, int R, int segs, int seg_len,
-                           float* scratch, cudaStream_t s, const GlaExtra& x) {
-  const int cols = NC * GLA_THREADS / R, dp = R * KP;
-  // tokens per round: what the threads' fetch registers hold, at most GLA_TB
-  const int tb = min(GLA_TB, min(GLA_THREADS * GLA_PF / dp, GLA_THREADS * GLA_PFV * NC / cols));
-  if (tb < 1) return TS_ERR_UNSUPPORTED_SIZE;
-  const size_t smem = (size_t)tb * (3 * dp + cols) * sizeof(float);  // at most 16 * (3 * 64 + 256) or 1 * (3 * 1024 + 8) floats: below 48 KB
-  const dim3 grid(B * segs, H, (e + cols - 1) / cols);
-  if (grid.y > 65535 || grid.z > 65535) return TS_ERR_UNSUPPORTED_SIZE;
-  // scratch of the segmented scan: end states [B, segs, H, d, e], decay products [B, segs, H, d], start states [B, H, d, e]
+                           const int* state_slots, const int* cu_seqlens, float* o, int B, int H, int d, int e, int R, cudaStream_t s,
+                           const GlaExtra& x) {
+  const GlaShape g = gla_shape(B, H, e, R, R * KP, 1);
+  if (!g.fits) return TS_ERR_UNSUPPORTED_SIZE;
+  return ts_launch(gla_scan_kernel<TA, KP>, g.grid, dim3(GLA_THREADS), g.smem, s, (const TA*)q, (const TA*)k, (const TA*)v, ld_qkv, decay, q_scale, state,
+                   state_slots, cu_seqlens, o, H, d, e, R, g.cols, g.tb, x.kscale, x.decay_scalar, x.groups, x.ev, x.slot_stride);
+}
+
+template <typename TA, int KP, int MODE, int NC>
+static int launch_gla_segments(const void* q, const void* k, const void* v, long long ld_qkv, const float* decay, float q_scale, float* state,
+                               const int* state_slots, const int* cu_seqlens, float* o, int B, int H, int d, int e, int R, int segs, int seg_len,
+                               float* scratch, cudaStream_t s, const GlaExtra& x) {
+  const GlaShape g = gla_shape(B * segs, H, e, R, R * KP, NC);
+  if (!g.fits) return TS_ERR_UNSUPPORTED_SIZE;
+  // scratch: end states [B, segs, H, d, e], decay products [B, segs, H, d], start states [B, H, d, e]
   float* seg_state = scratch;
-  float* seg_decay = scratch ? seg_state + (size_t)B * segs * H * d * e : nullptr;
-  float* seg_start = scratch ? seg_decay + (size_t)B * segs * H * d : nullptr;
-  return ts_launch(gla_scan_kernel<TA, KP, MODE, NC>, grid, dim3(GLA_THREADS), smem, s, (const TA*)q, (const TA*)k, (const TA*)v, ld_qkv, decay,
-                   q_scale, state, state_slots, cu_seqlens, o, H, d, e, R, cols, tb, segs, seg_len, seg_state, seg_decay, seg_start, x.kscale,
+  float* seg_decay = seg_state + (size_t)B * segs * H * d * e;
+  float* seg_start = seg_decay + (size_t)B * segs * H * d;
+  return ts_launch(gla_segment_kernel<TA, KP, MODE, NC>, g.grid, dim3(GLA_THREADS), g.smem, s, (const TA*)q, (const TA*)k, (const TA*)v, ld_qkv, decay,
+                   q_scale, state, state_slots, cu_seqlens, o, H, d, e, R, g.cols, g.tb, segs, seg_len, seg_state, seg_decay, seg_start, x.kscale,
                    x.decay_scalar, x.groups, x.ev, x.slot_stride);
 }
 
 // Whether a thread takes two columns: its loads of q, k and the decay from shared memory then serve both.  Not where the grid
-// would no longer fill the SMs, nor where the state of two columns does not fit the registers, nor in one piece: the longest portion's chain of
-// tokens then sets the time, and it is longer with two (64 heads of 128 x 64, 50 decoded tokens beside a prompt of 944: the
-// step 2.37 ms against 2.05).  Passes over 16 segments of 64 tokens of the same heads, without and with read-outs: 235 -> 131 and 487 -> 471 us.
+// would no longer fill the SMs, nor where the state of two columns does not fit the registers.
+#define GLA_TWO_COLUMNS_CTAS 296  // fewest CTAs of two columns a thread
 template <int KP>
-static bool two_columns(int B, int segs, int H, int e, int R) {
+static bool two_columns(long long parts, int H, int e, int R) {
   const long long cols = 2 * GLA_THREADS / R;
-  return KP <= 16 && e > GLA_THREADS / R && (long long)B * segs * H * ((e + cols - 1) / cols) >= GLA_TWO_COLUMNS_CTAS;
+  return KP <= 16 && e > GLA_THREADS / R && parts * H * ((e + cols - 1) / cols) >= GLA_TWO_COLUMNS_CTAS;
 }
 
 template <typename TA, int KP, int MODE>
-static int launch_gla_scan_columns(const void* q, const void* k, const void* v, long long ld_qkv, const float* decay, float q_scale, float* state,
-                                   const int* state_slots, const int* cu_seqlens, float* o, int B, int H, int d, int e, int R, int segs,
-                                   int seg_len, float* scratch, cudaStream_t s, const GlaExtra& x) {
-  if constexpr (KP <= 16 && MODE != 0)
-    if (two_columns<KP>(B, segs, H, e, R))
-      return launch_gla_scan<TA, KP, MODE, 2>(q, k, v, ld_qkv, decay, q_scale, state, state_slots, cu_seqlens, o, B, H, d, e, R, segs, seg_len,
-                                              scratch, s, x);
-  return launch_gla_scan<TA, KP, MODE, 1>(q, k, v, ld_qkv, decay, q_scale, state, state_slots, cu_seqlens, o, B, H, d, e, R, segs, seg_len, scratch, s, x);
+static int launch_gla_pass(const void* q, const void* k, const void* v, long long ld_qkv, const float* decay, float q_scale, float* state,
+                           const int* state_slots, const int* cu_seqlens, float* o, int B, int H, int d, int e, int R, int segs, int seg_len,
+                           float* scratch, cudaStream_t s, const GlaExtra& x) {
+  if constexpr (KP <= 16)
+    if (two_columns<KP>((long long)B * segs, H, e, R))
+      return launch_gla_segments<TA, KP, MODE, 2>(q, k, v, ld_qkv, decay, q_scale, state, state_slots, cu_seqlens, o, B, H, d, e, R, segs, seg_len,
+                                                  scratch, s, x);
+  return launch_gla_segments<TA, KP, MODE, 1>(q, k, v, ld_qkv, decay, q_scale, state, state_slots, cu_seqlens, o, B, H, d, e, R, segs, seg_len, scratch, s, x);
 }
 
 template <typename TA, int KP>
 static int launch_gla_scan_modes(const void* q, const void* k, const void* v, long long ld_qkv, const float* decay, float q_scale, float* state,
                                  const int* state_slots, const int* cu_seqlens, float* o, int B, int H, int d, int e, int R, int segs,
                                  int seg_len, float* scratch, cudaStream_t s, const GlaExtra& x) {
-  if (segs <= 1)
-    return launch_gla_scan_columns<TA, KP, 0>(q, k, v, ld_qkv, decay, q_scale, state, state_slots, cu_seqlens, o, B, H, d, e, R, 1, 0, nullptr, s, x);
-  const int st = launch_gla_scan_columns<TA, KP, 1>(q, k, v, ld_qkv, decay, q_scale, state, state_slots, cu_seqlens, o, B, H, d, e, R, segs, seg_len,
-                                            scratch, s, x);
+  if (segs <= 1) return launch_gla_scan<TA, KP>(q, k, v, ld_qkv, decay, q_scale, state, state_slots, cu_seqlens, o, B, H, d, e, R, s, x);
+  const int st = launch_gla_pass<TA, KP, 1>(q, k, v, ld_qkv, decay, q_scale, state, state_slots, cu_seqlens, o, B, H, d, e, R, segs, seg_len, scratch, s, x);
   if (st != 0) return st;
-  return launch_gla_scan_columns<TA, KP, 2>(q, k, v, ld_qkv, decay, q_scale, state, state_slots, cu_seqlens, o, B, H, d, e, R, segs, seg_len, scratch, s, x);
+  return launch_gla_pass<TA, KP, 2>(q, k, v, ld_qkv, decay, q_scale, state, state_slots, cu_seqlens, o, B, H, d, e, R, segs, seg_len, scratch, s, x);
 }
 
 template <typename TA>
