@@ -381,6 +381,57 @@ def test_gla_scan_long_portions_in_segments(dtype, H, d, e):
     assert torch.equal(results[0][1][1].cpu(), start[1]) and torch.equal(results[0][1][4].cpu(), start[4]), "a slot of no sequence was touched"
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H, groups, d, e, scalar, normaliser, lens", [
+    (36, 36, 50, 120, False, False, [1300]),       # two columns a thread in both passes, the last block short by eight columns
+    (40, 8, 100, 60, True, True, [1300, 3, 700]),  # one decay and one key scale a head, five heads a group, a column beyond v's
+    (80, 16, 60, 59, True, True, [700]),           # two columns in the second pass only (the first has 2 x 240 CTAs of one)
+    (40, 40, 48, 96, False, False, [1000]),        # three blocks of columns: one column a thread
+])
+def test_linear_scan_with_two_columns_a_thread(dtype, H, groups, d, e, scalar, normaliser, lens):
+    """Segments whose threads have two value columns, against the recurrence in float64 and the same tokens in one piece; 1,300
+    float32 updates per state entry with decays of 0.9 to 1: 5e-5, as for the other segmented runs."""
+    from tokensprint_b200 import ops
+
+    T, B = sum(lens), len(lens)
+    g = torch.Generator().manual_seed(H + d)
+    wide = torch.randn(T, 2 * groups * d + H * e, generator=g).to(dtype).to(DEV)
+    q, k, v = wide[:, : groups * d], wide[:, groups * d : 2 * groups * d], wide[:, 2 * groups * d :]
+    ee = e + 1 if normaliser else e
+    start = (0.3 * torch.randn(B + 1, H, d, ee, generator=g)).to(DEV)
+    slots, cu = torch.arange(B, 0, -1, dtype=torch.int32, device=DEV), torch.tensor([0] + lens).cumsum(0).to(torch.int32).to(DEV)
+    if scalar:
+        decay, kscale = (0.9 + 0.1 * torch.rand(T, H, generator=g)).to(DEV), torch.rand(T, H, generator=g).to(DEV)
+        a = decay.double()[:, :, None].expand(T, H, d)
+    else:
+        z, tau = (torch.randn(T, H * d, generator=g) + 3.0).to(dtype).to(DEV), 2.0
+        a, kscale = torch.sigmoid(z.double()).pow(1.0 / tau).view(T, H, d), torch.ones(T, H, device=DEV)
+    results = []
+    for max_seqlen in (max(lens), None):
+        state, out = start.clone(), torch.empty((T, H * ee), device=DEV)
+        if scalar:
+            ops.linear_scan(q, k, v, decay, kscale, d ** -0.5, state.view(B + 1, -1), slots, cu, out, B, H, groups, d, e, normaliser=normaliser, max_seqlen=max_seqlen)
+        else:
+            ops.gla_scan(q, k, v, z, None, tau, d ** -0.5, state, slots, cu, out, B, H, d, e, max_seqlen=max_seqlen)
+        results.append((out, state))
+    heads = lambda x: x.double().view(T, groups, 1, d).expand(T, groups, H // groups, d).reshape(T, H, d)  # noqa: E731
+    qh, kh, vh = heads(q) * d ** -0.5, heads(k) * kscale.double()[:, :, None], v.double().reshape(T, H, e)
+    if normaliser:
+        vh = torch.cat([vh, torch.ones(T, H, 1, device=DEV, dtype=torch.float64)], 2)
+    at = 0
+    for b, n in enumerate(lens):
+        S, want = start[B - b].double(), []
+        for t in range(at, at + n):
+            S = a[t][:, :, None] * S + kh[t][:, :, None] * vh[t][:, None, :]
+            want.append((S * qh[t][:, :, None]).sum(1).reshape(-1))
+        want = torch.stack(want).cpu()
+        for out, state in results:
+            assert _rel(out[at : at + n], want) < 5e-5, f"sequence {b}"
+            assert _rel(state[B - b], S.cpu()) < 5e-5, f"state of sequence {b}"
+        at += n
+    assert all(torch.equal(state[0], start[0]) for _, state in results), "a slot of no sequence was touched"
+
+
 def test_gla_state_remembers_a_far_token():
     """Decays of one on one key channel: a value written 600 tokens ago is read back exactly by a
     query on that channel; a channel whose decay is small has forgotten it."""

@@ -533,13 +533,17 @@ static int launch_gla_segments(const void* q, const void* k, const void* v, long
                    x.decay_scalar, x.groups, x.ev, x.slot_stride);
 }
 
-// Whether a thread takes two columns: its loads of q, k and the decay from shared memory then serve both.  Not where the grid
-// would no longer fill the SMs, nor where the state of two columns does not fit the registers.
-#define GLA_TWO_COLUMNS_CTAS 296  // fewest CTAs of two columns a thread
+// Whether a thread takes two columns (its loads of q, k and the decay from shared memory then serve both) in a pass of `parts`
+// segments that have work: where the CTAs of one column each would not all stand on the SMs at once (GLA_MIN_BLOCKS on
+// each), where pairs leave at most an eighth more columns empty, and where two columns' state fits the registers.  Both passes, one / two
+// columns, us: 64 heads of 128 x 64, one prompt of 512, 768, 1,024, 2,048, 4,096 tokens (segments of 256; 512, 768, ... CTAs of one
+// column): 323 / 327, 453 / 340, 590 / 484, 1,144 / 904, 2,303 / 1,669; 16 heads of 64 x 128, 512, 1,024, 2,048, 3,000, 4,096 tokens (128, 256, 512,
+// 768, 1,024): 157 / 188, 190 / 203, 281 / 284, 484 / 301, 563 / 519; 24 heads of 48 x 96 (three blocks of columns, a third more as
+// pairs), 2,048 and 4,096 tokens: 234 / 264, 482 / 498.
 template <int KP>
 static bool two_columns(long long parts, int H, int e, int R) {
-  const long long cols = 2 * GLA_THREADS / R;
-  return KP <= 16 && e > GLA_THREADS / R && parts * H * ((e + cols - 1) / cols) >= GLA_TWO_COLUMNS_CTAS;
+  const int lanes = GLA_THREADS / R, blocks = (e + lanes - 1) / lanes;
+  return KP <= 16 && (blocks + 1) / 2 * 16 <= blocks * 9 && parts * H * blocks > GLA_MIN_BLOCKS * 148;
 }
 
 template <typename TA, int KP, int MODE>
@@ -547,7 +551,7 @@ static int launch_gla_pass(const void* q, const void* k, const void* v, long lon
                            const int* state_slots, const int* cu_seqlens, float* o, int B, int H, int d, int e, int R, int segs, int seg_len,
                            float* scratch, cudaStream_t s, const GlaExtra& x) {
   if constexpr (KP <= 16)
-    if (two_columns<KP>((long long)B * segs, H, e, R))
+    if (two_columns<KP>((long long)B * (MODE == 1 ? segs - 1 : segs), H, e, R))  // a sequence's last segment has nothing to do in the first pass
       return launch_gla_segments<TA, KP, MODE, 2>(q, k, v, ld_qkv, decay, q_scale, state, state_slots, cu_seqlens, o, B, H, d, e, R, segs, seg_len,
                                                   scratch, s, x);
   return launch_gla_segments<TA, KP, MODE, 1>(q, k, v, ld_qkv, decay, q_scale, state, state_slots, cu_seqlens, o, B, H, d, e, R, segs, seg_len, scratch, s, x);
