@@ -67,13 +67,14 @@ class CacheTensors:
                 state.append(None)
         return cls(k, v, state, list(group_index))
 
-    def layer_cache(self, cache: int, writes: bool) -> LayerCache:
+    def layer_cache(self, cache: int, writes: bool, read_later: int = 0) -> LayerCache:
         return LayerCache(
             group=self.group_index[cache],
             k_pages=self.k[cache],
             v_pages=self.v[cache],
             state=self.state[cache],
             writes=writes,
+            read_later=read_later,
         )
 
     def zero_slot(self, slot: int) -> None:

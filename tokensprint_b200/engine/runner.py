@@ -144,6 +144,7 @@ class ModelRunner:
         self._graph_pool = None
         self._capture_stream: Optional[torch.cuda.Stream] = None
         self.graph_launches = 0  # kernels of this library replayed inside graphs so far
+        self._sizing_step = False
         self.sizing: Optional[dict] = None  # how the page count was derived, when it came from free memory
 
         if num_pages is None:
@@ -162,8 +163,9 @@ class ModelRunner:
         self.cache_manager = CacheManager(self.groups, self.page_size, self.num_pages, self.num_slots)
         self.cache_tensors = CacheTensors.allocate(
             self._needs, self.cache_group, self.num_pages, self.page_size, self.num_slots, self.device, self.model.dtype)
+        used = self.model.run_cache
         self.layer_caches = [
-            self.cache_tensors.layer_cache(self.model.run_cache[i], run.writes_cache)
+            self.cache_tensors.layer_cache(used[i], run.writes_cache, used[i + 1 :].count(used[i]))
             for i, run in enumerate(self.model.spec.run_order)
         ] + [self.cache_tensors.layer_cache(c, True) for c in getattr(self.model, "extra_caches", [])]
 
@@ -194,8 +196,9 @@ class ModelRunner:
             self.cache_manager.extend(rc, 0, n)
             entries.append(StepEntry(rc, [0] * n, 0, [n - 1]))
         graphs, self.use_graphs = self.use_graphs, False
+        self._sizing_step = True
         self.step(entries)
-        self.use_graphs = graphs
+        self.use_graphs, self._sizing_step = graphs, False
         torch.cuda.synchronize(self.device)
         peak = torch.cuda.max_memory_allocated(self.device) - before
         self.steps_run = 0
@@ -296,6 +299,7 @@ class ModelRunner:
         step.host_state_slots = [e.cache.slot for e in entries]
         step.rows_all = row_base is None and all(list(e.want) == list(range(n)) for e, n in zip(entries, lens))
         step.decode_seqs = singles
+        step.sizing = self._sizing_step
         return step, layout.view(dev, "rows"), R
 
     def _fill(self, host, layout: _Layout, entries: Sequence[StepEntry], lens: Sequence[int], row_marks=None, row_base=None) -> int:

@@ -153,6 +153,9 @@ class StepContext:
     # first in a step that also carries portions of prompts, so that a mixer may treat the two kinds apart)
     decode_seqs: int = 0
     rows_all: bool = False  # the logits of every token are wanted, in the tokens' order
+    # The step measures how much memory a step takes: a part that has several ways to work, which others
+    # of the same size may take, goes the one with the most scratch.
+    sizing: bool = False
     # A hint, set by whoever calls a part: the first weight matrix that will be read after the
     # part returns (the part may hand it to its last product for prefetching; may be None).
     weight_after: Optional[torch.Tensor] = None
@@ -232,6 +235,7 @@ class LayerCache:
     v_pages: Optional[torch.Tensor] = None  # [pages, page, *v_row], or None for a cache of one pool
     state: Optional[torch.Tensor] = None  # [slots, *state_shape]
     writes: bool = True  # False: reads a cache that another run filled
+    read_later: int = 0  # how many later runs of the step read these pages
     # [slots, *shape]: what the block around the mixer keeps per request (Block.state_need); always the
     # run's own, also where the run reads another run's pages
     block_state: Optional[torch.Tensor] = None

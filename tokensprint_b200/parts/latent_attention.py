@@ -19,9 +19,10 @@ LATENT_ATTENTION_MMA = os.environ.get("TS_LATENT_ATTENTION_MMA", "1") != "0"
 LATENT_DECODE_MAX_TOKENS = 4
 # TS_LATENT_REBUILD=0 (for measurements): prompt portions score the cached rows through absorbed queries too.
 LATENT_REBUILD = os.environ.get("TS_LATENT_REBUILD", "1") != "0"
-# Most bytes of rebuilt keys and values of a step; above it the portions go through absorbed queries.  A later portion of
-# a long prompt keeps more rows than the step that the page pool's size is measured with (a first portion):
-# the bound is the margin that the sizing leaves.
+# Most bytes of gathered rows and of the keys and values made of them at any time of a step, rows that later layers of the step will
+# read included; above it the portions go through absorbed queries.  The step that the page pool's size is measured with is an absorbed
+# one (StepContext.sizing), and a later portion of a long prompt keeps more rows than a step has tokens: the bound is the
+# margin that the sizing leaves.
 LATENT_REBUILD_MAX_BYTES = 256 << 20
 
 
@@ -203,7 +204,7 @@ class LatentAttentionMixer(Mixer):
             ops.rmsnorm_rows(proj[:, q_off:q_off + self.q_rank], self.dq_norm_weight, normed, self.norm_eps)
             q_src = linear(normed, self.uq_weight)
         q_rows = q_src if q_src is not None else proj[:, q_off : q_off + H * (self.nope_dim + self.rot_dim)]
-        absorbed, kept = self._rebuild_plan(step, q_rows)  # tokens in front that go through absorbed queries; rows the others' portions keep
+        absorbed, kept = self._rebuild_plan(step, q_rows, cache)  # tokens in front that go through absorbed queries; rows the others' portions keep
         rebuilt = absorbed < T
         q_abs = torch.empty((absorbed, H, D), device=dev, dtype=dtype)
         q_rot = torch.empty((T - absorbed, H, self.rot_dim), device=dev, dtype=dtype) if rebuilt else None
@@ -213,6 +214,8 @@ class LatentAttentionMixer(Mixer):
             step.positions, self.latent_weight, self.norm_eps, None if self.position is None else self.position.frequencies(),
             self.rot_dims, self.pairing, gates, H, self.nope_dim, self.rot_dim, R, magnitude=self.magnitude, q_src=q_src, q_rot=q_rot)
         heads_out = torch.empty((T, H, self.value_dim), device=dev, dtype=dtype)
+        if not rebuilt and not cache.read_later and "latent rows" in step.shared:
+            step.shared["latent rows"].pop(self._held_key(cache), None)
         if absorbed:
             if self.nope_dim:
                 q_plain = q_rows[:absorbed].view(absorbed, H, self.nope_dim + self.rot_dim)[:, :, : self.nope_dim]
@@ -226,12 +229,15 @@ class LatentAttentionMixer(Mixer):
             first = step.decode_seqs if absorbed else 0
             count = step.num_seqs - first
             cu, lens = step.cu_seqlens_q[first:], step.context_lens[first:]  # (the starts count from the step's first token)
-            # a layer that reads another one's rows finds them gathered already, where the windows agree
-            key = ("latent rows", cache.group, cache.k_pages.data_ptr(), self.window, first)
-            cached = None if has_latent else step.shared.get(key)
-            if cached is None:
-                cached = step.shared[key] = torch.empty((sum(kept), D), device=dev, dtype=dtype)
+            # a layer that reads another one's rows finds them gathered already, where the windows agree; they are held while a
+            # later layer may read them
+            held = step.shared.setdefault("latent rows", {})
+            what, cached = held.pop(self._held_key(cache), (None, None))
+            if has_latent or what != (self.window, first):
+                cached = torch.empty((sum(kept), D), device=dev, dtype=dtype)
                 ops.latent_gather(cache.k_pages, cached, cu, lens, tables.block_table[first:], step.page_size, count, max(kept), self.window)
+            if cache.read_later:
+                held[self._held_key(cache)] = (self.window, first), cached
             kv = ops.library_mm(cached[:, :R], self.kv_weight)
             ops.latent_rebuilt_attention(q_rows, q_rot, kv, cached, heads_out, gates, cu, lens, count, step.max_seqlen_q, H, R, self.scale,
                                          self.window, sink=self.sink)
@@ -244,18 +250,23 @@ class LatentAttentionMixer(Mixer):
             return linear_into_residual(rows, self.o_weight, fold, next_weight=step.weight_after)
         return linear(rows, self.o_weight, next_weight=step.weight_after)
 
-    def _rebuild_plan(self, step: StepContext, q_rows: torch.Tensor) -> tuple[int, list[int]]:
+    @staticmethod
+    def _held_key(cache: LayerCache) -> tuple[int, int]:
+        return cache.group, cache.k_pages.data_ptr()
+
+    def _rebuild_plan(self, step: StepContext, q_rows: torch.Tensor, cache: LayerCache) -> tuple[int, list[int]]:
         """How many tokens at the step's front go through absorbed queries (all of them, or the single decoded tokens
         beside prompt portions), and how many cached rows each portion behind them keeps."""
         T, B = step.num_tokens, step.num_seqs
-        if self.kv_weight is None or not LATENT_REBUILD or step.max_seqlen_q <= LATENT_DECODE_MAX_TOKENS or len(step.host_seq_lens) != B:
+        if self.kv_weight is None or not LATENT_REBUILD or step.sizing or step.max_seqlen_q <= LATENT_DECODE_MAX_TOKENS or len(step.host_seq_lens) != B:
             return T, []
         if q_rows.stride(0) % 8 or q_rows.data_ptr() % 16:  # the copy engine's rows are 16-byte aligned
             return T, []
         first = step.decode_seqs if step.decode_seqs < B else 0
         portions = [(n, ops.latent_kept_keys(self.window, n, start + n)) for start, n in zip(step.host_seq_starts[first:], step.host_seq_lens[first:])]
         kept = [k for _, k in portions]
-        if sum(kept) * self.kv_weight.shape[0] * 2 > LATENT_REBUILD_MAX_BYTES or not rebuilding_pays(
+        others = sum(rows.numel() for key, (_, rows) in step.shared.get("latent rows", {}).items() if key != self._held_key(cache))
+        if (sum(kept) * (self.kv_weight.shape[0] + self.key_dim) + others) * 2 > LATENT_REBUILD_MAX_BYTES or not rebuilding_pays(
                 portions, self.num_heads, ops._sm_count(q_rows.device), first > 0):
             return T, []
         return first, kept

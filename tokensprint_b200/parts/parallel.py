@@ -58,7 +58,8 @@ class ParallelMixers(Mixer):
                 ops.flush_gemm_chain()
             paged, stateful = i in self._paged, i in self._stateful
             part = LayerCache(group=cache.group if paged else -1, k_pages=cache.k_pages if paged else None,
-                              v_pages=cache.v_pages if paged else None, state=cache.state if stateful else None, writes=cache.writes)
+                              v_pages=cache.v_pages if paged else None, state=cache.state if stateful else None, writes=cache.writes,
+                              read_later=cache.read_later)
             step.weight_after = after if i + 1 == len(self.mixers) else self.mixers[i + 1].first_weight()
             outs.append(m.forward(x, step, part))
         step.weight_after = after
