@@ -28,8 +28,12 @@ LATENT_REBUILD_MAX_BYTES = 256 << 20
 
 def rebuilding_pays(portions: Sequence[tuple[int, int]], heads: int, sms: int, beside_decodes: bool = False) -> bool:
     """Whether a step's prompt portions, as (new tokens, keys kept) each, are faster with rebuilt keys and values.
-    Beside decoded tokens, which go through absorbed queries in any case, the step then has both paths: eight more calls a
-    layer, about 100 us of host time in a step that the host bounds (24 tokens beside 2 x 700: 2.13 against 2.01 ms).
+    Beside decoded tokens, which go through absorbed queries in any case, the step then has both paths, eight more calls a layer.  Such
+    a step is not captured, and its launches take the host 350 to 500 us a layer: while the absorbed attention fits in that, what it
+    takes on the device does not show and the calls do; beyond, the step takes what the device takes.  So there it has to save 300 us a
+    layer.  4, 24 and 64 decoded tokens beside 300 to 8,000 new ones, three models of 2 or 4 such layers, whole steps, absorbed against
+    rebuilt: saving 177 us a layer (1,024 tokens, 16 heads) 1.39 to 2.62 against 1.46 to 2.87 ms, no step the faster; saving 354 (2 x 700,
+    32 heads) 2.17 to 3.66 against 1.81 to 3.12, saving 381 (1,024, 32 heads) 1.82 to 4.37 against 1.52 to 4.34.
 
     Both sides in microseconds, fitted to a sweep on B200 (16 and 32 heads, 1 and 4 portions of 5 to 512 tokens, 5 to 8,192
     keys; the model is within a tenth or 4 us).  Absorbed queries: 32 rows a CTA, 3.75 us per block of 64 keys, one
@@ -43,7 +47,7 @@ def rebuilding_pays(portions: Sequence[tuple[int, int]], heads: int, sms: int, b
 
     absorbed = 18.0 + 3.75 * passes(32, 64, True)
     rebuilt = 26.0 + 2.2e-4 * heads * sum(k for _, k in portions) + 1.75 * passes(256, 96, False)
-    return rebuilt + (150.0 if beside_decodes else 0.0) < absorbed
+    return rebuilt + (300.0 if beside_decodes else 0.0) < absorbed
 
 
 def batched_linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
