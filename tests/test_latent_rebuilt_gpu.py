@@ -197,6 +197,12 @@ def test_plan_of_a_step(monkeypatch):
     assert _plan(monkeypatch, _step([0], [8191])) == (0, [8191])
     assert _plan(monkeypatch, _step([8000], [2000]), window=512) == (0, [10000 - 7489 // 96 * 96])
     assert _plan(monkeypatch, _step([0, 100], [3000, 2000])) == (0, [3000, 2100])
+    step, asked = _step([0, 100], [3000, 2000]), []
+    pays = latent.rebuilding_pays
+    monkeypatch.setattr(latent, "rebuilding_pays", lambda *a: asked.append(a) or pays(*a))
+    for window, heads in ((0, 16), (0, 16), (0, 8), (512, 16), (512, 16)):
+        _plan(monkeypatch, step, heads, window)
+    assert len(asked) == 3, "layers of one kind share the plan of a step"
     many = _step([900] * 4 + [0, 7000], [1] * 4 + [4000, 4000], decode_seqs=4)
     assert _plan(monkeypatch, many) == (4, [4000, 11000])
 

@@ -266,12 +266,19 @@ class LatentAttentionMixer(Mixer):
             return T, []
         if q_rows.stride(0) % 8 or q_rows.data_ptr() % 16:  # the copy engine's rows are 16-byte aligned
             return T, []
-        first = step.decode_seqs if step.decode_seqs < B else 0
-        portions = [(n, ops.latent_kept_keys(self.window, n, start + n)) for start, n in zip(step.host_seq_starts[first:], step.host_seq_lens[first:])]
-        kept = [k for _, k in portions]
-        others = sum(rows.numel() for key, (_, rows) in step.shared.get("latent rows", {}).items() if key != self._held_key(cache))
-        if (sum(kept) * (self.kv_weight.shape[0] + self.key_dim) + others) * 2 > LATENT_REBUILD_MAX_BYTES or not rebuilding_pays(
-                portions, self.num_heads, ops._sm_count(q_rows.device), first > 0):
+        plans = step.shared.setdefault("latent plans", {})  # worked out once a step for all layers of a kind
+        plan = plans.get((self.window, self.num_heads))
+        if plan is None:
+            first = step.decode_seqs if step.decode_seqs < B else 0
+            portions = [(n, ops.latent_kept_keys(self.window, n, start + n)) for start, n in zip(step.host_seq_starts[first:], step.host_seq_lens[first:])]
+            kept = [k for _, k in portions]
+            plan = plans[self.window, self.num_heads] = (
+                first, kept, sum(kept), rebuilding_pays(portions, self.num_heads, ops._sm_count(q_rows.device), first > 0))
+        first, kept, rows, pays = plan
+        if not pays:
+            return T, []
+        others = sum(x.numel() for key, (_, x) in step.shared.get("latent rows", {}).items() if key != self._held_key(cache))
+        if (rows * (self.kv_weight.shape[0] + self.key_dim) + others) * 2 > LATENT_REBUILD_MAX_BYTES:
             return T, []
         return first, kept
 
