@@ -44,8 +44,8 @@ struct RouterGroups {
 
 // The choice of one token by one warp: logits z [E + groups.count] (shared memory; the entries behind the
 // logits are scratch), the bias already in.  A chosen entry becomes NaN, which no comparison prefers, and lane k % 32 keeps
-// choice k: nothing is read back from device memory.  (With earlier choices and weights read back where they had been stored, eight
-// warps of a CTA took 25 us for a choice of 8.)
+// choice k: nothing is read back from device memory.  (With earlier choices and weights read back where they had been stored, a choice
+// of 8 of 16 experts took 32.5 us in tiles, 297 tokens of 2,048, and 12.7 now; with a CTA a token, 33 tokens, 9.3 and 7.2.)
 __device__ __forceinline__ void router_choose(float* z, int E, int top, int renormalize, int score_mode, int* my_ids, float* my_w,
                                               int lane, const float* __restrict__ correction, const RouterGroups& groups) {
   if (score_mode == ROUTER_SCORE_SOFTMAX_ALL) {
