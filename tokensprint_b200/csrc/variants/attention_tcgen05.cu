@@ -1036,12 +1036,14 @@ __global__ void __launch_bounds__(608, 1) attention_tcgen05_pair_kernel(const __
           }
         } else {
 #pragma unroll
-          for (int i = 0; i < PIECE; ++i)
-#pragma unroll
-            for (int g = 0; g < PIECES; ++g) {
-              const int key = kbase + g * PIECE + i;
-              if (key <= row_pos && key >= row_lo) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(v[g][i]));
-            }
+          for (int i = 0; i < PIECE; ++i) {
+            // (one line a piece: as a loop over the pieces this walk spilled 16 / 24 bytes instead of 8 / 8)
+            static_assert(PIECES == 2 || PIECES == 3, "the lines below");
+            const int key0 = kbase + i, key1 = key0 + PIECE, key2 = key1 + PIECE;
+            if (key0 <= row_pos && key0 >= row_lo) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(v[0][i]));
+            if (key1 <= row_pos && key1 >= row_lo) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(v[1][i]));
+            if (PIECES > 2 && key2 <= row_pos && key2 >= row_lo) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(v[PIECES - 1][i]));
+          }
         }
         m_blk = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
       }
