@@ -84,9 +84,10 @@ __device__ __forceinline__ float2 gla_mul2(float2 a, float2 b) {
 // loads of the next round's q, k, z and v are in flight into registers (issued before the updates,
 // used after them), so the recurrence never waits for device memory.
 //
-// The whole portion in one piece (short portions, and steps whose sequences fill the SMs: the same sums whatever the cut).  Scalar
-// arithmetic: in packed pairs (the kernel below with a segment as long as the portion) the longest chain of tokens
-// takes longer, one portion of 500 tokens, 16 heads of 64 x 128: 154 us here, 164 there.
+// The whole portion in one piece (short portions, and steps whose sequences fill the SMs: the same sums whatever the cut).  A kernel
+// of its own with scalar state: one portion of 500 tokens, 16 heads of 64 x 128, takes 154 us here; with the state as pairs of registers it took
+// 164 (scalar arithmetic, 232 bytes of spills instead of 128) or 160 (packed), and inside the kernel of the segments, with scalar state, 4
+// prompts of 500 tokens, 64 heads of 128 x 64, took 730 us instead of 670.
 template <typename TA, int KP>
 __global__ void __launch_bounds__(GLA_THREADS, GLA_MIN_BLOCKS) gla_scan_kernel(
     const TA* __restrict__ q, const TA* __restrict__ k, const TA* __restrict__ v, long long ld_qkv, const float* __restrict__ decay,

@@ -15,8 +15,9 @@
 //                (tile::gather4 copies, 40 ns each, took 981 us where this takes 397: 16,384 pairs of 32 experts, 4,096 -> 2 x 1,536);
 //   warp 5       one elected lane: every tcgen05.mma;
 //   the others   epilogue: a thread has a place and half of its columns, reads its sums from tensor memory and writes them.
-// Bound by the L2 at 48 KB a slice and SM (13 TB/s in all): 8,192 pairs of these experts 241 us, 0.86 PFLOP/s, and 121 us for
-// down (mma.sync tiles of 128 x 128: 863 and 450).
+// 8,192 pairs of these experts 242 us, 0.85 PFLOP/s, and 122 us for down (mma.sync tiles of 128 x 128: 863 and 450): the tensor pipes are
+// busy 62 % of the time that the SMs are, which ask the L2 for 48 KB a slice (42 % of its peak), and 768 items leave the last of six
+// rounds of CTAs a fifth full; 32,768 pairs 748 us, 1.10 PFLOP/s.
 //
 // Few rows (moe_few_kernel; up to 12 pairs per expert on average): the step streams the chosen experts' weights and little
 // else, at a rate that follows the bytes of weights in flight.  Row tiles of 32 places are the MMA's N and the weight rows
@@ -24,6 +25,7 @@
 // hides where a CTA has one item, is spread over 128 threads that each have a weight row and only as many
 // columns as the tile has places (with the places as M one warp did all of it, 5 to 8 us of the 35).  The tokens' rows come by
 // tile::gather4, four rows a copy, only as many as the tile has.
+// 32 experts, 4,096 -> 2 x 1,536, cold L2, gate/up and down: 32 pairs 84 and 46 us (6.3 and 5.7 TB/s), 256 pairs 132 and 66 (6.1 and 6.1 TB/s).
 // 16 experts, 2,048 -> 2 x 1,024, six calls in a graph, gate/up and down: 2 pairs 15.5 and 8.1 us, 8 pairs 15.8 and 8.9, 66 pairs 26.3 and 10.6
 // (the down matrices stay in the L2 in part); tiles of 16 rows on mma.sync, three CTAs an SM, took 22.2 and 11.8, 26.6 and 14.3, 33.1 and 17.6.
 //

@@ -289,8 +289,9 @@ CASE_FILTER = ""  # --case: only the latent-attention cases whose "H=.. B=.. T=.
 
 
 def latent_attention(cfg, timer, pk, rows, device):
-    """The tensor-core latent attention kernel: decode steps (cache bytes against the copy bandwidth)
-    and prompt portions (flops of both products against the bf16 peak)."""
+    """The tensor-core latent attention kernels: decode steps (cache bytes against the copy bandwidth)
+    and prompt portions (flops of both products against the bf16 peak), on the cached rows themselves and on
+    keys and values rebuilt from them."""
     R, rot, page = LATENT["rank"], LATENT["rot"], LATENT["page"]
     D = R + rot
     for H in LATENT["heads"]:
@@ -320,7 +321,31 @@ def latent_attention(cfg, timer, pk, rows, device):
                 pairs = B * (T * (ctx - T) + T * (T + 1) / 2)
                 tf = 2 * pairs * H * (D + R) / 1e12
                 rows.append(("latent attention, prompt", f"H={H} B={B} new={T} keys={ctx}", us, tf / (us * 1e-6), "TFLOP/s", tf / (us * 1e-6) / pk["bf16_tflops"]))
-            del cache, q, out
+                del q, out
+                _rebuilt_attention(timer, pk, rows, device, cache, cu, lens, table, page, gates, H, B, T, ctx, pairs)
+            del cache
+
+
+def _rebuilt_attention(timer, pk, rows, device, cache, cu, lens, table, page, gates, H, B, T, ctx, pairs):
+    dn, dr, dv = ops.LATENT_REBUILT_SIZES
+    R = LATENT["rank"]
+    q = torch.randn(B * T, H * (dn + dr), device=device).bfloat16()
+    q_rot = torch.randn(B * T, H, dr, device=device).bfloat16()
+    weight = (torch.randn(H * (dn + dv), R, device=device) / R ** 0.5).bfloat16()
+    kept = ops.latent_kept_keys(0, T, ctx)
+    gathered = torch.empty(B * kept, R + dr, device=device, dtype=torch.bfloat16)
+    out = torch.empty(B * T, H, dv, device=device, dtype=torch.bfloat16)
+
+    def gather():
+        ops.latent_gather(cache, gathered, cu, lens, table, page, B, kept)
+
+    us = timer(gather)
+    gb = 2 * gathered.numel() * 2 / 1e9
+    rows.append(("latent rows gathered", f"B={B} keys={ctx}", us, gb / (us * 1e-6), "GB/s", gb / (us * 1e-6) / pk["hbm_gbs"]))
+    kv = ops.library_mm(gathered[:, :R], weight)
+    us = timer(lambda: ops.latent_rebuilt_attention(q, q_rot, kv, gathered, out, gates, cu, lens, B, T, H, R, (dn + dr) ** -0.5))
+    tf = 2 * pairs * H * (dn + dr + dv) / 1e12
+    rows.append(("latent attention, prompt, rebuilt keys", f"H={H} B={B} new={T} keys={ctx}", us, tf / (us * 1e-6), "TFLOP/s", tf / (us * 1e-6) / pk["bf16_tflops"]))
 
 
 def routed_experts(cfg, timer, pk, rows, device):
