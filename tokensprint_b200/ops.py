@@ -2599,13 +2599,61 @@ def _gemm_scratch(device: torch.device, M: int, N: int, K: int) -> tuple[int, in
     return got[0], got[1], got[2], stream
 
 
-def gemm_skinny_bf16(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, prefetch: Optional[torch.Tensor] = None) -> None:
+_SIGNATURES["ts_gemm_rows_ssq_tiles"] = _SIGNATURES["ts_gemm_rows_takes_heads"] = [_c_int, _c_int, _c_int]
+_SIGNATURES["ts_gemm_rows_fused"] = [
+    _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_ll, _c_ll, _c_ll, _c_int,
+    _c_int, _c_void_p, _c_int, _c_float, _c_float, _c_void_p, _c_ll, _c_void_p, _c_void_p, _c_void_p, _c_float, _c_int,
+    _c_void_p, _c_ll, _c_void_p,
+]
+_SIGNATURES["ts_gemm_rows_qk_rope"] = [
+    _c_void_p, _c_void_p, _c_int, _c_int, _c_ll, _c_ll, _c_int, _c_int,
+    _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
+    _c_void_p, _c_void_p, _c_float, _c_void_p, _c_void_p,
+    _c_void_p, _c_int, _c_float, _c_float,
+    _c_void_p, _c_ll, _c_void_p,
+]
+_rows_tiles: dict[tuple[int, int, int, bool], int] = {}
+
+
+def _rows_takes(M: int, w: _MatrixFacts, heads: int = 0) -> int:
+    """0 where csrc/gemm_rows.cu does not take the product of M rows with `w`, else how many rows of sums of squares its
+    residual epilogue leaves.  `heads`: for the q/k/v form."""
+    if M > 16 or not w.ok or w.ld % 16 or w.ptr % 32 or w.rows * w.ld * 2 >= 1 << 32 or _chain_open:
+        return 0
+    key = (M, heads or w.rows, w.cols, heads > 0)
+    n = _rows_tiles.get(key)
+    if n is None:
+        n = _rows_tiles[key] = int(_fn("ts_gemm_rows_takes_heads" if heads else "ts_gemm_rows_ssq_tiles")(*key[:3]))
+    return n
+
+
+# Weights up to this size are not asked into the L2 ahead of a product of csrc/gemm_rows.cu: the rings of the chip (19 MB) hold most
+# of them by the time its input is there, and the requests were in the way (a step of one request, 0.6B: 766 us with them, 732
+# without; the larger weights of 8B: 2,889 with, 2,935 without).
+ROWS_HINT_FROM = 24 << 20
+
+
+def _rows_hint(prefetch: Optional[torch.Tensor]) -> tuple[Optional[int], int]:
+    """The address and size of what a product of csrc/gemm_rows.cu asks into the L2 for the one after it."""
+    pf = None if prefetch is None else _facts(prefetch)
+    return (None, 0) if pf is None or pf.nbytes < ROWS_HINT_FROM else (pf.ptr, min(pf.nbytes, GEMM_PREFETCH_BYTES))
+
+
+def gemm_ssq_tiles(num_rows: int, w: torch.Tensor) -> int:
+    """Rows of `ssq_out` that gemm_skinny_fused(..., direct=True) leaves in GEMM_EPILOGUE_RESIDUAL_NORM."""
+    return _rows_takes(num_rows, _facts(w)) or -(-w.shape[0] // 128)
+
+
+def gemm_skinny_bf16(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, prefetch: Optional[torch.Tensor] = None,
+                     direct: bool = False) -> None:
     """out[M,N] = x[M,K] @ w[N,K]^T for M <= 128 on the tcgen05 tensor cores.
 
     x, w bfloat16 with unit inner stride and rows that start on 16-byte boundaries; out
     bfloat16 or float32.  The work is spread evenly over all SMs; tiles that two CTAs share
     meet in a float32 scratch that this wrapper allocates.  `prefetch`: the weights the next
     product will read; the kernel asks for their start to be brought into L2 while it finishes.
+    `direct`: up to 16 rows may run on mma.sync straight from device memory (csrc/gemm_rows.cu), which is faster where it
+    takes the shape; a row's bits then depend on which of the two kernels its step takes.
     """
     if not (x.is_cuda and w.is_cuda and out.is_cuda):
         raise KernelError("gemm_skinny_bf16: CUDA tensors only (there is no CPU path)")
@@ -2617,6 +2665,12 @@ def gemm_skinny_bf16(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, prefet
     N = w.shape[0]
     if w.shape[1] != K or tuple(out.shape) != (M, N) or out.stride(1) != 1 or out.dtype not in (torch.bfloat16, torch.float32):
         raise KernelError(f"gemm_skinny_bf16: shapes disagree: x {tuple(x.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)} {out.dtype}")
+    if direct and _rows_takes(M, _facts(w)):
+        _check("gemm_skinny_bf16", _fn("ts_gemm_rows_fused")(
+            x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, x.stride(0), w.stride(0), out.stride(0), 1 if out.dtype == torch.float32 else 0,
+            GEMM_EPILOGUE_PLAIN, None, 0, 1.0, 0.0, None, 0, None, None, None, 1.0, 0,
+            *_rows_hint(prefetch), _stream()))
+        return
     partial, counters, error, stream = _gemm_scratch(x.device, M, N, K)
     pf = None if prefetch is None else _facts(prefetch)
     _check_product("gemm_skinny_bf16", _fn("ts_gemm_skinny_bf16")(
@@ -2651,6 +2705,7 @@ def gemm_skinny_fused(
     prefetch: Optional[torch.Tensor] = None,
     branch_scale: float = 1.0,
     activation: str = "silu",
+    direct: bool = False,
 ) -> None:
     """x[M,K] @ w[N,K]^T on the tcgen05 tensor cores (M <= 32) with the work of the neighbouring
     small kernels done where each tile is finished.
@@ -2663,6 +2718,7 @@ def gemm_skinny_fused(
       rows of the same outputs; out[M,N/2] bf16 = act(gate) * up (`activation`: one of GLU_ACTIVATIONS).
     mode GEMM_EPILOGUE_RESIDUAL_NORM: hidden[M,N] float32 += branch_scale * product; xprime[M,N] bf16 = hidden *
       norm_weight; ssq_out[ceil(N/128), M] float32 = sums of squares of the new hidden rows.
+    direct: as in gemm_skinny_bf16; ssq_out then has gemm_ssq_tiles(M, w) rows.
     """
     if not gemm_skinny_supported(x, w) or x.shape[0] > GEMM_FUSED_MAX_ROWS:
         raise KernelError(
@@ -2683,7 +2739,7 @@ def gemm_skinny_fused(
             raise KernelError("gemm_skinny_fused: the gate/up blocks need N to be a multiple of 128")
         ldo, out_f32 = out.stride(0), 1 if out.dtype == torch.float32 else 0
     elif mode == GEMM_EPILOGUE_RESIDUAL_NORM:
-        tiles = -(-N // 128)
+        tiles = gemm_ssq_tiles(M, w) if direct else -(-N // 128)
         ok = (
             hidden is not None and hidden.dtype == torch.float32 and tuple(hidden.shape) == (M, N) and hidden.is_contiguous()
             and xprime is not None and xprime.dtype == torch.bfloat16 and tuple(xprime.shape) == (M, N) and xprime.is_contiguous()
@@ -2699,6 +2755,13 @@ def gemm_skinny_fused(
         if scale_ssq.dtype != torch.float32 or not scale_ssq.is_contiguous() or scale_ssq.dim() != 2 or scale_ssq.shape[1] != M:
             raise KernelError("gemm_skinny_fused: scale_ssq must be float32 [tiles, M]")
         scale_tiles = scale_ssq.shape[0]
+    if direct and _rows_takes(M, _facts(w)):
+        _check("gemm_skinny_fused", _fn("ts_gemm_rows_fused")(
+            x.data_ptr(), w.data_ptr(), _ptr(out), M, N, K, x.stride(0), w.stride(0), ldo, out_f32,
+            int(mode), _ptr(scale_ssq), scale_tiles, float(scale_width), float(scale_eps),
+            _ptr(hidden), N, _ptr(norm_weight), _ptr(xprime), _ptr(ssq_out), float(branch_scale), GLU_ACTIVATIONS[activation],
+            *_rows_hint(prefetch), _stream()))
+        return
     partial, counters, error, stream = _gemm_scratch(x.device, M, N, K)
     pf = None if prefetch is None else _facts(prefetch)
     _check_product("gemm_skinny_fused", _fn("ts_gemm_skinny_fused")(
@@ -2756,13 +2819,14 @@ def gemm_qk_rope_store(
     scale_eps: float = 0.0,
     prefetch: Optional[torch.Tensor] = None,
     cos_sin: Optional[torch.Tensor] = None,
+    direct: bool = False,
 ) -> None:
     """The q/k/v projection (w [(nq + 2 nkv) * 128, K], heads of 128) with qk_norm_rope_store's work
     done in the product's epilogue: per-head RMS norm of q and k, rotate-half rotation over the
     whole head (inv_freq [64]) or none, q to q_out [M, nq * 128], k and v to their cache slots.
     At most 32 rows.  scale_ssq as in gemm_skinny_fused.  cos_sin: rope_cos_sin(positions, inv_freq,
     M) if the caller has it (the epilogue then reads the angles' cosines and sines instead of
-    computing them)."""
+    computing them).  direct: as in gemm_skinny_bf16."""
     nq, nkv, d = num_heads, num_kv_heads, GEMM_QK_ROPE_HEAD_DIM
     if not gemm_skinny_supported(x, w) or x.shape[0] > GEMM_FUSED_MAX_ROWS:
         raise KernelError(f"gemm_qk_rope_store: needs bfloat16, at most {GEMM_FUSED_MAX_ROWS} rows and 16-byte aligned rows")
@@ -2789,6 +2853,14 @@ def gemm_qk_rope_store(
     if cos_sin is not None and (inv_freq is None or cos_sin.dtype != torch.float32 or not cos_sin.is_cuda or not cos_sin.is_contiguous()
                                 or cos_sin.numel() < M * d):
         raise KernelError(f"gemm_qk_rope_store: cos_sin must be float32 [M, {d // 2}, 2] on the device, beside inv_freq")
+    if direct and _rows_takes(M, _facts(w), nq + 2 * nkv):
+        _check("gemm_qk_rope_store", _fn("ts_gemm_rows_qk_rope")(
+            x.data_ptr(), w.data_ptr(), M, K, x.stride(0), w.stride(0), nq, nkv,
+            q_out.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), slot_mapping.data_ptr(), positions.data_ptr(),
+            _ptr(q_norm_weight), _ptr(k_norm_weight), float(eps), _ptr(inv_freq), _ptr(cos_sin),
+            _ptr(scale_ssq), scale_tiles, float(scale_width), float(scale_eps),
+            *_rows_hint(prefetch), _stream()))
+        return
     partial, counters, error, stream = _gemm_scratch(x.device, M, w.shape[0], K)
     pf = None if prefetch is None else _facts(prefetch)
     _check_product("gemm_qk_rope_store", _fn("ts_gemm_skinny_qk_rope")(

@@ -1,8 +1,8 @@
 """Matrix product of activations with a row-major [out, in] weight.
 
 bfloat16: steps of up to SKINNY_ROWS tokens (decode, short portions) stream the weights through
-the engine's own tcgen05 kernel (csrc/gemm_tcgen05.cu); larger steps use the library
-GEMM (cuBLAS through torch.mm), as the reference does with nn.Linear
+the engine's own kernels (csrc/gemm_rows.cu up to 16 rows where it takes the shape, else
+csrc/gemm_tcgen05.cu); larger steps use the library GEMM (cuBLAS through torch.mm), as the reference does with nn.Linear
 (engine/nn/attention.py:122-135, engine/nn/layers.py:61-66).  float32 runs use the
 engine's own FFMA kernel, so no reduced-precision matrix mode can slip into the 32-bit
 path whatever torch's global switches say.
@@ -41,7 +41,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
         if not x.is_cuda:
             raise ops.KernelError("linear: there is no CPU path")
         if T <= SKINNY_ROWS and ops.gemm_skinny_supported(x, weight):
-            ops.gemm_skinny_bf16(x, weight, out, next_weight)
+            ops.gemm_skinny_bf16(x, weight, out, next_weight, direct=True)
         else:
             ops.library_mm(x, weight, out=out)
     else:
@@ -71,7 +71,7 @@ def linear_scaled(x: "PreNormed | torch.Tensor", weight: torch.Tensor, next_weig
     if isinstance(x, torch.Tensor):
         return linear_float32_out(x, weight) if float32_out else linear(x, weight, next_weight=next_weight)
     out = torch.empty((x.x.shape[0], weight.shape[0]), device=x.x.device, dtype=torch.float32 if float32_out else x.x.dtype)
-    ops.gemm_skinny_fused(x.x, weight, out=out, scale_ssq=x.ssq, scale_width=x.width, scale_eps=x.eps, prefetch=next_weight)
+    ops.gemm_skinny_fused(x.x, weight, out=out, scale_ssq=x.ssq, scale_width=x.width, scale_eps=x.eps, prefetch=next_weight, direct=True)
     return out
 
 
@@ -82,10 +82,10 @@ def linear_swiglu(x: "PreNormed | torch.Tensor", gate_up_blocks: torch.Tensor, n
     xt = x if isinstance(x, torch.Tensor) else x.x
     out = torch.empty((xt.shape[0], gate_up_blocks.shape[0] // 2), device=xt.device, dtype=xt.dtype)
     if isinstance(x, torch.Tensor):
-        ops.gemm_skinny_fused(x, gate_up_blocks, out=out, mode=ops.GEMM_EPILOGUE_SWIGLU, prefetch=next_weight, activation=activation)
+        ops.gemm_skinny_fused(x, gate_up_blocks, out=out, mode=ops.GEMM_EPILOGUE_SWIGLU, prefetch=next_weight, activation=activation, direct=True)
     else:
         ops.gemm_skinny_fused(x.x, gate_up_blocks, out=out, mode=ops.GEMM_EPILOGUE_SWIGLU, scale_ssq=x.ssq, scale_width=x.width,
-                              scale_eps=x.eps, prefetch=next_weight, activation=activation)
+                              scale_eps=x.eps, prefetch=next_weight, activation=activation, direct=True)
     return out
 
 
@@ -96,9 +96,9 @@ def linear_into_residual(x: torch.Tensor, weight: torch.Tensor, fold: "ResidualN
 
     T, N = x.shape[0], weight.shape[0]
     xprime = torch.empty((T, N), device=x.device, dtype=x.dtype)
-    ssq = torch.empty((-(-N // 128), T), device=x.device, dtype=torch.float32)
+    ssq = torch.empty((ops.gemm_ssq_tiles(T, weight), T), device=x.device, dtype=torch.float32)
     ops.gemm_skinny_fused(x, weight, mode=ops.GEMM_EPILOGUE_RESIDUAL_NORM, hidden=fold.hidden, norm_weight=fold.norm.weight,
-                          xprime=xprime, ssq_out=ssq, prefetch=next_weight, branch_scale=fold.scale)
+                          xprime=xprime, ssq_out=ssq, prefetch=next_weight, branch_scale=fold.scale, direct=True)
     return PreNormed(xprime, ssq, fold.norm.width, fold.norm.eps)
 
 
@@ -108,7 +108,7 @@ def linear_float32_out(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
         return linear(x, weight)
     if x.shape[0] <= SKINNY_ROWS and ops.gemm_skinny_supported(x, weight):
         out = torch.empty((x.shape[0], weight.shape[0]), device=x.device, dtype=torch.float32)
-        ops.gemm_skinny_bf16(x, weight, out)
+        ops.gemm_skinny_bf16(x, weight, out, direct=True)
         return out
     if not x.is_cuda or x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16:
         raise ops.KernelError(f"linear: bfloat16 CUDA tensors wanted (there is no CPU path), got {x.dtype} on {x.device}")
