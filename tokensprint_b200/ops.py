@@ -2142,12 +2142,13 @@ def attention_decode_splits(num_seqs: int, num_kv_heads: int, max_context: int, 
     best, best_cost = 1, None
     for s in range(1, min(blocks, 16) + 1):
         waves = -(-pairs * s // slots)
-        # per CTA: start and merge (about 3 us) + 2.5 us per 64-key block; merging the splits costs
-        # little inside a thread-block cluster (up to 8 CTAs, all running at once), more through
-        # scratch and a kernel of its own
+        # per CTA: start and merge (about 3 us) + 1.65 us per 64-key block; merging the splits costs
+        # little inside a thread-block cluster (up to 8 CTAs, all running at once), and a kernel and its seams
+        # through scratch (decode steps of 0.6B, 28 layers, 4 / 8 / 16 splits: one request of 200 keys 677 / 675 / 733 us, of
+        # 2,000 keys 972 / 787 / 875; four of 500 keys 749 / 726 / 853)
         in_cluster = ATTENTION_CLUSTER_MERGE and s <= 8 and pairs * s <= slots
-        merge = 0.0 if s == 1 else (0.8 if in_cluster else 1.5 + 0.15 * s)
-        cost = waves * (3.0 + 2.5 * -(-blocks // s)) + merge
+        merge = 0.0 if s == 1 else (0.8 if in_cluster else 7.2)
+        cost = waves * (3.0 + 1.65 * -(-blocks // s)) + merge
         if best_cost is None or cost < best_cost - 1e-9:
             best, best_cost = s, cost
     return best
