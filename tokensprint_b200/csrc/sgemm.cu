@@ -1,25 +1,25 @@
 // True float32 matrix product on CUDA cores: C[M, N] = A[M, K] * W[N, K]^T.
 //
 // This is the float32 path's GEMM: FFMA only, no tensor cores and no reduced-precision
-// mode.  Each output element is the sum of four chains of fused multiply-adds, (s0 + s1) + (s2 + s3):
-// chain i takes the runs of 16 along k whose number is i modulo 4, in increasing order.  Both kernels
-// below and all their tiles do exactly that, so a row's result does not depend on which other rows
+// mode.  Each output element is the sum of eight chains of fused multiply-adds: chain i of four takes the runs of 16 along k
+// whose number is i modulo 4, in increasing order, its even and its odd k apart (the packed instruction multiplies two
+// neighbours along k at once, as they lie in memory), and the element is (s0 + s1) + (s2 + s3) with s_i = even + odd.
+// All kernels below and all their tiles do exactly that, so a row's result does not depend on which other rows
 // share the launch, nor on the size of the step.
 // W is row-major [out, in] as the reference's Linear weights are (engine/nn/attention.py:
 // 122-135).
 //
-// Two kernels.  The tiled one: four groups of warps, one per chain, work on the same 64 x 64 (or
-// 32 x 32) outputs, each on its own run of 16 of every 64 along k; the runs come by 16-byte cp.async
-// into two buffers in the layout they have in memory, rows 20 floats apart, so that the eight rows a
-// warp reads at once meet no bank twice; a thread holds 8 x 8 (4 x 4) sums.  The four groups are there
-// because a layer's product of a few hundred rows has too few tiles to keep the schedulers busy: with one chain
-// a tile (64 x 64, 64 threads) 1.3 warps stood on a scheduler and issued an instruction every 3.4 cycles.
-// The other kernel is for steps of up to 16 rows, which are bound by reading W once: 16 or 32 rows of W
-// and all of A pass through a ring of four slices of 64 along k, a thread owns one row of W and a few of A.
-// Measured (B200, 333 rows; before: 64 x 64 tiles, 4 x 4 sums a thread, loads a word at a time and nothing in
-// flight, 270 to 400 us a product of this size): N x K = 4,096 x 1,024 104 us (27 TFLOP/s), 6,144 x 1,024 134 us,
-// 1,024 x 3,072 177 us (96 tiles); 512 rows of 8,192 x 2,048 450 us (38 TFLOP/s: one wavefront of shared memory
-// per value and warp holds it at about half of the FFMA rate); 64 rows of 4,096 x 2,048 41 us.
+// Scalar FFMA with three different registers issues 2.6 times a cycle and SM on B200, the packed one 1.9 times with twice the
+// work (83 against 124 products a cycle), hence the pairs.
+//
+// Three kernels.  The wide one, where its tiles fill the chip: 32 x 128 outputs, see there.  The small tiles: four groups of
+// warps, one per chain, work on the same 32 x 32 outputs, each on its own run of 16 of every 64 along k; the runs come
+// by 16-byte cp.async into two buffers in the layout they have in memory, rows 20 floats apart, so that the eight rows a
+// warp reads at once meet no bank twice; a thread holds 4 x 4 pairs of sums.  The third kernel is for steps of up to 16 rows, which are
+// bound by reading W once: 16 or 32 rows of W and all of A pass through a ring of four slices of 64 along k, a thread owns
+// one row of W and a few of A.
+// Measured (B200, 333 rows, us; before: 64 x 64 tiles, scalar): N x K = 4,096 x 1,024 104 -> 93, 6,144 x 1,024 134 -> 124, 1,024 x 2,048
+// 120 -> 63, 1,024 x 3,072 175 -> 91; 512 rows of 8,192 x 2,048 451 -> 408 (42 TFLOP/s); 64 rows of 6,144 x 1,024 59 -> 35.
 #include "common.cuh"
 
 namespace {
@@ -37,6 +37,11 @@ __device__ __forceinline__ void cp_async16(float* dst, const float* src, bool re
   const int bytes = real ? 16 : 0;  // 0: the piece is filled with zeros
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(src), "r"(bytes));
 }
+
+// Two products at once: (x, y) += (a.x b.x, a.y b.y), each rounded as fmaf rounds it.
+typedef unsigned long long Pair;
+__device__ __forceinline__ void fma_pair(Pair& acc, Pair a, Pair b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
+__device__ __forceinline__ float pair_sum(Pair v) { return __uint_as_float((unsigned)v) + __uint_as_float((unsigned)(v >> 32)); }
 
 constexpr int CHAINS = 4, RUN = 16, RSTRIDE = RUN + 4;
 
@@ -73,11 +78,11 @@ __global__ void __launch_bounds__(CHAINS * (BM / TM) * (BN / TN), 2) sgemm_tile_
     }
     if (VEC) asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  float acc[TM][TN];
+  Pair acc[TM][TN];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0;
   const int rounds = (p.K + CHAINS * RUN - 1) / (CHAINS * RUN);
   fetch(chain, 0);
   for (int it = 0; it < rounds; ++it) {
@@ -87,20 +92,20 @@ __global__ void __launch_bounds__(CHAINS * (BM / TM) * (BN / TN), 2) sgemm_tile_
     const float* as = sm + (it & 1) * STAGE + chain * ROWS * RSTRIDE + ty * RSTRIDE;
     const float* ws = sm + (it & 1) * STAGE + chain * ROWS * RSTRIDE + (BM + tx) * RSTRIDE;
 #pragma unroll
-    for (int k = 0; k < RUN; k += 2) {
-      float2 a[TM], b[TN];
+    for (int k = 0; k < RUN; k += 4) {
+      ulonglong2 a[TM], b[TN];
 #pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float2*>(as + i * TY * RSTRIDE + k);
+      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(as + i * TY * RSTRIDE + k);
 #pragma unroll
-      for (int j = 0; j < TN; ++j) b[j] = *reinterpret_cast<const float2*>(ws + j * TX * RSTRIDE + k);
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]);
+      for (int j = 0; j < TN; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(ws + j * TX * RSTRIDE + k);
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
+        for (int j = 0; j < TN; ++j) fma_pair(acc[i][j], a[i].x, b[j].x);
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) fma_pair(acc[i][j], a[i].y, b[j].y);
     }
   }
   __syncthreads();
@@ -108,13 +113,107 @@ __global__ void __launch_bounds__(CHAINS * (BM / TM) * (BN / TN), 2) sgemm_tile_
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) sums[(ty + i * TY) * (BN + 1) + tx + j * TX] = acc[i][j];
+    for (int j = 0; j < TN; ++j) sums[(ty + i * TY) * (BN + 1) + tx + j * TX] = pair_sum(acc[i][j]);
   __syncthreads();
   for (int i = threadIdx.x; i < BM * BN; i += THREADS) {
     const int r = i / BN, c = i % BN;
     if (m0 + r >= p.M || n0 + c >= p.N) continue;
     const float* s = sm + r * (BN + 1) + c;
     C[(size_t)(m0 + r) * p.ldc + n0 + c] = (s[0] + s[BM * (BN + 1)]) + (s[2 * BM * (BN + 1)] + s[3 * BM * (BN + 1)]);
+  }
+}
+
+// ---- many tiles: 32 x 128 outputs, a warp 16 rows x 128 columns ----
+
+constexpr int WM = 32, WN = 128, WROWS = WM + WN, WCHAIN = WROWS * RSTRIDE, WSTAGE = CHAINS * WCHAIN, WSTAGES = 3, W_RM = 16, W_RN = 4;
+
+// Two warps a chain, 16 of the tile's rows each; a lane has the columns lane, lane + 32, .. + 96.  The 16 values of A that a warp
+// multiplies are the same for all its lanes, and 16 bytes of them cost a third of what 16 different bytes a lane cost (1.4 against 0.46
+// such reads a cycle).  The chains wait for their own copies only (a named barrier of two warps).  What is left is latency at two
+// warps a scheduler; four warps a chain with 8 rows each: 64 -> 65 us, the loop over k unrolled: 64 -> 67.
+__global__ void __launch_bounds__(CHAINS * 32 * (WM / W_RM), 1) sgemm_wide_kernel(const Product p) {
+  constexpr int GROUP = 32 * (WM / W_RM), STEP = GROUP / 4;  // threads of a chain; rows they copy at once
+  ts_pdl_prologue();
+  extern __shared__ __align__(16) float sm[];  // [WSTAGES][CHAINS][WROWS][RSTRIDE], then the sums [CHAINS][WM][WN + 1]
+  const float* __restrict__ A = p.A + (size_t)blockIdx.z * p.batch_a;
+  const float* __restrict__ W = p.W + (size_t)blockIdx.z * p.batch_w;
+  float* __restrict__ C = p.C + (size_t)blockIdx.z * p.batch_c;
+  const int chain = threadIdx.x / GROUP, tid = threadIdx.x % GROUP, part = tid >> 5, lane = tid & 31;
+  const int m0 = blockIdx.y * WM, n0 = blockIdx.x * WN;
+  // a thread copies 16 bytes of every 32nd row: one of A, four of W
+  const int row = tid >> 2, col = (tid & 3) * 4;
+  const float* a_src = A + (size_t)(m0 + row) * p.lda + col;
+  const float* w_src = W + (size_t)(n0 + row) * p.ldw + col;
+  float* dst = sm + chain * WCHAIN + row * RSTRIDE + col;
+  auto fetch_w = [&](int round) {
+    const int k = (round * CHAINS + chain) * RUN;
+    const bool in = k + col < p.K;  // K is a multiple of 4: a piece lies inside the row or behind it
+#pragma unroll
+    for (int j = 0; j < WN / STEP; ++j) {
+      const bool real = in && n0 + row + j * STEP < p.N;
+      cp_async16(dst + round % WSTAGES * WSTAGE + (WM + j * STEP) * RSTRIDE, real ? w_src + (size_t)j * STEP * p.ldw + k : p.W, real);
+    }
+  };
+  auto fetch_a = [&](int round) {
+    const int k = (round * CHAINS + chain) * RUN;
+#pragma unroll
+    for (int j = 0; j < WM / STEP; ++j) {
+      const bool real = k + col < p.K && m0 + row + j * STEP < p.M;
+      cp_async16(dst + round % WSTAGES * WSTAGE + j * STEP * RSTRIDE, real ? a_src + (size_t)j * STEP * p.lda + k : p.A, real);
+    }
+  };
+  Pair acc[W_RM][W_RN];
+#pragma unroll
+  for (int i = 0; i < W_RM; ++i)
+#pragma unroll
+    for (int j = 0; j < W_RN; ++j) acc[i][j] = 0;
+  const int rounds = (p.K + CHAINS * RUN - 1) / (CHAINS * RUN);
+#pragma unroll
+  for (int r = 0; r < WSTAGES - 1; ++r) {
+    if (r < rounds) {
+      fetch_w(r);
+      fetch_a(r);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  for (int it = 0; it < rounds; ++it) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(WSTAGES - 2) : "memory");
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + chain), "n"(GROUP) : "memory");  // the chain's run is here, and the one before has been read
+    if (it + WSTAGES - 1 < rounds) {
+      fetch_w(it + WSTAGES - 1);
+      fetch_a(it + WSTAGES - 1);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const float* as = sm + it % WSTAGES * WSTAGE + chain * WCHAIN + part * W_RM * RSTRIDE;
+    const float* ws = sm + it % WSTAGES * WSTAGE + chain * WCHAIN + (WM + lane) * RSTRIDE;
+#pragma unroll 1
+    for (int k = 0; k < RUN; k += 4) {
+      ulonglong2 b[W_RN];
+#pragma unroll
+      for (int j = 0; j < W_RN; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(ws + j * 32 * RSTRIDE + k);
+#pragma unroll
+      for (int i = 0; i < W_RM; ++i) {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(as + i * RSTRIDE + k);
+#pragma unroll
+        for (int j = 0; j < W_RN; ++j) fma_pair(acc[i][j], a.x, b[j].x);
+#pragma unroll
+        for (int j = 0; j < W_RN; ++j) fma_pair(acc[i][j], a.y, b[j].y);
+      }
+    }
+  }
+  __syncthreads();
+  constexpr int PLANE = WM * (WN + 1);
+  static_assert(CHAINS * PLANE <= WSTAGES * WSTAGE, "the sums fit where the runs were");
+#pragma unroll
+  for (int i = 0; i < W_RM; ++i)
+#pragma unroll
+    for (int j = 0; j < W_RN; ++j) sm[chain * PLANE + (part * W_RM + i) * (WN + 1) + lane + j * 32] = pair_sum(acc[i][j]);
+  __syncthreads();
+  for (int i = threadIdx.x; i < WM * WN; i += CHAINS * GROUP) {
+    const int r = i / WN, c = i % WN;
+    if (m0 + r >= p.M || n0 + c >= p.N) continue;
+    const float* q = sm + r * (WN + 1) + c;
+    C[(size_t)(m0 + r) * p.ldc + n0 + c] = (q[0] + q[PLANE]) + (q[2 * PLANE] + q[3 * PLANE]);
   }
 }
 
@@ -155,11 +254,11 @@ __global__ void __launch_bounds__(128) sgemm_few_rows_kernel(const Product p) {
   }
   const int n = threadIdx.x % BN, g = threadIdx.x / BN;
   static_assert(FK == CHAINS * RUN, "a slice holds one run of every chain");
-  float acc[CHAINS][RM];
+  Pair acc[CHAINS][RM];
 #pragma unroll
   for (int c = 0; c < CHAINS; ++c)
 #pragma unroll
-    for (int i = 0; i < RM; ++i) acc[c][i] = 0.f;
+    for (int i = 0; i < RM; ++i) acc[c][i] = 0;
   for (int s = 0; s < slices; ++s) {
     asm volatile("cp.async.wait_group %0;" ::"n"(FSTAGES - 2) : "memory");
     __syncthreads();  // slice s is here for everybody, and slice s - 1 has been read
@@ -171,15 +270,13 @@ __global__ void __launch_bounds__(128) sgemm_few_rows_kernel(const Product p) {
     for (int k = 0; k < RUN; k += 4) {
 #pragma unroll
       for (int c = 0; c < CHAINS; ++c) {
-        const float4 w = *reinterpret_cast<const float4*>(ws + c * RUN + k);
+        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(ws + c * RUN + k);
 #pragma unroll
         for (int i = 0; i < RM; ++i) {
           if (g + i * G < p.M) {
-            const float4 a = *reinterpret_cast<const float4*>(as + (g + i * G) * FSTRIDE + c * RUN + k);
-            acc[c][i] = fmaf(a.x, w.x, acc[c][i]);
-            acc[c][i] = fmaf(a.y, w.y, acc[c][i]);
-            acc[c][i] = fmaf(a.z, w.z, acc[c][i]);
-            acc[c][i] = fmaf(a.w, w.w, acc[c][i]);
+            const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(as + (g + i * G) * FSTRIDE + c * RUN + k);
+            fma_pair(acc[c][i], a.x, w.x);
+            fma_pair(acc[c][i], a.y, w.y);
           }
         }
       }
@@ -188,7 +285,7 @@ __global__ void __launch_bounds__(128) sgemm_few_rows_kernel(const Product p) {
   if (n0 + n < p.N) {
 #pragma unroll
     for (int i = 0; i < RM; ++i)
-      if (g + i * G < p.M) C[(size_t)(g + i * G) * p.ldc + n0 + n] = (acc[0][i] + acc[1][i]) + (acc[2][i] + acc[3][i]);
+      if (g + i * G < p.M) C[(size_t)(g + i * G) * p.ldc + n0 + n] = (pair_sum(acc[0][i]) + pair_sum(acc[1][i])) + (pair_sum(acc[2][i]) + pair_sum(acc[3][i]));
   }
 }
 
@@ -202,6 +299,15 @@ int launch_tiles(const Product& p, int batch, cudaStream_t s) {
     if (e != cudaSuccess) return (int)e;
   }
   return ts_launch(sgemm_tile_kernel<BM, BN, TM, TN, VEC>, grid, dim3(CHAINS * (BM / TM) * (BN / TN)), smem, s, p);
+}
+
+int launch_wide(const Product& p, int batch, cudaStream_t s) {
+  const dim3 grid((p.N + WN - 1) / WN, (p.M + WM - 1) / WM, batch);
+  if (grid.y > 65535 || batch > 65535) return TS_ERR_UNSUPPORTED_SIZE;
+  constexpr size_t smem = (size_t)WSTAGES * WSTAGE * sizeof(float);
+  const cudaError_t e = cudaFuncSetAttribute(sgemm_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  return ts_launch(sgemm_wide_kernel, grid, dim3(CHAINS * 32 * (WM / W_RM)), smem, s, p);
 }
 
 template <int BN>
@@ -226,8 +332,12 @@ int launch(const Product& p, int batch, cudaStream_t s) {
   const bool vec = aligned16(p) && p.K % 4 == 0;
   if (p.M <= FEW_ROWS && vec)
     return (long long)batch * ((p.N + 31) / 32) >= 148 ? launch_few_rows<32>(p, batch, s) : launch_few_rows<16>(p, batch, s);
-  const long long tiles = (long long)batch * ((p.M + 63) / 64) * ((p.N + 63) / 64);
-  if (tiles >= 80) return vec ? launch_tiles<64, 64, 8, 8, true>(p, batch, s) : launch_tiles<64, 64, 8, 8, false>(p, batch, s);
+  // In multiples of what a full round of small tiles takes (two a SM: 22 us a 1,024 of K), a round of wide ones costs 1.4, with the
+  // small ones' last round partly empty: 1,024 x 2,048, 333 rows (352 small tiles, 88 wide) 63 against 66; 4,096 x 1,024, 128 rows
+  // (512, 128) 34 against 45; 2,048 x 2,048, 333 rows (704, 176) 117 against 105; 2,048 x 2,048, 100 rows (256, 64) 63 against 45.
+  const long long wide = (long long)batch * ((p.M + WM - 1) / WM) * ((p.N + WN - 1) / WN);
+  const long long small = (long long)batch * ((p.M + 31) / 32) * ((p.N + 31) / 32), rounds = (wide + 147) / 148;
+  if (vec && small * 100 >= 296 * rounds * (rounds == 1 ? 118 : 130)) return launch_wide(p, batch, s);
   return vec ? launch_tiles<32, 32, 4, 4, true>(p, batch, s) : launch_tiles<32, 32, 4, 4, false>(p, batch, s);
 }
 
