@@ -93,14 +93,10 @@ __device__ __forceinline__ void conv_store8(__nv_bfloat16* p, const float (&v)[8
 }
 
 template <typename TI, typename TO>
-__global__ void __launch_bounds__(128) causal_conv_vec_kernel(const TI* __restrict__ xin, long long ld, const float* __restrict__ taps_w,
-                                                              const float* __restrict__ bias, const float* __restrict__ in_bias, int K,
-                                                              float* __restrict__ conv_state, long long slot_stride, const int* __restrict__ state_slots,
-                                                              const int* __restrict__ cu_seqlens, const int* __restrict__ seq_index,
-                                                              TO* __restrict__ out, long long ld_out, int C, int act, int add_input) {
-  ts_pdl_prologue();
-  const int t = blockIdx.x, col = (blockIdx.y * 128 + threadIdx.x) * 8;
-  if (col >= C) return;
+__device__ __forceinline__ void conv_token(const TI* __restrict__ xin, long long ld, const float* __restrict__ taps_w, const float* __restrict__ bias,
+                                           const float* __restrict__ in_bias, int K, float* __restrict__ conv_state, long long slot_stride,
+                                           const int* __restrict__ state_slots, const int* __restrict__ cu_seqlens, const int* __restrict__ seq_index,
+                                           TO* __restrict__ out, long long ld_out, int C, int act, int add_input, int t, int col) {
   const int b = seq_index[t];
   float acc[8], cur[8], w[8], xb[8];
   if (b < 0) {
@@ -149,11 +145,81 @@ __global__ void __launch_bounds__(128) causal_conv_vec_kernel(const TI* __restri
 }
 
 template <typename TI, typename TO>
+__global__ void __launch_bounds__(128) causal_conv_vec_kernel(const TI* __restrict__ xin, long long ld, const float* __restrict__ taps_w,
+                                                              const float* __restrict__ bias, const float* __restrict__ in_bias, int K,
+                                                              float* __restrict__ conv_state, long long slot_stride, const int* __restrict__ state_slots,
+                                                              const int* __restrict__ cu_seqlens, const int* __restrict__ seq_index,
+                                                              TO* __restrict__ out, long long ld_out, int C, int act, int add_input) {
+  ts_pdl_prologue();
+  const int col = (blockIdx.y * 128 + threadIdx.x) * 8;
+  if (col >= C) return;
+  conv_token(xin, ld, taps_w, bias, in_bias, K, conv_state, slot_stride, state_slots, cu_seqlens, seq_index, out, ld_out, C, act, add_input, blockIdx.x, col);
+}
+
+// Four taps and long portions: a thread takes eight channels of TOK neighbouring tokens, so that the taps are read once and a row once
+// instead of four times (8,191 x 2,048 bfloat16: 63 us with a token a thread, most of it the 128 bytes of taps per token).  All rows
+// of a tile are asked for at once where it lies inside one portion, three tokens or more from its start; the
+// sums are those of the kernel above, in its order.  Other tiles go token by token through it.
+template <typename TI, typename TO, int TOK>
+__global__ void __launch_bounds__(128) causal_conv4_tile_kernel(const TI* __restrict__ xin, long long ld, const float* __restrict__ taps_w,
+                                                                const float* __restrict__ bias, const float* __restrict__ in_bias,
+                                                                float* __restrict__ conv_state, long long slot_stride, const int* __restrict__ state_slots,
+                                                                const int* __restrict__ cu_seqlens, const int* __restrict__ seq_index,
+                                                                TO* __restrict__ out, long long ld_out, int T, int C, int act, int add_input) {
+  ts_pdl_prologue();
+  constexpr int K = 4;
+  const int t0 = blockIdx.x * TOK, col = (blockIdx.y * 128 + threadIdx.x) * 8;
+  if (col >= C) return;
+  const int b0 = seq_index[t0];
+  if (b0 < 0 || t0 - cu_seqlens[b0] < K - 1 || t0 + TOK > cu_seqlens[b0 + 1]) {
+    for (int t = t0; t < min(t0 + TOK, T); ++t)
+      conv_token(xin, ld, taps_w, bias, in_bias, K, conv_state, slot_stride, state_slots, cu_seqlens, seq_index, out, ld_out, C, act, add_input, t, col);
+    return;
+  }
+  float w[K][8], xb[8], ab[8], win[K][8];
+  TI rows[TOK + K - 1][8];
+#pragma unroll
+  for (int r = 0; r < TOK + K - 1; ++r)
+#pragma unroll
+    for (int i = 0; i < (int)sizeof(TI) / 2; ++i)
+      reinterpret_cast<uint4*>(rows[r])[i] = reinterpret_cast<const uint4*>(xin + (size_t)(t0 - (K - 1) + r) * ld + col)[i];
+#pragma unroll
+  for (int j = 0; j < K; ++j) conv_load8(taps_w + (size_t)j * C + col, w[j]);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    xb[i] = in_bias ? in_bias[col + i] : 0.f;
+    ab[i] = bias ? bias[col + i] : 0.f;
+  }
+#pragma unroll
+  for (int r = 0; r < TOK + K - 1; ++r) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) win[r % K][i] = ts_to_float(rows[r][i]) + xb[i];
+    if (r < K - 1) continue;
+    float acc[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      acc[i] = ab[i];
+#pragma unroll
+      for (int j = 0; j < K; ++j) acc[i] = fmaf(w[j][i], win[(r + 1 + j) % K][i], acc[i]);
+      if (act == CONV_ACT_SILU) acc[i] = acc[i] / (1.f + expf(-acc[i]));
+      if (add_input) acc[i] += win[r % K][i];
+    }
+    conv_store8(out + (size_t)(t0 + r - (K - 1)) * ld_out + col, acc);
+  }
+}
+
+template <typename TI, typename TO>
 static int conv_launch(const void* xin, long long ld, const float* taps_w, const float* bias, const float* in_bias, int K, float* conv_state,
                        long long slot_stride, const int* state_slots, const int* cu_seqlens, const int* seq_index, void* out, long long ld_out,
                        int T, int C, int act, int add_input, cudaStream_t s) {
   const bool aligned = C % 8 == 0 && ld % 8 == 0 && ld_out % 8 == 0 && slot_stride % 4 == 0 &&
                        (((uintptr_t)xin | (uintptr_t)out | (uintptr_t)conv_state | (uintptr_t)taps_w) & 15) == 0;
+  // tiles of 8 tokens (4 of float32) where they still give every SM a few CTAs; in steps of few tokens a tile would be a chain
+  constexpr int TOK = sizeof(TI) == 2 ? 8 : 4;
+  const int cols = (C / 8 + 127) / 128;
+  if (aligned && K == 4 && (long long)((T + TOK - 1) / TOK) * cols >= 148)
+    return ts_launch(causal_conv4_tile_kernel<TI, TO, TOK>, dim3((T + TOK - 1) / TOK, cols), dim3(128), 0, s, (const TI*)xin, ld, taps_w, bias, in_bias,
+                     conv_state, slot_stride, state_slots, cu_seqlens, seq_index, (TO*)out, ld_out, T, C, act, add_input);
   if (aligned)
     return ts_launch(causal_conv_vec_kernel<TI, TO>, dim3(T, (C / 8 + 127) / 128), dim3(128), 0, s, (const TI*)xin, ld, taps_w, bias, in_bias, K, conv_state,
                      slot_stride, state_slots, cu_seqlens, seq_index, (TO*)out, ld_out, C, act, add_input);

@@ -380,6 +380,50 @@ __global__ void moe_combine_kernel(const TA* __restrict__ pair_out, const TA* __
   out[idx] = ts_from_float<TA>(sum);
 }
 
+// The same sums, 16 bytes of a row per thread and a block row per token: rows of whole 16-byte pieces.  Bound by reading the pairs'
+// rows once; an element a thread with its 64-bit division took 47 us for 2,048 tokens x 4 choices of 4,096 bfloat16.
+template <typename TA>
+__global__ void __launch_bounds__(128) moe_combine_vec_kernel(const TA* __restrict__ pair_out, const TA* __restrict__ shared, TA* __restrict__ out,
+                                                              const float* __restrict__ pair_weight, int N, int top, const int* __restrict__ ids, int E,
+                                                              const TA* __restrict__ x) {
+  ts_pdl_prologue();
+  constexpr int V = 16 / sizeof(TA);
+  const int t = blockIdx.y, n = (blockIdx.x * 128 + threadIdx.x) * V;
+  if (n >= N) return;
+  const size_t at = (size_t)t * N + n;
+  float sum[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) sum[i] = 0.f;
+  auto add = [&](const TA* from, float w) {
+    const uint4 raw = *reinterpret_cast<const uint4*>(from);
+    const TA* v = reinterpret_cast<const TA*>(&raw);
+#pragma unroll
+    for (int i = 0; i < V; ++i) sum[i] += ts_to_float(v[i]) * w;
+  };
+#pragma unroll 4
+  for (int k = 0; k < top; ++k) {
+    const int pair = t * top + k;
+    const bool identity = ids != nullptr && ids[pair] >= E;  // no expert ran for this pair: its output is the input row
+    add(identity ? x + at : pair_out + (size_t)pair * N + n, pair_weight ? pair_weight[pair] : 1.f);
+  }
+  if (shared) add(shared + at, 1.f);
+  uint4 raw;
+  TA* v = reinterpret_cast<TA*>(&raw);
+#pragma unroll
+  for (int i = 0; i < V; ++i) v[i] = ts_from_float<TA>(sum[i]);
+  *reinterpret_cast<uint4*>(out + at) = raw;
+}
+
+template <typename TA>
+static bool moe_combine_vec(const void* pair_out, const void* shared, void* out, const float* pair_weight, int T, int N, int top, const int* ids, int E,
+                            const void* x, cudaStream_t s, int* status) {
+  constexpr int V = 16 / sizeof(TA);
+  if (N % V || T > 65535 || (long long)T * top >= (1ll << 31) || (((uintptr_t)pair_out | (uintptr_t)shared | (uintptr_t)out | (uintptr_t)x) & 15)) return false;
+  *status = ts_launch(moe_combine_vec_kernel<TA>, dim3((N / V + 127) / 128, T), dim3(128), 0, s, (const TA*)pair_out, (const TA*)shared, (TA*)out, pair_weight,
+                      N, top, ids, E, (const TA*)x);
+  return true;
+}
+
 TS_EXPORT int ts_moe_combine(const void* pair_out, const void* shared, void* out, const float* pair_weight, int act_dtype, int T, int N,
                              int top, const int* ids, int E, const void* x, void* stream) {
   if (T <= 0) return 0;
@@ -387,6 +431,10 @@ TS_EXPORT int ts_moe_combine(const void* pair_out, const void* shared, void* out
   const size_t total = (size_t)T * N;
   const unsigned blocks = (unsigned)((total + 255) / 256);
   cudaStream_t s = (cudaStream_t)stream;
+  int status = 0;
+  if (act_dtype == TS_DTYPE_F32 ? moe_combine_vec<float>(pair_out, shared, out, pair_weight, T, N, top, ids, E, x, s, &status)
+                                : act_dtype == TS_DTYPE_BF16 && moe_combine_vec<__nv_bfloat16>(pair_out, shared, out, pair_weight, T, N, top, ids, E, x, s, &status))
+    return status;
   if (act_dtype == TS_DTYPE_F32)
     return ts_launch(moe_combine_kernel<float>, dim3(blocks), dim3(256), 0, s, (const float*)pair_out, (const float*)shared, (float*)out, pair_weight, N, top, total, ids, E, (const float*)x);
   if (act_dtype == TS_DTYPE_BF16)
