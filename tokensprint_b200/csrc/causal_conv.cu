@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(128) causal_conv_vec_kernel(const TI* __restri
 }
 
 // Four taps and long portions: a thread takes eight channels of TOK neighbouring tokens, so that the taps are read once and a row once
-// instead of four times (8,191 x 2,048 bfloat16: 63 us with a token a thread, most of it the 128 bytes of taps per token).  All rows
+// instead of four times (8,191 x 2,048 bfloat16: 63 us with a token a thread, most of it the 128 bytes of taps per token, 24 so).  All rows
 // of a tile are asked for at once where it lies inside one portion, three tokens or more from its start; the
 // sums are those of the kernel above, in its order.  Other tiles go token by token through it.
 template <typename TI, typename TO, int TOK>

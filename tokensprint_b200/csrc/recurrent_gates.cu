@@ -189,7 +189,7 @@ __global__ void ssm_conv_kernel(const TA* __restrict__ xin, long long ld, const 
 }
 
 // Four taps and rows of whole 16-byte pieces: a thread takes eight channels of TOK neighbouring tokens, with the taps and the
-// rows in registers (the kernel above reads a tap of another line per lane and load: 54 us for 1,024 tokens of 4,352 channels).
+// rows in registers (the kernel above reads a tap of another line per lane and load: 54 us for a portion of 1,024 tokens of the width-2,048 design, 18 so).
 // The rows of a tile that lies inside one portion, three tokens or more from its start, are asked for at once; other
 // tokens take the inputs before their portion from the state.  The same sums in the same order.  The last block rows (blockIdx.x
 // >= conv_blocks) work out the heads' step sizes and decays.
