@@ -9,17 +9,18 @@ import torch
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
 LENS = [1, 2, 3, 4, 5, 1201, 7, 8, 9, 30, 1, 400, 3]  # portions that start anywhere in a tile, end in one, fill none
+LONG = [1, 2, 3, 4, 5, 3201, 7, 8, 9, 30, 1, 2800, 3]  # the same, long enough for tiles at 2,056 bfloat16 channels
 
 
-def portions(dtype, C, pad, seed):
+def portions(dtype, C, pad, seed, lens=LENS):
     """Rows of a step with `pad` padded lanes behind them, on a 16-byte boundary and one entry off it, with kept inputs."""
     g = torch.Generator(device=DEV).manual_seed(seed)
-    n, T = len(LENS), sum(LENS) + pad
+    n, T = len(lens), sum(lens) + pad
     wide = torch.randn(T, C + 16, generator=g, device=DEV).to(dtype)
     off = torch.empty(T, C + 16, device=DEV, dtype=dtype)
     off[:, 1:1 + C] = wide[:, :C]
-    cu = torch.tensor([0] + torch.tensor(LENS).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
-    seq = torch.repeat_interleave(torch.arange(n, device=DEV), torch.tensor(LENS, device=DEV)).int()
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    seq = torch.repeat_interleave(torch.arange(n, device=DEV), torch.tensor(lens, device=DEV)).int()
     seq = torch.cat([seq, torch.full((pad,), -1, device=DEV, dtype=torch.int32)])
     state = torch.randn(n + 2, 3 * C, generator=g, device=DEV)
     slots = torch.randperm(n + 2, generator=g, device=DEV)[:n].int()
@@ -48,6 +49,35 @@ def test_causal_convolution(C, pad, add_input, biased, in_dtype, out_dtype):
     want = want + h[3:] if add_input else want * torch.sigmoid(want)
     err = float((got[0][0][a:a + 1201].double() - want).norm() / want.norm())
     assert err < (1e-6 if out_dtype == torch.float32 else 2 ** -8)
+
+
+@pytest.mark.parametrize("in_dtype,out_dtype", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32), (torch.bfloat16, torch.bfloat16)])
+@pytest.mark.parametrize("pad,add_input,biased", [(3, True, False), (0, False, True)])
+def test_causal_convolution_in_tiles(pad, add_input, biased, in_dtype, out_dtype):
+    from tokensprint_b200 import ops
+
+    C = 2056  # the last block of columns nearly empty
+    g, x, x_off, cu, seq, state, slots = portions(in_dtype, C, pad, 7 + pad, LONG)
+    narrow = in_dtype == torch.bfloat16
+    assert ops._fn("ts_causal_conv_tile_tokens")(1 if narrow else 0, x.shape[0], len(LONG), C) == (8 if narrow else 4)
+    taps = torch.randn(4, C, generator=g, device=DEV)
+    bias, in_bias = torch.randn(2, C, generator=g, device=DEV).unbind(0) if biased else (None, None)
+    got = []
+    for rows in (x, x_off):
+        out, kept = torch.full((x.shape[0], C), float("nan"), device=DEV, dtype=out_dtype), state.clone()
+        ops.causal_conv(rows, taps, bias, kept, slots, cu, seq, len(LONG), out, activation=None if add_input else "silu", add_input=add_input, in_bias=in_bias)
+        got.append((out, kept))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("T,n,C,narrow", [(128, 128, 10240, True), (512, 512, 10240, True), (512, 512, 10240, False), (320, 320, 4096, True),
+                                          (1424, 26, 4096, True), (2304, 257, 8192, True), (1024, 128, 10240, True), (512, 128, 10240, False),
+                                          (2048, 1, 8, True), (576, 65, 4096, False), (64, 64, 10240, False)])
+def test_steps_of_many_portions_take_no_tiles_of_tokens(T, n, C, narrow):
+    """Decode batches, and prompts beside so many requests that a tile's chain of single tokens would be the step."""
+    from tokensprint_b200 import ops
+
+    assert ops._fn("ts_causal_conv_tile_tokens")(1 if narrow else 0, T, n, C) == 1
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])

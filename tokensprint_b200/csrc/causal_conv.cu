@@ -208,16 +208,27 @@ __global__ void __launch_bounds__(128) causal_conv4_tile_kernel(const TI* __rest
   }
 }
 
+// How many neighbouring tokens a thread takes: 8 (4 of float32), or 1 for the kernels with a token a thread.  A tile that holds a portion's start, or
+// many portions, goes token by token, a chain of about 15 us (10 in float32) however small the step is, so tiles are for steps whose
+// rows alone take longer than that and whose portions are long.  The lines, us, a token a thread against tiles: bfloat16, one
+// prompt, 2,048 x 2,048 14 : 15, x 4,096 24 : 21; 7 x 509, x 2,048 23 : 23, x 4,096 43 : 34; 24 single tokens beside 2 x 700, x 4,096
+// 20 : 23, x 8,192 35 : 35, x 10,240 46 : 43; 64 x 16, x 10,240 33 : 32; 128 x 8 34 : 44; 512 single tokens, x 10,240 33 : 52.  float32,
+// 1,024 x 2,048 9.3 : 9.2, x 4,096 16 : 13; 64 single tokens beside 512, x 4,096 13 : 14, x 8,192 20 : 18; 128 x 4, x 10,240 23 : 27.
+static int conv_tile_tokens(bool narrow, int T, int num_seqs, int C) {
+  const long long work = (long long)T * C;
+  if (!narrow) return T >= 8ll * num_seqs && work >= 4000000 ? 4 : 1;
+  return T >= 16ll * num_seqs && work >= (num_seqs <= 8 ? 8000000 : 12000000) ? 8 : 1;
+}
+
 template <typename TI, typename TO>
 static int conv_launch(const void* xin, long long ld, const float* taps_w, const float* bias, const float* in_bias, int K, float* conv_state,
                        long long slot_stride, const int* state_slots, const int* cu_seqlens, const int* seq_index, void* out, long long ld_out,
-                       int T, int C, int act, int add_input, cudaStream_t s) {
+                       int T, int num_seqs, int C, int act, int add_input, cudaStream_t s) {
   const bool aligned = C % 8 == 0 && ld % 8 == 0 && ld_out % 8 == 0 && slot_stride % 4 == 0 &&
                        (((uintptr_t)xin | (uintptr_t)out | (uintptr_t)conv_state | (uintptr_t)taps_w) & 15) == 0;
-  // tiles of 8 tokens (4 of float32) where they still give every SM a few CTAs; in steps of few tokens a tile would be a chain
   constexpr int TOK = sizeof(TI) == 2 ? 8 : 4;
   const int cols = (C / 8 + 127) / 128;
-  if (aligned && K == 4 && (long long)((T + TOK - 1) / TOK) * cols >= 148)
+  if (aligned && K == 4 && conv_tile_tokens(sizeof(TI) == 2, T, num_seqs, C) == TOK)
     return ts_launch(causal_conv4_tile_kernel<TI, TO, TOK>, dim3((T + TOK - 1) / TOK, cols), dim3(128), 0, s, (const TI*)xin, ld, taps_w, bias, in_bias,
                      conv_state, slot_stride, state_slots, cu_seqlens, seq_index, (TO*)out, ld_out, T, C, act, add_input);
   if (aligned)
@@ -231,16 +242,21 @@ static int conv_launch(const void* xin, long long ld, const float* taps_w, const
 
 TS_EXPORT int ts_causal_conv(const void* xin, int in_dtype, long long ld, const float* taps_w, const float* bias, const float* in_bias, int K,
                              float* conv_state, long long slot_stride, const int* state_slots, const int* cu_seqlens, const int* seq_index, void* out,
-                             int out_dtype, long long ld_out, int T, int C, int act, int add_input, void* stream) {
+                             int out_dtype, long long ld_out, int T, int num_seqs, int C, int act, int add_input, void* stream) {
   if (T <= 0) return 0;
   if (C <= 0 || K < 1 || (act != CONV_ACT_NONE && act != CONV_ACT_SILU) || (K > 1 && conv_state == nullptr)) return TS_ERR_BAD_ARGUMENT;
   cudaStream_t s = (cudaStream_t)stream;
 #define CONV_CASE(TI, TO) \
-  return conv_launch<TI, TO>(xin, ld, taps_w, bias, in_bias, K, conv_state, slot_stride, state_slots, cu_seqlens, seq_index, out, ld_out, T, C, act, add_input, s)
+  return conv_launch<TI, TO>(xin, ld, taps_w, bias, in_bias, K, conv_state, slot_stride, state_slots, cu_seqlens, seq_index, out, ld_out, T, num_seqs, C, act, add_input, s)
   if (in_dtype == TS_DTYPE_F32 && out_dtype == TS_DTYPE_F32) CONV_CASE(float, float);
   if (in_dtype == TS_DTYPE_F32 && out_dtype == TS_DTYPE_BF16) CONV_CASE(float, __nv_bfloat16);
   if (in_dtype == TS_DTYPE_BF16 && out_dtype == TS_DTYPE_F32) CONV_CASE(__nv_bfloat16, float);
   if (in_dtype == TS_DTYPE_BF16 && out_dtype == TS_DTYPE_BF16) CONV_CASE(__nv_bfloat16, __nv_bfloat16);
 #undef CONV_CASE
   return TS_ERR_BAD_ARGUMENT;
+}
+
+// The tokens that a thread of ts_causal_conv takes with four taps and 16-byte aligned rows.
+TS_EXPORT int ts_causal_conv_tile_tokens(int in_dtype, int T, int num_seqs, int C) {
+  return C % 8 == 0 ? conv_tile_tokens(in_dtype == TS_DTYPE_BF16, T, num_seqs, C) : 1;
 }

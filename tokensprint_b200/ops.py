@@ -892,7 +892,8 @@ _SIGNATURES.update({
                        _c_void_p, _c_void_p, _c_void_p, _c_ll, _c_float, _c_void_p],
     "ts_softcap_rows": [_c_void_p, _c_ll, _c_float, _c_void_p],
     "ts_causal_conv": [_c_void_p, _c_int, _c_ll, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_ll, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
-                       _c_int, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_void_p],
+                       _c_int, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p],
+    "ts_causal_conv_tile_tokens": [_c_int, _c_int, _c_int, _c_int],
     "ts_delta_scan": [_c_void_p, _c_ll, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_ll, _c_void_p, _c_ll, _c_int, _c_int, _c_void_p, _c_void_p,
                       _c_void_p, _c_ll, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_float, _c_int,
                       _c_void_p],
@@ -1135,7 +1136,7 @@ def causal_conv(xin: torch.Tensor, taps: torch.Tensor, bias: Optional[torch.Tens
         raise KernelError(f"causal_conv: activation must be one of {list(CONV_ACTIVATIONS)}, got {activation!r}")
     _check("causal_conv", _fn("ts_causal_conv")(
         xin.data_ptr(), _act_code("xin", xin), xin.stride(0), taps.data_ptr(), _ptr(bias), _ptr(in_bias), K, state_ptr,
-        state_stride, state_slots.data_ptr(), cu_seqlens.data_ptr(), seq_index.data_ptr(), out.data_ptr(), _act_code("out", out), out.stride(0), T, C,
+        state_stride, state_slots.data_ptr(), cu_seqlens.data_ptr(), seq_index.data_ptr(), out.data_ptr(), _act_code("out", out), out.stride(0), T, int(num_seqs), C,
         CONV_ACTIVATIONS[activation], 1 if add_input else 0, _stream()))
 
 
