@@ -2126,7 +2126,14 @@ def attention_decode_plan_context(max_context: int, window: int = 0) -> int:
     return max(1, min(max_context, cap))
 
 
-def attention_decode_splits(num_seqs: int, num_kv_heads: int, max_context: int, head_dim: int = 128) -> int:
+# Up to this many keys a step's few pairs of a sequence and a KV head are split over one cluster of up to eight CTAs; steps that may
+# meet longer contexts take up to sixteen and a merge through scratch.  Attention alone, 8 KV heads of 128, us, 8 CTAs in a
+# cluster : 16 through scratch (11 for four sequences): one sequence of 200 keys 6.2 : 8.2, 1,000 6.9 : 11.3, 2,000 9.2 : 12.0, 3,500 13.9 :
+# 14.1, 4,000 15.6 : 14.9, 8,000 29 : 22, 32,000 108 : 63; four of 200 7.4 : 8.9, 2,000 12.1 : 12.8, 4,000 19.4 : 19.2, 32,000 121 : 95.
+ATTENTION_CLUSTER_REACH = 4096
+
+
+def attention_decode_splits(num_seqs: int, num_kv_heads: int, max_context: int, head_dim: int = 128, reach: int = 0) -> int:
     """How many CTAs share the keys of one sequence in a decode step.
 
     Each (sequence, KV head) pair is one unit of work that `splits` CTAs divide evenly.  The
@@ -2134,22 +2141,29 @@ def attention_decode_splits(num_seqs: int, num_kv_heads: int, max_context: int, 
     heads); the step takes ceil(pairs * splits / slots) waves, each as long as one CTA's
     share, so the count is chosen to fill whole waves: one wave for small batches, and for
     batches with more pairs than slots a count that makes the last wave nearly full.
+    `max_context`: the context the count is planned for; `reach`: the longest the step can meet, where that is more.
     """
     slots = _decode_slots(head_dim)
     pairs = max(1, num_seqs * num_kv_heads)
     blocks = max(1, -(-max_context // 64))
     if _os.environ.get("TS_DECODE_SPLITS"):
         return max(1, min(int(_os.environ["TS_DECODE_SPLITS"]), blocks, ATTENTION_MMA_MAX_SPLITS))
+    # Steps so small that a full cluster of every pair stands on the chip: a key block costs 1.65 us, and the second kernel of
+    # more than eight splits with its seams 7.2 (decode steps of 0.6B, 28 layers, 4 / 8 / 16 splits: one request of 200 keys
+    # 677 / 675 / 733 us, of 2,000 keys 972 / 787 / 875; four of 500 keys 749 / 726 / 853).  Larger steps keep
+    # the numbers below: with these, 20 sequences of 8 KV heads would take two splits and 40 one, faster than the even-share kernel for equal lengths
+    # (attention alone, 40 of 1,000 keys 33 : 54 us) and slower for unequal ones (100 to 2,000 keys 57 : 50, and 43 with the four splits of layers
+    # the even-share kernel does not know; one of 8,000 beside 200s 208 : 37).
+    small = ATTENTION_CLUSTER_MERGE and pairs * 8 <= slots and max(reach, max_context) <= ATTENTION_CLUSTER_REACH + 64
     best, best_cost = 1, None
     for s in range(1, min(blocks, 16) + 1):
         waves = -(-pairs * s // slots)
-        # per CTA: start and merge (about 3 us) + 1.65 us per 64-key block; merging the splits costs
-        # little inside a thread-block cluster (up to 8 CTAs, all running at once), and a kernel and its seams
-        # through scratch (decode steps of 0.6B, 28 layers, 4 / 8 / 16 splits: one request of 200 keys 677 / 675 / 733 us, of
-        # 2,000 keys 972 / 787 / 875; four of 500 keys 749 / 726 / 853)
+        # per CTA: start and merge (about 3 us) + a 64-key block's time; merging the splits costs
+        # little inside a thread-block cluster (up to 8 CTAs, all running at once), more through
+        # scratch and a kernel of its own
         in_cluster = ATTENTION_CLUSTER_MERGE and s <= 8 and pairs * s <= slots
-        merge = 0.0 if s == 1 else (0.8 if in_cluster else 7.2)
-        cost = waves * (3.0 + 1.65 * -(-blocks // s)) + merge
+        merge = 0.0 if s == 1 else (0.8 if in_cluster else (7.2 if small else 1.5 + 0.15 * s))
+        cost = waves * (3.0 + (1.65 if small else 2.5) * -(-blocks // s)) + merge
         if best_cost is None or cost < best_cost - 1e-9:
             best, best_cost = s, cost
     return best

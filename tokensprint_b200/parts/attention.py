@@ -412,7 +412,8 @@ class AttentionMixer(Mixer):
         # divides its own keys evenly.
         reach = min(self.window, self.chunk) if self.window and self.chunk else self.window or self.chunk  # the most keys a query sees
         context = ops.attention_decode_plan_context(step.max_context_len, reach)
-        splits = ops.attention_decode_splits(count, nkv, context, d)
+        longest = min(step.max_context_len, reach + 64) if reach else step.max_context_len
+        splits = ops.attention_decode_splits(count, nkv, context, d, reach=longest)
         # (the even-share decode kernel knows neither a block bound nor a sink nor a score cap)
         if (self.chunk == 0 and self.sink is None and self.head_sinks is None and self.softcap == 0.0 and self.distance is None
                 and ops.attention_decode_prefers_flat(count, nkv, splits, d)
