@@ -112,6 +112,23 @@ def test_sgemm_same_sums_in_every_kernel(M, N, K, pad):
     assert torch.equal(batch[0], out) and torch.equal(batch[1], out)
 
 
+@pytest.mark.parametrize("M", [1, 2, 4, 5, 8, 9, 12, 13, 16, 17, 65, 300])
+@pytest.mark.parametrize("N,K", [(4740, 1028), (4740, 452), (520, 1092), (33, 4096)])
+def test_sgemm_same_sums_over_many_rounds(M, N, K):
+    """As above with a K of many rounds of 64 and remainders: the rings of all kernels wrap, and rows and columns end inside a tile
+    (N = 4,740: rows of W by 32 or tiles of 32 x 128, which run three rounds ahead; the others: rows of W by 16 or tiles of 32 x 32)."""
+    from tokensprint_b200 import ops
+
+    a, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV)
+    out = torch.full((M, N), float("nan"), device=DEV)
+    ops.sgemm_nt(a, w, out)
+    assert float((out.double() - a.double() @ w.double().T).abs().max()) < 4e-7 * math.sqrt(K) * float(out.abs().max())
+    for m in {0, M // 2, M - 1}:
+        alone = torch.full((1, N), float("nan"), device=DEV)
+        ops.sgemm_nt(a[m : m + 1], w, alone)
+        assert torch.equal(alone[0], out[m])
+
+
 # ---------------------------------------------------------------------------
 # q/k norm + rope + store
 

@@ -9,17 +9,17 @@
 // W is row-major [out, in] as the reference's Linear weights are (engine/nn/attention.py:
 // 122-135).
 //
-// Scalar FFMA with three different registers issues 2.6 times a cycle and SM on B200, the packed one 1.9 times with twice the
-// work (83 against 124 products a cycle), hence the pairs.
-//
-// Three kernels.  The wide one, where its tiles fill the chip: 32 x 128 outputs, see there.  The small tiles: four groups of
-// warps, one per chain, work on the same 32 x 32 outputs, each on its own run of 16 of every 64 along k; the runs come
-// by 16-byte cp.async into two buffers in the layout they have in memory, rows 20 floats apart, so that the eight rows a
-// warp reads at once meet no bank twice; a thread holds 4 x 4 pairs of sums.  The third kernel is for steps of up to 16 rows, which are
+// Three kernels.  The wide one, where its tiles fill the chip: 32 x 128 outputs, see there; it multiplies in packed pairs, since scalar FFMA with
+// three different registers issues 2.6 times a cycle and SM on B200, the packed one 1.9 times with twice the work (83 against
+// 124 products a cycle).  The small tiles: four groups of warps, one per chain, work on the same 32 x 32 outputs, each on its own
+// run of 16 of every 64 along k; the runs come by 16-byte cp.async into two buffers in the layout they have in memory, rows 20 floats apart, so that the
+// eight rows a warp reads at once meet no bank twice; a thread holds 4 x 4 pairs of sums.  The third kernel is for steps of up to 16 rows, which are
 // bound by reading W once: 16 or 32 rows of W and all of A pass through a ring of four slices of 64 along k, a thread owns
-// one row of W and a few of A.
-// Measured (B200, 333 rows, us; before: 64 x 64 tiles, scalar): N x K = 4,096 x 1,024 104 -> 93, 6,144 x 1,024 134 -> 124, 1,024 x 2,048
-// 120 -> 63, 1,024 x 3,072 175 -> 91; 512 rows of 8,192 x 2,048 451 -> 408 (42 TFLOP/s); 64 rows of 6,144 x 1,024 59 -> 35.
+// one row of W and a few of A.  These two are bound by the latency of their chains, not by issue: packed pairs, in the same order, made them
+// slower (100 rows of 2,048 x 2,048 45 us, scalar 40; 1 row of 6,144 x 1,024 27 and 12, of 151,936 x 1,024 259 and 105).
+// Measured (B200, us; before: four chains, 64 x 64 scalar tiles): 333 rows, N x K = 4,096 x 1,024 104 -> 93, 6,144 x 1,024 134 -> 124, 1,024 x 2,048
+// 86 -> 63, 1,024 x 3,072 127 -> 90; 512 rows of 8,192 x 2,048 450 -> 407 (42 TFLOP/s); 64 rows of 6,144 x 1,024 45 -> 34; 1 / 8 / 16 rows of
+// 6,144 x 1,024 19 / 21 / 24 -> 12 / 20 / 25, of 151,936 x 1,024 189 / 217 / 254 -> 105 / 202 / 266.
 #include "common.cuh"
 
 namespace {
@@ -78,11 +78,11 @@ __global__ void __launch_bounds__(CHAINS * (BM / TM) * (BN / TN), 2) sgemm_tile_
     }
     if (VEC) asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  Pair acc[TM][TN];
+  float2 acc[TM][TN];  // the sums over the even and over the odd k of the chain
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0;
+    for (int j = 0; j < TN; ++j) acc[i][j] = make_float2(0.f, 0.f);
   const int rounds = (p.K + CHAINS * RUN - 1) / (CHAINS * RUN);
   fetch(chain, 0);
   for (int it = 0; it < rounds; ++it) {
@@ -92,20 +92,20 @@ __global__ void __launch_bounds__(CHAINS * (BM / TM) * (BN / TN), 2) sgemm_tile_
     const float* as = sm + (it & 1) * STAGE + chain * ROWS * RSTRIDE + ty * RSTRIDE;
     const float* ws = sm + (it & 1) * STAGE + chain * ROWS * RSTRIDE + (BM + tx) * RSTRIDE;
 #pragma unroll
-    for (int k = 0; k < RUN; k += 4) {
-      ulonglong2 a[TM], b[TN];
+    for (int k = 0; k < RUN; k += 2) {
+      float2 a[TM], b[TN];
 #pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(as + i * TY * RSTRIDE + k);
+      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float2*>(as + i * TY * RSTRIDE + k);
 #pragma unroll
-      for (int j = 0; j < TN; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(ws + j * TX * RSTRIDE + k);
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) fma_pair(acc[i][j], a[i].x, b[j].x);
+      for (int j = 0; j < TN; ++j) b[j] = *reinterpret_cast<const float2*>(ws + j * TX * RSTRIDE + k);
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) fma_pair(acc[i][j], a[i].y, b[j].y);
+        for (int j = 0; j < TN; ++j) acc[i][j].x = fmaf(a[i].x, b[j].x, acc[i][j].x);
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j].y = fmaf(a[i].y, b[j].y, acc[i][j].y);
     }
   }
   __syncthreads();
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(CHAINS * (BM / TM) * (BN / TN), 2) sgemm_tile_
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) sums[(ty + i * TY) * (BN + 1) + tx + j * TX] = pair_sum(acc[i][j]);
+    for (int j = 0; j < TN; ++j) sums[(ty + i * TY) * (BN + 1) + tx + j * TX] = acc[i][j].x + acc[i][j].y;
   __syncthreads();
   for (int i = threadIdx.x; i < BM * BN; i += THREADS) {
     const int r = i / BN, c = i % BN;
@@ -221,9 +221,14 @@ __global__ void __launch_bounds__(CHAINS * 32 * (WM / W_RM), 1) sgemm_wide_kerne
 
 constexpr int FEW_ROWS = 16, FK = 64, FSTAGES = 4, FSTRIDE = FK + 4;  // rows of FK + 4 floats: 16-byte reads of 8 neighbour rows meet no bank twice
 
+template <int R>
+struct Rows {
+  static constexpr int N = R;
+};
+
 // 128 threads; BN rows of W; thread (n, g) has the output row n and the rows g, g + G, ... of A (G = 128 / BN).
-template <int BN>
-__global__ void __launch_bounds__(128) sgemm_few_rows_kernel(const Product p) {
+template <int BN, bool ALL_ROWS>
+__global__ void __launch_bounds__(128, ALL_ROWS ? 1 : 4) sgemm_few_rows_kernel(const Product p) {
   constexpr int G = 128 / BN, RM = FEW_ROWS / G;
   extern __shared__ __align__(16) float sm[];  // FSTAGES x [BN + FEW_ROWS][FSTRIDE]
   constexpr int STAGE = (BN + FEW_ROWS) * FSTRIDE;
@@ -254,11 +259,32 @@ __global__ void __launch_bounds__(128) sgemm_few_rows_kernel(const Product p) {
   }
   const int n = threadIdx.x % BN, g = threadIdx.x / BN;
   static_assert(FK == CHAINS * RUN, "a slice holds one run of every chain");
-  Pair acc[CHAINS][RM];
+  float2 acc[CHAINS][RM];  // the sums over the even and over the odd k of each chain
 #pragma unroll
   for (int c = 0; c < CHAINS; ++c)
 #pragma unroll
-    for (int i = 0; i < RM; ++i) acc[c][i] = 0;
+    for (int i = 0; i < RM; ++i) acc[c][i] = make_float2(0.f, 0.f);
+  // A slice's products with `count` of this thread's rows, from number `first` on.  A row at a time, its runs unrolled, unless the warp has all of its
+  // rows: then a value of W is read once for them.  (All rows together behind a condition each: 30 against 22 us at 4 rows of 1,024 x 3,072.)
+  auto multiply = [&](const float* ws, const float* as, int first, auto count) {
+#pragma unroll
+    for (int k = 0; k < RUN; k += 4) {
+#pragma unroll
+      for (int c = 0; c < CHAINS; ++c) {
+        const float4 w = *reinterpret_cast<const float4*>(ws + c * RUN + k);
+#pragma unroll
+        for (int j = 0; j < decltype(count)::N; ++j) {
+          const float4 a = *reinterpret_cast<const float4*>(as + (g + (first + j) * G) * FSTRIDE + c * RUN + k);
+          float2& sum = acc[c][first + j];
+          sum.x = fmaf(a.x, w.x, sum.x);
+          sum.y = fmaf(a.y, w.y, sum.y);
+          sum.x = fmaf(a.z, w.z, sum.x);
+          sum.y = fmaf(a.w, w.w, sum.y);
+        }
+      }
+    }
+  };
+  const int g0 = threadIdx.x / 32 * 32 / BN;  // the lowest g of this warp
   for (int s = 0; s < slices; ++s) {
     asm volatile("cp.async.wait_group %0;" ::"n"(FSTAGES - 2) : "memory");
     __syncthreads();  // slice s is here for everybody, and slice s - 1 has been read
@@ -266,26 +292,25 @@ __global__ void __launch_bounds__(128) sgemm_few_rows_kernel(const Product p) {
     asm volatile("cp.async.commit_group;" ::: "memory");
     const float* ws = sm + (s % FSTAGES) * STAGE + n * FSTRIDE;
     const float* as = sm + (s % FSTAGES) * STAGE + BN * FSTRIDE;
+    if (ALL_ROWS || g0 + (RM - 1) * G < p.M) {
+      multiply(ws, as, 0, Rows<RM>());
+    } else {
 #pragma unroll
-    for (int k = 0; k < RUN; k += 4) {
-#pragma unroll
-      for (int c = 0; c < CHAINS; ++c) {
-        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(ws + c * RUN + k);
-#pragma unroll
-        for (int i = 0; i < RM; ++i) {
-          if (g + i * G < p.M) {
-            const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(as + (g + i * G) * FSTRIDE + c * RUN + k);
-            fma_pair(acc[c][i], a.x, w.x);
-            fma_pair(acc[c][i], a.y, w.y);
-          }
-        }
+      for (int i = 0; i < RM; ++i) {
+        if (g0 + i * G >= p.M) break;
+        multiply(ws, as, i, Rows<1>());
       }
     }
   }
   if (n0 + n < p.N) {
 #pragma unroll
     for (int i = 0; i < RM; ++i)
-      if (g + i * G < p.M) C[(size_t)(g + i * G) * p.ldc + n0 + n] = (pair_sum(acc[0][i]) + pair_sum(acc[1][i])) + (pair_sum(acc[2][i]) + pair_sum(acc[3][i]));
+      if (g + i * G < p.M) {
+        float v[CHAINS];
+#pragma unroll
+        for (int c = 0; c < CHAINS; ++c) v[c] = acc[c][i].x + acc[c][i].y;
+        C[(size_t)(g + i * G) * p.ldc + n0 + n] = (v[0] + v[1]) + (v[2] + v[3]);
+      }
   }
 }
 
@@ -310,15 +335,15 @@ int launch_wide(const Product& p, int batch, cudaStream_t s) {
   return ts_launch(sgemm_wide_kernel, grid, dim3(CHAINS * 32 * (WM / W_RM)), smem, s, p);
 }
 
-template <int BN>
+template <int BN, bool ALL_ROWS>
 int launch_few_rows(const Product& p, int batch, cudaStream_t s) {
   constexpr size_t smem = (size_t)FSTAGES * (BN + FEW_ROWS) * FSTRIDE * sizeof(float);
   if (batch > 65535) return TS_ERR_UNSUPPORTED_SIZE;
   if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(sgemm_few_rows_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = cudaFuncSetAttribute(sgemm_few_rows_kernel<BN, ALL_ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
-  return ts_launch(sgemm_few_rows_kernel<BN>, dim3((p.N + BN - 1) / BN, 1, batch), dim3(128), smem, s, p);
+  return ts_launch(sgemm_few_rows_kernel<BN, ALL_ROWS>, dim3((p.N + BN - 1) / BN, 1, batch), dim3(128), smem, s, p);
 }
 
 bool aligned16(const Product& p) {
@@ -326,18 +351,21 @@ bool aligned16(const Product& p) {
   return ((reinterpret_cast<size_t>(p.A) | reinterpret_cast<size_t>(p.W)) & 15) == 0 && (strides & 3) == 0;
 }
 
-// Which kernel: the choice changes the time only, never a bit of the result.  Small tiles where the
-// large ones would leave half of the SMs without one.
+// Which kernel: the choice changes the time only, never a bit of the result.
 int launch(const Product& p, int batch, cudaStream_t s) {
   const bool vec = aligned16(p) && p.K % 4 == 0;
-  if (p.M <= FEW_ROWS && vec)
-    return (long long)batch * ((p.N + 31) / 32) >= 148 ? launch_few_rows<32>(p, batch, s) : launch_few_rows<16>(p, batch, s);
-  // In multiples of what a full round of small tiles takes (two a SM: 22 us a 1,024 of K), a round of wide ones costs 1.4, with the
-  // small ones' last round partly empty: 1,024 x 2,048, 333 rows (352 small tiles, 88 wide) 63 against 66; 4,096 x 1,024, 128 rows
-  // (512, 128) 34 against 45; 2,048 x 2,048, 333 rows (704, 176) 117 against 105; 2,048 x 2,048, 100 rows (256, 64) 63 against 45.
+  if (p.M <= FEW_ROWS && vec) {
+    if ((long long)batch * ((p.N + 31) / 32) >= 148) return launch_few_rows<32, false>(p, batch, s);
+    // above eight rows nearly every thread has both of its rows (13 rows of 2,048 x 8,192: 83 us, 90 with the conditions)
+    return p.M > 8 ? launch_few_rows<16, true>(p, batch, s) : launch_few_rows<16, false>(p, batch, s);
+  }
+  // A round of wide tiles takes as long as 1.05 full rounds of small ones (two a SM), and more where it is one of several, since the
+  // small tiles' last round is never as empty.  Small and wide tiles, us: 100 rows of 2,048 x 2,048 (256 small tiles, 64 wide) 40 : 65, 333 of
+  // 1,024 x 2,048 (352, 88) 63 : 63, 128 of 4,096 x 1,024 (512, 128) 40 : 34; in two rounds of wide tiles, 333 of 2,048 x 2,048 (704, 176) 100 :
+  // 105, 700 of 1,024 x 1,024 (704, 176) 56 : 56; in three, 333 of 4,096 x 1,024 (1,408, 352) 98 : 93.
   const long long wide = (long long)batch * ((p.M + WM - 1) / WM) * ((p.N + WN - 1) / WN);
   const long long small = (long long)batch * ((p.M + 31) / 32) * ((p.N + 31) / 32), rounds = (wide + 147) / 148;
-  if (vec && small * 100 >= 296 * rounds * (rounds == 1 ? 118 : 130)) return launch_wide(p, batch, s);
+  if (vec && small * 100 >= 296 * rounds * (rounds == 1 ? 105 : 145)) return launch_wide(p, batch, s);
   return vec ? launch_tiles<32, 32, 4, 4, true>(p, batch, s) : launch_tiles<32, 32, 4, 4, false>(p, batch, s);
 }
 
