@@ -129,6 +129,25 @@ def test_sgemm_same_sums_over_many_rounds(M, N, K):
         assert torch.equal(alone[0], out[m])
 
 
+@pytest.mark.parametrize("M,N,K,pad", [(65, 4740, 451, 0), (300, 4740, 1028, 1), (333, 2048, 2050, 0), (129, 6100, 67, 0), (512, 1100, 130, 2)])
+def test_sgemm_wide_tiles_of_unaligned_rows(M, N, K, pad):
+    """Rows of any length and address in the wide tiles: bit by bit the aligned operands padded with zeros, and the row alone."""
+    from tokensprint_b200 import ops
+
+    a, w = torch.randn(M, K + pad, device=DEV)[:, pad:], torch.randn(N, K + pad, device=DEV)[:, pad:]
+    out, same = (torch.full((M, N), float("nan"), device=DEV) for _ in range(2))
+    ops.sgemm_nt(a, w, out)
+    zeros = -K % 4
+    ops.sgemm_nt(torch.nn.functional.pad(a, (0, zeros)).contiguous(), torch.nn.functional.pad(w, (0, zeros)).contiguous(), same)
+    assert torch.equal(out, same)
+    alone = torch.full((1, N), float("nan"), device=DEV)
+    ops.sgemm_nt(a[M - 1 :], w, alone)
+    assert torch.equal(alone[0], out[M - 1])
+    batch = torch.full((2, M, N), float("nan"), device=DEV)
+    ops.sgemm_nt_batched(a.expand(2, M, K), w.expand(2, N, K), batch)
+    assert torch.equal(batch[0], out) and torch.equal(batch[1], out)
+
+
 # ---------------------------------------------------------------------------
 # q/k norm + rope + store
 

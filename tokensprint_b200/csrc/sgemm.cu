@@ -38,6 +38,12 @@ __device__ __forceinline__ void cp_async16(float* dst, const float* src, bool re
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(src), "r"(bytes));
 }
 
+__device__ __forceinline__ void cp_async4(float* dst, const float* src, bool real) {
+  const unsigned to = (unsigned)__cvta_generic_to_shared(dst);
+  const int bytes = real ? 4 : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to), "l"(src), "r"(bytes));
+}
+
 // Two products at once: (x, y) += (a.x b.x, a.y b.y), each rounded as fmaf rounds it.
 typedef unsigned long long Pair;
 __device__ __forceinline__ void fma_pair(Pair& acc, Pair a, Pair b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
@@ -131,6 +137,7 @@ constexpr int WM = 32, WN = 128, WROWS = WM + WN, WCHAIN = WROWS * RSTRIDE, WSTA
 // multiplies are the same for all its lanes, and 16 bytes of them cost a third of what 16 different bytes a lane cost (1.4 against 0.46
 // such reads a cycle).  The chains wait for their own copies only (a named barrier of two warps).  What is left is latency at two
 // warps a scheduler; four warps a chain with 8 rows each: 64 -> 65 us, the loop over k unrolled: 64 -> 67.
+template <bool VEC>
 __global__ void __launch_bounds__(CHAINS * 32 * (WM / W_RM), 1) sgemm_wide_kernel(const Product p) {
   constexpr int GROUP = 32 * (WM / W_RM), STEP = GROUP / 4;  // threads of a chain; rows they copy at once
   ts_pdl_prologue();
@@ -140,7 +147,7 @@ __global__ void __launch_bounds__(CHAINS * 32 * (WM / W_RM), 1) sgemm_wide_kerne
   float* __restrict__ C = p.C + (size_t)blockIdx.z * p.batch_c;
   const int chain = threadIdx.x / GROUP, tid = threadIdx.x % GROUP, part = tid >> 5, lane = tid & 31;
   const int m0 = blockIdx.y * WM, n0 = blockIdx.x * WN;
-  // a thread copies 16 bytes of every 32nd row: one of A, four of W
+  // a thread copies 16 bytes of every 16th row: two of A, eight of W
   const int row = tid >> 2, col = (tid & 3) * 4;
   const float* a_src = A + (size_t)(m0 + row) * p.lda + col;
   const float* w_src = W + (size_t)(n0 + row) * p.ldw + col;
@@ -162,6 +169,30 @@ __global__ void __launch_bounds__(CHAINS * 32 * (WM / W_RM), 1) sgemm_wide_kerne
       cp_async16(dst + round % WSTAGES * WSTAGE + j * STEP * RSTRIDE, real ? a_src + (size_t)j * STEP * p.lda + k : p.A, real);
     }
   };
+  // rows of any address and length: a word at a time (512 rows of 6,144 x 1,025: 257 us, with words through registers in small tiles 369)
+  auto fetch_words = [&](int round) {
+    const int k = (round * CHAINS + chain) * RUN;
+    float* to = dst + round % WSTAGES * WSTAGE;
+    auto piece = [&](int r, const float* src, bool there) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const bool real = there && k + col + i < p.K;
+        cp_async4(to + r * RSTRIDE + i, real ? src + k + i : p.W, real);
+      }
+    };
+#pragma unroll
+    for (int j = 0; j < WN / STEP; ++j) piece(WM + j * STEP, w_src + (size_t)j * STEP * p.ldw, n0 + row + j * STEP < p.N);
+#pragma unroll
+    for (int j = 0; j < WM / STEP; ++j) piece(j * STEP, a_src + (size_t)j * STEP * p.lda, m0 + row + j * STEP < p.M);
+  };
+  auto fetch = [&](int round) {
+    if constexpr (VEC) {
+      fetch_w(round);
+      fetch_a(round);
+    } else {
+      fetch_words(round);
+    }
+  };
   Pair acc[W_RM][W_RN];
 #pragma unroll
   for (int i = 0; i < W_RM; ++i)
@@ -170,19 +201,13 @@ __global__ void __launch_bounds__(CHAINS * 32 * (WM / W_RM), 1) sgemm_wide_kerne
   const int rounds = (p.K + CHAINS * RUN - 1) / (CHAINS * RUN);
 #pragma unroll
   for (int r = 0; r < WSTAGES - 1; ++r) {
-    if (r < rounds) {
-      fetch_w(r);
-      fetch_a(r);
-    }
+    if (r < rounds) fetch(r);
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
   for (int it = 0; it < rounds; ++it) {
     asm volatile("cp.async.wait_group %0;" ::"n"(WSTAGES - 2) : "memory");
     asm volatile("bar.sync %0, %1;" ::"r"(1 + chain), "n"(GROUP) : "memory");  // the chain's run is here, and the one before has been read
-    if (it + WSTAGES - 1 < rounds) {
-      fetch_w(it + WSTAGES - 1);
-      fetch_a(it + WSTAGES - 1);
-    }
+    if (it + WSTAGES - 1 < rounds) fetch(it + WSTAGES - 1);
     asm volatile("cp.async.commit_group;" ::: "memory");
     const float* as = sm + it % WSTAGES * WSTAGE + chain * WCHAIN + part * W_RM * RSTRIDE;
     const float* ws = sm + it % WSTAGES * WSTAGE + chain * WCHAIN + (WM + lane) * RSTRIDE;
@@ -326,13 +351,14 @@ int launch_tiles(const Product& p, int batch, cudaStream_t s) {
   return ts_launch(sgemm_tile_kernel<BM, BN, TM, TN, VEC>, grid, dim3(CHAINS * (BM / TM) * (BN / TN)), smem, s, p);
 }
 
+template <bool VEC>
 int launch_wide(const Product& p, int batch, cudaStream_t s) {
   const dim3 grid((p.N + WN - 1) / WN, (p.M + WM - 1) / WM, batch);
   if (grid.y > 65535 || batch > 65535) return TS_ERR_UNSUPPORTED_SIZE;
   constexpr size_t smem = (size_t)WSTAGES * WSTAGE * sizeof(float);
-  const cudaError_t e = cudaFuncSetAttribute(sgemm_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = cudaFuncSetAttribute(sgemm_wide_kernel<VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  return ts_launch(sgemm_wide_kernel, grid, dim3(CHAINS * 32 * (WM / W_RM)), smem, s, p);
+  return ts_launch(sgemm_wide_kernel<VEC>, grid, dim3(CHAINS * 32 * (WM / W_RM)), smem, s, p);
 }
 
 template <int BN, bool ALL_ROWS>
@@ -365,7 +391,9 @@ int launch(const Product& p, int batch, cudaStream_t s) {
   // 105, 700 of 1,024 x 1,024 (704, 176) 56 : 56; in three, 333 of 4,096 x 1,024 (1,408, 352) 98 : 93.
   const long long wide = (long long)batch * ((p.M + WM - 1) / WM) * ((p.N + WN - 1) / WN);
   const long long small = (long long)batch * ((p.M + 31) / 32) * ((p.N + 31) / 32), rounds = (wide + 147) / 148;
-  if (vec && small * 100 >= 296 * rounds * (rounds == 1 ? 105 : 145)) return launch_wide(p, batch, s);
+  // Rows that the 16-byte copies do not take are read through registers by the small tiles, which costs them more: 333 rows of 2,048 x 2,050 208 :
+  // 163, 128 of 6,144 x 1,025 (768, 192) 104 : 88.
+  if (small * 100 >= 296 * rounds * (rounds == 1 || !vec ? 105 : 145)) return vec ? launch_wide<true>(p, batch, s) : launch_wide<false>(p, batch, s);
   return vec ? launch_tiles<32, 32, 4, 4, true>(p, batch, s) : launch_tiles<32, 32, 4, 4, false>(p, batch, s);
 }
 
