@@ -148,6 +148,25 @@ def test_sgemm_wide_tiles_of_unaligned_rows(M, N, K, pad):
     assert torch.equal(batch[0], out) and torch.equal(batch[1], out)
 
 
+@pytest.mark.parametrize("N,K,pad", [(12, 8, 0), (130, 5, 1)])
+@pytest.mark.parametrize("M", [65535 * 32, 65535 * 32 + 3, 65535 * 32 + 700])
+def test_sgemm_takes_more_rows_than_a_grid_has_tiles(M, N, K, pad):
+    from tokensprint_b200 import ops
+
+    a, w = torch.randn(M, K + pad, device=DEV)[:, pad:], torch.randn(N, K + pad, device=DEV)[:, pad:]
+    out = torch.full((M, N + 1), float("nan"), device=DEV)
+    ops.sgemm_nt(a, w, out[:, :N])
+    assert bool(out[:, N].isnan().all())
+    for at in (0, 65535 * 32 - 40, M - 40):
+        part = torch.empty(40, N, device=DEV)
+        ops.sgemm_nt(a[at : at + 40], w, part)
+        assert torch.equal(out[at : at + 40, :N], part)
+    assert float((out[:, :N] - a @ w.T).abs().max()) < 1e-4  # sums of at most 8 products of a few units
+    batch = torch.empty(2, M, N, device=DEV)
+    ops.sgemm_nt_batched(a.expand(2, M, K), w.expand(2, N, K), batch)
+    assert torch.equal(batch[1], out[:, :N])
+
+
 # ---------------------------------------------------------------------------
 # q/k norm + rope + store
 

@@ -377,8 +377,21 @@ bool aligned16(const Product& p) {
   return ((reinterpret_cast<size_t>(p.A) | reinterpret_cast<size_t>(p.W)) & 15) == 0 && (strides & 3) == 0;
 }
 
+constexpr int MOST_ROWS = 65535 * 32;
+
 // Which kernel: the choice changes the time only, never a bit of the result.
 int launch(const Product& p, int batch, cudaStream_t s) {
+  if (p.M > MOST_ROWS) {
+    // Tiles have 32 rows and a grid 65,535 of them in this direction; twice as many rows are taken, in two launches.
+    if (p.M > 2 * MOST_ROWS) return TS_ERR_UNSUPPORTED_SIZE;
+    Product first = p, rest = p;
+    first.M = MOST_ROWS;
+    rest.M = p.M - MOST_ROWS;
+    rest.A += (long long)MOST_ROWS * p.lda;
+    rest.C += (long long)MOST_ROWS * p.ldc;
+    const int status = launch(first, batch, s);
+    return status != 0 ? status : launch(rest, batch, s);
+  }
   const bool vec = aligned16(p) && p.K % 4 == 0;
   if (p.M <= FEW_ROWS && vec) {
     if ((long long)batch * ((p.N + 31) / 32) >= 148) return launch_few_rows<32, false>(p, batch, s);
