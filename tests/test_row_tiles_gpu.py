@@ -98,6 +98,32 @@ def test_state_space_convolution(C, H, pad, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,pad", [(1, 4), (130, 0)])
+def test_state_space_convolution_in_tiles(dtype, H, pad):
+    from tokensprint_b200 import ops
+
+    C = 2056
+    g, x, x_off, cu, seq, state, slots = portions(dtype, C, pad, C + H)
+    assert ops._fn("ts_ssm_conv_in_tiles")(x.shape[0], len(LENS), C)
+    taps, bias = torch.randn(C, 4, generator=g, device=DEV), torch.randn(C, generator=g, device=DEV)
+    dt_raw = torch.randn(x.shape[0], H, generator=g, device=DEV)
+    dt_bias, a_log = torch.randn(2, H, generator=g, device=DEV).unbind(0)
+    got = []
+    for rows in (x, x_off):
+        kept = state.clone()
+        got.append((*ops.ssm_conv(rows, taps, bias, kept, slots, cu, seq, len(LENS), dt_raw, dt_bias.contiguous(), a_log.contiguous()), kept))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("T,n,C", [(128, 128, 4352), (256, 256, 8448), (512, 512, 4352), (512, 128, 2304), (768, 64, 2304), (2048, 1, 256), (1424, 26, 256)])
+def test_small_steps_of_the_state_space_convolution_take_no_tiles(T, n, C):
+    from tokensprint_b200 import ops
+
+    assert not ops._fn("ts_ssm_conv_in_tiles")(T, n, C)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("T,N,top,shared,identity", [(1, 8, 1, False, False), (5, 2048, 4, True, True), (700, 1032, 2, False, True), (3, 1000, 7, True, False)])
 def test_sum_over_experts(T, N, top, shared, identity, dtype):
     from tokensprint_b200 import ops

@@ -268,22 +268,27 @@ __global__ void __launch_bounds__(128) ssm_conv4_tile_kernel(const TA* __restric
   }
 }
 
+// Whether tiles of tokens pay: a tile that holds a portion's start goes token by token, a chain of about 10 us, so tiles are for steps
+// whose rows alone take longer, and more so where portions are short.  The line, us, a token a thread against tiles: bfloat16, 1,024 tokens of one
+// prompt x 2,304 channels 23 : 14, 2,048 x 256 8 : 11; 64 x 12, x 2,304 19 : 21; 64 x 16 24 : 21; 128 x 4, x 4,352 25 : 22; 256 x 2 30 : 28; single
+// tokens, 256 x 4,352 21 : 25, 512 x 2,304 22 : 26, 512 x 8,448 73 : 62; float32, 256 x 2, x 4,352 30 : 30, 512 single tokens 39 : 40.
+static bool ssm_conv_in_tiles(int T, int num_seqs, int C) { return (long long)T * C >= (T >= 4ll * num_seqs ? 2000000 : 3000000); }
+
 template <typename TA>
 static bool ssm_conv4(const void* xin, long long ld, const float* taps_w, const float* bias, int K, const float* conv_state, long long slot_stride,
-                      const int* state_slots, const int* cu_seqlens, const int* seq_index, float* out, int T, int C, const float* dt_raw,
+                      const int* state_slots, const int* cu_seqlens, const int* seq_index, float* out, int T, int num_seqs, int C, const float* dt_raw,
                       const float* dt_bias, const float* a_log, float* dt, float* decay, int H, cudaStream_t s, int* status) {
-  // tiles of 8 tokens (4 of float32) where they still give every SM a CTA; in steps of few tokens a tile would be a chain
   constexpr int TOK = sizeof(TA) == 2 ? 8 : 4;
   const int conv_blocks = (C / 8 + 127) / 128, tiles = (T + TOK - 1) / TOK;
-  if (K != 4 || C % 8 || ld % 8 || (((uintptr_t)xin | (uintptr_t)out | (uintptr_t)taps_w) & 15) || (long long)conv_blocks * tiles < 148) return false;
+  if (K != 4 || C % 8 || ld % 8 || (((uintptr_t)xin | (uintptr_t)out | (uintptr_t)taps_w) & 15) || !ssm_conv_in_tiles(T, num_seqs, C)) return false;
   *status = ts_launch(ssm_conv4_tile_kernel<TA, TOK>, dim3(conv_blocks + (H + 127) / 128, tiles), dim3(128), 0, s, (const TA*)xin, ld, taps_w, bias, conv_state,
                       slot_stride, state_slots, cu_seqlens, seq_index, out, T, C, dt_raw, dt_bias, a_log, dt, decay, H, conv_blocks);
   return true;
 }
 
 TS_EXPORT int ts_ssm_conv(const void* xin, int act_dtype, long long ld, const float* taps_w, const float* bias, int K, const float* conv_state,
-                          long long slot_stride, const int* state_slots, const int* cu_seqlens, const int* seq_index, float* out, int T, int C,
-                          const float* dt_raw, const float* dt_bias, const float* a_log, float* dt, float* decay, int H, void* stream) {
+                          long long slot_stride, const int* state_slots, const int* cu_seqlens, const int* seq_index, float* out, int T, int num_seqs,
+                          int C, const float* dt_raw, const float* dt_bias, const float* a_log, float* dt, float* decay, int H, void* stream) {
   if (T <= 0) return 0;
   if (C <= 0 || K < 1 || H < 0) return TS_ERR_BAD_ARGUMENT;
   if (T > 65535) return TS_ERR_UNSUPPORTED_SIZE;
@@ -291,8 +296,8 @@ TS_EXPORT int ts_ssm_conv(const void* xin, int act_dtype, long long ld, const fl
   cudaStream_t s = (cudaStream_t)stream;
   int status = 0;
   if (act_dtype == TS_DTYPE_F32
-          ? ssm_conv4<float>(xin, ld, taps_w, bias, K, conv_state, slot_stride, state_slots, cu_seqlens, seq_index, out, T, C, dt_raw, dt_bias, a_log, dt, decay, H, s, &status)
-          : act_dtype == TS_DTYPE_BF16 && ssm_conv4<__nv_bfloat16>(xin, ld, taps_w, bias, K, conv_state, slot_stride, state_slots, cu_seqlens, seq_index, out, T, C,
+          ? ssm_conv4<float>(xin, ld, taps_w, bias, K, conv_state, slot_stride, state_slots, cu_seqlens, seq_index, out, T, num_seqs, C, dt_raw, dt_bias, a_log, dt, decay, H, s, &status)
+          : act_dtype == TS_DTYPE_BF16 && ssm_conv4<__nv_bfloat16>(xin, ld, taps_w, bias, K, conv_state, slot_stride, state_slots, cu_seqlens, seq_index, out, T, num_seqs, C,
                                                                    dt_raw, dt_bias, a_log, dt, decay, H, s, &status))
     return status;
   if (act_dtype == TS_DTYPE_F32)
@@ -303,6 +308,9 @@ TS_EXPORT int ts_ssm_conv(const void* xin, int act_dtype, long long ld, const fl
                      slot_stride, state_slots, cu_seqlens, seq_index, out, T, C, dt_raw, dt_bias, a_log, dt, decay, H);
   return TS_ERR_BAD_ARGUMENT;
 }
+
+// Whether ts_ssm_conv takes its tokens in tiles (four taps, 16-byte aligned rows).
+TS_EXPORT int ts_ssm_conv_in_tiles(int T, int num_seqs, int C) { return C % 8 == 0 && ssm_conv_in_tiles(T, num_seqs, C) ? 1 : 0; }
 
 template <typename TA>
 __global__ void ssm_conv_state_kernel(const TA* __restrict__ xin, long long ld, int K, float* __restrict__ conv_state, long long slot_stride,

@@ -881,7 +881,8 @@ _SIGNATURES.update({
     "ts_mlstm_gate_scan": [_c_void_p, _c_void_p, _c_float, _c_void_p, _c_ll, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p],
     "ts_mlstm_norm_gate": [_c_void_p, _c_void_p, _c_void_p, _c_ll, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_float, _c_void_p],
     "ts_ssm_conv": [_c_void_p, _c_int, _c_ll, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_ll, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int,
-                    _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p],
+                    _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p],
+    "ts_ssm_conv_in_tiles": [_c_int, _c_int, _c_int],
     "ts_ssm_conv_state": [_c_void_p, _c_int, _c_ll, _c_int, _c_void_p, _c_ll, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p],
     "ts_ssm_gate_norm": [_c_void_p, _c_void_p, _c_ll, _c_void_p, _c_void_p, _c_ll, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int,
                          _c_float, _c_void_p],
@@ -1056,7 +1057,7 @@ def ssm_conv(xin: torch.Tensor, taps: torch.Tensor, bias: torch.Tensor, conv_sta
     code, stream = _act_code("xin", xin), _stream()
     _check("ssm_conv", _fn("ts_ssm_conv")(
         xin.data_ptr(), code, xin.stride(0), taps.data_ptr(), bias.data_ptr(), K, conv_state.data_ptr(), conv_state.stride(0),
-        state_slots.data_ptr(), cu_seqlens.data_ptr(), seq_index.data_ptr(), out.data_ptr(), T, C, dt_raw.data_ptr(), dt_bias.data_ptr(),
+        state_slots.data_ptr(), cu_seqlens.data_ptr(), seq_index.data_ptr(), out.data_ptr(), T, int(num_seqs), C, dt_raw.data_ptr(), dt_bias.data_ptr(),
         a_log.data_ptr(), dt.data_ptr(), decay.data_ptr(), H, stream))
     if K > 1:
         _check("ssm_conv", _fn("ts_ssm_conv_state")(xin.data_ptr(), code, xin.stride(0), K, conv_state.data_ptr(), conv_state.stride(0),
