@@ -140,3 +140,35 @@ def test_sum_over_experts(T, N, top, shared, identity, dtype):
         v = torch.where((ids >= 4)[:, :, None], x.double()[:, None, :], v)
     want = (v * weight.double().view(T, top, 1)).sum(1) + (sh.double() if shared else 0.0)
     assert float((out.double() - want).norm() / want.norm()) < (1e-6 if dtype == torch.float32 else 2 ** -8)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,N,top,shared,identity", [(800, 256, 8, True, False), (200, 1032, 3, False, True), (33, 7168, 1, True, True), (66000, 256, 2, False, False)])
+def test_sum_over_experts_in_pieces(T, N, top, shared, identity, dtype):
+    """16 bytes a thread against an element a thread (rows off the 16-byte boundary, 66,000 tokens): the same bits."""
+    from tokensprint_b200 import ops
+
+    assert ops._fn("ts_moe_combine_in_pieces")(T, N)
+    g = torch.Generator(device=DEV).manual_seed(T + N)
+
+    def rows(n):  # the same values on a 16-byte boundary and one entry off it
+        v = torch.randn(n, N, generator=g, device=DEV).to(dtype)
+        off = torch.empty(n * N + 1, device=DEV, dtype=dtype)[1:].view(n, N)
+        return v, off.copy_(v)
+
+    pairs, x, sh = rows(T * top), rows(T), rows(T)
+    weight = torch.rand(T * top, generator=g, device=DEV)
+    ids = torch.randint(0, 6, (T, top), generator=g, device=DEV, dtype=torch.int32) if identity else None
+    got = []
+    for k in range(2):
+        out = torch.full((T * N + 1,), float("nan"), device=DEV, dtype=dtype)[k : k + T * N].view(T, N)
+        ops.moe_combine(pairs[k], sh[k] if shared else None, out, top, weight, ids=ids, num_experts=4, x=x[k] if identity else None)
+        got.append(out)
+    assert torch.equal(*got)
+
+
+@pytest.mark.parametrize("T,N", [(1, 2048), (5, 2048), (64, 2048), (200, 512), (8192, 64), (40000, 128), (2048, 248)])
+def test_small_sums_over_experts_take_an_element_a_thread(T, N):
+    from tokensprint_b200 import ops
+
+    assert not ops._fn("ts_moe_combine_in_pieces")(T, N)

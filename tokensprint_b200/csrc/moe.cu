@@ -381,8 +381,7 @@ __global__ void moe_combine_kernel(const TA* __restrict__ pair_out, const TA* __
 }
 
 // The same sums, 16 bytes of a row per thread and a block row per token: rows of whole 16-byte pieces.  Bound by reading the pairs'
-// rows once; with an element a thread and its 64-bit
-// division a step went on 48 us after the products, now 13 (2,048 tokens of 4,096 bfloat16; 25 and 7 for 2,500 of 2,048).
+// rows once; an element a thread is bound by its 64-bit division (2,048 tokens of 4,096 bfloat16, 4 choices: 50 us, 15 so; 8,192 tokens of 1,024: 50, 15).
 template <typename TA>
 __global__ void __launch_bounds__(128) moe_combine_vec_kernel(const TA* __restrict__ pair_out, const TA* __restrict__ shared, TA* __restrict__ out,
                                                               const float* __restrict__ pair_weight, int N, int top, const int* __restrict__ ids, int E,
@@ -415,11 +414,16 @@ __global__ void __launch_bounds__(128) moe_combine_vec_kernel(const TA* __restri
   *reinterpret_cast<uint4*>(out + at) = raw;
 }
 
+// Rows of 256 entries or more (of 64, at 8,192 tokens, a block row per token takes 9 us with most threads idle, an element a
+// thread 4), and 200,000 entries or more: below, the kernel with more threads ends earlier (us, an element : 16 bytes a thread, eight choices: one token of 2,048 1.9 :
+// 2.3, 64 of 1,024 2.2 : 2.3, 200 of 1,024 3.1 : 2.5, 64 of 4,096 3.1 : 2.5).
+static bool moe_combine_in_pieces(int T, int N) { return N >= 256 && (long long)T * N >= 200000; }
+
 template <typename TA>
 static bool moe_combine_vec(const void* pair_out, const void* shared, void* out, const float* pair_weight, int T, int N, int top, const int* ids, int E,
                             const void* x, cudaStream_t s, int* status) {
   constexpr int V = 16 / sizeof(TA);
-  if (N % V || T > 65535 || (long long)T * top >= (1ll << 31) || (((uintptr_t)pair_out | (uintptr_t)shared | (uintptr_t)out | (uintptr_t)x) & 15)) return false;
+  if (!moe_combine_in_pieces(T, N) || N % V || T > 65535 || (long long)T * top >= (1ll << 31) || (((uintptr_t)pair_out | (uintptr_t)shared | (uintptr_t)out | (uintptr_t)x) & 15)) return false;
   *status = ts_launch(moe_combine_vec_kernel<TA>, dim3((N / V + 127) / 128, T), dim3(128), 0, s, (const TA*)pair_out, (const TA*)shared, (TA*)out, pair_weight,
                       N, top, ids, E, (const TA*)x);
   return true;
@@ -443,6 +447,9 @@ TS_EXPORT int ts_moe_combine(const void* pair_out, const void* shared, void* out
                      (const __nv_bfloat16*)shared, (__nv_bfloat16*)out, pair_weight, N, top, total, ids, E, (const __nv_bfloat16*)x);
   return TS_ERR_BAD_ARGUMENT;
 }
+
+// Whether ts_moe_combine takes 16 bytes a thread (rows on 16-byte boundaries).
+TS_EXPORT int ts_moe_combine_in_pieces(int T, int N) { return N % 8 == 0 && moe_combine_in_pieces(T, N) ? 1 : 0; }
 
 // ---------------------------------------------------------------------------------------------
 // The router in one kernel: float32 logits of RT tokens against every expert's row, then the

@@ -80,6 +80,7 @@ _SIGNATURES = {
                            _c_void_p],
     "ts_stream_add": [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p],
     "ts_moe_combine": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p],
+    "ts_moe_combine_in_pieces": [_c_int, _c_int],
 }
 
 _functions: dict[str, object] = {}
