@@ -107,6 +107,15 @@ def test_heads_with_norm_rotation_and_store(M, nq, nkv, K, rope, norm):
             assert bool((kc[s] == 7.0).all()) and bool((vc[s] == 7.0).all()), "a slot nobody owns was written"
 
 
+@pytest.mark.parametrize("M,heads,K,warps", [(1, 32, 1024, 16), (2, 33, 2048, 16), (4, 32, 1024, 8), (15, 32, 1024, 8), (11, 48, 1024, 8), (16, 32, 1024, 16),
+                                             (1, 34, 4096, 8), (4, 56, 5120, 8), (4, 66, 5120, 8), (1, 67, 1024, 0), (4, 80, 5120, 0), (8, 48, 4096, 0)])
+def test_heads_are_taken_only_where_their_clusters_stand_at_once(M, heads, K, warps):
+    """33 clusters of four CTAs of 16 warps, 66 of 8 warps (two CTAs an SM)."""
+    from tokensprint_b200 import ops
+
+    assert ops._fn("ts_gemm_rows_takes_heads")(M, heads, K) == warps
+
+
 def test_what_it_does_not_take_runs_on_the_other_kernel():
     """17 rows, rows that are not whole chunks, short rows, rows that do not start on 32 bytes, an input that leaves no room for
     the rings: the same call, the tcgen05 kernel's bits."""

@@ -393,8 +393,9 @@ bool choose(int M, int N, int K, bool qk, Shape* s) {
   if (!qk) return smem_bytes(M, K, false, 16) <= SMEM_ONE;
   // Four CTAs a head: two an SM (0.6B of 8 requests 986 -> 898, 8B of 4 3,206 -> 3,146), or, where all stand at once, one of 16
   // warps for a small input (0.6B of 1 request: 781 beside 813) or one too large for two an SM (of 14: 1,256 -> 1,218).
-  // One an SM in two rounds is slower than the other kernel (8B of 8 requests: 3,545 against 3,311).
-  const bool two = smem_bytes(M, K, true, 8) <= SMEM_TWO;
+  // In two rounds either is slower than the other kernel (one an SM: 8B of 8 requests 3,545 against 3,311; two an SM: 80 heads over
+  // 5,120 columns, 320 CTAs, 26 and 27 us at 1 and 4 rows against 24 and 21; 56 heads, 224 CTAs, 15 and 16 against 21 and 18).
+  const bool two = smem_bytes(M, K, true, 8) <= SMEM_TWO && N / HEAD * CLUSTER <= 2 * CLUSTER_SLOTS;
   if (N / HEAD * CLUSTER <= CLUSTER_SLOTS && (M <= 2 || !two)) return smem_bytes(M, K, true, 16) <= SMEM_ONE;
   s->warps = 8;
   return two;
@@ -456,10 +457,10 @@ TS_EXPORT int ts_gemm_rows_ssq_tiles(int M, int N, int K) {
   return (N + 8 * RU_PLAIN - 1) / (8 * RU_PLAIN);
 }
 
-// Whether ts_gemm_rows_qk_rope takes the product of M rows with `heads` heads of W.
+// With how many warps a CTA ts_gemm_rows_qk_rope takes the product of M rows with `heads` heads of W (0: not at all).
 TS_EXPORT int ts_gemm_rows_takes_heads(int M, int heads, int K) {
   Shape s;
-  return choose(M, heads * HEAD, K, true, &s) ? 1 : 0;
+  return choose(M, heads * HEAD, K, true, &s) ? s.warps : 0;
 }
 
 // Arguments as for ts_gemm_skinny_fused (ssq_out: ts_gemm_rows_ssq_tiles(M, N, K) rows).
