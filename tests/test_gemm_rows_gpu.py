@@ -116,6 +116,15 @@ def test_heads_are_taken_only_where_their_clusters_stand_at_once(M, heads, K, wa
     assert ops._fn("ts_gemm_rows_takes_heads")(M, heads, K) == warps
 
 
+@pytest.mark.parametrize("M,N,K,taken", [(8, 151936, 1024, True), (9, 151936, 1024, False), (16, 24576, 1024, False), (16, 6144, 1024, True),
+                                         (16, 9472, 1024, True), (9, 9473, 1536, False), (16, 32768, 2048, True), (8, 24576, 4096, True),
+                                         (9, 24576, 4096, False)])
+def test_many_short_tasks_of_more_than_eight_rows_stay_with_the_other_kernel(M, N, K, taken):
+    from tokensprint_b200 import ops
+
+    assert (ops._fn("ts_gemm_rows_ssq_tiles")(M, N, K) > 0) == taken
+
+
 def test_what_it_does_not_take_runs_on_the_other_kernel():
     """17 rows, rows that are not whole chunks, short rows, rows that do not start on 32 bytes, an input that leaves no room for
     the rings: the same call, the tcgen05 kernel's bits."""

@@ -390,6 +390,10 @@ size_t smem_bytes(int M, int K, bool qk, int warps) {
 bool choose(int M, int N, int K, bool qk, Shape* s) {
   if (M < 1 || M > MAX_ROWS || K % CHUNK != 0 || K / CHUNK < 16) return false;
   s->warps = 16;
+  // Tasks of few columns end often: above 8 rows their sums over the warps and the epilogue outlast the copies where a CTA has many of them.  us, here :
+  // gemm_tcgen05.cu, K = 1,024: the logits' 151,936 columns at 9 / 16 rows 53 / 57 : 49 / 50, gate and up of 24,576 at 16 rows 15.3 : 13.6, of
+  // 8,192 8.9 : 9.5; K = 1,536, gate and up of 32,768 at 16 rows 24 : 21; K = 2,048 25 : 26.  Up to 8 rows they are even (50.1 : 48.6 at 8).
+  if (!qk && M > 8 && K < 2048 && N > 4 * 148 * 8 * RU_PLAIN) return false;
   if (!qk) return smem_bytes(M, K, false, 16) <= SMEM_ONE;
   // Four CTAs a head: two an SM (0.6B of 8 requests 986 -> 898, 8B of 4 3,206 -> 3,146), or, where all stand at once, one of 16
   // warps for a small input (0.6B of 1 request: 781 beside 813) or one too large for two an SM (of 14: 1,256 -> 1,218).
