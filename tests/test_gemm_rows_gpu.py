@@ -72,7 +72,8 @@ def test_gated_epilogue(M, I, K, activation):
 
 @pytest.mark.parametrize("M,nq,nkv,K,rope,norm", [(1, 16, 8, 1024, True, True), (16, 16, 8, 1024, True, False), (5, 16, 4, 2048, False, True),
                                                   (2, 8, 8, 2048, True, True), (4, 32, 8, 4096, True, True), (3, 32, 4, 4096, True, False),
-                                                  (1, 30, 5, 1088, True, True)])
+                                                  (1, 30, 5, 1088, True, True), (9, 16, 8, 1024, True, True), (15, 16, 8, 1024, True, True),
+                                                  (11, 32, 8, 1024, True, False), (13, 18, 8, 1024, False, True)])
 def test_heads_with_norm_rotation_and_store(M, nq, nkv, K, rope, norm):
     from tokensprint_b200 import ops
 
@@ -123,6 +124,62 @@ def test_many_short_tasks_of_more_than_eight_rows_stay_with_the_other_kernel(M, 
     from tokensprint_b200 import ops
 
     assert (ops._fn("ts_gemm_rows_ssq_tiles")(M, N, K) > 0) == taken
+
+
+@pytest.mark.parametrize("nq,nkv,K", [(16, 8, 1024), (8, 4, 1088), (4, 2, 1984)])
+def test_a_head_has_the_same_bits_whatever_the_rows_beside_it(nq, nkv, K):
+    """Steps of 1 to 16 rows share a head among 16 or among 8 warps a CTA: the same sums in the same order."""
+    from tokensprint_b200 import ops
+
+    d, most = 128, 16
+    normal, x, w = make(most, (nq + 2 * nkv) * d, K)
+    forms = {ops._fn("ts_gemm_rows_takes_heads")(M, nq + 2 * nkv, K) for M in range(1, most + 1)}
+    assert forms == {8, 16}
+    qw, kw = 1 + 0.2 * normal(d), 1 + 0.2 * normal(d)
+    inv_freq = (1.0 / (1e4 ** (torch.arange(0, d, 2).float() / d))).to(DEV)
+    positions = torch.randint(0, 3000, (most,)).to(DEV, torch.int32)
+    slots = torch.randperm(most).to(DEV, torch.int32)
+    ssq = torch.rand(64, most, device=DEV) + 0.1
+
+    def run(first, last):
+        q = torch.full((last - first, nq * d), float("nan"), device=DEV, dtype=torch.bfloat16)
+        kc, vc = (torch.full((most, nkv, d), 7.0, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+        ops.gemm_qk_rope_store(x[first:last].contiguous(), w, q, kc, vc, slots[first:last].contiguous(), positions[first:last].contiguous(), qw, kw, 1e-5,
+                               inv_freq, nq, nkv, scale_ssq=ssq[:, first:last].contiguous(), scale_width=K, scale_eps=1e-6, direct=True)
+        at = slots[first:last].long()
+        return q, kc[at], vc[at]
+
+    whole = run(0, most)
+    for first, last in ((0, 1), (15, 16), (3, 5), (0, 3), (7, 15), (1, 16), (0, 9), (4, 12)):
+        for a, b in zip(run(first, last), whole):
+            assert torch.equal(a, b[first:last])
+
+
+@pytest.mark.parametrize("N,K", [(1000, 1024), (2056, 1984), (4104, 2048)])
+def test_a_row_has_the_same_bits_whatever_the_rows_beside_it(N, K):
+    """Plain, gated and residual products sum over 16 warps at every number of rows."""
+    from tokensprint_b200 import ops
+
+    normal, x, w = make(16, N, K)
+    gate_up = (normal(256, K) * 0.05).bfloat16()
+    hidden0, norm_w = normal(16, N), 1 + 0.1 * normal(N)
+
+    def run(first, last):
+        M, rows = last - first, x[first:last].contiguous()
+        assert ops._rows_takes(M, ops._facts(w)) > 0 and ops._rows_takes(M, ops._facts(gate_up)) > 0
+        plain = torch.empty(M, N, device=DEV)
+        ops.gemm_skinny_bf16(rows, w, plain, direct=True)
+        gated = torch.empty(M, 128, device=DEV, dtype=torch.bfloat16)
+        ops.gemm_skinny_fused(rows, gate_up, out=gated, mode=ops.GEMM_EPILOGUE_SWIGLU, direct=True)
+        hidden, xprime = hidden0[first:last].clone(), torch.empty(M, N, device=DEV, dtype=torch.bfloat16)
+        ssq = torch.empty(ops.gemm_ssq_tiles(M, w), M, device=DEV)
+        ops.gemm_skinny_fused(rows, w, mode=ops.GEMM_EPILOGUE_RESIDUAL_NORM, hidden=hidden, norm_weight=norm_w, xprime=xprime, ssq_out=ssq, direct=True)
+        return plain, gated, hidden, xprime, ssq.T
+
+    whole = run(0, 16)
+    for first, last in ((0, 1), (15, 16), (3, 5), (0, 8), (0, 9), (5, 14)):
+        for a, b in zip(run(first, last), whole):
+            assert torch.equal(a, b[first:last])
 
 
 def test_what_it_does_not_take_runs_on_the_other_kernel():

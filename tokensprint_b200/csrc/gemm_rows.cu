@@ -19,6 +19,7 @@
 // The epilogues are those of gemm_tcgen05.cu: row scale, gated activation, residual sum with the next norm's input and
 // row sums of squares (per 16 columns), q/k norm with rotation and cache store (a head's 128 rows are shared by
 // a cluster of four CTAs with 16 pairs (j, j + 64) each, which exchange their sums of squares through distributed shared memory).
+// A row's sums are added up in one order whatever the rows beside it, the number of warps included.
 //
 // Measured (B200; a whole decode step, us, with gemm_tcgen05.cu's products and with these): 0.6B of 1 request 1,133 -> 732, of 8
 // 1,240 -> 872; 8B of 1 3,324 -> 2,889, of 8 3,485 -> 3,298; four small products of a layer (0.6B, 1 row) 27.8 -> 14.6, floor 4.9.
@@ -208,10 +209,15 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) gemm_rows_kern
         norm0 = a.norm_w[col];
       }
     }
-    float acc[4][4];  // 4 / RU chains per group of rows: a product waits for the one before it in its chain
+    // 4 / RU chains per group of rows: a product waits for the one before it in its chain.  Eight warps that share a head keep the sums of every
+    // other chunk apart: what 16 warps sum, added up in the same order, so a row's bits do not depend on the form.
+    constexpr int SETS = QK && WARPS == 8 ? 2 : 1;
+    float acc[SETS][4][4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) acc[u][0] = acc[u][1] = acc[u][2] = acc[u][3] = 0.f;
-    for (int c = 0; c < nc; ++c) {
+    for (int i = 0; i < SETS; ++i)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) acc[i][u][0] = acc[i][u][1] = acc[i][u][2] = acc[i][u][3] = 0.f;
+    auto chunk = [&](int c, float (&sums)[4][4]) {
       asm volatile("cp.async.wait_group %0;" ::"n"(SLOTS - 1) : "memory");
       const int x_off = c * (WARPS * CHUNK * 2);
       uint4 lo[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)}, hi[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
@@ -232,13 +238,17 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) gemm_rows_kern
       }
 #pragma unroll
       for (int u = 0; u < RU; ++u) {
-        mma_16816(acc[u * CHAINS], lo[0].x, hi[0].x, lo[0].y, hi[0].y, w[u][0].x, w[u][0].y);
-        mma_16816(acc[u * CHAINS + 1 % CHAINS], lo[0].z, hi[0].z, lo[0].w, hi[0].w, w[u][0].z, w[u][0].w);
-        mma_16816(acc[u * CHAINS + 2 % CHAINS], lo[1].x, hi[1].x, lo[1].y, hi[1].y, w[u][1].x, w[u][1].y);
-        mma_16816(acc[u * CHAINS + 3 % CHAINS], lo[1].z, hi[1].z, lo[1].w, hi[1].w, w[u][1].z, w[u][1].w);
+        mma_16816(sums[u * CHAINS], lo[0].x, hi[0].x, lo[0].y, hi[0].y, w[u][0].x, w[u][0].y);
+        mma_16816(sums[u * CHAINS + 1 % CHAINS], lo[0].z, hi[0].z, lo[0].w, hi[0].w, w[u][0].z, w[u][0].w);
+        mma_16816(sums[u * CHAINS + 2 % CHAINS], lo[1].x, hi[1].x, lo[1].y, hi[1].y, w[u][1].x, w[u][1].y);
+        mma_16816(sums[u * CHAINS + 3 % CHAINS], lo[1].z, hi[1].z, lo[1].w, hi[1].w, w[u][1].z, w[u][1].w);
       }
       load_next();  // into the slot just read
       slot = slot + 1 == SLOTS ? 0 : slot + 1;
+    };
+    for (int c = 0; c < nc; c += SETS) {
+      chunk(c, acc[0]);
+      if (SETS == 2 && c + 1 < nc) chunk(c + 1, acc[SETS - 1]);
     }
     // ---- the warps' sums meet in shared memory (two buffers in turn: one barrier a task)
     float* r = red + (size_t)(it & 1) * (WARPS * ROWS * COLS);
@@ -247,9 +257,10 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) gemm_rows_kern
       float v[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        v[i] = acc[u * CHAINS][i];
+        v[i] = acc[0][u * CHAINS][i];
 #pragma unroll
-        for (int k = 1; k < CHAINS; ++k) v[i] += acc[u * CHAINS + k][i];
+        for (int k = 1; k < CHAINS; ++k) v[i] += acc[0][u * CHAINS + k][i];
+        if (SETS == 2) v[i] += acc[SETS - 1][u * CHAINS][i];
       }
       float* mine = r + (warp * ROWS + g) * COLS + u * 8 + 2 * t;
       *reinterpret_cast<float2*>(mine) = make_float2(v[0], v[1]);
@@ -258,8 +269,13 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) gemm_rows_kern
     __syncthreads();
     auto total = [&](int m, int n) {
       float sum = 0.f;
+      if (QK && WARPS == 16) {  // warps 8 apart first, as the eight-warp form adds them
 #pragma unroll
-      for (int w = 0; w < WARPS; ++w) sum += r[(w * ROWS + m) * COLS + n];
+        for (int w = 0; w < 8; ++w) sum += r[(w * ROWS + m) * COLS + n] + r[((w + 8) * ROWS + m) * COLS + n];
+      } else {
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) sum += r[(w * ROWS + m) * COLS + n];
+      }
       return sum * rstd_s[m];
     };
     if (QK) {

@@ -2671,7 +2671,9 @@ def gemm_skinny_bf16(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, prefet
     meet in a float32 scratch that this wrapper allocates.  `prefetch`: the weights the next
     product will read; the kernel asks for their start to be brought into L2 while it finishes.
     `direct`: up to 16 rows may run on mma.sync straight from device memory (csrc/gemm_rows.cu), which is faster where it
-    takes the shape; a row's bits then depend on which of the two kernels its step takes.
+    takes the shape (its input must fit beside the rings: 16 rows of 2,048 columns, 8 of 4,096, 3 of 12,288).  Either kernel gives a row the
+    same bits whatever the rows beside it; between the two, and so between steps of different numbers of rows, they differ by
+    the order of float32 sums.
     """
     if not (x.is_cuda and w.is_cuda and out.is_cuda):
         raise KernelError("gemm_skinny_bf16: CUDA tensors only (there is no CPU path)")
