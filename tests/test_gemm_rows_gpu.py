@@ -3,6 +3,8 @@ and many more, warps with unequal shares of K, M at the edges of the halves of e
 tolerances: float32 sums of up to 12,288 products of standard normal x 0.05 stay below 1e-6 of the result's norm (1e-5
 asserted), one rounding to bfloat16 is 2^-9 (1e-2)."""
 
+import math
+
 import pytest
 import torch
 
@@ -180,6 +182,26 @@ def test_a_row_has_the_same_bits_whatever_the_rows_beside_it(N, K):
     for first, last in ((0, 1), (15, 16), (3, 5), (0, 8), (0, 9), (5, 14)):
         for a, b in zip(run(first, last), whole):
             assert torch.equal(a, b[first:last])
+
+
+@pytest.mark.parametrize("M", [1, 5, 17])
+@pytest.mark.parametrize("off", ["table", "q", "k"])
+def test_buffers_off_their_boundaries_are_refused(off, M):
+    """A table of cosines and sines, query rows or a cache that do not start where the kernels read and write them: refused on the host,
+    whichever kernel takes the step."""
+    from tokensprint_b200 import ops
+
+    nq, nkv, K, d = 16, 8, 1024, 128
+    _, x, w = make(M, (nq + 2 * nkv) * d, K)
+    inv_freq = (1.0 / (1e4 ** (torch.arange(0, d, 2).float() / d))).to(DEV)
+    positions, slots = (torch.arange(M, device=DEV, dtype=torch.int32) for _ in range(2))
+    rows = lambda shape, shift: torch.zeros(math.prod(shape) + 1, device=DEV, dtype=torch.bfloat16)[int(shift):][:math.prod(shape)].view(shape)
+    table = ops.rope_cos_sin(positions, inv_freq, M).flatten()
+    if off == "table":
+        table = torch.cat([table[:1], table])[1:]
+    q, kc, vc = rows((M, nq * d), off == "q"), rows((M, nkv, d), off == "k"), rows((M, nkv, d), False)
+    with pytest.raises(ops.KernelError):
+        ops.gemm_qk_rope_store(x, w, q, kc, vc, slots, positions, None, None, 1e-5, inv_freq, nq, nkv, cos_sin=table, direct=True)
 
 
 def test_what_it_does_not_take_runs_on_the_other_kernel():

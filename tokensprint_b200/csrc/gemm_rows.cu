@@ -523,6 +523,8 @@ TS_EXPORT int ts_gemm_rows_qk_rope(const void* x, const void* w, int M, int K, l
   if (nq <= 0 || nkv <= 0 || q_out == nullptr || k_cache == nullptr || v_cache == nullptr || slot_mapping == nullptr ||
       (inv_freq != nullptr && positions == nullptr))
     return TS_ERR_BAD_ARGUMENT;
+  // what the tcgen05 kernel refuses; the table's (cos, sin) are read as pairs of 8 bytes
+  if (((uintptr_t)q_out | (uintptr_t)k_cache | (uintptr_t)v_cache) % 8 || (uintptr_t)rope_cos_sin % 16) return TS_ERR_UNSUPPORTED_SIZE;
   RowsArgs a = {};
   a.mode = MODE_QK_ROPE;
   a.scale_ssq = scale_ssq;
