@@ -336,15 +336,15 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) gemm_rows_kern
           reinterpret_cast<__nv_bfloat16*>(a.out)[(size_t)m * a.ldo + col] = __float2bfloat16_rn(ts_glu_gate_fast(gate, a.glu_act) * up);
       }
     } else if (a.mode == MODE_RESIDUAL_NORM) {
-      for (int idx = tid; (idx & ~31) < M * COLS; idx += THREADS) {  // whole warps: COLS divides 32
-        const int m = idx / COLS, n = idx % COLS, col = task * COLS + n;
+      static_assert(QK || THREADS >= MAX_ROWS * COLS, "a thread finishes at most one element");
+      if ((tid & ~31) < M * COLS) {  // whole warps: COLS divides 32
+        const int m = tid / COLS, n = tid % COLS, col = task * COLS + n;
         float ss = 0.f;
         if (m < M && col < a.N) {
           const size_t at = (size_t)m * a.ldh + col;
-          const float old = idx == tid ? hidden0 : __ldcg(a.hidden + at), nw = idx == tid ? norm0 : a.norm_w[col];
-          const float h = fmaf(a.branch_scale, total(m, n), old);
+          const float h = fmaf(a.branch_scale, total(m, n), hidden0);
           a.hidden[at] = h;
-          a.xprime[at] = __float2bfloat16_rn(h * nw);
+          a.xprime[at] = __float2bfloat16_rn(h * norm0);
           ss = h * h;
         }
 #pragma unroll
@@ -453,6 +453,7 @@ int run_rows(RowsArgs& a, const void* x, const void* w, int M, int N, int K, lon
   if (K <= 0 || ldx < K || ldw < K) return TS_ERR_BAD_ARGUMENT;
   Shape s;
   if (!choose(M, N, K, qk, &s)) return TS_ERR_UNSUPPORTED_SIZE;
+  // rows of W on whole sectors of 32 bytes: the 64 bytes that four lanes ask for at a time would touch three of them otherwise, not two
   if ((ldx % 8) || (ldw % 16) || ((uintptr_t)x % 16) || ((uintptr_t)w % 32) || (long long)N * ldw * 2 >= (1ll << 32)) return TS_ERR_UNSUPPORTED_SIZE;
   if (a.scale_ssq != nullptr && (a.scale_tiles <= 0 || !(a.scale_width > 0.f))) return TS_ERR_BAD_ARGUMENT;
   a.x = (const __nv_bfloat16*)x;
