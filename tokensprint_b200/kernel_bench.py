@@ -173,7 +173,7 @@ def skinny_gemm(cfg, timer, pk, rows, device):
             out = torch.empty(M, N, device=device, dtype=torch.bfloat16)
             if not ops.gemm_skinny_supported(x, w):
                 continue
-            us = timer(lambda: ops.gemm_skinny_bf16(x, w, out))
+            us = timer(lambda: ops.gemm_skinny_bf16(x, w, out, direct=True))
             gb = (N * K + M * K + M * N) * 2 / 1e9
             rows.append(("GEMM, few rows", f"{name} M={M} N={N} K={K}", us, gb / (us * 1e-6), "GB/s", gb / (us * 1e-6) / pk["hbm_gbs"]))
         del w
@@ -250,7 +250,6 @@ def layer_products(cfg, timer, pk, rows, device):
     for M in (1, 8, 32):
         attn, hidden = bf(M, nq * d, s=1.0), torch.randn(M, H, device=device)
         x1, x2 = (torch.empty((M, H), device=device, dtype=torch.bfloat16) for _ in range(2))
-        ssq1, ssq2 = (torch.empty((-(-H // 128), M), device=device) for _ in range(2))
         act = torch.empty((M, I), device=device, dtype=torch.bfloat16)
         q = torch.empty((M, nq * d), device=device, dtype=torch.bfloat16)
         kc = torch.zeros(64, nkv, d, device=device, dtype=torch.bfloat16)
@@ -259,12 +258,17 @@ def layer_products(cfg, timer, pk, rows, device):
         pos = torch.arange(M, device=device, dtype=torch.int32)
         cos_sin = ops.rope_cos_sin(pos, inv_freq, M)  # once a step in the engine: not part of a layer
 
-        def layer(w, nxt):
-            ops.gemm_skinny_fused(attn, w["o"], mode=ops.GEMM_EPILOGUE_RESIDUAL_NORM, hidden=hidden, norm_weight=n1, xprime=x1, ssq_out=ssq1, prefetch=w["gu"])
-            ops.gemm_skinny_fused(x1, w["gu"], out=act, mode=ops.GEMM_EPILOGUE_SWIGLU, scale_ssq=ssq1, scale_width=H, scale_eps=1e-6, prefetch=w["down"])
-            ops.gemm_skinny_fused(act, w["down"], mode=ops.GEMM_EPILOGUE_RESIDUAL_NORM, hidden=hidden, norm_weight=n2, xprime=x2, ssq_out=ssq2, prefetch=w["qkv"])
+        def layer(w, nxt):  # the row sums of squares come in as many pieces as the product before leaves (inside a chain: one per 128 columns)
+            ssq1 = torch.empty((ops.gemm_ssq_tiles(M, w["o"]), M), device=device)
+            ssq2 = torch.empty((ops.gemm_ssq_tiles(M, w["down"]), M), device=device)
+            ops.gemm_skinny_fused(attn, w["o"], mode=ops.GEMM_EPILOGUE_RESIDUAL_NORM, hidden=hidden, norm_weight=n1, xprime=x1, ssq_out=ssq1, prefetch=w["gu"],
+                                  direct=True)
+            ops.gemm_skinny_fused(x1, w["gu"], out=act, mode=ops.GEMM_EPILOGUE_SWIGLU, scale_ssq=ssq1, scale_width=H, scale_eps=1e-6, prefetch=w["down"],
+                                  direct=True)
+            ops.gemm_skinny_fused(act, w["down"], mode=ops.GEMM_EPILOGUE_RESIDUAL_NORM, hidden=hidden, norm_weight=n2, xprime=x2, ssq_out=ssq2, prefetch=w["qkv"],
+                                  direct=True)
             ops.gemm_qk_rope_store(x2, w["qkv"], q, kc, vc, slots, pos, qn, kn, 1e-6, inv_freq, nq, nkv,
-                                   scale_ssq=ssq2, scale_width=H, scale_eps=1e-6, prefetch=nxt["o"], cos_sin=cos_sin)
+                                   scale_ssq=ssq2, scale_width=H, scale_eps=1e-6, prefetch=nxt["o"], cos_sin=cos_sin, direct=True)
 
         for chained in (False, True):
             def body():
