@@ -2727,11 +2727,11 @@ def gemm_skinny_fused(
     activation: str = "silu",
     direct: bool = False,
 ) -> None:
-    """x[M,K] @ w[N,K]^T on the tcgen05 tensor cores (M <= 32) with the work of the neighbouring
-    small kernels done where each tile is finished.
+    """x[M,K] @ w[N,K]^T in bfloat16 with float32 sums (M <= 32; on tcgen05, with `direct` up to 16 rows on mma.sync where that kernel
+    takes the shape) with the work of the neighbouring small kernels done where each tile is finished.
 
     scale_ssq [tiles, M] float32: x lacks its norm's 1/rms (x = source * norm weight); the sums
-    of squares of the source rows per 128 columns, as a GEMM in mode 2 leaves them; every row m of
+    of squares of the source rows in pieces, as a GEMM in mode 2 leaves them (per 128 columns, or per 16); every row m of
     the product is multiplied by rsqrt(sum_m / scale_width + scale_eps).
     mode GEMM_EPILOGUE_PLAIN: out[M,N] bf16 or float32.
     mode GEMM_EPILOGUE_SWIGLU: the rows of w come in blocks of 128, 64 gate rows and then the 64 up
