@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) gemm_rows_kern
       }
     }
     // 4 / RU chains per group of rows: a product waits for the one before it in its chain.  Eight warps that share a head keep the sums of every
-    // other chunk apart: what 16 warps sum, added up in the same order, so a row's bits do not depend on the form.
+    // other chunk apart, which are those of 16 warps, so that a row's bits do not depend on the form.
     constexpr int SETS = QK && WARPS == 8 ? 2 : 1;
     float acc[SETS][4][4];
 #pragma unroll
@@ -252,6 +252,8 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) gemm_rows_kern
     }
     // ---- the warps' sums meet in shared memory (two buffers in turn: one barrier a task)
     float* r = red + (size_t)(it & 1) * (WARPS * ROWS * COLS);
+    // Rows of a head's sums are as long as the banks: permuted so that neither four rows written at once nor two read at once share any.
+    auto place = [](int m, int n) { return m * COLS + (QK ? n ^ ((m & 1) << 4 | (m & 2) << 2) : n); };
 #pragma unroll
     for (int u = 0; u < RU; ++u) {
       float v[4];
@@ -260,21 +262,34 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) gemm_rows_kern
         v[i] = acc[0][u * CHAINS][i];
 #pragma unroll
         for (int k = 1; k < CHAINS; ++k) v[i] += acc[0][u * CHAINS + k][i];
-        if (SETS == 2) v[i] += acc[SETS - 1][u * CHAINS][i];
       }
-      float* mine = r + (warp * ROWS + g) * COLS + u * 8 + 2 * t;
+      float* mine = r + warp * ROWS * COLS + place(g, u * 8 + 2 * t);
       *reinterpret_cast<float2*>(mine) = make_float2(v[0], v[1]);
       if (MH == 2) *reinterpret_cast<float2*>(mine + 8 * COLS) = make_float2(v[2], v[3]);
+    }
+    // The second set takes the place of the warp's ring, which is empty: a head's CTA has one task, and its last chunks were waited for and read
+    // (by other lanes too, hence the warp's barrier).
+    float* odd = reinterpret_cast<float*>(smem);
+    constexpr int ODD_WARP = SLOTS * RU * 1024 / (int)sizeof(float);
+    static_assert(SETS == 1 || (CHAINS == 1 && ROWS * COLS <= ODD_WARP), "a set fits a ring");
+    if (SETS == 2) {
+      __syncwarp();
+#pragma unroll
+      for (int u = 0; u < RU; ++u) {
+        const float(&v)[4] = acc[SETS - 1][u];
+        float* mine = odd + warp * ODD_WARP + place(g, u * 8 + 2 * t);
+        *reinterpret_cast<float2*>(mine) = make_float2(v[0], v[1]);
+        if (MH == 2) *reinterpret_cast<float2*>(mine + 8 * COLS) = make_float2(v[2], v[3]);
+      }
     }
     __syncthreads();
     auto total = [&](int m, int n) {
       float sum = 0.f;
-      if (QK && WARPS == 16) {  // warps 8 apart first, as the eight-warp form adds them
 #pragma unroll
-        for (int w = 0; w < 8; ++w) sum += r[(w * ROWS + m) * COLS + n] + r[((w + 8) * ROWS + m) * COLS + n];
-      } else {
+      for (int w = 0; w < WARPS; ++w) sum += r[w * ROWS * COLS + place(m, n)];
+      if (SETS == 2) {  // the warps 8 to 15 of the form with 16
 #pragma unroll
-        for (int w = 0; w < WARPS; ++w) sum += r[(w * ROWS + m) * COLS + n];
+        for (int w = 0; w < WARPS; ++w) sum += odd[w * ODD_WARP + place(m, n)];
       }
       return sum * rstd_s[m];
     };
