@@ -21,8 +21,9 @@
 // a cluster of four CTAs with 16 pairs (j, j + 64) each, which exchange their sums of squares through distributed shared memory).
 // A row's sums are added up in one order whatever the rows beside it, the number of warps included.
 //
-// Measured (B200; a whole decode step, us, with gemm_tcgen05.cu's products and with these): 0.6B of 1 request 1,133 -> 732, of 8
-// 1,240 -> 872; 8B of 1 3,324 -> 2,889, of 8 3,485 -> 3,298; four small products of a layer (0.6B, 1 row) 27.8 -> 14.6, floor 4.9.
+// Measured (B200; a whole decode step, us, with gemm_tcgen05.cu's products and with these, about 60 of a small step's gain being its
+// attention's): 0.6B of 1 request 1,124 -> 670, of 8 1,226 -> 802, of 14 1,312 -> 1,109; 8B of 1 3,278 -> 2,856, of 4 3,422 -> 3,132, of 8
+// 3,467 -> 3,336; four small products of a layer (0.6B, 1 row) 27.8 -> 14.6, floor 4.9; gate and up of 24,576 x 4,096, 8 rows, alone 33.7: 6.0 TB/s.
 //
 // The reference runs these products through nn.Linear (engine/nn/attention.py:122-135, engine/nn/layers.py:61-66).
 #include "common.cuh"
